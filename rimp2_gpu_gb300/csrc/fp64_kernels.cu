@@ -20,7 +20,7 @@
 // staging is simple (cp.async double buffering in the GEMM), padding keeps
 // fragment loads bank-conflict free, and two CTAs per SM keep the FP64 pipe
 // busy.
-#include "common.cuh"
+#include "mod_gemm.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -632,6 +632,10 @@ int launch_gemm_f64(const GemmDesc &g, cudaStream_t s) {
     set_error("injected launch failure (RIMP2_FAULT_INJECT=launch)");
     return RIMP2_ERR_CUDA;
   }
+  // large products go to the FP16 tensor cores as residues
+  bool done = false;
+  RIMP2_TRY(mod_gemm(g, s, &done));
+  if (done) return RIMP2_OK;
   long long mt = (g.M + TM - 1) / TM, nt = (g.N + TN - 1) / TN;
   long long nb = (long long)g.nb0 * g.nb1;
   if (mt > 2147483647LL) {

@@ -1,0 +1,1098 @@
+// mod_gemm.cu -- FP64 contractions on the FP16 tensor cores by residue
+// arithmetic.
+//
+// GB300 runs FP64 tensor operations (DMMA) at 1.05 TFLOP/s and FP16 ones at
+// 1900 TFLOP/s.  A contraction C(m,n) = sum_k A(m,k) B(k,n) of FP64 numbers is
+// therefore evaluated with integers (the modular form of Ozaki's scheme:
+// Ozaki, Uchino, Imamura, "Ozaki Scheme II", 2025):
+//   1. every row of A and every column of B is scaled by a power of two and
+//      rounded to integers a', b' with 2-norm at most 2^62 (62 bits where the
+//      FP64 fraction has 53: an element keeps every bit it has down to 2^-9 of
+//      its row's norm);
+//   2. X = sum a' b' is an integer with |X| <= 2^124 (Cauchy-Schwarz), fixed
+//      by its residues modulo 16 pairwise coprime numbers of at most 8 bits
+//      whose product P is 2^125.1;
+//   3. residues are at most 128 in magnitude, exact in FP16, and 1024 of their
+//      products sum to at most 2^24: the FP32 accumulation of the tensor core
+//      is exact, whatever its internal rounding;
+//   4. the fraction X/P = sum_p r_p / p mod 1 is summed in 96-bit fixed point,
+//      multiplied by P and rounded once to FP64 (a fraction below 2^-28 is
+//      redone in exact integers): a sum that FP64 can hold comes out exact.
+// Everything between the rounding to 62-bit integers and the final rounding
+// is exact.  The rounding error of (1) in X is about 0.41 * 2^62, i.e.
+// 0.41 * 2^-9 u * (2^124 / sum|a'||b'|) relative to u sum|a||b| (u = 2^-53),
+// below what FP64 summation itself loses unless sum|a||b| is a tiny part of
+// ||a|| ||b|| (rows whose large elements meet only small ones).  A 17th
+// product of the magnitudes, in FP16, measures sum|a||b| for every element
+// (from below); an element whose measure is under 2^-8 of ||a|| ||b|| is
+// summed in FP64 instead (one warp per element, or a DMMA tile where an
+// eighth of a 64 x 64 tile needs it).  Rows with infinities, NaNs or extreme
+// exponents take that way too, so every element is what FP64 arithmetic would
+// make it, up to FP64's own rounding.
+//
+// Kernels: row_scale (norms -> exponents), residue (17 FP16 planes per
+// operand), mod_gemm (persistent CTA pairs, 256 x 256 tiles, TMA + tcgen05,
+// one product per plane; the epilogue reduces modulo p and stores bytes),
+// crt_epilogue (fixed-point reconstruction, scaling, denominators, the
+// elements to be summed in FP64), dmma_tiles (whole tiles in FP64).
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <cstring>
+
+#include "tc.cuh"
+#include "mod_gemm.cuh"
+
+namespace rimp2 {
+void count_launch(int n);
+
+namespace {
+
+// --------------------------------------------------------------------------
+// constants of the residue system
+// --------------------------------------------------------------------------
+typedef unsigned __int128 u128;
+
+// Pairwise coprime, at most 251 but for 256: the FP32 reduction of a sum below
+// 2^24 leaves |r| <= 0.507 p, which has to fit a signed byte (256 wraps onto
+// itself).
+struct ModTables {
+  float p[MG_P], inv[MG_P];
+  float ca[MG_P][5];      // 2^(13 l) mod p, symmetric: A's limbs
+  float cb[MG_P][5];      // the same times (P/p)^-1 mod p: B's limbs
+  unsigned phi[4][12];    // byte b of round(2^96 / p) for p = 4q .. 4q+3
+  unsigned long long pm;  // P 2^-62
+  unsigned long long plo, phi64;         // P
+  unsigned long long wlo[MG_P], whi[MG_P];  // P / p
+};
+
+constexpr int sym(long long v, int p) {
+  v %= p;
+  if (v < 0) v += p;
+  return (int)(2 * v > p ? v - p : v);
+}
+
+constexpr ModTables make_tables() {
+  ModTables t{};
+  const int ps[MG_P] = {256, 251, 249, 247, 245, 241, 239, 233, 229, 227, 223, 211, 199, 197, 193, 191};
+  u128 P = 1;
+  for (int i = 0; i < MG_P; ++i) P *= (u128)ps[i];
+  for (int i = 0; i < MG_P; ++i) {
+    const int p = ps[i];
+    t.p[i] = (float)p;
+    t.inv[i] = 1.0f / (float)p;
+    const int q = (int)((P / (u128)p) % (u128)p);
+    int inv = 0;
+    for (int x = 1; x < p; ++x)
+      if ((long long)x * q % p == 1) inv = x;
+    long long w = 1;
+    for (int l = 0; l < 5; ++l) {
+      t.ca[i][l] = (float)sym(w, p);
+      t.cb[i][l] = (float)sym(w * inv, p);
+      w = w * 8192 % p;
+    }
+    const u128 one = (u128)1 << 96;
+    const u128 phi = (one + (u128)(p / 2)) / (u128)p;
+    for (int b = 0; b < 12; ++b)
+      t.phi[i >> 2][b] |= (unsigned)((phi >> (8 * b)) & 0xFF) << (8 * (i & 3));
+    const u128 w128 = P / (u128)p;
+    t.wlo[i] = (unsigned long long)w128;
+    t.whi[i] = (unsigned long long)(w128 >> 64);
+  }
+  t.pm = (unsigned long long)(P >> 62);
+  t.plo = (unsigned long long)P;
+  t.phi64 = (unsigned long long)(P >> 64);
+  return t;
+}
+constexpr ModTables HT = make_tables();
+__constant__ ModTables DT = HT;
+
+constexpr float MAGIC = 12582912.0f;  // 1.5 * 2^23: adds round to an integer
+
+// --------------------------------------------------------------------------
+// operands
+// --------------------------------------------------------------------------
+__device__ __forceinline__ long long row_off(const RowMap &M, int r) {
+  const int d0 = r % M.ext[0], q = r / M.ext[0];
+  const int d1 = q % M.ext[1], d2 = q / M.ext[1];
+  return d0 * M.st[0] + d1 * M.st[1] + d2 * M.st[2];
+}
+
+// Norm of a row in pieces: largest exponent, sum of squares relative to it
+// (FP32: its rounding, below 2^-10, is inside the margin of the scale), the
+// lowest set bit, and whether a value is infinite or NaN.
+struct RowStat {
+  int e;      // largest biased exponent so far (0: all zero)
+  float ss;   // sum of (x 2^(1023-e))^2
+  int lsb;    // exponent of the lowest set bit of any value
+  int bad;
+};
+
+__device__ __forceinline__ float pow2f(int k) {  // 2^k, 0 below the normal range
+  return k < -126 ? 0.0f : __uint_as_float((unsigned)(k + 127) << 23);
+}
+
+__device__ __forceinline__ void stat_add(RowStat &s, double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFull;
+  if (b == 0) return;
+  const int ed = (int)(b >> 52);
+  if (ed == 0x7FF) {
+    s.bad = 1;
+    return;
+  }
+  const unsigned long long f = b & 0xFFFFFFFFFFFFFull;
+  const int tz = f ? __ffsll((long long)f) - 1 : 52;
+  s.lsb = min(s.lsb, (ed ? ed : 1) - 1075 + tz);
+  if (ed > s.e) {
+    s.ss *= pow2f(2 * (s.e - ed));
+    s.e = ed;
+  }
+  const float m = __uint_as_float(0x3F800000u | (unsigned)(f >> 29)) * pow2f(ed - s.e);
+  s.ss = fmaf(m, m, s.ss);
+}
+
+__device__ __forceinline__ void stat_merge(RowStat &s, int e, float ss, int lsb, int bad) {
+  const int m = max(s.e, e);
+  s.ss = s.ss * pow2f(2 * (s.e - m)) + ss * pow2f(2 * (e - m));
+  s.e = m;
+  s.lsb = min(s.lsb, lsb);
+  s.bad |= bad;
+}
+
+// Scale exponent: ||x|| 2^e <= 2^62 / 1.002.  Rows with values beyond
+// 2^+-400 are left to FP64: the reconstruction assembles exponents.
+__device__ __forceinline__ void stat_store(const RowStat &s, int *e, unsigned char *flag) {
+  if (s.bad || (s.e != 0 && (s.e < 1023 - 400 || s.e > 1023 + 400))) {
+    *e = 0;
+    *flag = MG_ROW_FP64;
+    return;
+  }
+  if (s.e == 0) {  // zeros (a row of subnormal values has lsb < 0 and goes to FP64)
+    *e = 0;
+    *flag = s.lsb == MG_NO_LSB ? MG_ROW_ZERO : MG_ROW_FP64;
+    return;
+  }
+  const float h = sqrtf(s.ss) * 1.002f;
+  const int c = (int)((__float_as_uint(h) >> 23) & 0xFFu) - 127 + 1;
+  const int ee = 62 - (s.e - 1023) - c;
+  *e = ee;
+  *flag = s.lsb + ee >= 0 ? MG_ROW_EXACT : 0;
+}
+
+// K-contiguous rows: one warp per row, four loads in flight per lane.
+__global__ void __launch_bounds__(256) row_scale_k_kernel(RowMap M, int row0, int nrows, int *e,
+                                                          unsigned char *flag) {
+  const int r = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
+  if (r >= nrows) return;
+  const double *x = M.base + row_off(M, row0 + r);
+  RowStat s{0, 0.0f, MG_NO_LSB, 0};
+  for (int k0 = lane; k0 < M.K; k0 += 128) {
+    double v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = k0 + 32 * u < M.K ? x[k0 + 32 * u] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) stat_add(s, v[u]);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const int e2 = __shfl_xor_sync(0xffffffffu, s.e, o);
+    const float s2 = __shfl_xor_sync(0xffffffffu, s.ss, o);
+    const int l2 = __shfl_xor_sync(0xffffffffu, s.lsb, o);
+    const int b2 = __shfl_xor_sync(0xffffffffu, s.bad, o);
+    stat_merge(s, e2, s2, l2, b2);
+  }
+  if (lane == 0) stat_store(s, e + r, flag + r);
+}
+
+// Rows along the fast direction: a block takes 32 rows, each warp a part of K.
+__global__ void __launch_bounds__(512) row_scale_r_kernel(RowMap M, int row0, int nrows, int *e,
+                                                          unsigned char *flag) {
+  __shared__ RowStat sh[16][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int r = blockIdx.x * 32 + lane;
+  RowStat s{0, 0.0f, MG_NO_LSB, 0};
+  if (r < nrows) {
+    const double *x = M.base + row_off(M, row0 + r);
+    for (int k0 = w; k0 < M.K; k0 += 64) {
+      double v[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v[u] = k0 + 16 * u < M.K ? x[(long long)(k0 + 16 * u) * M.sk] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) stat_add(s, v[u]);
+    }
+  }
+  sh[w][lane] = s;
+  __syncthreads();
+  if (w == 0 && r < nrows) {
+    for (int q = 1; q < 16; ++q) {
+      const RowStat &t = sh[q][lane];
+      stat_merge(s, t.e, t.ss, t.lsb, t.bad);
+    }
+    stat_store(s, e + r, flag + r);
+  }
+}
+
+// |x| 2^e rounded to an integer (< 2^63)
+__device__ __forceinline__ unsigned long long to_int(double x, int e) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int ed = (int)((b >> 52) & 0x7FF);
+  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+  const int sh = ed - 1075 + e;
+  if (ed == 0 || sh < -54) return 0;
+  return sh >= 0 ? m << sh : (m + (1ull << (-sh - 1))) >> (-sh);
+}
+
+// Residues of eight consecutive K values of one row: 16 bytes per plane.
+// Five 13-bit limbs times the residues of 2^(13 l), summed in FP32 (exact:
+// below 2^23), reduced once, packed to FP16 with the value's sign.  FP32
+// arithmetic bounds it: 9 operations per value and modulus.
+template <bool COL>
+__device__ __forceinline__ void residues8(const double (&v)[8], int e, bool live,
+                                          __half *__restrict__ out, size_t plane) {
+  float l[5][8];
+  unsigned sg[4] = {0u, 0u, 0u, 0u};
+  uint4 gq;
+  __half2 *gh = reinterpret_cast<__half2 *>(&gq);
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const unsigned long long x = live ? to_int(v[u], e) : 0ull;
+#pragma unroll
+    for (int q = 0; q < 5; ++q)
+      l[q][u] = __uint_as_float(0x4B000000u | (unsigned)((x >> (13 * q)) & 0x1FFFu)) - 8388608.0f;
+    if (__double2hiint(v[u]) < 0) sg[u >> 1] |= (u & 1) ? 0x80000000u : 0x8000u;
+  }
+#pragma unroll
+  for (int u = 0; u < 8; u += 2) {  // |x| 2^-50 (norm 2^12): the magnitudes' plane
+    const float a = fmaf(l[4][u], 4.0f, fmaf(l[3][u], 4.8828125e-4f, l[2][u] * 5.9604645e-8f));
+    const float b = fmaf(l[4][u + 1], 4.0f, fmaf(l[3][u + 1], 4.8828125e-4f, l[2][u + 1] * 5.9604645e-8f));
+    gh[u >> 1] = __floats2half2_rn(a, b);
+  }
+  *reinterpret_cast<uint4 *>(out + (size_t)MG_P * plane) = gq;
+#pragma unroll
+  for (int p = 0; p < MG_P; ++p) {
+    const float pf = DT.p[p], inv = DT.inv[p];
+    uint4 o;
+    unsigned *ow = reinterpret_cast<unsigned *>(&o);
+#pragma unroll
+    for (int u = 0; u < 8; u += 2) {
+      float r[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float y = l[0][u + h] * (COL ? DT.cb[p][0] : DT.ca[p][0]);
+#pragma unroll
+        for (int q = 1; q < 5; ++q)
+          y = fmaf(l[q][u + h], (COL ? DT.cb[p][q] : DT.ca[p][q]), y);
+        const float q = fmaf(y, inv, MAGIC) - MAGIC;
+        r[h] = fmaf(-q, pf, y);
+      }
+      const __half2 hh = __floats2half2_rn(r[0], r[1]);
+      ow[u >> 1] = *reinterpret_cast<const unsigned *>(&hh) ^ sg[u >> 1];
+    }
+    *reinterpret_cast<uint4 *>(out + (size_t)p * plane) = o;
+  }
+}
+
+// out[(p * nkc + kc) * R + row][64]
+template <bool COL>
+__global__ void __launch_bounds__(256) residue_k_kernel(RowMap M, int row0, int R, int nkc,
+                                                        const int *__restrict__ e,
+                                                        const unsigned char *__restrict__ flag,
+                                                        __half *__restrict__ out, size_t plane) {
+  const long long g = blockIdx.x * 32ll + (threadIdx.x >> 3);  // (kc, row)
+  if (g >= (long long)nkc * R) return;
+  const int kc = (int)(g / R), r = (int)(g % R), k0 = kc * 64 + (threadIdx.x & 7) * 8;
+  const double *x = M.base + row_off(M, row0 + r);
+  double v[8];
+  if ((((uintptr_t)x) & 15) == 0 && k0 + 8 <= M.K) {
+#pragma unroll
+    for (int u = 0; u < 8; u += 2) {
+      const double2 d = *reinterpret_cast<const double2 *>(x + k0 + u);
+      v[u] = d.x;
+      v[u + 1] = d.y;
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = k0 + u < M.K ? x[k0 + u] : 0.0;
+  }
+  residues8<COL>(v, e[r], !(flag[r] & MG_ROW_FP64), out + g * 64 + (threadIdx.x & 7) * 8, plane);
+}
+
+template <bool COL>
+__global__ void __launch_bounds__(256) residue_r_kernel(RowMap M, int row0, int R, int nkc,
+                                                        const int *__restrict__ e,
+                                                        const unsigned char *__restrict__ flag,
+                                                        __half *__restrict__ out, size_t plane) {
+  __shared__ double sh[64][33];
+  const int nrb = (R + 31) / 32;
+  const int kc = blockIdx.x / nrb, rb = blockIdx.x % nrb;
+  {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = rb * 32 + lane;
+    const double *x = M.base + (r < R ? row_off(M, row0 + r) : 0);
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int k = kc * 64 + w + 8 * u;
+      sh[w + 8 * u][lane] = r < R && k < M.K ? x[(long long)k * M.sk] : 0.0;
+    }
+  }
+  __syncthreads();
+  const int rr = threadIdx.x >> 3, kq = threadIdx.x & 7, r = rb * 32 + rr;
+  if (r >= R) return;
+  double v[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) v[u] = sh[kq * 8 + u][rr];
+  residues8<COL>(v, e[r], !(flag[r] & MG_ROW_FP64), out + ((size_t)kc * R + r) * 64 + kq * 8, plane);
+}
+
+// --------------------------------------------------------------------------
+// products: persistent CTA pairs
+// --------------------------------------------------------------------------
+// Work item = (plane, 256 columns n x 256 rows m of C): the columns' operand
+// lies on the TMEM lanes (M = 256 over the pair), the rows' operand on the
+// accumulator columns (N = 256, half of it in each CTA), so that a thread
+// stores runs of bytes along m.  Two 256-column accumulators per CTA: the
+// MMAs of one item run while the epilogue reduces the other.  Sums longer
+// than 1024 are cut there (exactness) and joined modulo p in the epilogue's
+// registers.  A 64-deep stage is 32 KB per CTA, six stages.
+constexpr int MG_NST = 6;
+constexpr int MG_STAGE = 2 * PANEL_BYTES;
+constexpr int MG_THREADS = 320;
+constexpr int MG_SEG = 16;  // K chunks per exact sum
+constexpr int MG_SMEM = MG_NST * MG_STAGE + 1024 + 256;
+
+struct MgParams {
+  int rows_l, rows_q;        // rows per K chunk of the two operands
+  int tiles_l, tiles_q;      // 256-wide tiles
+  int nkc;
+  int lower;                 // only tiles with an element m >= n
+  signed char *out;          // [plane][n][ldm]
+  long long ldm;
+  int *err;
+};
+
+__device__ __forceinline__ bool mg_item(const MgParams &P, long long item, int &plane, int &tl, int &tq) {
+  const int tiles = P.tiles_l * P.tiles_q;
+  plane = (int)(item / tiles);
+  const int t = (int)(item % tiles);
+  // groups of eight column tiles: the tiles in flight share their operands in L2
+  const int per = 8 * P.tiles_q, g = t / per, rem = t % per;
+  const int gs = min(8, P.tiles_l - 8 * g);
+  tl = 8 * g + rem % gs;
+  tq = rem / gs;
+  return !(P.lower && tq < tl);
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
+    mod_gemm_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__ CUtensorMap tmQ,
+                    MgParams P) {
+  constexpr int NST = MG_NST;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  // bars: full[NST], empty[NST], tfull[2], tempty[2], drain
+  uint64_t *bars = (uint64_t *)(base + NST * MG_STAGE);
+  uint32_t *tmem_slot = (uint32_t *)(bars + 2 * NST + 5);
+  volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  const bool leader = rank == 0;
+  const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[NST]);
+  const uint32_t tfull0 = smem_u32(&bars[2 * NST]), tempty0 = smem_u32(&bars[2 * NST + 2]);
+  const uint32_t drain = smem_u32(&bars[2 * NST + 4]);
+  const uint32_t full0_L = map_shared(full0, 0), tempty0_L = map_shared(tempty0, 0);
+  const uint32_t abort_peer = map_shared(smem_u32((const void *)abort_flag), rank ^ 1u);
+  const long long nitems = (long long)MG_PLANES * P.tiles_l * P.tiles_q;
+  const int pair = blockIdx.x >> 1, npair = gridDim.x >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NST; ++s) {
+      mbar_init(full0 + 8 * s, 1);   // rank 0: its producer's arrive + both CTAs' bytes
+      mbar_init(empty0 + 8 * s, 1);  // multicast MMA commit
+    }
+    for (int u = 0; u < 2; ++u) {
+      mbar_init(tfull0 + 8 * u, 1);
+      mbar_init(tempty0 + 8 * u, 16);  // the epilogue warps of both CTAs
+    }
+    mbar_init(drain, 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&tmL) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&tmQ) : "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                     smem_u32(tmem_slot))
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // both CTAs' barriers are initialised before any remote access
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0) {
+    // --------------------- TMA producers (both CTAs) ---------------------
+    if (lane == 0) {
+      int stage = 0;
+      uint32_t phase = 0, armed = 0, armed_par = 0;
+      bool ok = true;
+      for (long long item = pair; item < nitems && ok; item += npair) {
+        int p, tl, tq;
+        if (!mg_item(P, item, p, tl, tq)) continue;
+        const int rl = tl * 256 + 128 * (int)rank, rq = tq * 256 + 128 * (int)rank;
+        for (int kc = 0; kc < P.nkc; ++kc) {
+          if (!pair_wait(empty0 + 8 * stage, phase ^ 1, false, abort_flag, abort_peer, P.err, 21)) {
+            ok = false;
+            break;
+          }
+          if (leader) {
+            mbar_expect_tx(full0 + 8 * stage, 2 * MG_STAGE);
+            armed |= 1u << stage;
+            armed_par = (armed_par & ~(1u << stage)) | (phase << stage);
+          }
+          const uint32_t dst = smem_u32(base + stage * MG_STAGE), fb = full0_L + 8 * stage;
+          tma_load_3d_pair(dst, &tmL, fb, 0, kc * P.rows_l + rl, p);
+          tma_load_3d_pair(dst + PANEL_BYTES, &tmQ, fb, 0, kc * P.rows_q + rq, p);
+          if (++stage == NST) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+      }
+      if (leader && (!ok || *abort_flag)) {  // copies in flight complete before the pair exits
+        for (int s = 0; s < NST; ++s) {
+          if (!((armed >> s) & 1u)) continue;
+          const long long t0 = clock64();
+          while (!mbar_test(full0 + 8 * s, (armed_par >> s) & 1u) && clock64() - t0 < WAIT_BUDGET) {
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // --------------------- MMA issuer (rank 0 only) ----------------------
+    if (lane == 0 && leader) {
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      long long t = 0;  // sums so far
+      for (long long item = pair; item < nitems && ok; item += npair) {
+        int p, tl, tq;
+        if (!mg_item(P, item, p, tl, tq)) continue;
+        for (int s0 = 0; s0 < P.nkc && ok; s0 += MG_SEG, ++t) {
+          const int u = (int)(t & 1);
+          if (t >= 2 && !pair_wait(tempty0 + 8 * u, (uint32_t)(((t >> 1) - 1) & 1), true, abort_flag,
+                                   abort_peer, P.err, 22)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t d = tmem + (uint32_t)(u * 256);
+          const int s1 = min(P.nkc, s0 + MG_SEG);
+          for (int kc = s0; kc < s1; ++kc) {
+            if (!pair_wait(full0 + 8 * stage, phase, false, abort_flag, abort_peer, P.err, 23)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t sb = smem_u32(base + stage * MG_STAGE);
+#pragma unroll
+            for (int k16 = 0; k16 < KSTEP / 16; ++k16)
+              mma_f16_pair(d, smem_desc(sb + k16 * 32), smem_desc(sb + PANEL_BYTES + k16 * 32),
+                           IDESC_PAIR_N256, (kc > s0 || k16 > 0) ? 1u : 0u);
+            mma_commit_pair(empty0 + 8 * stage);  // frees the stage in both CTAs
+            if (++stage == NST) {
+              stage = 0;
+              phase ^= 1;
+            }
+          }
+          if (!ok) break;
+          mma_commit_pair(tfull0 + 8 * u);
+        }
+      }
+      mma_commit_pair(drain);  // both CTAs learn when the last MMA has completed
+    }
+  } else {
+    // --------------------- epilogue (both CTAs) ---------------------------
+    const int quad = warp & 3, half = (warp - 2) >> 2;
+    const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
+    const int nl = P.rows_l;
+    long long t = 0;
+    bool ok = true;
+    for (long long item = pair; item < nitems && ok; item += npair) {
+      int p, tl, tq;
+      if (!mg_item(P, item, p, tl, tq)) continue;
+      const int n = tl * 256 + 128 * (int)rank + quad * 32 + lane;
+      const bool mag = p == MG_P;
+      const float pf = mag ? 1.0f : DT.p[p], inv = mag ? 1.0f : DT.inv[p];
+      uint32_t pk[8][4];
+      for (int s0 = 0; s0 < P.nkc; s0 += MG_SEG, ++t) {
+        const int u = (int)(t & 1);
+        ok = pair_wait(tfull0 + 8 * u, (uint32_t)((t >> 1) & 1), false, abort_flag, abort_peer, P.err, 24);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t ta = tmem + lane_off + (uint32_t)(u * 256 + half * 128);
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          float v[16];
+          tmem_ld16(ta + g * 16, v);
+          tmem_wait_ld();
+          if (mag) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              uint32_t w = s0 ? pk[g][q] : 0u;
+#pragma unroll
+              for (int k = 0; k < 4; ++k) w |= v[4 * q + k] >= MG_TAU ? 1u << (8 * k) : 0u;
+              pk[g][q] = w;
+            }
+          } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              uint32_t b[4];
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                const float y = v[4 * q + k];
+                float r = fmaf(-(fmaf(y, inv, MAGIC) - MAGIC), pf, y);
+                if (s0) {  // join with the earlier sums' residue, modulo p
+                  r += (float)(signed char)(pk[g][q] >> (8 * k));
+                  r = fmaf(-(fmaf(r, inv, MAGIC) - MAGIC), pf, r);
+                }
+                b[k] = __float_as_uint(r + MAGIC);  // low byte: the residue
+              }
+              pk[g][q] = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410);
+            }
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_remote(tempty0_L + 8 * u);
+      }
+      if (ok && n < nl) {
+        signed char *o = P.out + ((long long)p * nl + n) * P.ldm + tq * 256 + half * 128;
+#pragma unroll
+        for (int g = 0; g < 8; ++g)
+          *reinterpret_cast<uint4 *>(o + g * 16) = make_uint4(pk[g][0], pk[g][1], pk[g][2], pk[g][3]);
+      }
+    }
+  }
+  __syncthreads();
+  if (warp == 1 && lane == 0) {
+    // the last MMA of the pair has completed (it may write this CTA's TMEM)
+    const long long t0 = clock64();
+    while (!mbar_test(drain, 0) && clock64() - t0 < WAIT_BUDGET) {
+    }
+  }
+  if (*abort_flag) {
+    // after an abort the peer may still have copies in flight into its own
+    // shared memory (their completion is counted in rank 0): give them time
+    const long long t0 = clock64();
+    while (clock64() - t0 < 4000000LL) {
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+  }
+}
+
+// --------------------------------------------------------------------------
+// reconstruction and epilogue
+// --------------------------------------------------------------------------
+__device__ __forceinline__ int dp4a_su(unsigned a, unsigned b, int c) {
+  int d;
+  asm("dp4a.s32.u32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
+  return d;
+}
+
+// m 2^(x - 63) rounded to 53 bits, m's top bit set
+__device__ __forceinline__ double assemble(unsigned long long m, int x, bool neg) {
+  const unsigned long long f = (m >> 11) + ((m >> 10) & 1);  // 2^52 .. 2^53
+  const unsigned long long bits = ((unsigned long long)(1022 + x) << 52) + f;
+  return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0ull)));
+}
+
+// X 2^-eab where |X / P| < 2^-28: X = sum_p r_p P/p - k P in 128-bit integers
+// (wrapping), k the whole part of sum_p r_p / p.  Sums that cancel exactly,
+// or nearly, come here: the fraction's 96 bits would leave them too few.
+__device__ __noinline__ double crt_small(unsigned r0, unsigned r1, unsigned r2, unsigned r3, int eab) {
+  const unsigned r[4] = {r0, r1, r2, r3};
+  unsigned long long lo = 0, hi = 0;
+  float ks = 0.0f;
+  for (int p = 0; p < MG_P; ++p) {
+    const long long v = (signed char)(r[p >> 2] >> (8 * (p & 3)));
+    ks = fmaf((float)v, DT.inv[p], ks);
+    const unsigned long long w = DT.wlo[p], q = lo + w * (unsigned long long)v;
+    hi += DT.whi[p] * (unsigned long long)v + (unsigned long long)__mul64hi((long long)w, v) +
+          (w >> 63 ? (unsigned long long)v : 0ull) + (q < lo);
+    lo = q;
+  }
+  const long long k = (long long)rintf(ks);
+  const unsigned long long w = DT.plo, t = w * (unsigned long long)k;
+  hi -= DT.phi64 * (unsigned long long)k + (unsigned long long)__mul64hi((long long)w, k) +
+        (w >> 63 ? (unsigned long long)k : 0ull) + (lo < t);
+  lo -= t;
+  const bool neg = (long long)hi < 0;
+  if (neg) {
+    lo = ~lo + 1;
+    hi = ~hi + (lo == 0);
+  }
+  if ((hi | lo) == 0) return 0.0;
+  const int n = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo);
+  unsigned long long m = n >= 64 ? lo << (n - 64) : n ? (hi << n) | (lo >> (64 - n)) : hi;
+  if (n < 64 && (lo << n)) m |= 1;  // what lies below only matters beside a tie
+  return assemble(m, 127 - n - eab, neg);
+}
+
+// X 2^-eab for the residues r[q] (four signed bytes each): the fraction X/P in
+// 96-bit fixed point (wrapping: the whole part drops out) times P.
+__device__ __forceinline__ double crt_value(const unsigned (&r)[4], int eab) {
+  int s[12];
+#pragma unroll
+  for (int b = 0; b < 12; ++b) {
+    s[b] = 0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) s[b] = dp4a_su(r[q], DT.phi[q][b], s[b]);
+  }
+  const long long low = (long long)(s[0] + (s[1] << 8)) + ((long long)(s[2] + (s[3] << 8)) << 16);
+  const unsigned lo = (unsigned)low;
+  long long h = (long long)(s[4] + (s[5] << 8)) + (low >> 32);
+  h += (long long)(s[6] + (s[7] << 8)) << 16;
+  h += (long long)((unsigned long long)(long long)(s[8] + (s[9] << 8)) << 32);
+  h += (long long)((unsigned long long)(long long)(s[10] + (s[11] << 8)) << 48);
+  const bool neg = h < 0;
+  const unsigned l2 = neg ? 0u - lo : lo;
+  const unsigned long long H = neg ? ~(unsigned long long)h + (lo == 0) : (unsigned long long)h;
+  if (H < (1ull << 36)) return crt_small(r[0], r[1], r[2], r[3], eab);
+  const int n = __clzll((long long)H);  // 1 .. 27
+  const unsigned long long m = (H << n) | ((unsigned long long)l2 >> (32 - n));
+  // m 2^-(64 + n) is the fraction, pm 2^62 the modulus P
+  const unsigned long long q = __umul64hi(m, DT.pm);
+  const int z = q >> 63 ? 0 : 1;
+  return assemble(q << z, 125 - n - z - eab, neg);
+}
+
+struct CrtParams {
+  RowMap A, B;               // C's rows m (A) and columns n (B)
+  int row0, col0;            // of this part
+  int nm, nn;                // rows and columns of this part
+  const signed char *res;    // [plane][n][ldm]
+  long long ldm;
+  const int *ea, *eb;
+  const unsigned char *fa, *fb;
+  double *C;
+  double alpha, beta;
+  const double *eo, *ev;
+  int denom, lower;
+  unsigned *list;            // [0] count, then tiles (tn * tiles_m + tm) left to FP64
+};
+
+__device__ __forceinline__ long long c_off(const RowMap &M, int r) {
+  const int d0 = r % M.ext[0], q = r / M.ext[0];
+  const int d1 = q % M.ext[1], d2 = q / M.ext[1];
+  return d0 * M.cst[0] + d1 * M.cst[1] + d2 * M.cst[2];
+}
+
+// the index along the dimension with the given role (0: m or n, 1: batch)
+__device__ __forceinline__ int role_index(const RowMap &M, int r, int role) {
+  const int d0 = r % M.ext[0], q = r / M.ext[0];
+  const int d1 = q % M.ext[1], d2 = q / M.ext[1];
+  return (M.role[0] == role ? d0 : 0) + (M.role[1] == role ? d1 : 0) + (M.role[2] == role ? d2 : 0);
+}
+
+__device__ __forceinline__ void put_c(const CrtParams &P, int m, int n, double v) {
+  if (P.denom) {
+    // RIMP2.F90:403-404: deltaEPS = EVocc(I)+EVocc(J)-EVvirt(B)-EVvirt(A)
+    const double d = P.eo[role_index(P.A, m, 1)] + P.eo[role_index(P.B, n, 1)] -
+                     P.ev[role_index(P.B, n, 0)] - P.ev[role_index(P.A, m, 0)];
+    v = v / d;
+  }
+  double *c = P.C + c_off(P.A, m) + c_off(P.B, n);
+  v = P.alpha * v;
+  if (P.beta != 0.0) v += P.beta * *c;
+  *c = v;
+}
+
+// A block takes 64 rows x 64 columns of C; a thread four consecutive rows of
+// four columns.  It reads 17 bytes and writes 8 per element.
+__global__ void __launch_bounds__(256) crt_epilogue_kernel(CrtParams P) {
+  __shared__ int count;
+  const int tm = blockIdx.x, tn = blockIdx.y;
+  if (P.lower && tm < tn) return;
+  const int mq = (threadIdx.x & 15) * 4, nq = threadIdx.x >> 4;
+  const int m0 = tm * 64 + mq, n0 = tn * 64 + nq;
+  const long long plane = (long long)P.nn * P.ldm;
+  if (threadIdx.x == 0) count = 0;
+  __syncthreads();
+  // which elements are summed in FP64
+  unsigned todo = 0;
+  unsigned fm = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) fm |= (unsigned)(m0 + k < P.nm ? P.fa[m0 + k] : (unsigned)MG_ROW_ZERO) << (8 * k);
+#pragma unroll
+  for (int y = 0; y < 4; ++y) {
+    const int n = n0 + 16 * y;
+    if (n >= P.nn) continue;
+    const unsigned g = *reinterpret_cast<const unsigned *>(P.res + MG_P * plane + n * P.ldm + m0);
+    const unsigned fn = P.fb[n];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const unsigned f = (fm >> (8 * k)) & 0xFFu;
+      const bool need = ((f | fn) & MG_ROW_FP64) ||
+                        (!((f | fn) & MG_ROW_ZERO) && !(f & fn & MG_ROW_EXACT) && !((g >> (8 * k)) & 1u));
+      if (need && m0 + k < P.nm) todo |= 1u << (4 * y + k);
+    }
+  }
+  if (todo) atomicAdd(&count, __popc(todo));
+  __syncthreads();
+  if (count > MG_TILE_MAX) {
+    if (threadIdx.x == 0) P.list[1 + atomicAdd(P.list, 1u)] = tn * gridDim.x + tm;
+    return;
+  }
+  const int lane = threadIdx.x & 31;
+  int ea[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) ea[k] = m0 + k < P.nm ? P.ea[m0 + k] : 0;
+#pragma unroll 1
+  for (int y = 0; y < 4; ++y) {
+    const int n = n0 + 16 * y;
+    if (n < P.nn) {
+      unsigned w[MG_P];
+      const signed char *src = P.res + n * P.ldm + m0;
+#pragma unroll
+      for (int p = 0; p < MG_P; ++p) w[p] = *reinterpret_cast<const unsigned *>(src + p * plane);
+      const int eb = P.eb[n];
+      // 4 x 4 byte transposes: r[k][q] holds planes 4q .. 4q+3 of row m0 + k
+      unsigned r[4][4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const unsigned a = __byte_perm(w[4 * q], w[4 * q + 1], 0x5140), b = __byte_perm(w[4 * q + 2], w[4 * q + 3], 0x5140);
+        const unsigned c = __byte_perm(w[4 * q], w[4 * q + 1], 0x7362), d = __byte_perm(w[4 * q + 2], w[4 * q + 3], 0x7362);
+        r[0][q] = __byte_perm(a, b, 0x5410);
+        r[1][q] = __byte_perm(a, b, 0x7632);
+        r[2][q] = __byte_perm(c, d, 0x5410);
+        r[3][q] = __byte_perm(c, d, 0x7632);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (m0 + k < P.nm && !((todo >> (4 * y + k)) & 1u))
+          put_c(P, P.row0 + m0 + k, P.col0 + n, crt_value(r[k], ea[k] + eb));
+    }
+    // the others: one warp per element
+#pragma unroll 1
+    for (int k = 0; k < 4; ++k) {
+      unsigned mask = __ballot_sync(0xffffffffu, (todo >> (4 * y + k)) & 1u);
+      while (mask) {
+        const int src = __ffs(mask) - 1;
+        mask &= mask - 1;
+        const int m = __shfl_sync(0xffffffffu, P.row0 + m0 + k, src);
+        const int nn = __shfl_sync(0xffffffffu, P.col0 + n, src);
+        const double *a = P.A.base + row_off(P.A, m), *b = P.B.base + row_off(P.B, nn);
+        double s = 0.0;
+        for (int q = lane; q < P.A.K; q += 32) s = fma(a[q * P.A.sk], b[q * P.B.sk], s);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == src) put_c(P, m, nn, s);
+      }
+    }
+  }
+}
+
+// The listed 64 x 64 tiles with FP64 tensor operations (DMMA m8n8k4).
+constexpr int DK = 16, DP = 20;
+__global__ void __launch_bounds__(256) dmma_tiles_kernel(CrtParams P, int tiles_m) {
+  __shared__ double As[64][DP], Bs[64][DP];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int wm = (warp & 1) * 32, wn = (warp >> 1) * 16, gid = lane >> 2, tig = lane & 3;
+  const unsigned ntile = P.list[0];
+  for (unsigned t = blockIdx.x; t < ntile; t += gridDim.x) {
+    const int id = (int)P.list[1 + t], m0 = (id % tiles_m) * 64, n0 = (id / tiles_m) * 64;
+    double acc[4][2][2];
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+      for (int y = 0; y < 2; ++y) acc[x][y][0] = acc[x][y][1] = 0.0;
+    // this thread's four (row, k) places of each operand
+    const double *pa[4], *pb[4];
+    int ra[4], rb[4], ka[4], kb[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      ra[q] = P.A.sk == 1 ? (tid >> 4) + 16 * q : tid & 63;
+      ka[q] = P.A.sk == 1 ? tid & 15 : (tid >> 6) + 4 * q;
+      rb[q] = P.B.sk == 1 ? (tid >> 4) + 16 * q : tid & 63;
+      kb[q] = P.B.sk == 1 ? tid & 15 : (tid >> 6) + 4 * q;
+      pa[q] = m0 + ra[q] < P.nm ? P.A.base + row_off(P.A, P.row0 + m0 + ra[q]) : nullptr;
+      pb[q] = n0 + rb[q] < P.nn ? P.B.base + row_off(P.B, P.col0 + n0 + rb[q]) : nullptr;
+    }
+    for (int k0 = 0; k0 < P.A.K; k0 += DK) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        As[ra[q]][ka[q]] = pa[q] && k0 + ka[q] < P.A.K ? pa[q][(long long)(k0 + ka[q]) * P.A.sk] : 0.0;
+        Bs[rb[q]][kb[q]] = pb[q] && k0 + kb[q] < P.A.K ? pb[q][(long long)(k0 + kb[q]) * P.B.sk] : 0.0;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int ks = 0; ks < DK; ks += 4) {
+        double af[4], bf[2];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) af[x] = As[wm + 8 * x + gid][ks + tig];
+#pragma unroll
+        for (int y = 0; y < 2; ++y) bf[y] = Bs[wn + 8 * y + gid][ks + tig];
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+          for (int y = 0; y < 2; ++y)
+            asm volatile(
+                "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                : "+d"(acc[x][y][0]), "+d"(acc[x][y][1])
+                : "d"(af[x]), "d"(bf[y]));
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+#pragma unroll
+      for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int m = m0 + wm + 8 * x + gid, n = n0 + wn + 8 * y + 2 * tig + h;
+          if (m < P.nm && n < P.nn) put_c(P, P.row0 + m, P.col0 + n, acc[x][y][h]);
+        }
+  }
+}
+
+// --------------------------------------------------------------------------
+// host side
+// --------------------------------------------------------------------------
+int encode_planes(CUtensorMap &tm, const ModOperand &op) {
+  auto encode = get_encode();
+  if (!encode) {
+    set_error("cuTensorMapEncodeTiled entry point unavailable");
+    return RIMP2_ERR_UNSUPPORTED;
+  }
+  const cuuint64_t rows = (cuuint64_t)op.rows * op.nkc;
+  cuuint64_t dims[3] = {64, rows, MG_PLANES};
+  cuuint64_t strides[2] = {128, rows * 128};
+  cuuint32_t box[3] = {KSTEP, TILE, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult cr = encode(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, op.planes.p, dims, strides, box, estr,
+                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (cr != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed (%d)", (int)cr);
+    return RIMP2_ERR_CUDA;
+  }
+  return RIMP2_OK;
+}
+
+// Stream-ordered allocation that leaves no error behind: the caller has
+// another way to compute the product.
+int try_alloc(DevBuf &b, size_t bytes, cudaStream_t s) {
+  const int rc = b.alloc(bytes, s);
+  if (rc != RIMP2_OK) {
+    (void)cudaGetLastError();
+    clear_error();
+  }
+  return rc;
+}
+
+}  // namespace
+
+size_t mod_operand_bytes(int rows, int K) {
+  const size_t nkc = (K + 63) / 64;
+  return (size_t)MG_PLANES * nkc * rows * 128;
+}
+
+int mod_operand_alloc(ModOperand &op, int rows, int K, cudaStream_t s) {
+  op.rows = rows;
+  op.nkc = (K + 63) / 64;
+  if (try_alloc(op.planes, mod_operand_bytes(rows, K), s) != RIMP2_OK) return RIMP2_ERR_NOMEM;
+  if (try_alloc(op.e, sizeof(int) * (size_t)rows, s) != RIMP2_OK) return RIMP2_ERR_NOMEM;
+  return try_alloc(op.flag, (size_t)rows, s);
+}
+
+int mod_operand_fill(ModOperand &op, const RowMap &M, int row0, bool col, cudaStream_t s) {
+  const int R = op.rows;
+  const size_t plane = (size_t)op.nkc * R * 64;
+  int *e = op.e.as<int>();
+  unsigned char *fl = op.flag.as<unsigned char>();
+  __half *out = op.planes.as<__half>();
+  if (M.sk == 1) {
+    row_scale_k_kernel<<<(unsigned)((R + 7ll) / 8), 256, 0, s>>>(M, row0, R, e, fl);
+    const unsigned grid = (unsigned)(((long long)op.nkc * R + 31) / 32);
+    if (col)
+      residue_k_kernel<true><<<grid, 256, 0, s>>>(M, row0, R, op.nkc, e, fl, out, plane);
+    else
+      residue_k_kernel<false><<<grid, 256, 0, s>>>(M, row0, R, op.nkc, e, fl, out, plane);
+  } else {
+    const unsigned nrb = (unsigned)((R + 31ll) / 32);
+    row_scale_r_kernel<<<nrb, 512, 0, s>>>(M, row0, R, e, fl);
+    if (col)
+      residue_r_kernel<true><<<nrb * op.nkc, 256, 0, s>>>(M, row0, R, op.nkc, e, fl, out, plane);
+    else
+      residue_r_kernel<false><<<nrb * op.nkc, 256, 0, s>>>(M, row0, R, op.nkc, e, fl, out, plane);
+  }
+  count_launch(2);
+  RIMP2_CK(cudaGetLastError());
+  return RIMP2_OK;
+}
+
+int mod_product(const ModOperand &L, const ModOperand &Q, signed char *out, long long ldm, bool lower,
+                cudaStream_t s) {
+  CUtensorMap tl, tq;
+  RIMP2_TRY(encode_planes(tl, L));
+  RIMP2_TRY(encode_planes(tq, Q));
+  MgParams P;
+  P.rows_l = L.rows;
+  P.rows_q = Q.rows;
+  P.tiles_l = (L.rows + 255) / 256;
+  P.tiles_q = (Q.rows + 255) / 256;
+  P.nkc = L.nkc;
+  P.lower = lower;
+  P.out = out;
+  P.ldm = ldm;
+  P.err = device_error_word();
+  RIMP2_CK(cudaFuncSetAttribute(mod_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM));
+  int dev = 0, nsm = 0;
+  RIMP2_CK(cudaGetDevice(&dev));
+  RIMP2_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const long long nitems = (long long)MG_PLANES * P.tiles_l * P.tiles_q;
+  const int npair = (int)std::min<long long>(nitems, nsm / 2);
+  mod_gemm_kernel<<<2 * npair, MG_THREADS, MG_SMEM, s>>>(tl, tq, P);
+  count_launch(1);
+  RIMP2_CK(cudaGetLastError());
+  return RIMP2_OK;
+}
+
+namespace {
+
+struct Dim {
+  int ext;
+  long long st, cst;
+  int role;
+};
+
+// Up to three dimensions into a row map, the fastest one first: by the
+// operand's stride where rows lie along the fast direction of memory, else by
+// C's (the operand is read along K either way).
+bool make_map(RowMap &M, Dim *d, int nd, const double *base, long long sk, int K) {
+  std::sort(d, d + nd, [&](const Dim &x, const Dim &y) {
+    return sk == 1 ? x.cst < y.cst : x.st < y.st;
+  });
+  long long rows = 1;
+  for (int k = 0; k < 3; ++k) {
+    M.ext[k] = k < nd ? d[k].ext : 1;
+    M.st[k] = k < nd ? d[k].st : 0;
+    M.cst[k] = k < nd ? d[k].cst : 0;
+    M.role[k] = k < nd ? d[k].role : -1;
+    rows *= M.ext[k];
+  }
+  M.base = base;
+  M.sk = sk;
+  M.K = K;
+  if (rows > 2147480000LL) return false;
+  M.rows = (int)rows;
+  return true;
+}
+
+constexpr size_t MG_PLANE_CAP = (size_t)6 << 30;  // bytes of one operand's planes per part
+constexpr size_t MG_RES_CAP = (size_t)4 << 30;    // bytes of the residues of a part of C
+
+}  // namespace
+
+int mod_gemm(const GemmDesc &g, cudaStream_t s, bool *handled) {
+  *handled = false;
+  if (g.K < 8 || g.K > 16384 || g.alpha == 0.0) return RIMP2_OK;
+  // batch dimensions that move only one operand are more rows or columns
+  Dim da[3] = {{g.M, g.sAm, g.sCm, 0}}, db[3] = {{g.N, g.sBn, g.sCn, 0}};
+  int na = 1, nb = 1;
+  const int ext[2] = {g.nb0, g.nb1};
+  const long long sa[2] = {g.sAb0, g.sAb1}, sb[2] = {g.sBb0, g.sBb1}, sc[2] = {g.sCb0, g.sCb1};
+  for (int k = 0; k < 2; ++k) {
+    if (g.denom ? false : ext[k] == 1) continue;
+    // with denominators the first batch index is the row's i, the second the column's j
+    if (g.denom ? k == 0 : sb[k] == 0)
+      da[na++] = {ext[k], sa[k], sc[k], 1};
+    else if (g.denom || sa[k] == 0)
+      db[nb++] = {ext[k], sb[k], sc[k], 1};
+    else
+      return RIMP2_OK;
+    if (g.denom && (k == 0 ? sb[k] : sa[k]) != 0 && ext[k] > 1) return RIMP2_OK;
+  }
+  RowMap A, B;
+  if (!make_map(A, da, na, g.A, g.sAk, g.K) || !make_map(B, db, nb, g.B, g.sBk, g.K)) return RIMP2_OK;
+  if (!mod_gemm_pays(g, A.rows, B.rows)) return RIMP2_OK;
+  // parts: bounded workspaces, whatever the product's size
+  const long long cap_rows = std::max<long long>(256, (long long)(MG_PLANE_CAP / mod_operand_bytes(1, g.K)) / 256 * 256);
+  const int ra = (int)std::min<long long>(A.rows, cap_rows);
+  const long long ldm = ((long long)ra + 255) / 256 * 256;
+  const long long cap_cols = std::max<long long>(256, (long long)(MG_RES_CAP / (MG_PLANES * ldm)) / 256 * 256);
+  const int rb = (int)std::min<long long>(B.rows, std::min(cap_rows, cap_cols));
+  if (g.lower && (ra < A.rows || rb < B.rows)) return RIMP2_OK;
+  if ((rb + 63) / 64 > 65535) return RIMP2_OK;
+  const long long tiles_m = (ra + 63) / 64, tiles_n = (rb + 63) / 64;
+  ModOperand Q, L;
+  DevBuf res, list;
+  if (mod_operand_alloc(Q, ra, g.K, s) != RIMP2_OK || mod_operand_alloc(L, rb, g.K, s) != RIMP2_OK ||
+      try_alloc(res, (size_t)MG_PLANES * rb * ldm, s) != RIMP2_OK ||
+      try_alloc(list, sizeof(unsigned) * (size_t)(tiles_m * tiles_n + 1), s) != RIMP2_OK)
+    return RIMP2_OK;  // no room: the FP64 kernel needs none
+  CrtParams P;
+  memset(&P, 0, sizeof P);
+  P.A = A;
+  P.B = B;
+  P.res = res.as<signed char>();
+  P.C = g.C;
+  P.alpha = g.alpha;
+  P.beta = g.beta;
+  P.eo = g.eo;
+  P.ev = g.ev;
+  P.denom = g.denom;
+  P.lower = g.lower;
+  P.list = list.as<unsigned>();
+  P.ea = Q.e.as<int>();
+  P.fa = Q.flag.as<unsigned char>();
+  P.eb = L.e.as<int>();
+  P.fb = L.flag.as<unsigned char>();
+  for (int r0 = 0; r0 < A.rows; r0 += ra) {
+    Q.rows = std::min(ra, A.rows - r0);
+    RIMP2_TRY(mod_operand_fill(Q, A, r0, false, s));
+    for (int c0 = 0; c0 < B.rows; c0 += rb) {
+      const int nc = std::min(rb, B.rows - c0);
+      if (r0 == 0 || rb < B.rows) {
+        L.rows = nc;
+        RIMP2_TRY(mod_operand_fill(L, B, c0, true, s));
+      }
+      P.row0 = r0;
+      P.col0 = c0;
+      P.nm = Q.rows;
+      P.nn = nc;
+      P.ldm = ((long long)Q.rows + 255) / 256 * 256;
+      RIMP2_TRY(mod_product(L, Q, res.as<signed char>(), P.ldm, g.lower != 0, s));
+      RIMP2_CK(cudaMemsetAsync(list.p, 0, sizeof(unsigned), s));
+      dim3 grid((unsigned)((P.nm + 63) / 64), (unsigned)((P.nn + 63) / 64));
+      crt_epilogue_kernel<<<grid, 256, 0, s>>>(P);
+      const long long nt = (long long)grid.x * grid.y;
+      dmma_tiles_kernel<<<(unsigned)std::min<long long>(nt, 304), 256, 0, s>>>(P, (int)grid.x);
+      count_launch(2);
+      RIMP2_CK(cudaGetLastError());
+    }
+  }
+  *handled = true;
+  return RIMP2_OK;
+}
+
+// Which products go this way: estimated times of both forms.
+bool mod_gemm_pays(const GemmDesc &g, double m, double n) {
+  const double k = g.K, kp = (g.K + 63) / 64 * 64.0;
+  auto up = [](double x, double t) { return (double)((long long)((x + t - 1) / t)) * t; };
+  const double part = g.lower ? 0.55 : 1.0;
+  const double nbat = (double)g.nb0 * g.nb1;
+  const double t_dmma = part * 2.0 * up(g.M, 64) * up(g.N, 64) * nbat * up(k, 16) / 1.0e12;
+  const double t_mod = 30e-6 + (m + n) * kp * 16e-12 +
+                       part * (m * n * 16e-12 + 17.0 * 2.0 * up(m, 256) * up(n, 256) * (kp + 64) / 1.3e15);
+  return t_mod < 0.8 * t_dmma;
+}
+
+}  // namespace rimp2

@@ -1,0 +1,149 @@
+"""FP64 contractions through residues on the FP16 tensor cores (mod_gemm.cu):
+the general product over its forms and tile edges, against exactly rounded
+sums, and the elements and tiles that it leaves to FP64 arithmetic."""
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+U = 2.0 ** -53
+
+
+@pytest.fixture(scope="module")
+def api():
+    from rimp2_gpu_gb300 import api
+    return api
+
+
+def exact_dot(a, b):
+    """sum a b rounded once: error-free products (Dekker), math.fsum."""
+    c = 134217729.0
+    p = a * b
+    ah = a * c - (a * c - a)
+    bh = b * c - (b * c - b)
+    e = ((ah * bh - p) + ah * (b - bh) + (a - ah) * bh) + (a - ah) * (b - bh)
+    return math.fsum(np.concatenate([p, e]))
+
+
+def product(api, ta, tb, A, B, alpha, beta, C, pad=0):
+    """C := alpha A B + beta C through the library; the number of launches."""
+    m, k = A.shape
+    n = B.shape[1]
+
+    def store(x, t):
+        x = x.T if t == "T" else x
+        s = np.zeros((x.shape[0] + pad, x.shape[1]), order="F")
+        s[:x.shape[0]] = x
+        return s
+    As, Bs = store(A, ta), store(B, tb)
+    before = api.kernel_launch_count()
+    api.dgemm(ta, tb, m, n, k, alpha, As, As.shape[0], Bs, Bs.shape[0], beta, C, m)
+    return api.kernel_launch_count() - before
+
+
+@pytest.mark.parametrize("ta,tb,m,n,k,alpha,beta,pad", [
+    ("N", "N", 257, 255, 1025, 1.0, 0.0, 0),    # one value past a tile, a sum and a K chunk
+    ("T", "N", 256, 512, 1024, -1.0, 1.0, 0),   # whole tiles and sums
+    ("N", "T", 511, 321, 639, 0.5, -2.0, 3),    # ragged, leading dimensions beyond the extents
+    ("T", "T", 385, 700, 2049, 1.0, 0.0, 1),    # three sums, odd leading dimensions
+    ("T", "N", 4100, 4097, 8, 1.0, 0.0, 0),     # the shortest sum
+    ("N", "N", 70000, 3, 61, 1.0, 0.0, 0),      # far fewer columns than a tile
+])
+def test_product_forms(api, ta, tb, m, n, k, alpha, beta, pad):
+    r = np.random.Generator(np.random.Philox(key=[k, m]))
+    A, B = r.standard_normal((m, k)), r.standard_normal((k, n))
+    C0 = np.asfortranarray(r.standard_normal((m, n)))
+    C = C0.copy(order="F")
+    assert product(api, ta, tb, A, B, alpha, beta, C, pad) > 1, "expected the residue form"
+    I = np.concatenate([r.integers(0, m, 300), [0, m - 1, m - 1, 0]])
+    J = np.concatenate([r.integers(0, n, 300), [0, n - 1, 0, n - 1]])
+    for i, j in zip(I, J):
+        d = alpha * exact_dot(A[i], B[:, j])
+        ref = d + beta * C0[i, j]
+        # rounding to 62-bit integers: sqrt(K)/2 u sum|a||b| at most (an element
+        # under 2^-8 of the norms' product is summed in FP64); then alpha, beta
+        tol = abs(alpha) * (math.sqrt(k) / 2 + 2) * U * np.abs(A[i] * B[:, j]).sum() + \
+            3 * U * (abs(d) + abs(beta * C0[i, j]))
+        assert abs(C[i, j] - ref) <= tol
+
+
+def test_product_exact_and_special_values(api):
+    r = np.random.Generator(np.random.Philox(key=[5, 9]))
+    m = n = k = 640
+    # integers, sums that cancel, a permutation: results that FP64 holds come out exact
+    A = r.integers(-1000, 1000, (m, k)).astype(float)
+    B = r.integers(-1000, 1000, (k, n)).astype(float)
+    A[5, 0], A[5, 1], B[0, 7], B[1, 7] = 2.0 ** 45, 2.0 ** 45, 1.0, -1.0
+    C = np.zeros((m, n), order="F")
+    assert product(api, "N", "N", A, B, 1.0, 0.0, C) > 1
+    ref = A.astype(np.int64) @ B.astype(np.int64)
+    held = ref.astype(float).astype(np.int64) == ref  # row 5 has sums beyond 53 bits
+    assert held[6:].all() and not held.all()
+    assert np.array_equal(C[held], ref[held].astype(float))
+    assert (np.abs(C.astype(np.int64) - ref) <= np.spacing(np.abs(C))).all()
+    perm = np.eye(k)[r.permutation(k)]
+    X = r.standard_normal((m, k)) * np.exp(4 * r.standard_normal((m, k)))
+    product(api, "N", "N", X, perm, 1.0, 0.0, C)
+    assert np.array_equal(C, X @ perm)
+    # infinities, NaN, zeros, extreme magnitudes: as FP64 sums them
+    X = r.standard_normal((m, k))
+    X[3, 5], X[70, 2], X[100], X[400, 9] = np.nan, np.inf, 0.0, -np.inf
+    X[200] *= 1e-200
+    X[201] *= 1e300
+    X[:, 7] = 1e-310
+    Y = r.standard_normal((k, n))
+    Y[11, 13] = np.inf
+    product(api, "N", "N", X, Y, 1.0, 0.0, C)
+    with np.errstate(all="ignore"):
+        ref, mag = X @ Y, np.abs(X) @ np.abs(Y)
+    assert np.array_equal(np.isnan(C), np.isnan(ref))
+    assert np.array_equal(np.isinf(C), np.isinf(ref))
+    f = np.isfinite(ref)
+    assert np.array_equal(np.sign(C[~f & ~np.isnan(ref)]), np.sign(ref[~f & ~np.isnan(ref)]))
+    assert (np.abs(C - ref)[f] <= 2 * k * U * mag[f]).all()
+
+
+@pytest.mark.parametrize("spread", [2.0, 6.0])
+def test_rows_of_wide_range(api, spread):
+    """Log-normal values: a part, or nearly all, of the elements is summed in FP64."""
+    r = np.random.Generator(np.random.Philox(key=[17, int(spread)]))
+    m, n, k = 500, 520, 700
+    A = r.standard_normal((m, k)) * np.exp(spread * r.standard_normal((m, k)))
+    B = r.standard_normal((k, n)) * np.exp(spread * r.standard_normal((k, n)))
+    C = np.zeros((m, n), order="F")
+    assert product(api, "T", "N", A, B, 1.0, 0.0, C) > 1
+    for i, j in zip(r.integers(0, m, 400), r.integers(0, n, 400)):
+        ref = exact_dot(A[i], B[:, j])
+        assert abs(C[i, j] - ref) <= k * U * np.abs(A[i] * B[:, j]).sum()  # FP64's own bound
+
+
+def test_subroutine_forms(api):
+    """Every stride pattern that the drop-in subroutines hand to the product,
+    at sizes that take the residue form, against numpy's FP64."""
+    r = np.random.Generator(np.random.Philox(key=[3, 8]))
+    nv, no, ne, ve, nb = 201, 19, 9, 37, 333
+    F = np.asfortranarray
+    Ca = F(r.standard_normal((nb, nv, no)) * 0.03)
+    eo, ev = np.sort(-r.random(no) - 0.3), np.sort(r.random(nv) + 0.1)
+    UoE, UvT = F(r.standard_normal((no, ne))), F(r.standard_normal((nv, nv)))
+    UoT, UvE = F(r.standard_normal((no, no))), F(r.standard_normal((nv, ve)))
+    tocc, tvirt, gocc, gvirt = api.steps5to8(nv, no, ne, ve, nb, Ca, eo, ev, UoE, UvT, UoT, UvE)
+    g = np.tensordot(Ca, Ca, (0, 0))  # a i b j
+    t = g / (eo[None, :, None, None] + eo - ev[:, None, None, None] - ev[None, None, :, None])
+
+    def local(x, uo, uv):
+        x = np.tensordot(uv, x, (0, 0))
+        x = np.moveaxis(np.tensordot(uo, x, (0, 1)), 0, 1)
+        x = np.moveaxis(np.tensordot(uv, x, (0, 2)), 0, 2)
+        return np.moveaxis(np.tensordot(uo, x, (0, 3)), 0, 3)
+    for got, x, uo, uv, chain in ((tocc, t, UoE, UvT, nb + 2 * no + 2 * nv),
+                                  (tvirt, t, UoT, UvE, nb + 2 * no + 2 * nv),
+                                  (gocc, g, UoE, UvT, nb + 2 * no + 2 * nv),
+                                  (gvirt, g, UoT, UvE, nb + 2 * no + 2 * nv)):
+        ref, mag = local(x, uo, uv), None
+        gm = np.tensordot(np.abs(Ca), np.abs(Ca), (0, 0))
+        mag = local(gm / np.abs(g / x), np.abs(uo), np.abs(uv))
+        # the classical bound of the chain of sums, for either side
+        assert (np.abs(got - ref) <= 2 * chain * U * mag).all()
