@@ -38,7 +38,9 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
+#include <mutex>
 
 #include "tc.cuh"
 #include "mod_gemm.cuh"
@@ -421,13 +423,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
                      smem_u32(tmem_slot))
                  : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers are initialised before any remote access
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if (warp == 1)  // both CTAs hold their columns
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
 
   if (warp == 0) {
     // --------------------- TMA producers (both CTAs) ---------------------
@@ -616,12 +619,13 @@ __device__ __forceinline__ double assemble(unsigned long long m, int x, bool neg
 // X 2^-eab where |X / P| < 2^-28: X = sum_p r_p P/p - k P in 128-bit integers
 // (wrapping), k the whole part of sum_p r_p / p.  Sums that cancel exactly,
 // or nearly, come here: the fraction's 96 bits would leave them too few.
-__device__ __noinline__ double crt_small(unsigned r0, unsigned r1, unsigned r2, unsigned r3, int eab) {
-  const unsigned r[4] = {r0, r1, r2, r3};
+// src: the element's residues, one byte per plane.
+__device__ __forceinline__ double crt_small(const signed char *src, long long plane, int eab) {
   unsigned long long lo = 0, hi = 0;
   float ks = 0.0f;
+#pragma unroll 4
   for (int p = 0; p < MG_P; ++p) {
-    const long long v = (signed char)(r[p >> 2] >> (8 * (p & 3)));
+    const long long v = src[p * plane];
     ks = fmaf((float)v, DT.inv[p], ks);
     const unsigned long long w = DT.wlo[p], q = lo + w * (unsigned long long)v;
     hi += DT.whi[p] * (unsigned long long)v + (unsigned long long)__mul64hi((long long)w, v) +
@@ -646,8 +650,9 @@ __device__ __noinline__ double crt_small(unsigned r0, unsigned r1, unsigned r2, 
 }
 
 // X 2^-eab for the residues r[q] (four signed bytes each): the fraction X/P in
-// 96-bit fixed point (wrapping: the whole part drops out) times P.
-__device__ __forceinline__ double crt_value(const unsigned (&r)[4], int eab) {
+// 96-bit fixed point (wrapping: the whole part drops out) times P.  False where
+// the fraction is too small for that (crt_small).
+__device__ __forceinline__ bool crt_value(const unsigned (&r)[4], int eab, double &v) {
   int s[12];
 #pragma unroll
   for (int b = 0; b < 12; ++b) {
@@ -664,13 +669,14 @@ __device__ __forceinline__ double crt_value(const unsigned (&r)[4], int eab) {
   const bool neg = h < 0;
   const unsigned l2 = neg ? 0u - lo : lo;
   const unsigned long long H = neg ? ~(unsigned long long)h + (lo == 0) : (unsigned long long)h;
-  if (H < (1ull << 36)) return crt_small(r[0], r[1], r[2], r[3], eab);
+  if (H < (1ull << 36)) return false;
   const int n = __clzll((long long)H);  // 1 .. 27
   const unsigned long long m = (H << n) | ((unsigned long long)l2 >> (32 - n));
   // m 2^-(64 + n) is the fraction, pm 2^62 the modulus P
   const unsigned long long q = __umul64hi(m, DT.pm);
   const int z = q >> 63 ? 0 : 1;
-  return assemble(q << z, 125 - n - z - eab, neg);
+  v = assemble(q << z, 125 - n - z - eab, neg);
+  return true;
 }
 
 struct CrtParams {
@@ -754,6 +760,7 @@ __global__ void __launch_bounds__(256) crt_epilogue_kernel(CrtParams P) {
   int ea[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) ea[k] = m0 + k < P.nm ? P.ea[m0 + k] : 0;
+  unsigned small = 0;
 #pragma unroll 1
   for (int y = 0; y < 4; ++y) {
     const int n = n0 + 16 * y;
@@ -775,26 +782,36 @@ __global__ void __launch_bounds__(256) crt_epilogue_kernel(CrtParams P) {
         r[3][q] = __byte_perm(c, d, 0x7632);
       }
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
-        if (m0 + k < P.nm && !((todo >> (4 * y + k)) & 1u))
-          put_c(P, P.row0 + m0 + k, P.col0 + n, crt_value(r[k], ea[k] + eb));
-    }
-    // the others: one warp per element
-#pragma unroll 1
-    for (int k = 0; k < 4; ++k) {
-      unsigned mask = __ballot_sync(0xffffffffu, (todo >> (4 * y + k)) & 1u);
-      while (mask) {
-        const int src = __ffs(mask) - 1;
-        mask &= mask - 1;
-        const int m = __shfl_sync(0xffffffffu, P.row0 + m0 + k, src);
-        const int nn = __shfl_sync(0xffffffffu, P.col0 + n, src);
-        const double *a = P.A.base + row_off(P.A, m), *b = P.B.base + row_off(P.B, nn);
-        double s = 0.0;
-        for (int q = lane; q < P.A.K; q += 32) s = fma(a[q * P.A.sk], b[q * P.B.sk], s);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == src) put_c(P, m, nn, s);
+      for (int k = 0; k < 4; ++k) {
+        double v;
+        if (m0 + k >= P.nm || ((todo >> (4 * y + k)) & 1u)) continue;
+        if (crt_value(r[k], ea[k] + eb, v))
+          put_c(P, P.row0 + m0 + k, P.col0 + n, v);
+        else
+          small |= 1u << (4 * y + k);
       }
+    }
+  }
+  // the few others: exact integers, or a sum in FP64 by one warp
+  if (!__any_sync(0xffffffffu, small | todo)) return;
+#pragma unroll 1
+  for (int x = 0; x < 16; ++x) {
+    const int k = x & 3, n = n0 + 16 * (x >> 2);
+    if ((small >> x) & 1u)
+      put_c(P, P.row0 + m0 + k, P.col0 + n,
+            crt_small(P.res + n * P.ldm + m0 + k, plane, P.ea[m0 + k] + P.eb[n]));
+    unsigned mask = __ballot_sync(0xffffffffu, (todo >> x) & 1u);
+    while (mask) {
+      const int src = __ffs(mask) - 1;
+      mask &= mask - 1;
+      const int m = __shfl_sync(0xffffffffu, P.row0 + m0 + k, src);
+      const int nn = __shfl_sync(0xffffffffu, P.col0 + n, src);
+      const double *a = P.A.base + row_off(P.A, m), *b = P.B.base + row_off(P.B, nn);
+      double s = 0.0;
+      for (int q = lane; q < P.A.K; q += 32) s = fma(a[q * P.A.sk], b[q * P.B.sk], s);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == src) put_c(P, m, nn, s);
     }
   }
 }
@@ -805,7 +822,7 @@ __global__ void __launch_bounds__(256) dmma_tiles_kernel(CrtParams P, int tiles_
   __shared__ double As[64][DP], Bs[64][DP];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = (warp & 1) * 32, wn = (warp >> 1) * 16, gid = lane >> 2, tig = lane & 3;
-  const unsigned ntile = P.list[0];
+  const unsigned ntile = min(P.list[0], (unsigned)(tiles_m * ((P.nn + 63) / 64)));
   for (unsigned t = blockIdx.x; t < ntile; t += gridDim.x) {
     const int id = (int)P.list[1 + t], m0 = (id % tiles_m) * 64, n0 = (id / tiles_m) * 64;
     double acc[4][2][2];
@@ -959,9 +976,8 @@ int mod_product(const ModOperand &L, const ModOperand &Q, signed char *out, long
   RIMP2_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const long long nitems = (long long)MG_PLANES * P.tiles_l * P.tiles_q;
   const int npair = (int)std::min<long long>(nitems, nsm / 2);
-  mod_gemm_kernel<<<2 * npair, MG_THREADS, MG_SMEM, s>>>(tl, tq, P);
+  RIMP2_CK(launch_hi(mod_gemm_kernel, 2 * npair, MG_THREADS, MG_SMEM, s, tl, tq, P));
   count_launch(1);
-  RIMP2_CK(cudaGetLastError());
   return RIMP2_OK;
 }
 
@@ -996,6 +1012,35 @@ bool make_map(RowMap &M, Dim *d, int nd, const double *base, long long sk, int K
   return true;
 }
 
+// One contraction's kernels at a time on the device: a later one, on whatever
+// stream and from whatever thread, starts when the earlier one's have ended.
+// Each fills the GPU by itself, so nothing is lost; several at once (persistent
+// CTA pairs between the operands' and the epilogue's many small blocks on other
+// streams) were seen to stop the GPU's scheduling.  Held while a contraction
+// is queued.
+class ModOrder {
+  static std::mutex mu;
+  static cudaEvent_t last;
+  std::unique_lock<std::mutex> lk;
+  cudaStream_t s;
+
+ public:
+  explicit ModOrder(cudaStream_t st) : lk(mu), s(st) {}
+  int begin() {
+    if (!last) {
+      RIMP2_CK(cudaEventCreateWithFlags(&last, cudaEventDisableTiming));
+      return RIMP2_OK;
+    }
+    RIMP2_CK(cudaStreamWaitEvent(s, last, 0));
+    return RIMP2_OK;
+  }
+  ~ModOrder() {
+    if (last) cudaEventRecord(last, s);
+  }
+};
+std::mutex ModOrder::mu;
+cudaEvent_t ModOrder::last = nullptr;
+
 constexpr size_t MG_PLANE_CAP = (size_t)6 << 30;  // bytes of one operand's planes per part
 constexpr size_t MG_RES_CAP = (size_t)4 << 30;    // bytes of the residues of a part of C
 
@@ -1003,7 +1048,7 @@ constexpr size_t MG_RES_CAP = (size_t)4 << 30;    // bytes of the residues of a 
 
 int mod_gemm(const GemmDesc &g, cudaStream_t s, bool *handled) {
   *handled = false;
-  if (g.K < 8 || g.K > 16384 || g.alpha == 0.0) return RIMP2_OK;
+  if (g.K < MG_K_MIN || g.K > MG_K_MAX || g.alpha == 0.0) return RIMP2_OK;
   // batch dimensions that move only one operand are more rows or columns
   Dim da[3] = {{g.M, g.sAm, g.sCm, 0}}, db[3] = {{g.N, g.sBn, g.sCn, 0}};
   int na = 1, nb = 1;
@@ -1023,6 +1068,13 @@ int mod_gemm(const GemmDesc &g, cudaStream_t s, bool *handled) {
   RowMap A, B;
   if (!make_map(A, da, na, g.A, g.sAk, g.K) || !make_map(B, db, nb, g.B, g.sBk, g.K)) return RIMP2_OK;
   if (!mod_gemm_pays(g, A.rows, B.rows)) return RIMP2_OK;
+  // a captured call keeps to the FP64 kernel: the order between contractions
+  // (ModOrder) cannot reach into a graph
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    (void)cudaGetLastError();
+    return RIMP2_OK;
+  }
   // parts: bounded workspaces, whatever the product's size
   const long long cap_rows = std::max<long long>(256, (long long)(MG_PLANE_CAP / mod_operand_bytes(1, g.K)) / 256 * 256);
   const int ra = (int)std::min<long long>(A.rows, cap_rows);
@@ -1038,6 +1090,8 @@ int mod_gemm(const GemmDesc &g, cudaStream_t s, bool *handled) {
       try_alloc(res, (size_t)MG_PLANES * rb * ldm, s) != RIMP2_OK ||
       try_alloc(list, sizeof(unsigned) * (size_t)(tiles_m * tiles_n + 1), s) != RIMP2_OK)
     return RIMP2_OK;  // no room: the FP64 kernel needs none
+  ModOrder order(s);
+  RIMP2_TRY(order.begin());
   CrtParams P;
   memset(&P, 0, sizeof P);
   P.A = A;
@@ -1083,16 +1137,29 @@ int mod_gemm(const GemmDesc &g, cudaStream_t s, bool *handled) {
   return RIMP2_OK;
 }
 
-// Which products go this way: estimated times of both forms.
+// Estimated time of the residue form: launches and latencies, the residues of
+// both operands, the products, the reconstruction.
+double mod_gemm_time(double m, double n, double k, bool lower) {
+  auto up = [](double x, double t) { return std::ceil(x / t) * t; };
+  const double kp = up(k, 64), part = lower ? 0.55 : 1.0;
+  return 30e-6 + (m + n) * kp * 16e-12 +
+         part * (m * n * 16e-12 + 17.0 * 2.0 * up(m, 256) * up(n, 256) * (kp + 64) / 1.3e15);
+}
+
+// Which products go this way: estimated times of both forms (DMMA on 64 x 64
+// tiles of each product of the batch).
 bool mod_gemm_pays(const GemmDesc &g, double m, double n) {
-  const double k = g.K, kp = (g.K + 63) / 64 * 64.0;
-  auto up = [](double x, double t) { return (double)((long long)((x + t - 1) / t)) * t; };
-  const double part = g.lower ? 0.55 : 1.0;
-  const double nbat = (double)g.nb0 * g.nb1;
-  const double t_dmma = part * 2.0 * up(g.M, 64) * up(g.N, 64) * nbat * up(k, 16) / 1.0e12;
-  const double t_mod = 30e-6 + (m + n) * kp * 16e-12 +
-                       part * (m * n * 16e-12 + 17.0 * 2.0 * up(m, 256) * up(n, 256) * (kp + 64) / 1.3e15);
-  return t_mod < 0.8 * t_dmma;
+  auto up = [](double x, double t) { return std::ceil(x / t) * t; };
+  const double t_dmma = (g.lower ? 0.55 : 1.0) * 2.0 * up(g.M, 64) * up(g.N, 64) * g.nb0 * (double)g.nb1 *
+                        up(g.K, 16) / 1.0e12;
+  return mod_gemm_time(m, n, g.K, g.lower != 0) < 0.8 * t_dmma;
+}
+
+// Rows and columns of a square product that runs as one part.
+int mod_gemm_block(int K) {
+  const double rows = std::min((double)(MG_PLANE_CAP / mod_operand_bytes(1, K)),
+                               std::sqrt((double)(MG_RES_CAP / MG_PLANES)));
+  return (int)rows / 256 * 256;
 }
 
 }  // namespace rimp2

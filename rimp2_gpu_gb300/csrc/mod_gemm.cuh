@@ -12,6 +12,8 @@ constexpr int MG_PLANES = MG_P + 1;  // and the plane of magnitudes
 constexpr float MG_TAU = 65536.0f;
 constexpr int MG_TILE_MAX = 512;     // of a 64 x 64 tile's elements; beyond it the whole tile is
 
+constexpr int MG_K_MIN = 8, MG_K_MAX = 16384;  // lengths of a sum
+
 // a row's (or column's) flags
 constexpr unsigned MG_ROW_ZERO = 1;   // all zeros
 constexpr unsigned MG_ROW_FP64 = 2;   // infinities, NaNs, extreme exponents: FP64 only
@@ -44,6 +46,8 @@ int mod_operand_fill(ModOperand &op, const RowMap &M, int row0, bool col, cudaSt
 int mod_product(const ModOperand &L, const ModOperand &Q, signed char *out, long long ldm, bool lower,
                 cudaStream_t s);
 bool mod_gemm_pays(const GemmDesc &g, double m, double n);
+double mod_gemm_time(double m, double n, double k, bool lower);  // seconds, estimated
+int mod_gemm_block(int K);
 // The contraction of g; *handled = false where FP64 tensor operations are the
 // better way (or there is no room for the workspace): nothing was launched.
 int mod_gemm(const GemmDesc &g, cudaStream_t s, bool *handled);

@@ -263,5 +263,35 @@ PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
   return fn;
 }
 
+// Launch with the device's highest scheduling priority.  The persistent
+// energy kernels of a batch graph run beside the slicing of the next launch
+// group on a side branch; without priority the slicer's many small blocks,
+// ready at the same moment, fill the SMs first and the energy kernel's CTAs
+// wait for them to drain.  (The priority is recorded into graph nodes.)
+int energy_priority() {
+  static int prio = 1;
+  if (prio == 1) {
+    int least = 0, greatest = 0;
+    prio = cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess ? greatest : 0;
+  }
+  return prio;
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_hi(void (*k)(KArgs...), unsigned grid, unsigned block, size_t smem,
+                      cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributePriority;
+  at[0].val.priority = energy_priority();
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
 }  // namespace
 }  // namespace rimp2
