@@ -23,6 +23,7 @@
 #include "mod_gemm.cuh"
 
 #include <algorithm>
+#include <cstring>
 #include <vector>
 
 namespace rimp2 {
@@ -399,6 +400,98 @@ __global__ void __launch_bounds__(NTHR, 2) eos_energy_kernel(const double *__res
   }
 }
 
+// Pair energies from integrals in memory: G(x, y) = sum_al C(al, x) C(al, y)
+// for the columns x = (b, j) of a block of occupied orbitals and y = (a, i) of
+// another (the same or an earlier one: then only x >= y is read).  A block
+// takes the 64 x 64 tile pair (A, B) of a pair i <= j: rows (b,j), columns
+// (a,i) hold g_ij(a,b); rows (a,j), columns (b,i) hold g_ij(b,a) and pass
+// through shared memory, so that both are read along the fast direction.  Off
+// the diagonal tile the two orders share a denominator:
+// 2 (g1^2 - g1 g2 + g2^2) / D.  It reads each integral once (8 bytes; twice on
+// diagonal tiles) and keeps to about ten FP64 operations per pair of elements:
+// at 1/64 of the FP32 rate these take as long as the reads.  The reciprocal is
+// the FP32 one refined by a third-order Newton step (error about an ulp).
+struct GEnergyArgs {
+  const double *G;
+  long long ld;
+  int i0, j0, ni, nvirt, nocc;
+  const double *eo, *ev;
+  double *part, *tamp;
+};
+
+__device__ __forceinline__ double recip_f64(double d) {
+  float r32;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r32) : "f"((float)d));
+  const double r0 = (double)r32;
+  const double e = fma(-d, r0, 1.0);
+  return fma(r0, fma(e, e, e), r0);
+}
+
+constexpr int GE_PITCH = 65;
+
+__global__ void __launch_bounds__(NTHR) g_energy_kernel(GEnergyArgs P) {
+  __shared__ double S[TN * GE_PITCH];  // g_ij(b,a) at [b][a]
+  __shared__ double red[NTHR / 32];
+  const int i = P.i0 + (int)(blockIdx.x % P.ni), j = P.j0 + (int)(blockIdx.x / P.ni);
+  if (i > j) return;
+  int tA, tB;
+  decode_tri((int)blockIdx.y, tA, tB);
+  const bool same = (i == j), diag = (tA == tB);
+  const int a0 = tA * TM, b0 = tB * TN, nv = P.nvirt;
+  const int r = threadIdx.x & 63, c0 = threadIdx.x >> 6;  // row, first column of a tile
+  const double *gj = P.G + (long long)(j - P.j0) * nv;            // rows (., j)
+  const double *gi = gj + P.ld * (long long)(i - P.i0) * nv;      // columns (., i)
+  if (!same) {
+#pragma unroll 8
+    for (int c = c0; c < TN; c += NTHR / 64)
+      if (a0 + r < nv && b0 + c < nv) S[c * GE_PITCH + r] = gi[(a0 + r) + P.ld * (b0 + c)];
+    __syncthreads();
+  }
+  const double eij = P.eo[i] + P.eo[j];
+  const int b = b0 + r;
+  double e = 0.0;
+  if (b < nv) {
+    const double eb = P.ev[b];
+#pragma unroll 8
+    for (int c = c0; c < TM; c += NTHR / 64) {
+      const int a = a0 + c;
+      if (a >= nv) break;
+      double g1, g2;
+      if (same) {
+        g1 = gi[b >= a ? b + P.ld * a : a + P.ld * b];
+        g2 = g1;
+      } else {
+        g1 = gi[b + P.ld * a];
+        g2 = S[r * GE_PITCH + c];
+      }
+      const double d = eij - eb - P.ev[a];  // RIMP2.F90:403 order
+      const double q = recip_f64(d);
+      if (diag)
+        e = fma(g1 * fma(2.0, g1, -g2), q, e);
+      else
+        e = fma(2.0 * fma(g1, g1 - g2, g2 * g2), q, e);
+      if (P.tamp) {
+        const double u1 = g1 / d, u2 = g2 / d;
+        const size_t v = nv, no = P.nocc;
+        P.tamp[a + v * (i + no * (b + v * j))] = u1;
+        if (!diag) P.tamp[b + v * (i + no * (a + v * j))] = u2;
+        if (!same) {
+          P.tamp[a + v * (j + no * (b + v * i))] = u2;
+          if (!diag) P.tamp[b + v * (j + no * (a + v * i))] = u1;
+        }
+      }
+    }
+  }
+  e = warp_sum(e);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = e;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int w = 0; w < NTHR / 32; ++w) s += red[w];
+    P.part[((size_t)j * (j + 1) / 2 + i) * gridDim.y + blockIdx.y] = s;
+  }
+}
+
 // Batched form: one persistent launch drains a queue of (fragment, pair,
 // tile pair) items over every fragment of the batch.  Fragments are ordered
 // heaviest first (by NBA, the K length of each item), so the long items lead
@@ -695,7 +788,95 @@ int plain_energy_f64_scratch(const PlainEnergyArgs &a, int *pairs_scratch, doubl
   return RIMP2_OK;
 }
 
+// All pairs of a fragment through integrals in memory, where the product is
+// worth its residue form (mod_gemm.cu): blocks of occupied orbitals J >= I, G
+// of each (2 GB at most) by one product, its lower triangle where I = J.
+// *handled = false: the fused kernel is the better way, nothing was launched.
+static int g_energy(const PlainEnergyArgs &a, cudaStream_t s, bool *handled) {
+  *handled = false;
+  const int ntile = (a.nvirt + TM - 1) / TM, ntp = ntile * (ntile + 1) / 2;
+  const long long npairs = (long long)a.nocc * (a.nocc + 1) / 2, nitems = npairs * ntp;
+  if (a.pairs || nitems > 2147483647LL || ntp > 65535) return RIMP2_OK;
+  const int bo = std::min(a.nocc, mod_gemm_block(a.NBA) / a.nvirt);  // orbitals of a block
+  if (bo < 1) return RIMP2_OK;
+  // the fused kernel: 64 x 64 tile pairs on two blocks an SM; here: products of
+  // the triangle, then 16 bytes and the FP64 work of the terms per element
+  const double n = (double)a.nocc * a.nvirt;
+  const double t_fused = std::max((double)nitems, 304.0) * 4.0 * TM * TN * a.NBA / 1.0e12;
+  const double t_here = mod_gemm_time(bo * (double)a.nvirt, bo * (double)a.nvirt, a.NBA, true) *
+                            std::max(1.0, n * n / ((double)bo * a.nvirt * bo * a.nvirt)) +
+                        10e-6 + 0.5 * n * n * 20e-12;
+  if (a.NBA < MG_K_MIN || a.NBA > MG_K_MAX || t_here > 0.8 * t_fused) return RIMP2_OK;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    (void)cudaGetLastError();
+    return RIMP2_OK;  // a captured call keeps to the fused kernel (mod_gemm.cu)
+  }
+  DevBuf G, pairs, part;
+  RIMP2_TRY(pairs.alloc(sizeof(int) * 2 * (size_t)npairs, s));
+  RIMP2_TRY(part.alloc(sizeof(double) * (size_t)nitems, s));
+  const long long ld = (long long)bo * a.nvirt;
+  if (G.alloc(sizeof(double) * (size_t)ld * ld, s) != RIMP2_OK) {
+    (void)cudaGetLastError();  // no room: the fused kernel needs none
+    clear_error();
+    return RIMP2_OK;
+  }
+  if (inject_fault("launch")) {
+    set_error("injected launch failure (RIMP2_FAULT_INJECT=launch)");
+    return RIMP2_ERR_CUDA;
+  }
+  make_pairs_kernel<<<(unsigned)((npairs + 255) / 256), 256, 0, s>>>(a.nocc, pairs.as<int>());
+  count_launch(1);
+  GemmDesc g;
+  memset(&g, 0, sizeof g);
+  g.alpha = 1.0;
+  g.nb0 = g.nb1 = 1;
+  g.K = a.NBA;
+  g.sAm = g.sBn = a.NBA;
+  g.sAk = g.sBk = 1;
+  g.C = G.as<double>();
+  g.sCm = 1;
+  g.sCn = ld;
+  GEnergyArgs P;
+  P.G = G.as<double>();
+  P.ld = ld;
+  P.nvirt = a.nvirt;
+  P.nocc = a.nocc;
+  P.eo = a.eo;
+  P.ev = a.ev;
+  P.part = part.as<double>();
+  P.tamp = a.tamp;
+  const long long col = (long long)a.NBA * a.nvirt;
+  for (int j0 = 0; j0 < a.nocc; j0 += bo)
+    for (int i0 = 0; i0 <= j0; i0 += bo) {
+      const int nj = std::min(bo, a.nocc - j0), ni = std::min(bo, a.nocc - i0);
+      g.M = nj * a.nvirt;
+      g.N = ni * a.nvirt;
+      g.A = a.Ca + col * j0;
+      g.B = a.Ca + col * i0;
+      g.lower = i0 == j0;
+      RIMP2_TRY(launch_gemm_f64(g, s));
+      P.i0 = i0;
+      P.j0 = j0;
+      P.ni = ni;
+      g_energy_kernel<<<dim3((unsigned)(ni * nj), (unsigned)ntp), NTHR, 0, s>>>(P);
+      count_launch(1);
+      RIMP2_CK(cudaGetLastError());
+    }
+  pair_reduce_kernel<<<(unsigned)((npairs + 7) / 8), 256, 0, s>>>(part.as<double>(), ntp,
+                                                                 pairs.as<int>(), (int)npairs, a.nocc,
+                                                                 a.Epair);
+  total_reduce_kernel<<<1, 1024, 0, s>>>(a.Epair, a.nocc, a.Etot);
+  count_launch(2);
+  RIMP2_CK(cudaGetLastError());
+  *handled = true;
+  return RIMP2_OK;
+}
+
 int plain_energy_f64(const PlainEnergyArgs &a, cudaStream_t s) {
+  bool done = false;
+  RIMP2_TRY(g_energy(a, s, &done));
+  if (done) return RIMP2_OK;
   if (!a.tamp && !a.pairs) {
     // energies only, all pairs: the persistent form (one launch draining the
     // queue of (pair, tile pair) items, as for a batch of one fragment)

@@ -147,3 +147,58 @@ def test_subroutine_forms(api):
         mag = local(gm / np.abs(g / x), np.abs(uo), np.abs(uv))
         # the classical bound of the chain of sums, for either side
         assert (np.abs(got - ref) <= 2 * chain * U * mag).all()
+
+
+def fp64_energies(nocc, nvirt, nba, Ca, eo, ev):
+    """The DMMA kernels (the allocation-free entry point keeps to them)."""
+    import torch
+    from rimp2_gpu_gb300._lib import call
+    d = [torch.from_numpy(np.ascontiguousarray(x)).cuda() for x in (Ca.ravel(order="F"), eo, ev)]
+    E = torch.zeros(nocc * nocc, dtype=torch.float64, device="cuda")
+    T = torch.zeros(1, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    call("rimp2_energy_fp64_noalloc_dev", nvirt, nocc, nba, *(x.data_ptr() for x in d), E.data_ptr(),
+         T.data_ptr(), None)
+    torch.cuda.synchronize()
+    return E.cpu().numpy().reshape(nocc, nocc, order="F"), float(T[0])
+
+
+@pytest.mark.parametrize("nocc,nvirt,nba,spread", [
+    (1, 515, 900, 0.0),     # one pair, i = j
+    (7, 129, 700, 0.0),     # one virtual past two tiles, odd row padding
+    (16, 65, 1025, 0.0),    # two sums
+    (5, 256, 2048, 0.0),    # whole tiles
+    (64, 256, 70, 0.0),     # two blocks of occupied orbitals
+    (6, 190, 640, 2.5),     # some elements summed in FP64
+    (4, 250, 640, 7.0),     # most tiles left to FP64
+])
+def test_fp64_energies(api, nocc, nvirt, nba, spread):
+    r = np.random.Generator(np.random.Philox(key=[nocc, nvirt]))
+    Ca = r.standard_normal((nba, nvirt, nocc)) * np.exp(spread * r.standard_normal((nba, nvirt, nocc)))
+    Ca = np.asfortranarray(Ca * 0.03 / np.abs(Ca).max())
+    eo, ev = np.sort(-r.random(nocc) - 0.3), np.sort(r.random(nvirt) + 0.1)
+    Er, Tr = fp64_energies(nocc, nvirt, nba, Ca, eo, ev)
+    before = api.kernel_launch_count()
+    E, T = api.energy(nvirt, nocc, nba, Ca, eo, ev)
+    assert api.kernel_launch_count() - before > 8, "expected the residue form"
+    # both sides sum FP64 terms of g and 1/D that are a few ulp off; the terms
+    # of a pair cancel by no more than their number: sums of magnitudes over
+    # |e_ij| stay below ~10 here, the sums' rounding below sqrt(nvirt) u each
+    assert (np.abs(E - Er) <= 1e-13 * np.abs(Er)).all()
+    assert abs(T - Tr) <= 1e-13 * abs(Tr)
+
+
+@pytest.mark.parametrize("nocc,nvirt,nba", [(6, 131, 640), (9, 64, 900)])
+def test_fp64_amplitudes(api, nocc, nvirt, nba):
+    r = np.random.Generator(np.random.Philox(key=[nvirt, nba]))
+    Ca = np.asfortranarray(r.standard_normal((nba, nvirt, nocc)) * 0.03)
+    eo, ev = np.sort(-r.random(nocc) - 0.3), np.sort(r.random(nvirt) + 0.1)
+    before = api.kernel_launch_count()
+    E, T, t = api.energy(nvirt, nocc, nba, Ca, eo, ev, amplitudes=True)
+    assert api.kernel_launch_count() - before > 8, "expected the residue form"
+    g = np.tensordot(Ca, Ca, (0, 0))
+    mag = np.tensordot(np.abs(Ca), np.abs(Ca), (0, 0))
+    d = eo[None, :, None, None] + eo - ev[:, None, None, None] - ev[None, None, :, None]
+    assert (np.abs(t - g / d) <= (nba + 4) * U * np.abs(mag / d)).all()
+    e = (t * (2 * g - g.transpose(2, 1, 0, 3))).sum((0, 2))
+    assert np.abs(E - e).max() <= 1e-12 * np.abs(e).max()
