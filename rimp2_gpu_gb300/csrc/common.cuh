@@ -89,6 +89,15 @@ struct GemmDesc {
 };
 int launch_gemm_f64(const GemmDesc &g, cudaStream_t s);
 
+// Threads of a total-energy reduction over nocc^2 pair energies: about eight
+// values each.  A warp's compensated tree costs 40 FP64 operations per lane at
+// two a clock and SM, so idle warps are not free (64 values: 15.8 us with 1024
+// threads, 3 us with 32).
+inline unsigned total_threads(int nocc) {
+  const long long n = ((long long)nocc * nocc / 8 + 31) / 32 * 32;
+  return (unsigned)(n < 32 ? 32 : n > 1024 ? 1024 : n);
+}
+
 struct PlainEnergyArgs {
   const double *Ca;  // Calpha(NBA, nvirt, nocc)
   int NBA, nvirt, nocc;

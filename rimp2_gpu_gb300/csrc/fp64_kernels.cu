@@ -23,6 +23,7 @@
 #include "mod_gemm.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -46,7 +47,7 @@ __device__ __forceinline__ void dmma884(double &d0, double &d1, double a, double
 }
 
 // ---------------------------------------------------------------------------
-// Generic strided batched GEMM
+// Strided batched GEMM
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void cp_async8(double *dst, const double *src, bool valid) {
   // 8-byte global -> shared copy; an invalid element is zero-filled (no read)
@@ -56,111 +57,106 @@ __device__ __forceinline__ void cp_async8(double *dst, const double *src, bool v
                : "memory");
 }
 
-// The 16-wide K slabs are double-buffered with cp.async: the next slab is in
-// flight while the DMMA loop consumes the current one.
-__global__ void __launch_bounds__(NTHR) gemm_f64_kernel(GemmDesc g) {
-  __shared__ double As[2][TM][KP];
-  __shared__ double Bs[2][TN][KP];
+struct MapGemm {
+  RowMap A, B;  // C's rows and columns
+  double *C;
+  double alpha, beta;
+  const double *eo, *ev;
+  int denom, lower;
+};
+
+// One BM x BN tile of C per block, WM x WN of it per warp.  The 16-wide K
+// slabs are double-buffered with cp.async: the next slab is in flight while
+// the DMMA loop consumes the current one.  A DMMA tile pays for its padding at
+// 6.9 GFLOP/s an SM, so the tile follows the product's shape (dmma_form).
+template <int BM, int BN, int WM, int WN>
+__global__ void __launch_bounds__(BM / WM * (BN / WN) * 32) gemm_f64_kernel(MapGemm g) {
+  constexpr int NT = BM / WM * (BN / WN) * 32;
+  constexpr int LA = (BM * TK + NT - 1) / NT, LB = (BN * TK + NT - 1) / NT;
+  __shared__ double As[2][BM][KP];
+  __shared__ double Bs[2][BN][KP];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp & 1) * 32, wn = (warp >> 1) * 16;
+  const int wm = (warp % (BM / WM)) * WM, wn = (warp / (BM / WM)) * WN;
   const int gid = lane >> 2, tig = lane & 3;
-  const bool a_kcontig = (g.sAk == 1);
-  const bool b_kcontig = (g.sBk == 1);
-  const long long nbat = (long long)g.nb0 * g.nb1;
-
-  for (long long bz = blockIdx.z; bz < nbat; bz += gridDim.z) {
-    const int b0 = (int)(bz % g.nb0), b1 = (int)(bz / g.nb0);
-    const double *Ab = g.A + b0 * g.sAb0 + b1 * g.sAb1;
-    const double *Bb = g.B + b0 * g.sBb0 + b1 * g.sBb1;
-    double *Cb = g.C + b0 * g.sCb0 + b1 * g.sCb1;
-    for (int by = blockIdx.y; by * TN < g.N; by += gridDim.y) {
-      const int m0 = blockIdx.x * TM, n0 = by * TN;
-      if (g.lower && n0 > m0 + TM - 1) continue;  // tile strictly above the diagonal
-      double acc[4][2][2];
+  const bool a_kcontig = (g.A.sk == 1), b_kcontig = (g.B.sk == 1);
+  const int M = g.A.rows, N = g.B.rows, K = g.A.K;
+  const int m0 = blockIdx.x * BM;
+  // this thread's places of a slab of A (row, k), and where their rows start
+  long long oa[LA];
 #pragma unroll
-      for (int x = 0; x < 4; ++x)
+  for (int p = 0; p < LA; ++p) {
+    const int x = tid + p * NT, mm = a_kcontig ? x >> 4 : x % BM;
+    oa[p] = mm < BM && m0 + mm < M ? row_off(g.A, m0 + mm) : -1;
+  }
+  for (int by = blockIdx.y; by * BN < N; by += gridDim.y) {
+    const int n0 = by * BN;
+    if (g.lower && n0 > m0 + BM - 1) continue;  // tile strictly above the diagonal
+    long long ob[LB];
 #pragma unroll
-        for (int y = 0; y < 2; ++y) acc[x][y][0] = acc[x][y][1] = 0.0;
-
-      // stage A(m0:m0+64, k0:k0+16) and B(k0:k0+16, n0:n0+64) into buffer buf
-      auto load_slab = [&](int buf, int k0) {
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          int mm, kk;
-          if (a_kcontig) {
-            kk = tid & 15;
-            mm = (tid >> 4) + 16 * p;
-          } else {
-            mm = tid & 63;
-            kk = (tid >> 6) + 4 * p;
-          }
-          const int m = m0 + mm, k = k0 + kk;
-          const bool va = (m < g.M && k < g.K);
-          cp_async8(&As[buf][mm][kk], va ? Ab + (long long)m * g.sAm + (long long)k * g.sAk : Ab,
-                    va);
-          int nn, kb;
-          if (b_kcontig) {
-            kb = tid & 15;
-            nn = (tid >> 4) + 16 * p;
-          } else {
-            nn = tid & 63;
-            kb = (tid >> 6) + 4 * p;
-          }
-          const int n = n0 + nn, kq = k0 + kb;
-          const bool vb = (n < g.N && kq < g.K);
-          cp_async8(&Bs[buf][nn][kb], vb ? Bb + (long long)kq * g.sBk + (long long)n * g.sBn : Bb,
-                    vb);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-      };
-
-      if (g.K > 0) load_slab(0, 0);
-      int cur = 0;
-      for (int k0 = 0; k0 < g.K; k0 += TK, cur ^= 1) {
-        if (k0 + TK < g.K) {
-          load_slab(cur ^ 1, k0 + TK);
-          asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-          asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
-#pragma unroll
-        for (int ks = 0; ks < TK; ks += 4) {
-          double af[4], bf[2];
-#pragma unroll
-          for (int x = 0; x < 4; ++x) af[x] = As[cur][wm + 8 * x + gid][ks + tig];
-#pragma unroll
-          for (int y = 0; y < 2; ++y) bf[y] = Bs[cur][wn + 8 * y + gid][ks + tig];
-#pragma unroll
-          for (int x = 0; x < 4; ++x)
-#pragma unroll
-            for (int y = 0; y < 2; ++y) dmma884(acc[x][y][0], acc[x][y][1], af[x], bf[y]);
-        }
-        __syncthreads();  // buffer cur is refilled two slabs later
-      }
-      // epilogue
-#pragma unroll
-      for (int x = 0; x < 4; ++x)
-#pragma unroll
-        for (int y = 0; y < 2; ++y)
-#pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const int m = m0 + wm + 8 * x + gid;
-            const int n = n0 + wn + 8 * y + 2 * tig + h;
-            if (m < g.M && n < g.N) {
-              double v = acc[x][y][h];
-              if (g.denom == 1) {
-                // RIMP2.F90:403-404: deltaEPS = EVocc(I)+EVocc(J)-EVvirt(B)-EVvirt(A)
-                const double d = g.eo[b0] + g.eo[b1] - g.ev[n] - g.ev[m];
-                v = v / d;
-              }
-              double *cp = Cb + m * g.sCm + n * g.sCn;
-              v = g.alpha * v;
-              if (g.beta != 0.0) v += g.beta * *cp;
-              *cp = v;
-            }
-          }
+    for (int p = 0; p < LB; ++p) {
+      const int x = tid + p * NT, nn = b_kcontig ? x >> 4 : x % BN;
+      ob[p] = nn < BN && n0 + nn < N ? row_off(g.B, n0 + nn) : -1;
     }
+    double acc[WM / 8][WN / 8][2];
+#pragma unroll
+    for (int x = 0; x < WM / 8; ++x)
+#pragma unroll
+      for (int y = 0; y < WN / 8; ++y) acc[x][y][0] = acc[x][y][1] = 0.0;
+
+    // stage A(m0:m0+BM, k0:k0+16) and B(k0:k0+16, n0:n0+BN) into buffer buf
+    auto load_slab = [&](int buf, int k0) {
+#pragma unroll
+      for (int p = 0; p < LA; ++p) {
+        const int x = tid + p * NT, mm = a_kcontig ? x >> 4 : x % BM, kk = a_kcontig ? x & 15 : x / BM;
+        if (x >= BM * TK) break;
+        const bool v = oa[p] >= 0 && k0 + kk < K;
+        cp_async8(&As[buf][mm][kk], v ? g.A.base + oa[p] + (long long)(k0 + kk) * g.A.sk : g.A.base, v);
+      }
+#pragma unroll
+      for (int p = 0; p < LB; ++p) {
+        const int x = tid + p * NT, nn = b_kcontig ? x >> 4 : x % BN, kk = b_kcontig ? x & 15 : x / BN;
+        if (x >= BN * TK) break;
+        const bool v = ob[p] >= 0 && k0 + kk < K;
+        cp_async8(&Bs[buf][nn][kk], v ? g.B.base + ob[p] + (long long)(k0 + kk) * g.B.sk : g.B.base, v);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    if (K > 0) load_slab(0, 0);
+    int cur = 0;
+    for (int k0 = 0; k0 < K; k0 += TK, cur ^= 1) {
+      if (k0 + TK < K) {
+        load_slab(cur ^ 1, k0 + TK);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      } else {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+      }
+      __syncthreads();
+#pragma unroll
+      for (int ks = 0; ks < TK; ks += 4) {
+        if (k0 + ks >= K) break;  // zeros from here on
+        double af[WM / 8], bf[WN / 8];
+#pragma unroll
+        for (int x = 0; x < WM / 8; ++x) af[x] = As[cur][wm + 8 * x + gid][ks + tig];
+#pragma unroll
+        for (int y = 0; y < WN / 8; ++y) bf[y] = Bs[cur][wn + 8 * y + gid][ks + tig];
+#pragma unroll
+        for (int x = 0; x < WM / 8; ++x)
+#pragma unroll
+          for (int y = 0; y < WN / 8; ++y) dmma884(acc[x][y][0], acc[x][y][1], af[x], bf[y]);
+      }
+      __syncthreads();  // buffer cur is refilled two slabs later
+    }
+#pragma unroll
+    for (int x = 0; x < WM / 8; ++x)
+#pragma unroll
+      for (int y = 0; y < WN / 8; ++y)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int m = m0 + wm + 8 * x + gid;
+          const int n = n0 + wn + 8 * y + 2 * tig + h;
+          if (m < M && n < N) put_c(g, m, n, acc[x][y][h]);
+        }
   }
 }
 
@@ -403,7 +399,7 @@ __global__ void __launch_bounds__(NTHR, 2) eos_energy_kernel(const double *__res
 // Pair energies from integrals in memory: G(x, y) = sum_al C(al, x) C(al, y)
 // for the columns x = (b, j) of a block of occupied orbitals and y = (a, i) of
 // another (the same or an earlier one: then only x >= y is read).  A block
-// takes the 64 x 64 tile pair (A, B) of a pair i <= j: rows (b,j), columns
+// takes the T x T tile pair (A, B) of a pair i <= j: rows (b,j), columns
 // (a,i) hold g_ij(a,b); rows (a,j), columns (b,i) hold g_ij(b,a) and pass
 // through shared memory, so that both are read along the fast direction.  Off
 // the diagonal tile the two orders share a denominator:
@@ -427,24 +423,24 @@ __device__ __forceinline__ double recip_f64(double d) {
   return fma(r0, fma(e, e, e), r0);
 }
 
-constexpr int GE_PITCH = 65;
-
+// T: the tile's edge, 32 where 64 would leave SMs without a block.
+template <int T>
 __global__ void __launch_bounds__(NTHR) g_energy_kernel(GEnergyArgs P) {
-  __shared__ double S[TN * GE_PITCH];  // g_ij(b,a) at [b][a]
+  __shared__ double S[T * (T + 1)];  // g_ij(b,a) at [b][a]
   __shared__ double red[NTHR / 32];
   const int i = P.i0 + (int)(blockIdx.x % P.ni), j = P.j0 + (int)(blockIdx.x / P.ni);
   if (i > j) return;
   int tA, tB;
   decode_tri((int)blockIdx.y, tA, tB);
   const bool same = (i == j), diag = (tA == tB);
-  const int a0 = tA * TM, b0 = tB * TN, nv = P.nvirt;
-  const int r = threadIdx.x & 63, c0 = threadIdx.x >> 6;  // row, first column of a tile
+  const int a0 = tA * T, b0 = tB * T, nv = P.nvirt;
+  const int r = threadIdx.x % T, c0 = threadIdx.x / T;  // row, first column of a tile
   const double *gj = P.G + (long long)(j - P.j0) * nv;            // rows (., j)
   const double *gi = gj + P.ld * (long long)(i - P.i0) * nv;      // columns (., i)
   if (!same) {
 #pragma unroll 8
-    for (int c = c0; c < TN; c += NTHR / 64)
-      if (a0 + r < nv && b0 + c < nv) S[c * GE_PITCH + r] = gi[(a0 + r) + P.ld * (b0 + c)];
+    for (int c = c0; c < T; c += NTHR / T)
+      if (a0 + r < nv && b0 + c < nv) S[c * (T + 1) + r] = gi[(a0 + r) + P.ld * (b0 + c)];
     __syncthreads();
   }
   const double eij = P.eo[i] + P.eo[j];
@@ -453,7 +449,7 @@ __global__ void __launch_bounds__(NTHR) g_energy_kernel(GEnergyArgs P) {
   if (b < nv) {
     const double eb = P.ev[b];
 #pragma unroll 8
-    for (int c = c0; c < TM; c += NTHR / 64) {
+    for (int c = c0; c < T; c += NTHR / T) {
       const int a = a0 + c;
       if (a >= nv) break;
       double g1, g2;
@@ -462,7 +458,7 @@ __global__ void __launch_bounds__(NTHR) g_energy_kernel(GEnergyArgs P) {
         g2 = g1;
       } else {
         g1 = gi[b + P.ld * a];
-        g2 = S[r * GE_PITCH + c];
+        g2 = S[r * (T + 1) + c];
       }
       const double d = eij - eb - P.ev[a];  // RIMP2.F90:403 order
       const double q = recip_f64(d);
@@ -719,29 +715,105 @@ int probe_fp64_peak(double *tflops, cudaStream_t s) {
   return RIMP2_OK;
 }
 
+// Time of a product on BM x BN DMMA tiles: 1.05 TFLOP/s over all SMs, 6.9
+// GFLOP/s on the one with the most tiles (64 x 64 x 16 takes 19 us).
+static double dmma_time(double m, double n, double k, int bm, int bn, bool lower, int nsm) {
+  const double tiles = std::ceil(m / bm) * std::ceil(n / bn) * (lower ? 0.5 : 1.0) + (lower ? std::ceil(m / bm) * 0.5 : 0.0);
+  return 5e-6 + std::ceil(tiles / nsm) * bm * bn * 2.0 * std::ceil(k / 4) * 4 / 6.9e9;
+}
+
+constexpr int DMMA_FORMS = 4;
+constexpr int DMMA_BM[DMMA_FORMS] = {64, 32, 16, 128}, DMMA_BN[DMMA_FORMS] = {64, 32, 16, 8};
+
+// The tile that loses least to padding and to idle SMs, and its time; the
+// larger one (fewer blocks, fewer reads) where they are within a fifteenth.
+static int dmma_form(double m, double n, double k, bool lower, int nsm, double *time) {
+  int best = 0;
+  *time = 1e30;
+  for (int v = 0; v < DMMA_FORMS; ++v) {
+    const double x = dmma_time(m, n, k, DMMA_BM[v], DMMA_BN[v], lower, nsm);
+    if (x < 0.93 * *time) {
+      *time = x;
+      best = v;
+    }
+  }
+  return best;
+}
+
+static double gemm_time(double m, double n, double k, bool lower, int nsm) {
+  double t;
+  dmma_form(m, n, k, lower, nsm, &t);
+  return k < MG_K_MIN || k > MG_K_MAX ? t : std::min(t, mod_gemm_time(m, n, k, lower));
+}
+
+template <int BM, int BN, int WM, int WN>
+static int launch_dmma(const MapGemm &P, cudaStream_t s) {
+  const long long mt = ((long long)P.A.rows + BM - 1) / BM, nt = ((long long)P.B.rows + BN - 1) / BN;
+  gemm_f64_kernel<BM, BN, WM, WN>
+      <<<dim3((unsigned)mt, (unsigned)std::min<long long>(nt, 65535)), BM / WM * (BN / WN) * 32, 0, s>>>(P);
+  count_launch(1);
+  RIMP2_CK(cudaGetLastError());
+  return RIMP2_OK;
+}
+
+static int launch_folded(const GemmDesc &g, RowMap A, RowMap B, cudaStream_t s) {
+  int dev = 0, nsm = 0;
+  RIMP2_CK(cudaGetDevice(&dev));
+  RIMP2_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  // a product with few columns has all of them in a tile, one with few rows is
+  // transposed
+  const bool thin_rows = !g.lower && !g.denom && A.rows < B.rows && A.rows <= 16;
+  const double m = thin_rows ? B.rows : A.rows, n = thin_rows ? A.rows : B.rows;
+  double t;
+  const int form = dmma_form(m, n, g.K, g.lower != 0, nsm, &t);
+  // large ones go to the FP16 tensor cores as residues
+  if (mod_gemm_time(A.rows, B.rows, g.K, g.lower != 0) < 0.9 * t) {
+    bool done = false;
+    RIMP2_TRY(mod_gemm(g, A, B, s, &done));
+    if (done) return RIMP2_OK;
+  }
+  MapGemm P;
+  P.A = thin_rows ? B : A;
+  P.B = thin_rows ? A : B;
+  P.C = g.C;
+  P.alpha = g.alpha;
+  P.beta = g.beta;
+  P.eo = g.eo;
+  P.ev = g.ev;
+  P.denom = g.denom;
+  P.lower = g.lower;
+  if (form == 1) return launch_dmma<32, 32, 16, 16>(P, s);
+  if (form == 2) return launch_dmma<16, 16, 16, 16>(P, s);
+  if (form == 3) return launch_dmma<128, 8, 32, 8>(P, s);
+  return launch_dmma<64, 64, 32, 16>(P, s);
+}
+
 int launch_gemm_f64(const GemmDesc &g, cudaStream_t s) {
   if (g.M <= 0 || g.N <= 0 || g.nb0 <= 0 || g.nb1 <= 0) return RIMP2_OK;
   if (inject_fault("launch")) {
     set_error("injected launch failure (RIMP2_FAULT_INJECT=launch)");
     return RIMP2_ERR_CUDA;
   }
-  // large products go to the FP16 tensor cores as residues
-  bool done = false;
-  RIMP2_TRY(mod_gemm(g, s, &done));
-  if (done) return RIMP2_OK;
-  long long mt = (g.M + TM - 1) / TM, nt = (g.N + TN - 1) / TN;
-  long long nb = (long long)g.nb0 * g.nb1;
-  if (mt > 2147483647LL) {
+  RowMap A, B;
+  if (fold_gemm(g, A, B)) return launch_folded(g, A, B, s);
+  // a batch index that moves both operands, or too many rows for one product
+  if (g.nb0 == 1 && g.nb1 == 1) {
     set_error("gemm M too large");
     return RIMP2_ERR_ARG;
   }
-  dim3 grid((unsigned)mt, (unsigned)(nt < 65535 ? nt : 65535), (unsigned)(nb < 65535 ? nb : 65535));
-  if (g.K <= 0) {
-    // C = beta*C (alpha*0): still run the kernel (it handles K=0 as zero sum)
+  if (g.denom) {
+    set_error("gemm: denominators need independent batch indices");
+    return RIMP2_ERR_UNSUPPORTED;
   }
-  gemm_f64_kernel<<<grid, NTHR, 0, s>>>(g);
-  count_launch(1);
-  RIMP2_CK(cudaGetLastError());
+  GemmDesc h = g;
+  const bool outer = g.nb1 > 1;
+  (outer ? h.nb1 : h.nb0) = 1;
+  for (int b = 0; b < (outer ? g.nb1 : g.nb0); ++b) {
+    RIMP2_TRY(launch_gemm_f64(h, s));
+    h.A += outer ? g.sAb1 : g.sAb0;
+    h.B += outer ? g.sBb1 : g.sBb0;
+    h.C += outer ? g.sCb1 : g.sCb0;
+  }
   return RIMP2_OK;
 }
 
@@ -782,31 +854,40 @@ int plain_energy_f64_scratch(const PlainEnergyArgs &a, int *pairs_scratch, doubl
                                                         a.tamp);
   pair_reduce_kernel<<<(npairs + 7) / 8, 256, 0, s>>>(part_scratch, ntp, pairs_scratch, npairs,
                                                      a.nocc, a.Epair);
-  total_reduce_kernel<<<1, 1024, 0, s>>>(a.Epair, a.nocc, a.Etot);
+  total_reduce_kernel<<<1, total_threads(a.nocc), 0, s>>>(a.Epair, a.nocc, a.Etot);
   count_launch(4);
   RIMP2_CK(cudaGetLastError());
   return RIMP2_OK;
 }
 
-// All pairs of a fragment through integrals in memory, where the product is
-// worth its residue form (mod_gemm.cu): blocks of occupied orbitals J >= I, G
+// All pairs of a fragment through integrals in memory, where that is faster
+// (the product as residues, mod_gemm.cu, or on tiles that fill the SMs): blocks of occupied orbitals J >= I, G
 // of each (2 GB at most) by one product, its lower triangle where I = J.
 // *handled = false: the fused kernel is the better way, nothing was launched.
 static int g_energy(const PlainEnergyArgs &a, cudaStream_t s, bool *handled) {
   *handled = false;
-  const int ntile = (a.nvirt + TM - 1) / TM, ntp = ntile * (ntile + 1) / 2;
-  const long long npairs = (long long)a.nocc * (a.nocc + 1) / 2, nitems = npairs * ntp;
-  if (a.pairs || nitems > 2147483647LL || ntp > 65535) return RIMP2_OK;
+  int dev = 0, nsm = 0;
+  RIMP2_CK(cudaGetDevice(&dev));
+  RIMP2_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const long long npairs = (long long)a.nocc * (a.nocc + 1) / 2;
+  auto tile_pairs = [&](int T) {
+    const long long n = (a.nvirt + T - 1) / T;
+    return n * (n + 1) / 2;
+  };
+  const bool wide = npairs * tile_pairs(64) >= 2 * nsm;
+  const long long ntp = tile_pairs(wide ? 64 : 32), nitems = npairs * ntp;
+  if (a.pairs || nitems > 2147483647LL || ntp > 65535 || a.NBA < 1) return RIMP2_OK;
   const int bo = std::min(a.nocc, mod_gemm_block(a.NBA) / a.nvirt);  // orbitals of a block
   if (bo < 1) return RIMP2_OK;
-  // the fused kernel: 64 x 64 tile pairs on two blocks an SM; here: products of
-  // the triangle, then 16 bytes and the FP64 work of the terms per element
-  const double n = (double)a.nocc * a.nvirt;
-  const double t_fused = std::max((double)nitems, 304.0) * 4.0 * TM * TN * a.NBA / 1.0e12;
-  const double t_here = mod_gemm_time(bo * (double)a.nvirt, bo * (double)a.nvirt, a.NBA, true) *
-                            std::max(1.0, n * n / ((double)bo * a.nvirt * bo * a.nvirt)) +
-                        10e-6 + 0.5 * n * n * 20e-12;
-  if (a.NBA < MG_K_MIN || a.NBA > MG_K_MAX || t_here > 0.8 * t_fused) return RIMP2_OK;
+  // the fused kernel: 64 x 64 tile pairs, 6.9 GFLOP/s of DMMA an SM; here: the
+  // products of the triangle, then the terms (16 bytes and ten FP64 operations
+  // per pair of elements)
+  const double n = (double)a.nocc * a.nvirt, nb = (double)bo * a.nvirt;
+  const double items = (double)npairs * tile_pairs(64);
+  const double t_fused = 10e-6 + std::max(items / nsm, std::ceil(items / nsm)) * 4.0 * TM * TN * a.NBA / 6.9e9;
+  const double t_here = gemm_time(nb, nb, a.NBA, true, nsm) * std::max(1.0, n * n / (nb * nb)) + 20e-6 +
+                        std::max(0.5 * n * n * 20e-12, wide ? 11e-6 : 3e-6);
+  if (t_here > 0.8 * t_fused) return RIMP2_OK;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
     (void)cudaGetLastError();
@@ -859,14 +940,18 @@ static int g_energy(const PlainEnergyArgs &a, cudaStream_t s, bool *handled) {
       P.i0 = i0;
       P.j0 = j0;
       P.ni = ni;
-      g_energy_kernel<<<dim3((unsigned)(ni * nj), (unsigned)ntp), NTHR, 0, s>>>(P);
+      const dim3 grid((unsigned)(ni * nj), (unsigned)ntp);
+      if (wide)
+        g_energy_kernel<64><<<grid, NTHR, 0, s>>>(P);
+      else
+        g_energy_kernel<32><<<grid, NTHR, 0, s>>>(P);
       count_launch(1);
       RIMP2_CK(cudaGetLastError());
     }
-  pair_reduce_kernel<<<(unsigned)((npairs + 7) / 8), 256, 0, s>>>(part.as<double>(), ntp,
+  pair_reduce_kernel<<<(unsigned)((npairs + 7) / 8), 256, 0, s>>>(part.as<double>(), (int)ntp,
                                                                  pairs.as<int>(), (int)npairs, a.nocc,
                                                                  a.Epair);
-  total_reduce_kernel<<<1, 1024, 0, s>>>(a.Epair, a.nocc, a.Etot);
+  total_reduce_kernel<<<1, total_threads(a.nocc), 0, s>>>(a.Epair, a.nocc, a.Etot);
   count_launch(2);
   RIMP2_CK(cudaGetLastError());
   *handled = true;
@@ -927,7 +1012,7 @@ int plain_energy_f64(const PlainEnergyArgs &a, cudaStream_t s) {
                                                      a.Epair);
   count_launch(1);
   RIMP2_CK(cudaGetLastError());
-  total_reduce_kernel<<<1, 1024, 0, s>>>(a.Epair, a.nocc, a.Etot);
+  total_reduce_kernel<<<1, total_threads(a.nocc), 0, s>>>(a.Epair, a.nocc, a.Etot);
   count_launch(1);
   RIMP2_CK(cudaGetLastError());
   return RIMP2_OK;
@@ -964,7 +1049,7 @@ int eos_energy_f64(const double *Ca, const double *Ct, int NBA, int nvirt, int n
                                                               part.as<double>());
   pair_reduce_kernel<<<(npairs + 7) / 8, 256, 0, s>>>(part.as<double>(), ntp, pairs.as<int>(),
                                                      npairs, nocc, Epair);
-  total_reduce_kernel<<<1, 1024, 0, s>>>(Epair, nocc, Etot);
+  total_reduce_kernel<<<1, total_threads(nocc), 0, s>>>(Epair, nocc, Etot);
   count_launch(4);
   RIMP2_CK(cudaGetLastError());
   return RIMP2_OK;
@@ -972,7 +1057,7 @@ int eos_energy_f64(const double *Ca, const double *Ct, int NBA, int nvirt, int n
 
 // A planned plain FP64 batch: fragment table, per-item partials, queue.
 struct PlainPlan {
-  int nfrag = 0, npairs_total = 0, grid = 0;
+  int nfrag = 0, npairs_total = 0, grid = 0, nocc_max = 0;
   long long nitems = 0;
   std::vector<PlainFrag> fh;  // host copy of the descriptor table
   DevBuf frags, part, queue;
@@ -1002,6 +1087,7 @@ int plain_plan_create(PlainPlan **out, int nfrag, const PlainFrag *in, cudaStrea
   PlainPlan *P = new PlainPlan();
   P->nfrag = nfrag;
   P->npairs_total = pb;
+  for (const auto &F : fh) P->nocc_max = std::max(P->nocc_max, F.nocc);
   P->nitems = item;
   int dev = 0, nsm = 0, occ = 0;
   cudaGetDevice(&dev);
@@ -1041,7 +1127,7 @@ int plain_plan_record(PlainPlan *P, cudaStream_t s) {
                                               P->part.as<double>());
   pair_reduce_plain_batch_kernel<<<(unsigned)((P->npairs_total + 7) / 8), 256, 0, s>>>(
       fr, P->nfrag, P->npairs_total, P->part.as<double>());
-  total_reduce_plain_batch_kernel<<<P->nfrag, 1024, 0, s>>>(fr);
+  total_reduce_plain_batch_kernel<<<P->nfrag, total_threads(P->nocc_max), 0, s>>>(fr);
   count_launch(3);
   RIMP2_CK(cudaGetLastError());
   return RIMP2_OK;

@@ -114,12 +114,6 @@ constexpr float MAGIC = 12582912.0f;  // 1.5 * 2^23: adds round to an integer
 // --------------------------------------------------------------------------
 // operands
 // --------------------------------------------------------------------------
-__device__ __forceinline__ long long row_off(const RowMap &M, int r) {
-  const int d0 = r % M.ext[0], q = r / M.ext[0];
-  const int d1 = q % M.ext[1], d2 = q / M.ext[1];
-  return d0 * M.st[0] + d1 * M.st[1] + d2 * M.st[2];
-}
-
 // Norm of a row in pieces: largest exponent, sum of squares relative to it
 // (FP32: its rounding, below 2^-10, is inside the margin of the scale), the
 // lowest set bit, and whether a value is infinite or NaN.
@@ -181,56 +175,71 @@ __device__ __forceinline__ void stat_store(const RowStat &s, int *e, unsigned ch
   *flag = s.lsb + ee >= 0 ? MG_ROW_EXACT : 0;
 }
 
-// K-contiguous rows: one warp per row, four loads in flight per lane.
-__global__ void __launch_bounds__(256) row_scale_k_kernel(RowMap M, int row0, int nrows, int *e,
-                                                          unsigned char *flag) {
-  const int r = (int)((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (r >= nrows) return;
-  const double *x = M.base + row_off(M, row0 + r);
-  RowStat s{0, 0.0f, MG_NO_LSB, 0};
-  for (int k0 = lane; k0 < M.K; k0 += 128) {
-    double v[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) v[u] = k0 + 32 * u < M.K ? x[k0 + 32 * u] : 0.0;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) stat_add(s, v[u]);
-  }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const int e2 = __shfl_xor_sync(0xffffffffu, s.e, o);
-    const float s2 = __shfl_xor_sync(0xffffffffu, s.ss, o);
-    const int l2 = __shfl_xor_sync(0xffffffffu, s.lsb, o);
-    const int b2 = __shfl_xor_sync(0xffffffffu, s.bad, o);
-    stat_merge(s, e2, s2, l2, b2);
-  }
-  if (lane == 0) stat_store(s, e + r, flag + r);
-}
+// One operand's work of the two kernels below.
+struct OpArgs {
+  RowMap M;
+  int row0, rows, nkc;
+  int blocks;            // of the kernel's grid
+  int *e;
+  unsigned char *flag;
+  __half *out;
+  size_t plane;
+};
 
-// Rows along the fast direction: a block takes 32 rows, each warp a part of K.
-__global__ void __launch_bounds__(512) row_scale_r_kernel(RowMap M, int row0, int nrows, int *e,
-                                                          unsigned char *flag) {
-  __shared__ RowStat sh[16][32];
+// K-contiguous rows: one warp per row, four loads in flight per lane.  Rows
+// along the fast direction: a block takes 32 rows, each warp a part of K.
+// Both operands of a product in one launch (short ones are launch-bound).
+__global__ void __launch_bounds__(256) row_scale_kernel(const __grid_constant__ OpArgs A,
+                                                        const __grid_constant__ OpArgs B, unsigned *list) {
+  __shared__ RowStat sh[8][32];
+  if (blockIdx.x == 0 && threadIdx.x == 0) *list = 0;  // the count of tiles left to FP64
+  const bool second = (int)blockIdx.x >= A.blocks;
+  const OpArgs &P = second ? B : A;
+  const RowMap &M = P.M;
+  const int blk = (int)blockIdx.x - (second ? A.blocks : 0);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int r = blockIdx.x * 32 + lane;
   RowStat s{0, 0.0f, MG_NO_LSB, 0};
-  if (r < nrows) {
-    const double *x = M.base + row_off(M, row0 + r);
-    for (int k0 = w; k0 < M.K; k0 += 64) {
+  if (M.sk == 1) {
+    const int r = blk * 8 + w;
+    if (r >= P.rows) return;
+    const double *x = M.base + row_off(M, P.row0 + r);
+    for (int k0 = lane; k0 < M.K; k0 += 128) {
       double v[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) v[u] = k0 + 16 * u < M.K ? x[(long long)(k0 + 16 * u) * M.sk] : 0.0;
+      for (int u = 0; u < 4; ++u) v[u] = k0 + 32 * u < M.K ? x[k0 + 32 * u] : 0.0;
 #pragma unroll
       for (int u = 0; u < 4; ++u) stat_add(s, v[u]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const int e2 = __shfl_xor_sync(0xffffffffu, s.e, o);
+      const float s2 = __shfl_xor_sync(0xffffffffu, s.ss, o);
+      const int l2 = __shfl_xor_sync(0xffffffffu, s.lsb, o);
+      const int b2 = __shfl_xor_sync(0xffffffffu, s.bad, o);
+      stat_merge(s, e2, s2, l2, b2);
+    }
+    if (lane == 0) stat_store(s, P.e + r, P.flag + r);
+    return;
+  }
+  const int r = blk * 32 + lane;
+  if (r < P.rows) {
+    const double *x = M.base + row_off(M, P.row0 + r);
+    for (int k0 = w; k0 < M.K; k0 += 64) {
+      double v[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = k0 + 8 * u < M.K ? x[(long long)(k0 + 8 * u) * M.sk] : 0.0;
+#pragma unroll
+      for (int u = 0; u < 8; ++u) stat_add(s, v[u]);
     }
   }
   sh[w][lane] = s;
   __syncthreads();
-  if (w == 0 && r < nrows) {
-    for (int q = 1; q < 16; ++q) {
+  if (w == 0 && r < P.rows) {
+    for (int q = 1; q < 8; ++q) {
       const RowStat &t = sh[q][lane];
       stat_merge(s, t.e, t.ss, t.lsb, t.bad);
     }
-    stat_store(s, e + r, flag + r);
+    stat_store(s, P.e + r, P.flag + r);
   }
 }
 
@@ -294,55 +303,51 @@ __device__ __forceinline__ void residues8(const double (&v)[8], int e, bool live
   }
 }
 
-// out[(p * nkc + kc) * R + row][64]
-template <bool COL>
-__global__ void __launch_bounds__(256) residue_k_kernel(RowMap M, int row0, int R, int nkc,
-                                                        const int *__restrict__ e,
-                                                        const unsigned char *__restrict__ flag,
-                                                        __half *__restrict__ out, size_t plane) {
-  const long long g = blockIdx.x * 32ll + (threadIdx.x >> 3);  // (kc, row)
-  if (g >= (long long)nkc * R) return;
-  const int kc = (int)(g / R), r = (int)(g % R), k0 = kc * 64 + (threadIdx.x & 7) * 8;
-  const double *x = M.base + row_off(M, row0 + r);
+// out[(p * nkc + kc) * rows + row][64]; a block takes 32 rows of one K chunk.
+// A: the rows' operand, B: the columns'.
+__global__ void __launch_bounds__(256) residue_kernel(const __grid_constant__ OpArgs A,
+                                                      const __grid_constant__ OpArgs B) {
+  __shared__ double sh[64][33];
+  const bool second = (int)blockIdx.x >= A.blocks;
+  const OpArgs &P = second ? B : A;
+  const RowMap &M = P.M;
+  const int blk = (int)blockIdx.x - (second ? A.blocks : 0);
+  const int nrb = (P.rows + 31) / 32, kc = blk / nrb, rb = blk % nrb;
+  const int rr = threadIdx.x >> 3, kq = threadIdx.x & 7, r = rb * 32 + rr, k0 = kc * 64 + kq * 8;
   double v[8];
-  if ((((uintptr_t)x) & 15) == 0 && k0 + 8 <= M.K) {
+  if (M.sk == 1) {
+    if (r >= P.rows) return;
+    const double *x = M.base + row_off(M, P.row0 + r);
+    if ((((uintptr_t)x) & 15) == 0 && k0 + 8 <= M.K) {
 #pragma unroll
-    for (int u = 0; u < 8; u += 2) {
-      const double2 d = *reinterpret_cast<const double2 *>(x + k0 + u);
-      v[u] = d.x;
-      v[u + 1] = d.y;
+      for (int u = 0; u < 8; u += 2) {
+        const double2 d = *reinterpret_cast<const double2 *>(x + k0 + u);
+        v[u] = d.x;
+        v[u + 1] = d.y;
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) v[u] = k0 + u < M.K ? x[k0 + u] : 0.0;
     }
   } else {
-#pragma unroll
-    for (int u = 0; u < 8; ++u) v[u] = k0 + u < M.K ? x[k0 + u] : 0.0;
-  }
-  residues8<COL>(v, e[r], !(flag[r] & MG_ROW_FP64), out + g * 64 + (threadIdx.x & 7) * 8, plane);
-}
-
-template <bool COL>
-__global__ void __launch_bounds__(256) residue_r_kernel(RowMap M, int row0, int R, int nkc,
-                                                        const int *__restrict__ e,
-                                                        const unsigned char *__restrict__ flag,
-                                                        __half *__restrict__ out, size_t plane) {
-  __shared__ double sh[64][33];
-  const int nrb = (R + 31) / 32;
-  const int kc = blockIdx.x / nrb, rb = blockIdx.x % nrb;
-  {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, r = rb * 32 + lane;
-    const double *x = M.base + (r < R ? row_off(M, row0 + r) : 0);
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, rl = rb * 32 + lane;
+    const double *x = M.base + (rl < P.rows ? row_off(M, P.row0 + rl) : 0);
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const int k = kc * 64 + w + 8 * u;
-      sh[w + 8 * u][lane] = r < R && k < M.K ? x[(long long)k * M.sk] : 0.0;
+      sh[w + 8 * u][lane] = rl < P.rows && k < M.K ? x[(long long)k * M.sk] : 0.0;
     }
-  }
-  __syncthreads();
-  const int rr = threadIdx.x >> 3, kq = threadIdx.x & 7, r = rb * 32 + rr;
-  if (r >= R) return;
-  double v[8];
+    __syncthreads();
+    if (r >= P.rows) return;
 #pragma unroll
-  for (int u = 0; u < 8; ++u) v[u] = sh[kq * 8 + u][rr];
-  residues8<COL>(v, e[r], !(flag[r] & MG_ROW_FP64), out + ((size_t)kc * R + r) * 64 + kq * 8, plane);
+    for (int u = 0; u < 8; ++u) v[u] = sh[kq * 8 + u][rr];
+  }
+  const bool live = !(P.flag[r] & MG_ROW_FP64);
+  __half *out = P.out + ((size_t)kc * P.rows + r) * 64 + kq * 8;
+  if (second)
+    residues8<true>(v, P.e[r], live, out, P.plane);
+  else
+    residues8<false>(v, P.e[r], live, out, P.plane);
 }
 
 // --------------------------------------------------------------------------
@@ -694,32 +699,6 @@ struct CrtParams {
   unsigned *list;            // [0] count, then tiles (tn * tiles_m + tm) left to FP64
 };
 
-__device__ __forceinline__ long long c_off(const RowMap &M, int r) {
-  const int d0 = r % M.ext[0], q = r / M.ext[0];
-  const int d1 = q % M.ext[1], d2 = q / M.ext[1];
-  return d0 * M.cst[0] + d1 * M.cst[1] + d2 * M.cst[2];
-}
-
-// the index along the dimension with the given role (0: m or n, 1: batch)
-__device__ __forceinline__ int role_index(const RowMap &M, int r, int role) {
-  const int d0 = r % M.ext[0], q = r / M.ext[0];
-  const int d1 = q % M.ext[1], d2 = q / M.ext[1];
-  return (M.role[0] == role ? d0 : 0) + (M.role[1] == role ? d1 : 0) + (M.role[2] == role ? d2 : 0);
-}
-
-__device__ __forceinline__ void put_c(const CrtParams &P, int m, int n, double v) {
-  if (P.denom) {
-    // RIMP2.F90:403-404: deltaEPS = EVocc(I)+EVocc(J)-EVvirt(B)-EVvirt(A)
-    const double d = P.eo[role_index(P.A, m, 1)] + P.eo[role_index(P.B, n, 1)] -
-                     P.ev[role_index(P.B, n, 0)] - P.ev[role_index(P.A, m, 0)];
-    v = v / d;
-  }
-  double *c = P.C + c_off(P.A, m) + c_off(P.B, n);
-  v = P.alpha * v;
-  if (P.beta != 0.0) v += P.beta * *c;
-  *c = v;
-}
-
 // A block takes 64 rows x 64 columns of C; a thread four consecutive rows of
 // four columns.  It reads 17 bytes and writes 8 per element.
 __global__ void __launch_bounds__(256) crt_epilogue_kernel(CrtParams P) {
@@ -929,31 +908,40 @@ int mod_operand_alloc(ModOperand &op, int rows, int K, cudaStream_t s) {
   return try_alloc(op.flag, (size_t)rows, s);
 }
 
-int mod_operand_fill(ModOperand &op, const RowMap &M, int row0, bool col, cudaStream_t s) {
-  const int R = op.rows;
-  const size_t plane = (size_t)op.nkc * R * 64;
-  int *e = op.e.as<int>();
-  unsigned char *fl = op.flag.as<unsigned char>();
-  __half *out = op.planes.as<__half>();
-  if (M.sk == 1) {
-    row_scale_k_kernel<<<(unsigned)((R + 7ll) / 8), 256, 0, s>>>(M, row0, R, e, fl);
-    const unsigned grid = (unsigned)(((long long)op.nkc * R + 31) / 32);
-    if (col)
-      residue_k_kernel<true><<<grid, 256, 0, s>>>(M, row0, R, op.nkc, e, fl, out, plane);
-    else
-      residue_k_kernel<false><<<grid, 256, 0, s>>>(M, row0, R, op.nkc, e, fl, out, plane);
-  } else {
-    const unsigned nrb = (unsigned)((R + 31ll) / 32);
-    row_scale_r_kernel<<<nrb, 512, 0, s>>>(M, row0, R, e, fl);
-    if (col)
-      residue_r_kernel<true><<<nrb * op.nkc, 256, 0, s>>>(M, row0, R, op.nkc, e, fl, out, plane);
-    else
-      residue_r_kernel<false><<<nrb * op.nkc, 256, 0, s>>>(M, row0, R, op.nkc, e, fl, out, plane);
+namespace {
+
+OpArgs op_args(ModOperand &op, const RowMap &M, int row0, bool used) {
+  OpArgs P;
+  P.M = M;
+  P.row0 = row0;
+  P.rows = op.rows;
+  P.nkc = op.nkc;
+  P.blocks = used ? (M.sk == 1 ? (op.rows + 7) / 8 : (op.rows + 31) / 32) : 0;
+  P.e = op.e.as<int>();
+  P.flag = op.flag.as<unsigned char>();
+  P.out = op.planes.as<__half>();
+  P.plane = (size_t)op.nkc * op.rows * 64;
+  return P;
+}
+
+// Residues of rows [r0, ..) of A into Q and of columns [c0, ..) of B into L;
+// either may be in place already.  Clears the list of tiles left to FP64.
+int fill_operands(ModOperand &Q, const RowMap &A, int r0, bool rows, ModOperand &L, const RowMap &B,
+                  int c0, bool cols, unsigned *list, cudaStream_t s) {
+  OpArgs a = op_args(Q, A, r0, rows), b = op_args(L, B, c0, cols);
+  row_scale_kernel<<<(unsigned)std::max(1, a.blocks + b.blocks), 256, 0, s>>>(a, b, list);
+  count_launch(1);
+  a.blocks = rows ? a.nkc * ((a.rows + 31) / 32) : 0;
+  b.blocks = cols ? b.nkc * ((b.rows + 31) / 32) : 0;
+  if (a.blocks + b.blocks > 0) {
+    residue_kernel<<<(unsigned)(a.blocks + b.blocks), 256, 0, s>>>(a, b);
+    count_launch(1);
   }
-  count_launch(2);
   RIMP2_CK(cudaGetLastError());
   return RIMP2_OK;
 }
+
+}  // namespace
 
 int mod_product(const ModOperand &L, const ModOperand &Q, signed char *out, long long ldm, bool lower,
                 cudaStream_t s) {
@@ -993,7 +981,8 @@ struct Dim {
 // operand's stride where rows lie along the fast direction of memory, else by
 // C's (the operand is read along K either way).
 bool make_map(RowMap &M, Dim *d, int nd, const double *base, long long sk, int K) {
-  std::sort(d, d + nd, [&](const Dim &x, const Dim &y) {
+  std::stable_sort(d, d + nd, [&](const Dim &x, const Dim &y) {
+    if ((x.ext == 1) != (y.ext == 1)) return y.ext == 1;  // extents of one last
     return sk == 1 ? x.cst < y.cst : x.st < y.st;
   });
   long long rows = 1;
@@ -1046,28 +1035,26 @@ constexpr size_t MG_RES_CAP = (size_t)4 << 30;    // bytes of the residues of a 
 
 }  // namespace
 
-int mod_gemm(const GemmDesc &g, cudaStream_t s, bool *handled) {
-  *handled = false;
-  if (g.K < MG_K_MIN || g.K > MG_K_MAX || g.alpha == 0.0) return RIMP2_OK;
-  // batch dimensions that move only one operand are more rows or columns
+bool fold_gemm(const GemmDesc &g, RowMap &A, RowMap &B) {
   Dim da[3] = {{g.M, g.sAm, g.sCm, 0}}, db[3] = {{g.N, g.sBn, g.sCn, 0}};
   int na = 1, nb = 1;
   const int ext[2] = {g.nb0, g.nb1};
   const long long sa[2] = {g.sAb0, g.sAb1}, sb[2] = {g.sBb0, g.sBb1}, sc[2] = {g.sCb0, g.sCb1};
   for (int k = 0; k < 2; ++k) {
-    if (g.denom ? false : ext[k] == 1) continue;
     // with denominators the first batch index is the row's i, the second the column's j
-    if (g.denom ? k == 0 : sb[k] == 0)
+    const bool row = g.denom ? k == 0 : sb[k] == 0;
+    if (ext[k] > 1 && (row ? sb[k] : sa[k]) != 0) return false;
+    if (row)
       da[na++] = {ext[k], sa[k], sc[k], 1};
-    else if (g.denom || sa[k] == 0)
-      db[nb++] = {ext[k], sb[k], sc[k], 1};
     else
-      return RIMP2_OK;
-    if (g.denom && (k == 0 ? sb[k] : sa[k]) != 0 && ext[k] > 1) return RIMP2_OK;
+      db[nb++] = {ext[k], sb[k], sc[k], 1};
   }
-  RowMap A, B;
-  if (!make_map(A, da, na, g.A, g.sAk, g.K) || !make_map(B, db, nb, g.B, g.sBk, g.K)) return RIMP2_OK;
-  if (!mod_gemm_pays(g, A.rows, B.rows)) return RIMP2_OK;
+  return make_map(A, da, na, g.A, g.sAk, g.K) && make_map(B, db, nb, g.B, g.sBk, g.K);
+}
+
+int mod_gemm(const GemmDesc &g, const RowMap &A, const RowMap &B, cudaStream_t s, bool *handled) {
+  *handled = false;
+  if (g.K < MG_K_MIN || g.K > MG_K_MAX || g.alpha == 0.0) return RIMP2_OK;
   // a captured call keeps to the FP64 kernel: the order between contractions
   // (ModOrder) cannot reach into a graph
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -1111,20 +1098,17 @@ int mod_gemm(const GemmDesc &g, cudaStream_t s, bool *handled) {
   P.fb = L.flag.as<unsigned char>();
   for (int r0 = 0; r0 < A.rows; r0 += ra) {
     Q.rows = std::min(ra, A.rows - r0);
-    RIMP2_TRY(mod_operand_fill(Q, A, r0, false, s));
     for (int c0 = 0; c0 < B.rows; c0 += rb) {
       const int nc = std::min(rb, B.rows - c0);
-      if (r0 == 0 || rb < B.rows) {
-        L.rows = nc;
-        RIMP2_TRY(mod_operand_fill(L, B, c0, true, s));
-      }
+      const bool cols = r0 == 0 || rb < B.rows;
+      if (cols) L.rows = nc;
+      RIMP2_TRY(fill_operands(Q, A, r0, c0 == 0, L, B, c0, cols, list.as<unsigned>(), s));
       P.row0 = r0;
       P.col0 = c0;
       P.nm = Q.rows;
       P.nn = nc;
       P.ldm = ((long long)Q.rows + 255) / 256 * 256;
       RIMP2_TRY(mod_product(L, Q, res.as<signed char>(), P.ldm, g.lower != 0, s));
-      RIMP2_CK(cudaMemsetAsync(list.p, 0, sizeof(unsigned), s));
       dim3 grid((unsigned)((P.nm + 63) / 64), (unsigned)((P.nn + 63) / 64));
       crt_epilogue_kernel<<<grid, 256, 0, s>>>(P);
       const long long nt = (long long)grid.x * grid.y;
@@ -1142,17 +1126,8 @@ int mod_gemm(const GemmDesc &g, cudaStream_t s, bool *handled) {
 double mod_gemm_time(double m, double n, double k, bool lower) {
   auto up = [](double x, double t) { return std::ceil(x / t) * t; };
   const double kp = up(k, 64), part = lower ? 0.55 : 1.0;
-  return 30e-6 + (m + n) * kp * 16e-12 +
+  return 20e-6 + (m + n) * kp * 10e-12 +
          part * (m * n * 16e-12 + 17.0 * 2.0 * up(m, 256) * up(n, 256) * (kp + 64) / 1.3e15);
-}
-
-// Which products go this way: estimated times of both forms (DMMA on 64 x 64
-// tiles of each product of the batch).
-bool mod_gemm_pays(const GemmDesc &g, double m, double n) {
-  auto up = [](double x, double t) { return std::ceil(x / t) * t; };
-  const double t_dmma = (g.lower ? 0.55 : 1.0) * 2.0 * up(g.M, 64) * up(g.N, 64) * g.nb0 * (double)g.nb1 *
-                        up(g.K, 16) / 1.0e12;
-  return mod_gemm_time(m, n, g.K, g.lower != 0) < 0.8 * t_dmma;
 }
 
 // Rows and columns of a square product that runs as one part.

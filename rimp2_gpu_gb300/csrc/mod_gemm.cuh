@@ -12,7 +12,7 @@ constexpr int MG_PLANES = MG_P + 1;  // and the plane of magnitudes
 constexpr float MG_TAU = 65536.0f;
 constexpr int MG_TILE_MAX = 512;     // of a 64 x 64 tile's elements; beyond it the whole tile is
 
-constexpr int MG_K_MIN = 8, MG_K_MAX = 16384;  // lengths of a sum
+constexpr int MG_K_MIN = 16, MG_K_MAX = 16384;  // lengths of a sum
 
 // a row's (or column's) flags
 constexpr unsigned MG_ROW_ZERO = 1;   // all zeros
@@ -32,6 +32,47 @@ struct RowMap {
   long long sk;
 };
 
+// The product of g as rows and columns: batch dimensions that move only one
+// operand become more rows or columns of it.  False if one moves both.
+bool fold_gemm(const GemmDesc &g, RowMap &A, RowMap &B);
+
+#ifdef __CUDACC__
+__device__ __forceinline__ long long row_off(const RowMap &M, int r) {
+  const int d0 = r % M.ext[0], q = r / M.ext[0];
+  const int d1 = q % M.ext[1], d2 = q / M.ext[1];
+  return d0 * M.st[0] + d1 * M.st[1] + d2 * M.st[2];
+}
+
+__device__ __forceinline__ long long c_off(const RowMap &M, int r) {
+  const int d0 = r % M.ext[0], q = r / M.ext[0];
+  const int d1 = q % M.ext[1], d2 = q / M.ext[1];
+  return d0 * M.cst[0] + d1 * M.cst[1] + d2 * M.cst[2];
+}
+
+// the index along the dimension with the given role (0: m or n, 1: batch)
+__device__ __forceinline__ int role_index(const RowMap &M, int r, int role) {
+  const int d0 = r % M.ext[0], q = r / M.ext[0];
+  const int d1 = q % M.ext[1], d2 = q / M.ext[1];
+  return (M.role[0] == role ? d0 : 0) + (M.role[1] == role ? d1 : 0) + (M.role[2] == role ? d2 : 0);
+}
+
+// C(m,n) = alpha v + beta C(m,n), v divided by the orbital-energy denominator
+// if the product has one; P: RowMap A, B; C, alpha, beta, denom, eo, ev
+template <class Params>
+__device__ __forceinline__ void put_c(const Params &P, int m, int n, double v) {
+  if (P.denom) {
+    // RIMP2.F90:403-404: deltaEPS = EVocc(I)+EVocc(J)-EVvirt(B)-EVvirt(A)
+    const double d = P.eo[role_index(P.A, m, 1)] + P.eo[role_index(P.B, n, 1)] -
+                     P.ev[role_index(P.B, n, 0)] - P.ev[role_index(P.A, m, 0)];
+    v = v / d;
+  }
+  double *c = P.C + c_off(P.A, m) + c_off(P.B, n);
+  v = P.alpha * v;
+  if (P.beta != 0.0) v += P.beta * *c;
+  *c = v;
+}
+#endif
+
 // Residue planes of a set of rows: [plane][K chunk of 64][row][64] FP16.
 struct ModOperand {
   DevBuf planes, e, flag;
@@ -40,16 +81,14 @@ struct ModOperand {
 
 size_t mod_operand_bytes(int rows, int K);
 int mod_operand_alloc(ModOperand &op, int rows, int K, cudaStream_t s);
-// rows [row0, row0 + op.rows) of M; col: as the columns' operand of a product
-int mod_operand_fill(ModOperand &op, const RowMap &M, int row0, bool col, cudaStream_t s);
 // out[plane][n][ldm] = residues of sum_k Q(m,k) L(n,k)
 int mod_product(const ModOperand &L, const ModOperand &Q, signed char *out, long long ldm, bool lower,
                 cudaStream_t s);
-bool mod_gemm_pays(const GemmDesc &g, double m, double n);
 double mod_gemm_time(double m, double n, double k, bool lower);  // seconds, estimated
 int mod_gemm_block(int K);
-// The contraction of g; *handled = false where FP64 tensor operations are the
-// better way (or there is no room for the workspace): nothing was launched.
-int mod_gemm(const GemmDesc &g, cudaStream_t s, bool *handled);
+// The contraction of g, folded into rows A and columns B; *handled = false
+// where it cannot be (length, capture, no room for the workspace): nothing was
+// launched.
+int mod_gemm(const GemmDesc &g, const RowMap &A, const RowMap &B, cudaStream_t s, bool *handled);
 
 }  // namespace rimp2

@@ -1873,7 +1873,7 @@ struct Group {
   int nfrag = 0;
   std::vector<FragDesc> fh;
   long long nitems = 0, R = 0, ncol_total = 0;
-  int npairs_total = 0, max_ncol = 0, max_nv = 0;
+  int npairs_total = 0, max_ncol = 0, max_nv = 0, max_nocc = 0;
   DevBuf frags, items, slices, inv, eo2, ev2, part, queue;
   CUtensorMap tm;
   // paired-CTA kernel (one residual slice): its pair items and B-half map
@@ -1945,6 +1945,7 @@ int build_group(Group &g, cudaStream_t s) {
     col += F.ncol;
     item += (long long)np * F.ntp;
     g.max_ncol = std::max(g.max_ncol, F.ncol);
+    g.max_nocc = std::max(g.max_nocc, F.nocc);
     g.max_nv = std::max(g.max_nv, std::max(F.nvpad, F.nocc));
   }
   g.nfrag = (int)g.fh.size();
@@ -2098,7 +2099,7 @@ int record_group(Group &g, cudaStream_t s, int nsm, cudaEvent_t *ev /* 3 or null
   if (ev) RIMP2_CK(cudaEventRecord(ev[2], s));
   pair_reduce_batch_kernel<<<(unsigned)((g.npairs_total + 7) / 8), 256, 0, s>>>(
       fr, g.nfrag, g.npairs_total, g.part.as<double>());
-  total_reduce_batch_kernel<<<g.nfrag, 1024, 0, s>>>(fr);
+  total_reduce_batch_kernel<<<g.nfrag, total_threads(g.max_nocc), 0, s>>>(fr);
   count_launch(2);
   RIMP2_CK(cudaGetLastError());
   return RIMP2_OK;
@@ -3503,7 +3504,7 @@ int split_energy_streamed(const double *hCa, double *dCa, const SplitEnergyArgs 
   if (rc == RIMP2_OK) {
     pair_reduce_batch_kernel<<<(unsigned)((g.npairs_total + 7) / 8), 256, 0, s>>>(
         fr, g.nfrag, g.npairs_total, g.part.as<double>());
-    total_reduce_batch_kernel<<<g.nfrag, 1024, 0, s>>>(fr);
+    total_reduce_batch_kernel<<<g.nfrag, total_threads(g.max_nocc), 0, s>>>(fr);
     count_launch(2);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -3864,7 +3865,7 @@ int split_eos_energy(const double *Ca, const double *Ct, int NBA, int nvirt, int
   RIMP2_CK(cudaMemsetAsync(Epair, 0, sizeof(double) * (size_t)nocc * nocc, s));
   pair_reduce_kernel<<<(npairs + 7) / 8, 256, 0, s>>>(part.as<double>(), 2 * ntp, pairs.as<int>(),
                                                      npairs, nocc, Epair);
-  total_reduce_kernel<<<1, 1024, 0, s>>>(Epair, nocc, Etot);
+  total_reduce_kernel<<<1, total_threads(nocc), 0, s>>>(Epair, nocc, Etot);
   count_launch(3);
   RIMP2_CK(cudaGetLastError());
   return RIMP2_OK;

@@ -43,29 +43,36 @@ def product(api, ta, tb, A, B, alpha, beta, C, pad=0):
     return api.kernel_launch_count() - before
 
 
-@pytest.mark.parametrize("ta,tb,m,n,k,alpha,beta,pad", [
-    ("N", "N", 257, 255, 1025, 1.0, 0.0, 0),    # one value past a tile, a sum and a K chunk
-    ("T", "N", 256, 512, 1024, -1.0, 1.0, 0),   # whole tiles and sums
-    ("N", "T", 511, 321, 639, 0.5, -2.0, 3),    # ragged, leading dimensions beyond the extents
-    ("T", "T", 385, 700, 2049, 1.0, 0.0, 1),    # three sums, odd leading dimensions
-    ("T", "N", 4100, 4097, 8, 1.0, 0.0, 0),     # the shortest sum
-    ("N", "N", 70000, 3, 61, 1.0, 0.0, 0),      # far fewer columns than a tile
+@pytest.mark.parametrize("residues,ta,tb,m,n,k,alpha,beta,pad", [
+    (True, "N", "N", 257, 255, 1025, 1.0, 0.0, 0),   # one value past a tile, a sum and a K chunk
+    (True, "T", "N", 256, 512, 1024, -1.0, 1.0, 0),  # whole tiles and sums
+    (True, "N", "T", 511, 321, 639, 0.5, -2.0, 3),   # ragged, leading dimensions beyond the extents
+    (True, "T", "T", 385, 700, 2049, 1.0, 0.0, 1),   # three sums, odd leading dimensions
+    (True, "T", "N", 4100, 4097, 31, 1.0, 0.0, 0),   # a short sum
+    (False, "T", "N", 4100, 4097, 8, 1.0, 0.0, 0),   # DMMA on 64 x 64 tiles
+    (False, "N", "N", 70000, 3, 61, 1.0, 0.0, 0),    # on 128 x 8 tiles
+    (False, "N", "T", 50001, 13, 29, 2.0, 1.0, 2),   # on 16 x 16 tiles, odd leading dimensions
+    (False, "T", "N", 7, 40003, 30, 1.0, 0.0, 0),    # few rows: transposed
+    (False, "N", "N", 100, 77, 45, 1.0, -1.0, 0),    # on 16 x 16 tiles
+    (False, "T", "T", 380, 384, 12, 1.0, 0.0, 0),    # on 32 x 32 tiles
+    (False, "N", "N", 33, 1, 3, 1.0, 0.0, 0),
 ])
-def test_product_forms(api, ta, tb, m, n, k, alpha, beta, pad):
+def test_product_forms(api, residues, ta, tb, m, n, k, alpha, beta, pad):
     r = np.random.Generator(np.random.Philox(key=[k, m]))
     A, B = r.standard_normal((m, k)), r.standard_normal((k, n))
     C0 = np.asfortranarray(r.standard_normal((m, n)))
     C = C0.copy(order="F")
-    assert product(api, ta, tb, A, B, alpha, beta, C, pad) > 1, "expected the residue form"
+    assert (product(api, ta, tb, A, B, alpha, beta, C, pad) > 1) == residues
     I = np.concatenate([r.integers(0, m, 300), [0, m - 1, m - 1, 0]])
     J = np.concatenate([r.integers(0, n, 300), [0, n - 1, 0, n - 1]])
     for i, j in zip(I, J):
         d = alpha * exact_dot(A[i], B[:, j])
         ref = d + beta * C0[i, j]
         # rounding to 62-bit integers: sqrt(K)/2 u sum|a||b| at most (an element
-        # under 2^-8 of the norms' product is summed in FP64); then alpha, beta
-        tol = abs(alpha) * (math.sqrt(k) / 2 + 2) * U * np.abs(A[i] * B[:, j]).sum() + \
-            3 * U * (abs(d) + abs(beta * C0[i, j]))
+        # under 2^-8 of the norms' product is summed in FP64); FP64 sums: K u
+        # sum|a||b|; then alpha, beta
+        tol = abs(alpha) * (math.sqrt(k) / 2 + 2 if residues else k) * U * \
+            np.abs(A[i] * B[:, j]).sum() + 3 * U * (abs(d) + abs(beta * C0[i, j]))
         assert abs(C[i, j] - ref) <= tol
 
 
