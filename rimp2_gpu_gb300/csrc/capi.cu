@@ -207,18 +207,15 @@ int dev_g_over_d(int nvirt, int nocc, int NBA, const double *Ca, const double *e
   return launch_gemm_f64(g, s);
 }
 
-int dev_tocca(int nvirt, int nocc, int noccEOS, int NBA, const double *Ca, const double *eo,
-              const double *ev, double *tocc, const double *U, cudaStream_t s) {
-  DevBuf X;
-  const size_t no = nocc, nv = nvirt;
-  RIMP2_TRY(dalloc(X, no * no * nv * nv, s));
-  RIMP2_TRY(dev_g_over_d(nvirt, nocc, NBA, Ca, eo, ev, X.as<double>(), s));
-  // tocc(i,jL,ab) = sum_j X(i,j,ab) U(j,jL)   (RIMP2.F90:406-412)
+// tocc(i,jL,ab) = sum_j X(i,j,ab) U(j,jL)   (RIMP2.F90:406-412)
+int dev_project_occ(int nvirt, int nocc, int noccEOS, const double *X, const double *U, double *tocc,
+                    cudaStream_t s) {
+  const size_t no = nocc;
   GemmDesc g = gd();
   g.M = nvirt * nvirt;
   g.N = noccEOS;
   g.K = nocc;
-  g.A = X.as<double>();
+  g.A = X;
   g.sAm = (long long)no * no;
   g.sAk = nocc;
   g.sAb0 = 1;
@@ -233,18 +230,24 @@ int dev_tocca(int nvirt, int nocc, int noccEOS, int NBA, const double *Ca, const
   return launch_gemm_f64(g, s);
 }
 
-int dev_tvirta(int nvirt, int nocc, int nvirtEOS, int NBA, const double *Ca, const double *eo,
-               const double *ev, double *tvirt, const double *U, cudaStream_t s) {
+int dev_tocca(int nvirt, int nocc, int noccEOS, int NBA, const double *Ca, const double *eo,
+              const double *ev, double *tocc, const double *U, cudaStream_t s) {
   DevBuf X;
-  const long long no = nocc, nv = nvirt;
-  RIMP2_TRY(dalloc(X, (size_t)(no * no * nv * nv), s));
+  const size_t no = nocc, nv = nvirt;
+  RIMP2_TRY(dalloc(X, no * no * nv * nv, s));
   RIMP2_TRY(dev_g_over_d(nvirt, nocc, NBA, Ca, eo, ev, X.as<double>(), s));
-  // tvirt(i,j,aL,b) = sum_a X(i,j,a,b) U(a,aL)   (RIMP2.F90:442-448)
+  return dev_project_occ(nvirt, nocc, noccEOS, X.as<double>(), U, tocc, s);
+}
+
+// tvirt(i,j,aL,b) = sum_a X(i,j,a,b) U(a,aL)   (RIMP2.F90:442-448)
+int dev_project_virt(int nvirt, int nocc, int nvirtEOS, const double *X, const double *U,
+                     double *tvirt, cudaStream_t s) {
+  const long long no = nocc, nv = nvirt;
   GemmDesc g = gd();
   g.M = nocc * nocc;
   g.N = nvirtEOS;
   g.K = nvirt;
-  g.A = X.as<double>();
+  g.A = X;
   g.sAm = 1;
   g.sAk = no * no;
   g.sAb0 = no * no * nv;
@@ -257,6 +260,15 @@ int dev_tvirta(int nvirt, int nocc, int nvirtEOS, int NBA, const double *Ca, con
   g.sCb0 = no * no * nvirtEOS;
   g.nb0 = nvirt;
   return launch_gemm_f64(g, s);
+}
+
+int dev_tvirta(int nvirt, int nocc, int nvirtEOS, int NBA, const double *Ca, const double *eo,
+               const double *ev, double *tvirt, const double *U, cudaStream_t s) {
+  DevBuf X;
+  const long long no = nocc, nv = nvirt;
+  RIMP2_TRY(dalloc(X, (size_t)(no * no * nv * nv), s));
+  RIMP2_TRY(dev_g_over_d(nvirt, nocc, NBA, Ca, eo, ev, X.as<double>(), s));
+  return dev_project_virt(nvirt, nocc, nvirtEOS, X.as<double>(), U, tvirt, s);
 }
 
 int dev_toccb(int nvirt, int noccEOS, const double *tocc, const double *UvirtT, double *toccEOS,
@@ -697,10 +709,21 @@ int rimp2_steps5to8(const int *nvirt_, const int *nocc_, const int *noccEOS_, co
   RIMP2_TRY(h2d(dUoT, UoccT, no * no, s));
   RIMP2_TRY(h2d(dUvE, UvirtEOST, nv * ve, s));
   const double *Ca = dC.as<double>(), *eo = deo.as<double>(), *ev = dev.as<double>();
+  DevBuf tv1;  // Step 6's first array, from the g/D that Step 5 forms
   {  // Step 5 (RIMP2.F90:71-93)
-    DevBuf t1, t2, t3, out;
+    DevBuf X, t1, t2, t3, out;
+    RIMP2_TRY(dalloc(X, no * no * nv * nv, s));
+    RIMP2_TRY(dev_g_over_d(nvirt, nocc, NBA, Ca, eo, ev, X.as<double>(), s));
     RIMP2_TRY(dalloc(t1, no * ne * nv * nv, s));
-    RIMP2_TRY(dev_tocca(nvirt, nocc, noccEOS, NBA, Ca, eo, ev, t1.as<double>(), dUoE.as<double>(), s));
+    RIMP2_TRY(dev_project_occ(nvirt, nocc, noccEOS, X.as<double>(), dUoE.as<double>(), t1.as<double>(), s));
+    if (dalloc(tv1, no * no * ve * nv, s) == RIMP2_OK) {
+      RIMP2_TRY(dev_project_virt(nvirt, nocc, nvirtEOS, X.as<double>(), dUvE.as<double>(),
+                                 tv1.as<double>(), s));
+    } else {  // no room beside g/D: Step 6 forms it again
+      (void)cudaGetLastError();
+      clear_error();
+    }
+    X.release();
     RIMP2_TRY(dalloc(t2, ne * ne * nv * nv, s));
     RIMP2_TRY(dev_dgemm('T', 'N', noccEOS, noccEOS * nvirt * nvirt, nocc, 1.0, dUoE.as<double>(),
                         nocc, t1.as<double>(), nocc, 0.0, t2.as<double>(), noccEOS, s));
@@ -714,9 +737,11 @@ int rimp2_steps5to8(const int *nvirt_, const int *nocc_, const int *noccEOS_, co
     RIMP2_CK(cudaStreamSynchronize(s));
   }
   {  // Step 6 (RIMP2.F90:99-124)
-    DevBuf t1, t2, t3, out;
-    RIMP2_TRY(dalloc(t1, no * no * ve * nv, s));
-    RIMP2_TRY(dev_tvirta(nvirt, nocc, nvirtEOS, NBA, Ca, eo, ev, t1.as<double>(), dUvE.as<double>(), s));
+    DevBuf t2, t3, out, &t1 = tv1;
+    if (!t1.p) {
+      RIMP2_TRY(dalloc(t1, no * no * ve * nv, s));
+      RIMP2_TRY(dev_tvirta(nvirt, nocc, nvirtEOS, NBA, Ca, eo, ev, t1.as<double>(), dUvE.as<double>(), s));
+    }
     RIMP2_TRY(dalloc(t2, no * no * ve * ve, s));
     RIMP2_TRY(dev_dgemm('N', 'N', nocc * nocc * nvirtEOS, nvirtEOS, nvirt, 1.0, t1.as<double>(),
                         nocc * nocc * nvirtEOS, dUvE.as<double>(), nvirt, 0.0, t2.as<double>(),

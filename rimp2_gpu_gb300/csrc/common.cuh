@@ -57,10 +57,12 @@ struct DevBuf {
   DevBuf() = default;
   DevBuf(const DevBuf &) = delete;
   DevBuf &operator=(const DevBuf &) = delete;
-  ~DevBuf() {
-    if (p) cudaFreeAsync(p, s);
-  }
+  ~DevBuf() { release(); }
   int alloc(size_t bytes, cudaStream_t st);
+  void release() {
+    if (p) cudaFreeAsync(p, s);
+    p = nullptr;
+  }
   template <class T>
   T *as() const { return static_cast<T *>(p); }
 };

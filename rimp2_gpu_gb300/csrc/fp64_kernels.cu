@@ -415,14 +415,6 @@ struct GEnergyArgs {
   double *part, *tamp;
 };
 
-__device__ __forceinline__ double recip_f64(double d) {
-  float r32;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r32) : "f"((float)d));
-  const double r0 = (double)r32;
-  const double e = fma(-d, r0, 1.0);
-  return fma(r0, fma(e, e, e), r0);
-}
-
 // T: the tile's edge, 32 where 64 would leave SMs without a block.
 template <int T>
 __global__ void __launch_bounds__(NTHR) g_energy_kernel(GEnergyArgs P) {
@@ -465,7 +457,7 @@ __global__ void __launch_bounds__(NTHR) g_energy_kernel(GEnergyArgs P) {
       if (diag)
         e = fma(g1 * fma(2.0, g1, -g2), q, e);
       else
-        e = fma(2.0 * fma(g1, g1 - g2, g2 * g2), q, e);
+        e = fma(fma(g1, g1 - g2, g2 * g2), q, e);  // doubled below
       if (P.tamp) {
         const double u1 = g1 / d, u2 = g2 / d;
         const size_t v = nv, no = P.nocc;
@@ -478,7 +470,7 @@ __global__ void __launch_bounds__(NTHR) g_energy_kernel(GEnergyArgs P) {
       }
     }
   }
-  e = warp_sum(e);
+  e = warp_sum(diag ? e : 2.0 * e);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = e;
   __syncthreads();
   if (threadIdx.x == 0) {

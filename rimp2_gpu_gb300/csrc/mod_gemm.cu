@@ -363,29 +363,42 @@ __global__ void __launch_bounds__(256) residue_kernel(const __grid_constant__ Op
 constexpr int MG_NST = 6;
 constexpr int MG_STAGE = 2 * PANEL_BYTES;
 constexpr int MG_THREADS = 320;
-constexpr int MG_SEG = 16;  // K chunks per exact sum
+constexpr int MG_SEG = 16;  // most K chunks of an exact sum
 constexpr int MG_SMEM = MG_NST * MG_STAGE + 1024 + 256;
 
 struct MgParams {
   int rows_l, rows_q;        // rows per K chunk of the two operands
   int tiles_l, tiles_q;      // 256-wide tiles
-  int nkc;
-  int lower;                 // only tiles with an element m >= n
+  int nkc, seg;              // K chunks, and of one exact sum
+  int lower;                 // square, only tiles with an element m >= n
   signed char *out;          // [plane][n][ldm]
   long long ldm;
   int *err;
 };
 
-__device__ __forceinline__ bool mg_item(const MgParams &P, long long item, int &plane, int &tl, int &tq) {
-  const int tiles = P.tiles_l * P.tiles_q;
+// Items are numbered without gaps and dealt in turn: every pair of CTAs gets
+// as many, also of a triangle's tiles.
+__host__ __device__ inline int mg_tiles(const MgParams &P) {
+  return P.lower ? P.tiles_q * (P.tiles_q + 1) / 2 : P.tiles_l * P.tiles_q;
+}
+
+__device__ __forceinline__ void mg_item(const MgParams &P, long long item, int &plane, int &tl, int &tq) {
+  const int tiles = mg_tiles(P);
   plane = (int)(item / tiles);
   const int t = (int)(item % tiles);
+  if (P.lower) {
+    int q = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
+    while ((q + 1) * (q + 2) / 2 <= t) ++q;
+    while (q * (q + 1) / 2 > t) --q;
+    tq = q;
+    tl = t - q * (q + 1) / 2;
+    return;
+  }
   // groups of eight column tiles: the tiles in flight share their operands in L2
   const int per = 8 * P.tiles_q, g = t / per, rem = t % per;
   const int gs = min(8, P.tiles_l - 8 * g);
   tl = 8 * g + rem % gs;
   tq = rem / gs;
-  return !(P.lower && tq < tl);
 }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
@@ -406,7 +419,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
   const uint32_t drain = smem_u32(&bars[2 * NST + 4]);
   const uint32_t full0_L = map_shared(full0, 0), tempty0_L = map_shared(tempty0, 0);
   const uint32_t abort_peer = map_shared(smem_u32((const void *)abort_flag), rank ^ 1u);
-  const long long nitems = (long long)MG_PLANES * P.tiles_l * P.tiles_q;
+  const long long nitems = (long long)MG_PLANES * mg_tiles(P);
   const int pair = blockIdx.x >> 1, npair = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
@@ -445,7 +458,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
       bool ok = true;
       for (long long item = pair; item < nitems && ok; item += npair) {
         int p, tl, tq;
-        if (!mg_item(P, item, p, tl, tq)) continue;
+        mg_item(P, item, p, tl, tq);
         const int rl = tl * 256 + 128 * (int)rank, rq = tq * 256 + 128 * (int)rank;
         for (int kc = 0; kc < P.nkc; ++kc) {
           if (!pair_wait(empty0 + 8 * stage, phase ^ 1, false, abort_flag, abort_peer, P.err, 21)) {
@@ -484,8 +497,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
       long long t = 0;  // sums so far
       for (long long item = pair; item < nitems && ok; item += npair) {
         int p, tl, tq;
-        if (!mg_item(P, item, p, tl, tq)) continue;
-        for (int s0 = 0; s0 < P.nkc && ok; s0 += MG_SEG, ++t) {
+        mg_item(P, item, p, tl, tq);
+        for (int s0 = 0; s0 < P.nkc && ok; s0 += P.seg, ++t) {
           const int u = (int)(t & 1);
           if (t >= 2 && !pair_wait(tempty0 + 8 * u, (uint32_t)(((t >> 1) - 1) & 1), true, abort_flag,
                                    abort_peer, P.err, 22)) {
@@ -494,7 +507,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
           }
           tc_fence_after();
           const uint32_t d = tmem + (uint32_t)(u * 256);
-          const int s1 = min(P.nkc, s0 + MG_SEG);
+          const int s1 = min(P.nkc, s0 + P.seg);
           for (int kc = s0; kc < s1; ++kc) {
             if (!pair_wait(full0 + 8 * stage, phase, false, abort_flag, abort_peer, P.err, 23)) {
               ok = false;
@@ -527,12 +540,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
     bool ok = true;
     for (long long item = pair; item < nitems && ok; item += npair) {
       int p, tl, tq;
-      if (!mg_item(P, item, p, tl, tq)) continue;
+      mg_item(P, item, p, tl, tq);
       const int n = tl * 256 + 128 * (int)rank + quad * 32 + lane;
       const bool mag = p == MG_P;
       const float pf = mag ? 1.0f : DT.p[p], inv = mag ? 1.0f : DT.inv[p];
       uint32_t pk[8][4];
-      for (int s0 = 0; s0 < P.nkc; s0 += MG_SEG, ++t) {
+      for (int s0 = 0; s0 < P.nkc; s0 += P.seg, ++t) {
         const int u = (int)(t & 1);
         ok = pair_wait(tfull0 + 8 * u, (uint32_t)((t >> 1) & 1), false, abort_flag, abort_peer, P.err, 24);
         ok = __all_sync(0xffffffffu, ok);
@@ -696,19 +709,52 @@ struct CrtParams {
   double alpha, beta;
   const double *eo, *ev;
   int denom, lower;
+  int sym;                   // rows and columns are the same vectors: C(n,m) comes with C(m,n)
   unsigned *list;            // [0] count, then tiles (tn * tiles_m + tm) left to FP64
 };
 
+// Whether an element is left to FP64: the flags of its row and column, and
+// its bit of the magnitudes' plane.
+__device__ __forceinline__ bool needs_fp64(unsigned f, unsigned fn, unsigned measured) {
+  return ((f | fn) & MG_ROW_FP64) ||
+         (!((f | fn) & MG_ROW_ZERO) && !(f & fn & MG_ROW_EXACT) && !measured);
+}
+
+// What a row or column of C brings to its elements.
+struct Side {
+  long long off;   // in C
+  double eo, ev;   // orbital energies of its indices
+};
+__device__ __forceinline__ Side side(const CrtParams &P, const RowMap &M, int r) {
+  Side s;
+  s.off = c_off(M, r);
+  s.eo = P.denom ? P.eo[role_index(M, r, 1)] : 0.0;
+  s.ev = P.denom ? P.ev[role_index(M, r, 0)] : 0.0;
+  return s;
+}
+
 // A block takes 64 rows x 64 columns of C; a thread four consecutive rows of
-// four columns.  It reads 17 bytes and writes 8 per element.
-__global__ void __launch_bounds__(256) crt_epilogue_kernel(CrtParams P) {
+// four columns.  It reads 17 bytes and writes 8 per element; about 150
+// instructions an element bound it, so what only depends on the row or the
+// column (offsets, orbital energies) is formed once.  A symmetric product (g
+// of one set of vectors with itself) has only the tiles m >= n: C(n,m) is
+// written along with C(m,n) through shared memory, with the same denominator
+// (the reference subtracts the two virtual energies in the other order there).
+__global__ void __launch_bounds__(256) crt_epilogue_kernel(const __grid_constant__ CrtParams P) {
   __shared__ int count;
+  __shared__ long long rows[64], cols[64];  // symmetric: offsets of the mirror's columns
+  extern __shared__ double S[];             // symmetric: [64][65]
   const int tm = blockIdx.x, tn = blockIdx.y;
-  if (P.lower && tm < tn) return;
+  if ((P.lower || P.sym) && tm < tn) return;
   const int mq = (threadIdx.x & 15) * 4, nq = threadIdx.x >> 4;
   const int m0 = tm * 64 + mq, n0 = tn * 64 + nq;
   const long long plane = (long long)P.nn * P.ldm;
+  const bool mirror = P.sym && tm != tn;
   if (threadIdx.x == 0) count = 0;
+  if (mirror && threadIdx.x < 64) {
+    if (tm * 64 + threadIdx.x < P.nm) rows[threadIdx.x] = c_off(P.B, tm * 64 + threadIdx.x);
+    if (tn * 64 + threadIdx.x < P.nn) cols[threadIdx.x] = c_off(P.A, tn * 64 + threadIdx.x);
+  }
   __syncthreads();
   // which elements are summed in FP64
   unsigned todo = 0;
@@ -722,12 +768,8 @@ __global__ void __launch_bounds__(256) crt_epilogue_kernel(CrtParams P) {
     const unsigned g = *reinterpret_cast<const unsigned *>(P.res + MG_P * plane + n * P.ldm + m0);
     const unsigned fn = P.fb[n];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const unsigned f = (fm >> (8 * k)) & 0xFFu;
-      const bool need = ((f | fn) & MG_ROW_FP64) ||
-                        (!((f | fn) & MG_ROW_ZERO) && !(f & fn & MG_ROW_EXACT) && !((g >> (8 * k)) & 1u));
-      if (need && m0 + k < P.nm) todo |= 1u << (4 * y + k);
-    }
+    for (int k = 0; k < 4; ++k)
+      if (m0 + k < P.nm && needs_fp64((fm >> (8 * k)) & 0xFFu, fn, (g >> (8 * k)) & 1u)) todo |= 1u << (4 * y + k);
   }
   if (todo) atomicAdd(&count, __popc(todo));
   __syncthreads();
@@ -737,8 +779,20 @@ __global__ void __launch_bounds__(256) crt_epilogue_kernel(CrtParams P) {
   }
   const int lane = threadIdx.x & 31;
   int ea[4];
+  Side sm[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) ea[k] = m0 + k < P.nm ? P.ea[m0 + k] : 0;
+  for (int k = 0; k < 4; ++k) {
+    ea[k] = m0 + k < P.nm ? P.ea[m0 + k] : 0;
+    if (m0 + k < P.nm) sm[k] = side(P, P.A, P.row0 + m0 + k);
+  }
+  auto put = [&](const Side &a, const Side &b, int k, int y, double v) {
+    if (P.denom) v = div_f64(v, a.eo + b.eo - b.ev - a.ev);  // RIMP2.F90:403-404
+    if (P.alpha != 1.0) v *= P.alpha;
+    if (mirror) S[(mq + k) * 65 + nq + 16 * y] = v;
+    double *c = P.C + a.off + b.off;
+    if (P.beta != 0.0) v += P.beta * *c;
+    *c = v;
+  };
   unsigned small = 0;
 #pragma unroll 1
   for (int y = 0; y < 4; ++y) {
@@ -749,6 +803,7 @@ __global__ void __launch_bounds__(256) crt_epilogue_kernel(CrtParams P) {
 #pragma unroll
       for (int p = 0; p < MG_P; ++p) w[p] = *reinterpret_cast<const unsigned *>(src + p * plane);
       const int eb = P.eb[n];
+      const Side sn = side(P, P.B, P.col0 + n);
       // 4 x 4 byte transposes: r[k][q] holds planes 4q .. 4q+3 of row m0 + k
       unsigned r[4][4];
 #pragma unroll
@@ -765,39 +820,47 @@ __global__ void __launch_bounds__(256) crt_epilogue_kernel(CrtParams P) {
         double v;
         if (m0 + k >= P.nm || ((todo >> (4 * y + k)) & 1u)) continue;
         if (crt_value(r[k], ea[k] + eb, v))
-          put_c(P, P.row0 + m0 + k, P.col0 + n, v);
+          put(sm[k], sn, k, y, v);
         else
           small |= 1u << (4 * y + k);
       }
     }
   }
   // the few others: exact integers, or a sum in FP64 by one warp
-  if (!__any_sync(0xffffffffu, small | todo)) return;
+  if (__any_sync(0xffffffffu, small | todo)) {
 #pragma unroll 1
-  for (int x = 0; x < 16; ++x) {
-    const int k = x & 3, n = n0 + 16 * (x >> 2);
-    if ((small >> x) & 1u)
-      put_c(P, P.row0 + m0 + k, P.col0 + n,
+    for (int x = 0; x < 16; ++x) {
+      const int k = x & 3, y = x >> 2, n = n0 + 16 * y;
+      if ((small >> x) & 1u)
+        put(side(P, P.A, P.row0 + m0 + k), side(P, P.B, P.col0 + n), k, y,
             crt_small(P.res + n * P.ldm + m0 + k, plane, P.ea[m0 + k] + P.eb[n]));
-    unsigned mask = __ballot_sync(0xffffffffu, (todo >> x) & 1u);
-    while (mask) {
-      const int src = __ffs(mask) - 1;
-      mask &= mask - 1;
-      const int m = __shfl_sync(0xffffffffu, P.row0 + m0 + k, src);
-      const int nn = __shfl_sync(0xffffffffu, P.col0 + n, src);
-      const double *a = P.A.base + row_off(P.A, m), *b = P.B.base + row_off(P.B, nn);
-      double s = 0.0;
-      for (int q = lane; q < P.A.K; q += 32) s = fma(a[q * P.A.sk], b[q * P.B.sk], s);
+      unsigned mask = __ballot_sync(0xffffffffu, (todo >> x) & 1u);
+      while (mask) {
+        const int src = __ffs(mask) - 1;
+        mask &= mask - 1;
+        const int m = __shfl_sync(0xffffffffu, P.row0 + m0 + k, src);
+        const int nn = __shfl_sync(0xffffffffu, P.col0 + n, src);
+        const double *a = P.A.base + row_off(P.A, m), *b = P.B.base + row_off(P.B, nn);
+        double s = 0.0;
+        for (int q = lane; q < P.A.K; q += 32) s = fma(a[q * P.A.sk], b[q * P.B.sk], s);
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == src) put_c(P, m, nn, s);
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == src) put(side(P, P.A, m), side(P, P.B, nn), k, y, s);
+      }
     }
   }
+  if (!mirror) return;
+  __syncthreads();
+  // C(n, m): rows along n are the fast direction here
+  const int c = threadIdx.x & 63;
+  if (tn * 64 + c < P.nn)
+    for (int r = threadIdx.x >> 6; r < 64 && tm * 64 + r < P.nm; r += 4)
+      P.C[cols[c] + rows[r]] = S[r * 65 + c];
 }
 
 // The listed 64 x 64 tiles with FP64 tensor operations (DMMA m8n8k4).
 constexpr int DK = 16, DP = 20;
-__global__ void __launch_bounds__(256) dmma_tiles_kernel(CrtParams P, int tiles_m) {
+__global__ void __launch_bounds__(256) dmma_tiles_kernel(const __grid_constant__ CrtParams P, int tiles_m) {
   __shared__ double As[64][DP], Bs[64][DP];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = (warp & 1) * 32, wn = (warp >> 1) * 16, gid = lane >> 2, tig = lane & 3;
@@ -853,7 +916,10 @@ __global__ void __launch_bounds__(256) dmma_tiles_kernel(CrtParams P, int tiles_
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int m = m0 + wm + 8 * x + gid, n = n0 + wn + 8 * y + 2 * tig + h;
-          if (m < P.nm && n < P.nn) put_c(P, P.row0 + m, P.col0 + n, acc[x][y][h]);
+          if (m < P.nm && n < P.nn) {
+            put_c(P, P.row0 + m, P.col0 + n, acc[x][y][h]);
+            if (P.sym && m0 != n0) put_c(P, n, m, acc[x][y][h]);
+          }
         }
   }
 }
@@ -954,6 +1020,8 @@ int mod_product(const ModOperand &L, const ModOperand &Q, signed char *out, long
   P.tiles_l = (L.rows + 255) / 256;
   P.tiles_q = (Q.rows + 255) / 256;
   P.nkc = L.nkc;
+  const int nseg = (P.nkc + MG_SEG - 1) / MG_SEG;  // of about equal length
+  P.seg = (P.nkc + nseg - 1) / nseg;
   P.lower = lower;
   P.out = out;
   P.ldm = ldm;
@@ -962,7 +1030,7 @@ int mod_product(const ModOperand &L, const ModOperand &Q, signed char *out, long
   int dev = 0, nsm = 0;
   RIMP2_CK(cudaGetDevice(&dev));
   RIMP2_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const long long nitems = (long long)MG_PLANES * P.tiles_l * P.tiles_q;
+  const long long nitems = (long long)MG_PLANES * mg_tiles(P);
   const int npair = (int)std::min<long long>(nitems, nsm / 2);
   RIMP2_CK(launch_hi(mod_gemm_kernel, 2 * npair, MG_THREADS, MG_SMEM, s, tl, tq, P));
   count_launch(1);
@@ -981,8 +1049,8 @@ struct Dim {
 // operand's stride where rows lie along the fast direction of memory, else by
 // C's (the operand is read along K either way).
 bool make_map(RowMap &M, Dim *d, int nd, const double *base, long long sk, int K) {
+  nd = (int)(std::remove_if(d, d + nd, [](const Dim &x) { return x.ext == 1; }) - d);
   std::stable_sort(d, d + nd, [&](const Dim &x, const Dim &y) {
-    if ((x.ext == 1) != (y.ext == 1)) return y.ext == 1;  // extents of one last
     return sk == 1 ? x.cst < y.cst : x.st < y.st;
   });
   long long rows = 1;
@@ -1091,6 +1159,12 @@ int mod_gemm(const GemmDesc &g, const RowMap &A, const RowMap &B, cudaStream_t s
   P.ev = g.ev;
   P.denom = g.denom;
   P.lower = g.lower;
+  // the product of a set of vectors with itself
+  P.sym = !g.lower && g.beta == 0.0 && ra == A.rows && rb == B.rows && A.rows == B.rows && A.rows > 256 &&
+          A.base == B.base && A.sk == B.sk &&
+          memcmp(A.ext, B.ext, sizeof A.ext) == 0 && memcmp(A.st, B.st, sizeof A.st) == 0 &&
+          memcmp(A.role, B.role, sizeof A.role) == 0;
+  constexpr int mirror_smem = 64 * 65 * (int)sizeof(double);
   P.list = list.as<unsigned>();
   P.ea = Q.e.as<int>();
   P.fa = Q.flag.as<unsigned char>();
@@ -1108,9 +1182,9 @@ int mod_gemm(const GemmDesc &g, const RowMap &A, const RowMap &B, cudaStream_t s
       P.nm = Q.rows;
       P.nn = nc;
       P.ldm = ((long long)Q.rows + 255) / 256 * 256;
-      RIMP2_TRY(mod_product(L, Q, res.as<signed char>(), P.ldm, g.lower != 0, s));
+      RIMP2_TRY(mod_product(L, Q, res.as<signed char>(), P.ldm, g.lower || P.sym, s));
       dim3 grid((unsigned)((P.nm + 63) / 64), (unsigned)((P.nn + 63) / 64));
-      crt_epilogue_kernel<<<grid, 256, 0, s>>>(P);
+      crt_epilogue_kernel<<<grid, 256, P.sym ? mirror_smem : 0, s>>>(P);
       const long long nt = (long long)grid.x * grid.y;
       dmma_tiles_kernel<<<(unsigned)std::min<long long>(nt, 304), 256, 0, s>>>(P, (int)grid.x);
       count_launch(2);

@@ -209,3 +209,28 @@ def test_fp64_amplitudes(api, nocc, nvirt, nba):
     assert (np.abs(t - g / d) <= (nba + 4) * U * np.abs(mag / d)).all()
     e = (t * (2 * g - g.transpose(2, 1, 0, 3))).sum((0, 2))
     assert np.abs(E - e).max() <= 1e-12 * np.abs(e).max()
+
+
+@pytest.mark.parametrize("n,k", [(300, 700), (321, 1500)])
+def test_symmetric_product(api, n, k):
+    """A set of vectors with itself: both triangles, and the elements left to FP64."""
+    r = np.random.Generator(np.random.Philox(key=[n, k]))
+    X = r.standard_normal((k, n, 2))
+    X[:, 5, 1] = 0.0
+    X[:, 100, 0] *= np.exp(6 * r.standard_normal(k))
+    X[3, 200, 1] = np.inf
+    X = np.asfortranarray(X)
+    G = np.zeros((n, 2, n, 2), order="F")
+    before = api.kernel_launch_count()
+    api.calc_gocc(n, 2, k, X, G)
+    assert api.kernel_launch_count() - before > 1
+    F, G = X.reshape(k, 2 * n, order="F"), G.reshape(2 * n, 2 * n, order="F")
+    assert np.array_equal(G, G.T, equal_nan=True)
+    with np.errstate(all="ignore"):
+        ref, mag = F.T @ F, np.abs(F).T @ np.abs(F)
+    ok = np.isfinite(ref)
+    assert np.array_equal(ok, np.isfinite(G))
+    assert (np.abs(G - ref)[ok] <= 2 * k * U * mag[ok]).all()
+    for i, j in [(0, 1), (1, 0), (2 * n - 1, 3), (3, 2 * n - 1), (70, 100), (64, 63), (256, 255)]:
+        d = exact_dot(F[:, i], F[:, j])
+        assert abs(G[i, j] - d) <= (math.sqrt(k) / 2 + 1) * U * np.abs(F[:, i] * F[:, j]).sum()
