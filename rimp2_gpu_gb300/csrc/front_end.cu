@@ -9,16 +9,16 @@
 // of fp64_kernels.cu or on the tcgen05 split GEMM (two residual FP16 slices,
 // ~2^-33 relative per product); the Cholesky and the solve are FP64, blocked
 // (64) so that all but O(n*64^2) of their work is GEMM:
-//   Cholesky: diagonal-block factorisation and inverse (one CTA), panel
-//             P L_kk^{-T} (GEMM), trailing update C -= P P^T on the
-//             lower-triangle tiles;
-//   solve:    all diagonal-block inverses in one launch, then
-//             X_k = inv(L_kk) B_k and B_rest -= L_rest,k X_k (GEMMs).
+//   Cholesky: panels of 256 columns, in them 64 at a time (diagonal block in
+//             one CTA, rows below solved against it, update of the panel), the
+//             rest updated once per panel;
+//   solve:    all diagonal-block inverses in one launch, then by halves:
+//             X_1, B_2 -= L_21 X_1, X_2 (GEMMs).
 #include <cmath>
 #include <cstring>
 #include <vector>
 
-#include "common.cuh"
+#include "mod_gemm.cuh"
 
 namespace rimp2 {
 void count_launch(int n);
@@ -36,11 +36,11 @@ GemmDesc gdesc() {
   return g;
 }
 
-// Diagonal 64x64 blocks: factorisation and triangular inverse in shared
-// memory, 256 threads.  Blocks narrower than 64 (the last one) are padded
-// with the identity, so the same code runs on every block.
+// Diagonal 64x64 blocks: triangular inverse in shared memory, 256 threads.
+// Blocks narrower than 64 (the last one) are padded with the identity, so the
+// same code runs on every block.
 constexpr int DP = NB + 1;                        // padded row (doubles)
-constexpr int DIAG_SMEM = (2 * NB * DP + 5 * NB + 1) * sizeof(double);
+constexpr int DIAG_SMEM = (2 * NB * DP + 5 * NB) * sizeof(double);
 
 __device__ __forceinline__ void load_block(double (*A)[DP], const double *V, int n, int k0, int b) {
   for (int t = threadIdx.x; t < NB * NB; t += blockDim.x) {
@@ -72,46 +72,95 @@ __device__ void tri_inverse(double (*A)[DP], double (*X)[DP], double *part, doub
   }
 }
 
-// In-place Cholesky of the b x b diagonal block at (k0,k0) of V (ld n) and
-// its inverse into Linv (NB x NB, column-major); *bad = pivot+1 on a
-// non-positive pivot.
-__global__ void __launch_bounds__(256) potrf_inv_block_kernel(double *V, int n, int k0, int b,
-                                                             double *Linv, int *bad) {
-  extern __shared__ double dsm[];
-  double(*A)[DP] = reinterpret_cast<double(*)[DP]>(dsm);
-  double(*X)[DP] = reinterpret_cast<double(*)[DP]>(dsm + NB * DP);
-  double *part = dsm + 2 * NB * DP;
-  double *rdiag = part + 4 * NB;
-  double *rpiv = rdiag + NB;
-  load_block(A, V, n, k0, b);
-  const int c = threadIdx.x & (NB - 1), r0 = threadIdx.x >> 6;
+// In-place Cholesky of the b x b diagonal block at (k0,k0) of V (ld n); *bad =
+// pivot+1 on a non-positive pivot.  One CTA, so its FP64 pipe (two FMAs a
+// clock) and the chain of 64 pivots bound it: the block lives in registers
+// (lane = row, a warp holds every fourth column of 32 rows, so that a finished
+// column costs whole warps nothing), column k passes through shared memory
+// with one barrier a step, and the chain is kept short by eliminating with
+// column k over d_k (a reciprocal; the columns get their 1/sqrt(d_k) at the end,
+// all at once).
+__global__ void __launch_bounds__(256) potrf_block_kernel(double *V, int n, int k0, int b, int *bad) {
+  __shared__ double col[2][NB];  // column k, not yet scaled
+  __shared__ double piv[NB];     // 1 / sqrt(d_k)
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, q = w & 3, half = w >> 2;
+  const int r = 32 * half + lane;
+  double a[NB / 4];
+#pragma unroll
+  for (int x = 0; x < NB / 4; ++x) {
+    const int c = 4 * x + q;
+    a[x] = r < b && c < b ? V[(size_t)(k0 + (r > c ? r : c)) + (size_t)n * (k0 + (r > c ? c : r))]
+                          : (r == c ? 1.0 : 0.0);
+  }
+  if (q == 0) col[0][r] = a[0];
+  __syncthreads();
+#pragma unroll 1
   for (int k = 0; k < NB; ++k) {
-    if (threadIdx.x == 0) {
-      const double d = A[k][k];
-      double l = 1.0;
-      if (!(d > 0.0))
-        atomicCAS(bad, 0, k0 + k + 1);
-      else
-        l = sqrt(d);
-      A[k][k] = l;
-      *rpiv = 1.0 / l;
+    const double *ck = col[k & 1];
+    const double d = ck[k];
+    const bool ok = d > 0.0;
+    if (!ok && threadIdx.x == 0) atomicCAS(bad, 0, k0 + k + 1);
+    if (threadIdx.x == 0) piv[k] = ok ? d : 1.0;
+    const double f = -(ok ? recip_f64(d) : 1.0) * ck[r];
+#pragma unroll
+    for (int x = 0; x < NB / 4; ++x) {
+      const int c = 4 * x + q;
+      if (c <= k || (half == 0 && c >= 32)) continue;  // uniform over the warp
+      a[x] = fma(f, ck[c], a[x]);
+      if (c == k + 1) col[(k + 1) & 1][r] = a[x];
     }
-    __syncthreads();
-    if (threadIdx.x > k && threadIdx.x < NB) A[threadIdx.x][k] *= *rpiv;
-    __syncthreads();
-    // trailing lower triangle: column c, rows r >= c with r = r0 (mod 4)
-    if (c > k) {
-      const double ck = A[c][k];
-      for (int r = c + ((r0 - c) & 3); r < NB; r += 4) A[r][c] -= A[r][k] * ck;
-    }
+    // rows 0..31 of column k+1 >= 32 lie above the diagonal: not needed
     __syncthreads();
   }
-  tri_inverse(A, X, part, rdiag);
-  for (int t = threadIdx.x; t < NB * NB; t += blockDim.x) {
-    const int r = t & (NB - 1), cc = t >> 6;
-    if (r < b && cc < b) V[(size_t)(k0 + r) + (size_t)n * (k0 + cc)] = (r >= cc) ? A[r][cc] : 0.0;
-    Linv[t] = X[r][cc];
+  if (threadIdx.x < NB) piv[threadIdx.x] = 1.0 / sqrt(piv[threadIdx.x]);
+  __syncthreads();
+#pragma unroll
+  for (int x = 0; x < NB / 4; ++x) {
+    const int c = 4 * x + q;
+    if (r < b && c < b) V[(size_t)(k0 + r) + (size_t)n * (k0 + c)] = r >= c ? a[x] * piv[c] : 0.0;
   }
+}
+
+// X := X L^{-T} for the rows [k0+64, n) of the block column at k0, L its
+// factored diagonal block: eight rows per CTA (136 CTAs at n = 1152), 16
+// threads a row with four columns each, one barrier-free chain of 64 columns
+// within each row's half warp.  (As a product with L^{-1} the inverse sat on
+// the critical path: 70 of 143 us.)
+__global__ void __launch_bounds__(128) panel_solve_kernel(double *V, int n, int k0) {
+  __shared__ double Ls[NB][NB + 1];  // Ls[c][j] = L(j, c) below, 1 / L(c, c) on the diagonal
+  for (int t = threadIdx.x; t < NB * NB; t += 128) {
+    const int j = t & (NB - 1), c = t >> 6;
+    const double l = V[(size_t)(k0 + j) + (size_t)n * (k0 + c)];
+    Ls[c][j] = j == c ? 1.0 / l : l;
+  }
+  const int row = k0 + NB + blockIdx.x * 8 + (threadIdx.x >> 4), g = threadIdx.x & 15;
+  double x[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) x[u] = row < n ? V[(size_t)row + (size_t)n * (k0 + g + 16 * u)] : 0.0;
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < 4; ++u)  // columns 16 u + v, owned by thread v
+#pragma unroll 4
+    for (int v = 0; v < 16; ++v) {
+      const int c = 16 * u + v;
+      const double y = __shfl_sync(0xffffffffu, x[u], v, 16) * Ls[c][c];
+      if (g == v) x[u] = y;
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        if (s < u) continue;
+        const int j = g + 16 * s;
+        if (s > u || g > v) x[s] = fma(-y, Ls[c][j], x[s]);
+      }
+    }
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    if (row < n) V[(size_t)row + (size_t)n * (k0 + g + 16 * u)] = x[u];
+}
+
+__global__ void zero_upper_kernel(double *V, int n) {
+  const int c = blockIdx.y * blockDim.y + threadIdx.y;
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < n && r < c) V[(size_t)r + (size_t)n * c] = 0.0;
 }
 
 // Inverses of every diagonal block of the lower-triangular L (one CTA per
@@ -139,12 +188,8 @@ __global__ void __launch_bounds__(256) tri_inverse_blocks_kernel(const double *L
 
 // The shared-memory opt-in is per device: set it on the current device.
 int diag_kernels_init() {
-  const bool ok =
-      cudaFuncSetAttribute(potrf_inv_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           DIAG_SMEM) == cudaSuccess &&
-      cudaFuncSetAttribute(tri_inverse_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           DIAG_SMEM) == cudaSuccess;
-  if (!ok) {
+  if (cudaFuncSetAttribute(tri_inverse_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           DIAG_SMEM) != cudaSuccess) {
     set_error("diagonal-block kernels: shared-memory attribute failed");
     return RIMP2_ERR_CUDA;
   }
@@ -154,68 +199,52 @@ int diag_kernels_init() {
 }  // namespace
 
 // V (n x n, ld n, device) -> lower Cholesky factor in place (strict upper
-// zeroed block by block).  Returns RIMP2_ERR_ARG if V is not positive definite.
-// Per 64-column block k: factor and invert the diagonal block (one CTA),
-// panel P := P L_kk^{-T} as a GEMM with the inverse (into a work panel), the
-// trailing update C -= P P^T on the lower-triangle tiles, and the panel
-// copied back into V.
+// zeroed).  Returns RIMP2_ERR_ARG if V is not positive definite.  Two levels:
+// inside a panel of 256 columns, per 64 of them the diagonal block is factored
+// (one CTA), the rows below solved against it and the panel's remaining
+// columns updated; the columns right of the panel are updated once, over its
+// whole width (a product of 256 terms a sum, which the residue form takes).
+constexpr int CH_PANEL = 256;
 int dev_cholesky(int n, double *V, cudaStream_t s) {
-  RIMP2_TRY(diag_kernels_init());
-  DevBuf bad, inv, panel;
+  DevBuf bad;
   RIMP2_TRY(bad.alloc(sizeof(int), s));
-  RIMP2_TRY(inv.alloc(sizeof(double) * NB * NB, s));
-  RIMP2_TRY(panel.alloc(sizeof(double) * (size_t)(n > NB ? n - NB : 1) * NB, s));
   RIMP2_CK(cudaMemsetAsync(bad.p, 0, sizeof(int), s));
-  for (int k0 = 0; k0 < n; k0 += NB) {
-    const int b = n - k0 < NB ? n - k0 : NB;
-    potrf_inv_block_kernel<<<1, 256, DIAG_SMEM, s>>>(V, n, k0, b, inv.as<double>(),
-                                                     bad.as<int>());
-    count_launch(1);
-    const int rest = n - k0 - b;
-    if (rest > 0) {
-      double *Pv = V + (size_t)(k0 + b) + (size_t)n * k0;
-      {  // panel(rest x b) = P Linv^T
-        GemmDesc g = gdesc();
-        g.M = rest;
-        g.N = b;
-        g.K = b;
-        g.A = Pv;
-        g.sAm = 1;
-        g.sAk = n;
-        g.B = inv.as<double>();
-        g.sBk = NB;
-        g.sBn = 1;
-        g.C = panel.as<double>();
-        g.sCm = 1;
-        g.sCn = rest;
-        RIMP2_TRY(launch_gemm_f64(g, s));
-      }
-      {  // trailing update C -= panel panel^T (lower-triangle tiles)
-        GemmDesc g = gdesc();
-        g.M = rest;
-        g.N = rest;
-        g.K = b;
-        g.alpha = -1.0;
-        g.beta = 1.0;
-        g.lower = 1;
-        g.A = panel.as<double>();
-        g.sAm = 1;
-        g.sAk = rest;
-        g.B = panel.as<double>();
-        g.sBk = rest;
-        g.sBn = 1;
-        g.C = V + (size_t)(k0 + b) + (size_t)n * (k0 + b);
-        g.sCm = 1;
-        g.sCn = n;
-        RIMP2_TRY(launch_gemm_f64(g, s));
-      }
-      RIMP2_CK(cudaMemcpy2DAsync(Pv, sizeof(double) * n, panel.p, sizeof(double) * rest,
-                                 sizeof(double) * rest, b, cudaMemcpyDeviceToDevice, s));
+  // C(r0.., c0 .. c0+nc) -= P(r0..) P(c0 .. c0+nc)^T, P the columns [k0, k0 + K)
+  auto update = [&](int r0, int c0, int nc, int k0, int K, bool lower) -> int {
+    GemmDesc g = gdesc();
+    g.M = n - r0;
+    g.N = nc;
+    g.K = K;
+    g.alpha = -1.0;
+    g.beta = 1.0;
+    g.lower = lower ? 1 : 0;
+    g.A = V + (size_t)r0 + (size_t)n * k0;
+    g.sAm = 1;
+    g.sAk = n;
+    g.B = V + (size_t)c0 + (size_t)n * k0;
+    g.sBk = n;
+    g.sBn = 1;
+    g.C = V + (size_t)r0 + (size_t)n * c0;
+    g.sCm = 1;
+    g.sCn = n;
+    return launch_gemm_f64(g, s);
+  };
+  for (int p0 = 0; p0 < n; p0 += CH_PANEL) {
+    const int p1 = n - p0 < CH_PANEL ? n : p0 + CH_PANEL;
+    for (int k0 = p0; k0 < p1; k0 += NB) {
+      const int b = n - k0 < NB ? n - k0 : NB;
+      potrf_block_kernel<<<1, 256, 0, s>>>(V, n, k0, b, bad.as<int>());
+      count_launch(1);
+      const int r0 = k0 + b;
+      if (r0 >= n) break;
+      panel_solve_kernel<<<(n - r0 + 7) / 8, 128, 0, s>>>(V, n, k0);
+      count_launch(1);
+      if (r0 < p1) RIMP2_TRY(update(r0, r0, p1 - r0, k0, NB, false));
     }
-    // zero the strict upper part of this block column above the block
-    if (k0 > 0) RIMP2_CK(cudaMemset2DAsync(V + (size_t)n * k0, sizeof(double) * n, 0,
-                                           sizeof(double) * k0, b, s));
+    if (p1 < n) RIMP2_TRY(update(p1, p1, n - p1, p0, p1 - p0, true));
   }
+  zero_upper_kernel<<<dim3((n + 63) / 64, (n + 3) / 4), dim3(64, 4), 0, s>>>(V, n);
+  count_launch(1);
   RIMP2_CK(cudaGetLastError());
   int h = 0;
   RIMP2_CK(cudaMemcpyAsync(&h, bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
@@ -227,9 +256,44 @@ int dev_cholesky(int n, double *V, cudaStream_t s) {
   return RIMP2_OK;
 }
 
+// Rows [k0, k0 + nn) of X = L^{-1} B: the first half, B -= L21 X of the second,
+// the second half; 64 rows by the inverse of their diagonal block.  Halving
+// keeps the products' sums long (n/2, n/4, ...): 2.1 n m updated elements at
+// n = 1152 where 64 columns at a time update 9 n m.
+static int trsm_rows(int n, int m, int k0, int nn, const double *L, const double *inv, double *B,
+                     double *X, cudaStream_t s) {
+  GemmDesc g = gdesc();
+  g.N = m;
+  g.sAm = 1;
+  g.sBk = 1;
+  g.sBn = n;
+  g.sCm = 1;
+  g.sCn = n;
+  if (nn <= NB) {  // X_k = inv(L_kk) B_k
+    g.M = nn;
+    g.K = nn;
+    g.A = inv + (size_t)(k0 / NB) * NB * NB;
+    g.sAk = NB;
+    g.B = B + k0;
+    g.C = X + k0;
+    return launch_gemm_f64(g, s);
+  }
+  const int n1 = (nn / 2 + NB - 1) / NB * NB;
+  RIMP2_TRY(trsm_rows(n, m, k0, n1, L, inv, B, X, s));
+  g.M = nn - n1;
+  g.K = n1;
+  g.alpha = -1.0;
+  g.beta = 1.0;
+  g.A = L + (size_t)(k0 + n1) + (size_t)n * k0;
+  g.sAk = n;
+  g.B = X + k0;
+  g.C = B + k0 + n1;
+  RIMP2_TRY(launch_gemm_f64(g, s));
+  return trsm_rows(n, m, k0 + n1, nn - n1, L, inv, B, X, s);
+}
+
 // X = L^{-1} B for B (n x m, ld n).  B is overwritten (used as workspace).
-// The inverses of all diagonal blocks come from one launch; then per block
-// X_k = inv(L_kk) B_k and B_rest -= L_rest,k X_k (both GEMMs).
+// The inverses of all diagonal blocks come from one launch.
 int dev_trsm_lower(int n, int m, const double *L, double *B, double *X, cudaStream_t s) {
   RIMP2_TRY(diag_kernels_init());
   const int nblk = (n + NB - 1) / NB;
@@ -238,45 +302,7 @@ int dev_trsm_lower(int n, int m, const double *L, double *B, double *X, cudaStre
   tri_inverse_blocks_kernel<<<nblk, 256, DIAG_SMEM, s>>>(L, n, inv.as<double>());
   count_launch(1);
   RIMP2_CK(cudaGetLastError());
-  for (int k0 = 0; k0 < n; k0 += NB) {
-    const int b = n - k0 < NB ? n - k0 : NB;
-    {  // X_k = inv(L_kk) B_k
-      GemmDesc g = gdesc();
-      g.M = b;
-      g.N = m;
-      g.K = b;
-      g.A = inv.as<double>() + (size_t)(k0 / NB) * NB * NB;
-      g.sAm = 1;
-      g.sAk = NB;
-      g.B = B + k0;
-      g.sBk = 1;
-      g.sBn = n;
-      g.C = X + k0;
-      g.sCm = 1;
-      g.sCn = n;
-      RIMP2_TRY(launch_gemm_f64(g, s));
-    }
-    const int rest = n - k0 - b;
-    if (rest > 0) {  // B_rest -= L_rest,k X_k
-      GemmDesc g = gdesc();
-      g.M = rest;
-      g.N = m;
-      g.K = b;
-      g.alpha = -1.0;
-      g.beta = 1.0;
-      g.A = L + (size_t)(k0 + b) + (size_t)n * k0;
-      g.sAm = 1;
-      g.sAk = n;
-      g.B = X + k0;
-      g.sBk = 1;
-      g.sBn = n;
-      g.C = B + k0 + b;
-      g.sCm = 1;
-      g.sCn = n;
-      RIMP2_TRY(launch_gemm_f64(g, s));
-    }
-  }
-  return RIMP2_OK;
+  return trsm_rows(n, m, 0, n, L, inv.as<double>(), B, X, s);
 }
 
 // (alpha|a i) from (alpha|mu nu) and the MO coefficients

@@ -353,22 +353,25 @@ __global__ void __launch_bounds__(256) residue_kernel(const __grid_constant__ Op
 // --------------------------------------------------------------------------
 // products: persistent CTA pairs
 // --------------------------------------------------------------------------
-// Work item = (plane, 256 columns n x 256 rows m of C): the columns' operand
+// Work item = (plane, 256 columns n x TQ rows m of C): the columns' operand
 // lies on the TMEM lanes (M = 256 over the pair), the rows' operand on the
-// accumulator columns (N = 256, half of it in each CTA), so that a thread
-// stores runs of bytes along m.  Two 256-column accumulators per CTA: the
+// accumulator columns (N = TQ, half of it in each CTA), so that a thread
+// stores runs of bytes along m.  Two TQ-column accumulators per CTA: the
 // MMAs of one item run while the epilogue reduces the other.  Sums longer
 // than 1024 are cut there (exactness) and joined modulo p in the epilogue's
-// registers.  A 64-deep stage is 32 KB per CTA, six stages.
-constexpr int MG_NST = 6;
-constexpr int MG_STAGE = 2 * PANEL_BYTES;
+// registers.  A 64-deep stage is 32 KB per CTA (TQ = 256), six stages.
+// TQ, the rows of C in a tile, is 128 or 64 where 256 would mostly be padding
+// (a product with few rows; one with few columns is transposed): its MMAs and
+// epilogue shrink with it, the lanes' operand is read as before.
 constexpr int MG_THREADS = 320;
 constexpr int MG_SEG = 16;  // most K chunks of an exact sum
-constexpr int MG_SMEM = MG_NST * MG_STAGE + 1024 + 256;
+constexpr int mg_stage(int tq) { return PANEL_BYTES + tq / 2 * KSTEP * 2; }
+constexpr int mg_nst(int tq) { return tq == 256 ? 6 : 8; }
+constexpr int mg_smem(int tq) { return mg_nst(tq) * mg_stage(tq) + 1024 + 256; }
 
 struct MgParams {
   int rows_l, rows_q;        // rows per K chunk of the two operands
-  int tiles_l, tiles_q;      // 256-wide tiles
+  int tiles_l, tiles_q;      // 256 columns, TQ rows
   int nkc, seg;              // K chunks, and of one exact sum
   int lower;                 // square, only tiles with an element m >= n
   signed char *out;          // [plane][n][ldm]
@@ -401,14 +404,16 @@ __device__ __forceinline__ void mg_item(const MgParams &P, long long item, int &
   tq = rem / gs;
 }
 
+template <int TQ>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
     mod_gemm_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__ CUtensorMap tmQ,
                     MgParams P) {
-  constexpr int NST = MG_NST;
+  constexpr int NST = mg_nst(TQ), STAGE = mg_stage(TQ);
+  constexpr int NG = TQ / 32;  // groups of 16 accumulator columns per epilogue warp
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   // bars: full[NST], empty[NST], tfull[2], tempty[2], drain
-  uint64_t *bars = (uint64_t *)(base + NST * MG_STAGE);
+  uint64_t *bars = (uint64_t *)(base + NST * STAGE);
   uint32_t *tmem_slot = (uint32_t *)(bars + 2 * NST + 5);
   volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -459,18 +464,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
       for (long long item = pair; item < nitems && ok; item += npair) {
         int p, tl, tq;
         mg_item(P, item, p, tl, tq);
-        const int rl = tl * 256 + 128 * (int)rank, rq = tq * 256 + 128 * (int)rank;
+        const int rl = tl * 256 + 128 * (int)rank, rq = tq * TQ + TQ / 2 * (int)rank;
         for (int kc = 0; kc < P.nkc; ++kc) {
           if (!pair_wait(empty0 + 8 * stage, phase ^ 1, false, abort_flag, abort_peer, P.err, 21)) {
             ok = false;
             break;
           }
           if (leader) {
-            mbar_expect_tx(full0 + 8 * stage, 2 * MG_STAGE);
+            mbar_expect_tx(full0 + 8 * stage, 2 * STAGE);
             armed |= 1u << stage;
             armed_par = (armed_par & ~(1u << stage)) | (phase << stage);
           }
-          const uint32_t dst = smem_u32(base + stage * MG_STAGE), fb = full0_L + 8 * stage;
+          const uint32_t dst = smem_u32(base + stage * STAGE), fb = full0_L + 8 * stage;
           tma_load_3d_pair(dst, &tmL, fb, 0, kc * P.rows_l + rl, p);
           tma_load_3d_pair(dst + PANEL_BYTES, &tmQ, fb, 0, kc * P.rows_q + rq, p);
           if (++stage == NST) {
@@ -506,7 +511,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
             break;
           }
           tc_fence_after();
-          const uint32_t d = tmem + (uint32_t)(u * 256);
+          const uint32_t d = tmem + (uint32_t)(u * TQ);
           const int s1 = min(P.nkc, s0 + P.seg);
           for (int kc = s0; kc < s1; ++kc) {
             if (!pair_wait(full0 + 8 * stage, phase, false, abort_flag, abort_peer, P.err, 23)) {
@@ -514,11 +519,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
               break;
             }
             tc_fence_after();
-            const uint32_t sb = smem_u32(base + stage * MG_STAGE);
+            const uint32_t sb = smem_u32(base + stage * STAGE);
 #pragma unroll
             for (int k16 = 0; k16 < KSTEP / 16; ++k16)
               mma_f16_pair(d, smem_desc(sb + k16 * 32), smem_desc(sb + PANEL_BYTES + k16 * 32),
-                           IDESC_PAIR_N256, (kc > s0 || k16 > 0) ? 1u : 0u);
+                           idesc_mn(256, TQ), (kc > s0 || k16 > 0) ? 1u : 0u);
             mma_commit_pair(empty0 + 8 * stage);  // frees the stage in both CTAs
             if (++stage == NST) {
               stage = 0;
@@ -544,16 +549,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
       const int n = tl * 256 + 128 * (int)rank + quad * 32 + lane;
       const bool mag = p == MG_P;
       const float pf = mag ? 1.0f : DT.p[p], inv = mag ? 1.0f : DT.inv[p];
-      uint32_t pk[8][4];
+      uint32_t pk[NG][4];
       for (int s0 = 0; s0 < P.nkc; s0 += P.seg, ++t) {
         const int u = (int)(t & 1);
         ok = pair_wait(tfull0 + 8 * u, (uint32_t)((t >> 1) & 1), false, abort_flag, abort_peer, P.err, 24);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t ta = tmem + lane_off + (uint32_t)(u * 256 + half * 128);
+        const uint32_t ta = tmem + lane_off + (uint32_t)(u * TQ + half * (TQ / 2));
 #pragma unroll
-        for (int g = 0; g < 8; ++g) {
+        for (int g = 0; g < NG; ++g) {
           float v[16];
           tmem_ld16(ta + g * 16, v);
           tmem_wait_ld();
@@ -588,9 +593,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
         if (lane == 0) mbar_arrive_remote(tempty0_L + 8 * u);
       }
       if (ok && n < nl) {
-        signed char *o = P.out + ((long long)p * nl + n) * P.ldm + tq * 256 + half * 128;
+        signed char *o = P.out + ((long long)p * nl + n) * P.ldm + tq * TQ + half * (TQ / 2);
 #pragma unroll
-        for (int g = 0; g < 8; ++g)
+        for (int g = 0; g < NG; ++g)
           *reinterpret_cast<uint4 *>(o + g * 16) = make_uint4(pk[g][0], pk[g][1], pk[g][2], pk[g][3]);
       }
     }
@@ -709,6 +714,7 @@ struct CrtParams {
   double alpha, beta;
   const double *eo, *ev;
   int denom, lower;
+  int nfast;                 // C's fast direction is n
   int sym;                   // rows and columns are the same vectors: C(n,m) comes with C(m,n)
   unsigned *list;            // [0] count, then tiles (tn * tiles_m + tm) left to FP64
 };
@@ -746,7 +752,8 @@ __global__ void __launch_bounds__(256) crt_epilogue_kernel(const __grid_constant
   extern __shared__ double S[];             // symmetric: [64][65]
   const int tm = blockIdx.x, tn = blockIdx.y;
   if ((P.lower || P.sym) && tm < tn) return;
-  const int mq = (threadIdx.x & 15) * 4, nq = threadIdx.x >> 4;
+  const int t0 = threadIdx.x & 15, t1 = threadIdx.x >> 4;
+  const int mq = (P.nfast ? t1 : t0) * 4, nq = P.nfast ? t0 : t1;
   const int m0 = tm * 64 + mq, n0 = tn * 64 + nq;
   const long long plane = (long long)P.nn * P.ldm;
   const bool mirror = P.sym && tm != tn;
@@ -927,7 +934,7 @@ __global__ void __launch_bounds__(256) dmma_tiles_kernel(const __grid_constant__
 // --------------------------------------------------------------------------
 // host side
 // --------------------------------------------------------------------------
-int encode_planes(CUtensorMap &tm, const ModOperand &op) {
+int encode_planes(CUtensorMap &tm, const ModOperand &op, int boxrows) {
   auto encode = get_encode();
   if (!encode) {
     set_error("cuTensorMapEncodeTiled entry point unavailable");
@@ -936,7 +943,7 @@ int encode_planes(CUtensorMap &tm, const ModOperand &op) {
   const cuuint64_t rows = (cuuint64_t)op.rows * op.nkc;
   cuuint64_t dims[3] = {64, rows, MG_PLANES};
   cuuint64_t strides[2] = {128, rows * 128};
-  cuuint32_t box[3] = {KSTEP, TILE, 1};
+  cuuint32_t box[3] = {KSTEP, (cuuint32_t)boxrows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult cr = encode(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, op.planes.p, dims, strides, box, estr,
                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
@@ -1009,16 +1016,37 @@ int fill_operands(ModOperand &Q, const RowMap &A, int r0, bool rows, ModOperand 
 
 }  // namespace
 
+// Rows of a tile: least work, smaller tiles paying for their operand reads.
+static int tile_rows(double m) {
+  auto cost = [&](int tq, double per_row) { return std::ceil(m / tq) * tq * per_row; };
+  const double c256 = cost(256, 1.0), c128 = cost(128, 1.2), c64 = cost(64, 1.6);
+  return c64 < c128 && c64 < c256 ? 64 : c128 < c256 ? 128 : 256;
+}
+
+template <int TQ>
+static int launch_product(const CUtensorMap &tl, const CUtensorMap &tq, const MgParams &P, cudaStream_t s) {
+  RIMP2_CK(cudaFuncSetAttribute(mod_gemm_kernel<TQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, mg_smem(TQ)));
+  int dev = 0, nsm = 0;
+  RIMP2_CK(cudaGetDevice(&dev));
+  RIMP2_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const long long nitems = (long long)MG_PLANES * mg_tiles(P);
+  const int npair = (int)std::min<long long>(nitems, nsm / 2);
+  RIMP2_CK(launch_hi(mod_gemm_kernel<TQ>, 2 * npair, MG_THREADS, mg_smem(TQ), s, tl, tq, P));
+  count_launch(1);
+  return RIMP2_OK;
+}
+
 int mod_product(const ModOperand &L, const ModOperand &Q, signed char *out, long long ldm, bool lower,
                 cudaStream_t s) {
+  const int TQ = lower ? 256 : tile_rows(Q.rows);
   CUtensorMap tl, tq;
-  RIMP2_TRY(encode_planes(tl, L));
-  RIMP2_TRY(encode_planes(tq, Q));
+  RIMP2_TRY(encode_planes(tl, L, TILE));
+  RIMP2_TRY(encode_planes(tq, Q, TQ / 2));
   MgParams P;
   P.rows_l = L.rows;
   P.rows_q = Q.rows;
   P.tiles_l = (L.rows + 255) / 256;
-  P.tiles_q = (Q.rows + 255) / 256;
+  P.tiles_q = (Q.rows + TQ - 1) / TQ;
   P.nkc = L.nkc;
   const int nseg = (P.nkc + MG_SEG - 1) / MG_SEG;  // of about equal length
   P.seg = (P.nkc + nseg - 1) / nseg;
@@ -1026,15 +1054,9 @@ int mod_product(const ModOperand &L, const ModOperand &Q, signed char *out, long
   P.out = out;
   P.ldm = ldm;
   P.err = device_error_word();
-  RIMP2_CK(cudaFuncSetAttribute(mod_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MG_SMEM));
-  int dev = 0, nsm = 0;
-  RIMP2_CK(cudaGetDevice(&dev));
-  RIMP2_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const long long nitems = (long long)MG_PLANES * mg_tiles(P);
-  const int npair = (int)std::min<long long>(nitems, nsm / 2);
-  RIMP2_CK(launch_hi(mod_gemm_kernel, 2 * npair, MG_THREADS, MG_SMEM, s, tl, tq, P));
-  count_launch(1);
-  return RIMP2_OK;
+  if (TQ == 64) return launch_product<64>(tl, tq, P, s);
+  if (TQ == 128) return launch_product<128>(tl, tq, P, s);
+  return launch_product<256>(tl, tq, P, s);
 }
 
 namespace {
@@ -1120,8 +1142,11 @@ bool fold_gemm(const GemmDesc &g, RowMap &A, RowMap &B) {
   return make_map(A, da, na, g.A, g.sAk, g.K) && make_map(B, db, nb, g.B, g.sBk, g.K);
 }
 
-int mod_gemm(const GemmDesc &g, const RowMap &A, const RowMap &B, cudaStream_t s, bool *handled) {
+int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t s, bool *handled) {
   *handled = false;
+  // few columns: transposed, so that they are the tile's narrow side
+  const bool swap = !g.lower && !g.denom && B0.rows <= 128 && A0.rows > B0.rows;
+  const RowMap &A = swap ? B0 : A0, &B = swap ? A0 : B0;
   if (g.K < MG_K_MIN || g.K > MG_K_MAX || g.alpha == 0.0) return RIMP2_OK;
   // a captured call keeps to the FP64 kernel: the order between contractions
   // (ModOrder) cannot reach into a graph
@@ -1159,6 +1184,7 @@ int mod_gemm(const GemmDesc &g, const RowMap &A, const RowMap &B, cudaStream_t s
   P.ev = g.ev;
   P.denom = g.denom;
   P.lower = g.lower;
+  P.nfast = B.cst[0] < A.cst[0];
   // the product of a set of vectors with itself
   P.sym = !g.lower && g.beta == 0.0 && ra == A.rows && rb == B.rows && A.rows == B.rows && A.rows > 256 &&
           A.base == B.base && A.sk == B.sk &&
@@ -1199,9 +1225,11 @@ int mod_gemm(const GemmDesc &g, const RowMap &A, const RowMap &B, cudaStream_t s
 // both operands, the products, the reconstruction.
 double mod_gemm_time(double m, double n, double k, bool lower) {
   auto up = [](double x, double t) { return std::ceil(x / t) * t; };
-  const double kp = up(k, 64), part = lower ? 0.55 : 1.0;
+  if (!lower && n <= 128 && m > n) std::swap(m, n);
+  const double kp = up(k, 64), part = lower ? 0.55 : 1.0, tq = lower ? 256 : tile_rows(m);
+  const double rate = tq == 256 ? 1.3e15 : tq == 128 ? 1.3e15 / 1.2 : 1.3e15 / 1.6;
   return 20e-6 + (m + n) * kp * 10e-12 +
-         part * (m * n * 16e-12 + 17.0 * 2.0 * up(m, 256) * up(n, 256) * (kp + 64) / 1.3e15);
+         part * (m * n * 14e-12 + 17.0 * 2.0 * up(m, tq) * up(n, 256) * (kp + 64) / rate);
 }
 
 // Rows and columns of a square product that runs as one part.
