@@ -59,9 +59,17 @@ struct DevBuf {
   DevBuf &operator=(const DevBuf &) = delete;
   ~DevBuf() { release(); }
   int alloc(size_t bytes, cudaStream_t st);
+  bool own = true;  // false: a part of another buffer
   void release() {
-    if (p) cudaFreeAsync(p, s);
+    if (p && own) cudaFreeAsync(p, s);
     p = nullptr;
+  }
+  void alias(void *q, size_t bytes, cudaStream_t st) {
+    release();
+    own = false;
+    p = q;
+    n = bytes;
+    s = st;
   }
   template <class T>
   T *as() const { return static_cast<T *>(p); }
@@ -99,6 +107,11 @@ inline unsigned total_threads(int nocc) {
   const long long n = ((long long)nocc * nocc / 8 + 31) / 32 * 32;
   return (unsigned)(n < 32 ? 32 : n > 1024 ? 1024 : n);
 }
+
+#ifdef __CUDACC__
+// Width of a warp's reduction tree over n values: the power of two >= n.
+__device__ __forceinline__ int tree_width(int n) { return n >= 17 ? 32 : n <= 1 ? 1 : 1 << (32 - __clz(n - 1)); }
+#endif
 
 struct PlainEnergyArgs {
   const double *Ca;  // Calpha(NBA, nvirt, nocc)

@@ -534,9 +534,10 @@ __device__ __forceinline__ void two_sum(double a, double b, double &s, double &e
   e = (a - (s - bb)) + (b - bb);
 }
 
-__device__ __forceinline__ void warp_sum_comp(double &s, double &c) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+// width: a power of two, the lanes from it on hold zeros (each step of the tree
+// is eight FP64 operations a lane, 16 clocks each)
+__device__ __forceinline__ void warp_sum_comp(double &s, double &c, int width = 32) {
+  for (int o = width >> 1; o > 0; o >>= 1) {
     const double s2 = __shfl_xor_sync(0xffffffffu, s, o);
     const double c2 = __shfl_xor_sync(0xffffffffu, c, o);
     double t, e;
@@ -563,7 +564,7 @@ __global__ void pair_reduce_kernel(const double *__restrict__ part, int nper, co
     s = t;
     c += e;
   }
-  warp_sum_comp(s, c);
+  warp_sum_comp(s, c, tree_width(nper));
   if (lane == 0) {
     const double v = s + c;
     const int i = pairs[2 * p], j = pairs[2 * p + 1];
@@ -638,7 +639,7 @@ __global__ void pair_reduce_plain_batch_kernel(const PlainFrag *__restrict__ fr,
     s = t;
     c += e;
   }
-  warp_sum_comp(s, c);
+  warp_sum_comp(s, c, tree_width(F.ntp));
   if (lane == 0) {
     int i, j;
     decode_pair_ij(p, i, j);

@@ -296,16 +296,11 @@ __device__ __forceinline__ int col_scale_exponent(unsigned long long mxb, float 
 // beside the current group's energy kernel.  (A single-pass form holding the
 // column in registers was measured slower: a 12 KB column took ~40 KB of
 // register file, leaving too few columns in flight per SM.)
-__global__ void __launch_bounds__(256, 6)
-    slice_batch_kernel(const FragDesc *__restrict__ fr, int nsl, long long plane,
-                                   __half *__restrict__ slices, float *__restrict__ inv_scale,
-                                   int col0, int col1, int vplane = 0,
-                                   float *__restrict__ dcorr = nullptr) {
-  // columns [col0, min(col1, ncol)) of each fragment
-  const FragDesc &F = fr[blockIdx.y];
-  const int col = col0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+__device__ __forceinline__ void slice_column(const FragDesc &F, int col, int nsl, long long plane,
+                                             __half *__restrict__ slices,
+                                             float *__restrict__ inv_scale, int vplane,
+                                             float *__restrict__ dcorr) {
   const int lane = threadIdx.x & 31;
-  if (col >= F.ncol || col >= col1) return;
   const int a = col % F.nvpad, i = col / F.nvpad;
   const int Kpad = F.nks * 64;
   const __half hz = __float2half_rn(0.0f);
@@ -400,11 +395,21 @@ __global__ void __launch_bounds__(256, 6)
   if (lane == 0) inv_scale[F.col_base + col] = ldexpf(1.0f, -e);
 }
 
+__global__ void __launch_bounds__(256, 6)
+    slice_batch_kernel(const FragDesc *__restrict__ fr, int nsl, long long plane,
+                                   __half *__restrict__ slices, float *__restrict__ inv_scale,
+                                   int col0, int col1, int vplane = 0,
+                                   float *__restrict__ dcorr = nullptr) {
+  // columns [col0, min(col1, ncol)) of each fragment
+  const FragDesc &F = fr[blockIdx.y];
+  const int col = col0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (col >= F.ncol || col >= col1) return;
+  slice_column(F, col, nsl, plane, slices, inv_scale, vplane, dcorr);
+}
+
 // orbital energies as hi/lo float pairs (padded virtuals get a large value so
 // their denominators stay finite; their g is exactly zero). grid.y = fragment
-__global__ void eps_batch_kernel(const FragDesc *__restrict__ fr, float2 *eo2, float2 *ev2) {
-  const FragDesc &F = fr[blockIdx.y];
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void eps_entry(const FragDesc &F, int t, float2 *eo2, float2 *ev2) {
   if (t < F.nocc) {
     const double v = F.eo[t];
     const float h = (float)v;
@@ -417,21 +422,29 @@ __global__ void eps_batch_kernel(const FragDesc *__restrict__ fr, float2 *eo2, f
   }
 }
 
+__global__ void eps_batch_kernel(const FragDesc *__restrict__ fr, float2 *eo2, float2 *ev2) {
+  eps_entry(fr[blockIdx.y], blockIdx.x * blockDim.x + threadIdx.x, eo2, ev2);
+}
+
 // Work items in queue order: fragments are enumerated heaviest first (the
 // host orders the descriptors by K length), pairs j-major, tile pairs
 // B-major.  item = {fragment, i | j<<16, tA | tB<<16, item id}.
-__global__ void build_items_kernel(const FragDesc *__restrict__ fr, int nfrag, long long nitems,
-                                   int4 *__restrict__ items) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= nitems) return;
-  const int f = find_frag_item(fr, nfrag, t);
-  const FragDesc &F = fr[f];
+// Work item t of fragment f.
+__device__ __forceinline__ int4 work_item(const FragDesc &F, int f, long long t) {
   const long long loc = t - F.item_base;
   const int p = (int)(loc / F.ntp), q = (int)(loc % F.ntp);
   int i, j, tA, tB;
   decode_pair(p, i, j);
   decode_tri(q, tA, tB);
-  items[t] = make_int4(f, i | (j << 16), tA | (tB << 16), (int)t);
+  return make_int4(f, i | (j << 16), tA | (tB << 16), (int)t);
+}
+
+__global__ void build_items_kernel(const FragDesc *__restrict__ fr, int nfrag, long long nitems,
+                                   int4 *__restrict__ items) {
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= nitems) return;
+  const int f = find_frag_item(fr, nfrag, t);
+  items[t] = work_item(fr[f], f, t);
 }
 
 struct BatchParams {
@@ -1324,6 +1337,21 @@ __host__ __device__ inline long long pair_items_before(long long j) {
   return (j % 2 == 0) ? m * (m + 1) : (m + 1) * (m + 1);
 }
 
+// Pair item t of fragment f.
+__device__ __forceinline__ int4 pair_item(const FragDesc &F, int f, long long t) {
+  const long long loc = t - F.pitem_base;
+  const long long p2 = loc / F.ntp;
+  const int q = (int)(loc % F.ntp);
+  int j = (int)(2.0 * sqrt((double)p2));
+  if (j > F.nocc - 1) j = F.nocc - 1;
+  while (j > 0 && pair_items_before(j) > p2) --j;
+  while (j + 1 < F.nocc && pair_items_before(j + 1) <= p2) ++j;
+  const int i0 = (int)(2 * (p2 - pair_items_before(j)));
+  int tA, tB;
+  decode_tri(q, tA, tB);
+  return make_int4(f, i0 | (j << 16), tA | (tB << 16), q);
+}
+
 __global__ void build_pair_items_kernel(const FragDesc *__restrict__ fr, int nfrag,
                                         long long nitems, int4 *__restrict__ items) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -1336,18 +1364,7 @@ __global__ void build_pair_items_kernel(const FragDesc *__restrict__ fr, int nfr
     else
       hi = mid - 1;
   }
-  const FragDesc &F = fr[lo];
-  const long long loc = t - F.pitem_base;
-  const long long p2 = loc / F.ntp;
-  const int q = (int)(loc % F.ntp);
-  int j = (int)(2.0 * sqrt((double)p2));
-  if (j > F.nocc - 1) j = F.nocc - 1;
-  while (j > 0 && pair_items_before(j) > p2) --j;
-  while (j + 1 < F.nocc && pair_items_before(j + 1) <= p2) ++j;
-  const int i0 = (int)(2 * (p2 - pair_items_before(j)));
-  int tA, tB;
-  decode_tri(q, tA, tB);
-  items[t] = make_int4(lo, i0 | (j << 16), tA | (tB << 16), q);
+  items[t] = pair_item(fr[lo], lo, t);
 }
 
 // ==========================================================================
@@ -1780,9 +1797,9 @@ __device__ __forceinline__ void two_sum_d(double a, double b, double &s, double 
   e = (a - (s - bb)) + (b - bb);
 }
 
-__device__ __forceinline__ void warp_sum_comp_d(double &s, double &c) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+// width: a power of two, the lanes from it on hold zeros
+__device__ __forceinline__ void warp_sum_comp_d(double &s, double &c, int width = 32) {
+  for (int o = width >> 1; o > 0; o >>= 1) {
     const double s2 = __shfl_xor_sync(0xffffffffu, s, o);
     const double c2 = __shfl_xor_sync(0xffffffffu, c, o);
     double t, e;
@@ -1819,7 +1836,7 @@ __global__ void pair_reduce_batch_kernel(const FragDesc *__restrict__ fr, int nf
     s = t;
     c += e;
   }
-  warp_sum_comp_d(s, c);
+  warp_sum_comp_d(s, c, tree_width(F.ntp));
   if (lane == 0) {
     int i, j;
     decode_pair(p, i, j);
@@ -1857,6 +1874,93 @@ __global__ void total_reduce_batch_kernel(const FragDesc *__restrict__ fr) {
   }
 }
 
+// One fragment: everything before the energy kernel in one launch (slices, the
+// descriptor, orbital energies, work items, counters), and both reductions in
+// one.  A small call is bound by its launches: seven kernels, a memset and a
+// copy took 50 us of GPU time at nocc = 8, nvirt = 96, NBA = 256.
+struct SingleArgs {
+  FragDesc F;
+  FragDesc *frag;
+  int slice_blocks, nsl, vplane, nitems, npitems;
+  long long plane;
+  __half *slices;
+  float *inv, *dcorr;
+  float2 *eo2, *ev2;
+  int4 *items, *pitems;
+  unsigned *queue;  // item counter, reduction blocks done
+  double *part;
+};
+
+__global__ void __launch_bounds__(256, 6) single_inputs_kernel(const __grid_constant__ SingleArgs P) {
+  if ((int)blockIdx.x < P.slice_blocks) {
+    const int col = (blockIdx.x * 256 + threadIdx.x) >> 5;
+    if (col < P.F.ncol) slice_column(P.F, col, P.nsl, P.plane, P.slices, P.inv, P.vplane, P.dcorr);
+    return;
+  }
+  const int t = ((int)blockIdx.x - P.slice_blocks) * 256 + threadIdx.x;
+  if (t == 0) {
+    *P.frag = P.F;
+    P.queue[0] = P.queue[1] = 0;
+  }
+  eps_entry(P.F, t, P.eo2, P.ev2);
+  if (t < P.nitems) P.items[t] = work_item(P.F, 0, t);
+  if (t < P.npitems) P.pitems[t] = pair_item(P.F, 0, t);
+}
+
+// One warp per pair; the last block to finish sums the total.
+__global__ void __launch_bounds__(256) single_reduce_kernel(const __grid_constant__ SingleArgs P) {
+  __shared__ double ss[8], sc[8];
+  __shared__ bool last;
+  const FragDesc &F = P.F;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, p = blockIdx.x * 8 + w;
+  if (p < F.nocc * (F.nocc + 1) / 2) {
+    const double *src = P.part + (long long)p * F.ntp;
+    double s = 0.0, c = 0.0;
+    for (int r = lane; r < F.ntp; r += 32) {
+      double t, e;
+      two_sum_d(s, src[r], t, e);
+      s = t;
+      c += e;
+    }
+    warp_sum_comp_d(s, c, tree_width(F.ntp));
+    if (lane == 0) {
+      int i, j;
+      decode_pair(p, i, j);
+      const double v = s + c;
+      F.Epair[i + (size_t)F.nocc * j] = v;
+      F.Epair[j + (size_t)F.nocc * i] = v;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(P.queue + 1, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  const int n = F.nocc * F.nocc, nw = min(8, (n + 255) / 256);  // warps of the total
+  double s = 0.0, c = 0.0;
+  if (w < nw) {
+    for (int k = threadIdx.x; k < n; k += 32 * nw) {
+      double t, e;
+      two_sum_d(s, __ldcg(F.Epair + k), t, e);
+      s = t;
+      c += e;
+    }
+    warp_sum_comp_d(s, c);
+    if (lane == 0) {
+      ss[w] = s;
+      sc[w] = c;
+    }
+  }
+  __syncthreads();
+  if (w == 0) {
+    s = lane < nw ? ss[lane] : 0.0;
+    c = lane < nw ? sc[lane] : 0.0;
+    warp_sum_comp_d(s, c, tree_width(nw));
+    if (lane == 0) *F.Etot = s + c;
+  }
+}
+
 // --------------------------------------------------------------------------
 // host side
 // --------------------------------------------------------------------------
@@ -1874,6 +1978,7 @@ struct Group {
   std::vector<FragDesc> fh;
   long long nitems = 0, R = 0, ncol_total = 0;
   int npairs_total = 0, max_ncol = 0, max_nv = 0, max_nocc = 0;
+  DevBuf arena;  // the others are parts of it
   DevBuf frags, items, slices, inv, eo2, ev2, part, queue;
   CUtensorMap tm;
   // paired-CTA kernel (one residual slice): its pair items and B-half map
@@ -1917,7 +2022,7 @@ int launch_pair(const Group &g, PairParams Q, int npair, cudaStream_t s) {
   return RIMP2_OK;
 }
 
-int build_group(Group &g, cudaStream_t s) {
+int build_group(Group &g, cudaStream_t s, bool single = false) {
   // heaviest fragments first: their items lead the queue
   std::stable_sort(g.fh.begin(), g.fh.end(),
                    [](const FragDesc &x, const FragDesc &y) { return x.nks > y.nks; });
@@ -1963,21 +2068,37 @@ int build_group(Group &g, cudaStream_t s) {
     return RIMP2_ERR_ARG;
   }
   const int planes = g.nsl + (g.pair ? 1 : 0);  // the paired kernel adds the V plane
-  RIMP2_TRY(g.frags.alloc(sizeof(FragDesc) * g.nfrag, s));
-  RIMP2_TRY(g.items.alloc(sizeof(int4) * (size_t)g.nitems, s));
-  RIMP2_TRY(g.slices.alloc(sizeof(__half) * (size_t)planes * (size_t)g.R * 64, s));
-  RIMP2_TRY(g.inv.alloc(sizeof(float) * (size_t)g.ncol_total, s));
-  if (g.pair) RIMP2_TRY(g.dcorr.alloc(sizeof(float) * (size_t)g.ncol_total, s));
-  RIMP2_TRY(g.eo2.alloc(sizeof(float2) * (size_t)eo, s));
-  RIMP2_TRY(g.ev2.alloc(sizeof(float2) * (size_t)ev, s));
-  RIMP2_TRY(g.part.alloc(sizeof(double) * (size_t)g.nitems, s));
-  RIMP2_TRY(g.queue.alloc(sizeof(unsigned int), s));
-  RIMP2_CK(cudaMemcpyAsync(g.frags.p, g.fh.data(), sizeof(FragDesc) * g.nfrag,
-                           cudaMemcpyHostToDevice, s));
-  build_items_kernel<<<(unsigned)((g.nitems + 255) / 256), 256, 0, s>>>(
-      g.frags.as<FragDesc>(), g.nfrag, g.nitems, g.items.as<int4>());
-  count_launch(1);
-  RIMP2_CK(cudaGetLastError());
+  // one allocation, divided (ten of them were a third of a small call's host time)
+  {
+    DevBuf *buf[] = {&g.slices, &g.frags, &g.items, &g.pitems, &g.inv, &g.dcorr,
+                     &g.eo2,    &g.ev2,   &g.part,  &g.queue};
+    const size_t bytes[] = {sizeof(__half) * (size_t)planes * (size_t)g.R * 64,
+                            sizeof(FragDesc) * g.nfrag,
+                            single && g.pair ? 16 : sizeof(int4) * (size_t)g.nitems,
+                            g.pair ? sizeof(int4) * (size_t)g.npitems : 16,
+                            sizeof(float) * (size_t)g.ncol_total,
+                            g.pair ? sizeof(float) * (size_t)g.ncol_total : 16,
+                            sizeof(float2) * (size_t)eo,
+                            sizeof(float2) * (size_t)ev,
+                            sizeof(double) * (size_t)g.nitems,
+                            2 * sizeof(unsigned int)};
+    size_t total = 0;
+    for (size_t n : bytes) total += (n + 255) / 256 * 256;
+    RIMP2_TRY(g.arena.alloc(total, s));
+    char *at = g.arena.as<char>();
+    for (int k = 0; k < 10; ++k) {
+      buf[k]->alias(at, bytes[k], s);
+      at += (bytes[k] + 255) / 256 * 256;
+    }
+  }
+  if (!single) {
+    RIMP2_CK(cudaMemcpyAsync(g.frags.p, g.fh.data(), sizeof(FragDesc) * g.nfrag,
+                             cudaMemcpyHostToDevice, s));
+    build_items_kernel<<<(unsigned)((g.nitems + 255) / 256), 256, 0, s>>>(
+        g.frags.as<FragDesc>(), g.nfrag, g.nitems, g.items.as<int4>());
+    count_launch(1);
+    RIMP2_CK(cudaGetLastError());
+  }
   auto encode = get_encode();
   if (!encode) {
     set_error("cuTensorMapEncodeTiled entry point unavailable");
@@ -1994,10 +2115,11 @@ int build_group(Group &g, cudaStream_t s) {
     set_error("cuTensorMapEncodeTiled failed (%d)", (int)cr);
     return RIMP2_ERR_CUDA;
   }
-  auto k2 = split_batch_kernel<2, 3>;
-  auto k3 = split_batch_kernel<3, 2>;
-  RIMP2_CK(cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(2, 3)));
-  RIMP2_CK(cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(3, 2)));
+  if (!g.pair) {
+    auto k = g.nsl == 2 ? split_batch_kernel<2, 3> : split_batch_kernel<3, 2>;
+    RIMP2_CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  smem_bytes(g.nsl, g.nsl == 2 ? 3 : 2)));
+  }
   if (g.pair) {
     g.pair_nstage = pair_stages_for(g.fh);
     if (g.pair_nstage == 4) {
@@ -2021,7 +2143,7 @@ int build_group(Group &g, cudaStream_t s) {
       set_error("cuTensorMapEncodeTiled failed (%d)", (int)cr);
       return RIMP2_ERR_CUDA;
     }
-    RIMP2_TRY(g.pitems.alloc(sizeof(int4) * (size_t)g.npitems, s));
+    if (single) return RIMP2_OK;
     build_pair_items_kernel<<<(unsigned)((g.npitems + 255) / 256), 256, 0, s>>>(
         g.frags.as<FragDesc>(), g.nfrag, g.npitems, g.pitems.as<int4>());
     count_launch(1);
@@ -2048,13 +2170,39 @@ int record_group_inputs(Group &g, cudaStream_t s) {
 
 // Enqueue one evaluation of the group on s (graph-capturable: no sync, no
 // alloc); with_inputs = false when its inputs were enqueued elsewhere.
+// single: a group of one fragment whose inputs and reductions take one launch each
 int record_group(Group &g, cudaStream_t s, int nsm, cudaEvent_t *ev /* 3 or null */,
-                 bool with_inputs = true) {
+                 bool with_inputs = true, bool single = false) {
   if (g.nfrag == 0) return RIMP2_OK;
   const FragDesc *fr = g.frags.as<FragDesc>();
   if (ev) RIMP2_CK(cudaEventRecord(ev[0], s));
-  if (with_inputs) RIMP2_TRY(record_group_inputs(g, s));
-  RIMP2_CK(cudaMemsetAsync(g.queue.p, 0, sizeof(unsigned int), s));
+  SingleArgs A;
+  if (single) {
+    A.F = g.fh[0];
+    A.frag = g.frags.as<FragDesc>();
+    A.slice_blocks = (int)((g.max_ncol * 32LL + 255) / 256);
+    A.nsl = g.nsl;
+    A.vplane = g.pair ? 1 : 0;
+    A.nitems = g.pair ? 0 : (int)g.nitems;
+    A.npitems = g.pair ? (int)g.npitems : 0;
+    A.plane = g.R * 64;
+    A.slices = g.slices.as<__half>();
+    A.inv = g.inv.as<float>();
+    A.dcorr = g.dcorr.as<float>();
+    A.eo2 = g.eo2.as<float2>();
+    A.ev2 = g.ev2.as<float2>();
+    A.items = g.items.as<int4>();
+    A.pitems = g.pitems.as<int4>();
+    A.queue = g.queue.as<unsigned>();
+    A.part = g.part.as<double>();
+    const int rest = std::max(std::max(A.nitems, A.npitems), g.max_nv);
+    single_inputs_kernel<<<(unsigned)(A.slice_blocks + (rest + 255) / 256), 256, 0, s>>>(A);
+    count_launch(1);
+    RIMP2_CK(cudaGetLastError());
+  } else {
+    if (with_inputs) RIMP2_TRY(record_group_inputs(g, s));
+    RIMP2_CK(cudaMemsetAsync(g.queue.p, 0, sizeof(unsigned int), s));
+  }
   BatchParams P;
   P.frags = fr;
   P.items = g.items.as<int4>();
@@ -2097,6 +2245,12 @@ int record_group(Group &g, cudaStream_t s, int nsm, cudaEvent_t *ev /* 3 or null
   }
   count_launch(1);
   if (ev) RIMP2_CK(cudaEventRecord(ev[2], s));
+  if (single) {
+    single_reduce_kernel<<<(unsigned)((g.npairs_total + 7) / 8), 256, 0, s>>>(A);
+    count_launch(1);
+    RIMP2_CK(cudaGetLastError());
+    return RIMP2_OK;
+  }
   pair_reduce_batch_kernel<<<(unsigned)((g.npairs_total + 7) / 8), 256, 0, s>>>(
       fr, g.nfrag, g.npairs_total, g.part.as<double>());
   total_reduce_batch_kernel<<<g.nfrag, total_threads(g.max_nocc), 0, s>>>(fr);
@@ -3873,13 +4027,45 @@ int split_eos_energy(const double *Ca, const double *Ct, int NBA, int nvirt, int
 
 int split_energy(const SplitEnergyArgs &a, cudaStream_t s, float *ms_kernel) {
   (void)ms_kernel;
-  SplitPlan *P = nullptr;
-  const int ns = a.nslices;
-  RIMP2_TRY(split_plan_create(&P, 1, &a.nocc, &a.nvirt, &a.NBA, &a.Ca, &a.eo, &a.ev, &a.Epair,
-                              &a.Etot, &ns, false, s));
-  int rc = split_plan_execute(P, s);
-  split_plan_destroy(P);  // workspace is released stream-ordered
-  return rc;
+  // work items pack i | j << 16 and tA | tB << 16
+  if (a.nocc > 65535 || (a.nvirt + TILE - 1) / TILE > 65535) {
+    set_error("split form: fragment 0 too large for the work-item encoding (nocc=%d)", a.nocc);
+    return RIMP2_ERR_ARG;
+  }
+  int dev = 0, nsm = 0;
+  RIMP2_CK(cudaGetDevice(&dev));
+  RIMP2_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  Group g;
+  g.nsl = a.nslices >= 2 ? 3 : 2;
+  g.pair = a.nslices < 2 && pair_kernel_for(a.nocc, a.nvirt, a.NBA);
+  FragDesc F;
+  memset(&F, 0, sizeof F);
+  F.nocc = a.nocc;
+  F.nvirt = a.nvirt;
+  F.NBA = a.NBA;
+  F.Ca = a.Ca;
+  F.eo = a.eo;
+  F.ev = a.ev;
+  F.Epair = a.Epair;
+  F.Etot = a.Etot;
+  g.fh.push_back(F);
+  RIMP2_TRY(build_group(g, s, true));  // its workspace is released stream-ordered
+  const bool timed = timing_enabled();
+  cudaEvent_t ev[4];
+  if (timed)
+    for (int k = 0; k < 4; ++k) RIMP2_CK(cudaEventCreate(&ev[k]));
+  RIMP2_TRY(record_group(g, s, nsm, timed ? ev : nullptr, true, true));
+  if (timed) {
+    RIMP2_CK(cudaEventRecord(ev[3], s));
+    RIMP2_CK(cudaEventSynchronize(ev[3]));
+    float ms;
+    for (int k = 0; k < 3; ++k) {
+      RIMP2_CK(cudaEventElapsedTime(&ms, ev[k], ev[k + 1]));
+      record_timing(k, ms);
+    }
+    for (int k = 0; k < 4; ++k) cudaEventDestroy(ev[k]);
+  }
+  return RIMP2_OK;
 }
 
 }  // namespace rimp2
