@@ -414,34 +414,29 @@ int dev_transalpha2_strided(int n2, int n1, int n3, int nba, const double *U, lo
   return launch_gemm_f64(g, s);
 }
 
-// max |P(i,j) - delta_ij| over an n x n matrix (one block)
-__global__ void identity_dev_kernel(const double *P, int n, double *out) {
-  __shared__ double red[32];
-  double m = 0.0;
+// out = max |P(i,j) - delta_ij| over an n x n matrix (out zero before; the bits
+// of non-negative doubles order like integers; NaN counts as the largest)
+__global__ void identity_dev_kernel(const double *P, int n, unsigned long long *out) {
+  unsigned long long m = 0;
   const long long nn = (long long)n * n;
-  for (long long t = threadIdx.x; t < nn; t += blockDim.x) {
-    const long long i = t % n, j = t / n;
-    m = fmax(m, fabs(P[t] - (i == j ? 1.0 : 0.0)));
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < nn;
+       t += (long long)gridDim.x * blockDim.x) {
+    const double d = fabs(P[t] - (t % n == t / n ? 1.0 : 0.0));
+    const unsigned long long b = (unsigned long long)__double_as_longlong(d);
+    m = b > m ? b : m;
   }
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double r = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r = fmax(r, red[w]);
-    *out = r;
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long b = __shfl_xor_sync(0xffffffffu, m, o);
+    m = b > m ? b : m;
   }
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(out, m);
 }
 
-// true if P = I within 1e-13 (P on the device; synchronises s)
-int is_identity(const double *P, int n, double *dwork, bool *yes, cudaStream_t s) {
-  identity_dev_kernel<<<1, 1024, 0, s>>>(P, n, dwork);
+int identity_deviation(const double *P, int n, double *out, cudaStream_t s) {
+  const long long blocks = std::min<long long>(304, ((long long)n * n + 1023) / 1024);
+  identity_dev_kernel<<<(unsigned)blocks, 256, 0, s>>>(P, n, reinterpret_cast<unsigned long long *>(out));
   count_launch(1);
   RIMP2_CK(cudaGetLastError());
-  double h = 1.0;
-  RIMP2_CK(cudaMemcpyAsync(&h, dwork, sizeof h, cudaMemcpyDeviceToHost, s));
-  RIMP2_CK(cudaStreamSynchronize(s));
-  *yes = (h <= 1e-13);
   return RIMP2_OK;
 }
 
@@ -875,7 +870,7 @@ int rimp2_energy_eos(const int *nvirt_, const int *nocc_, const int *noccEOS_,
   const int nvirt = *nvirt_, nocc = *nocc_, noccEOS = *noccEOS_, nvirtEOS = *nvirtEOS_,
             NBA = *NBA_;
   const size_t nv = nvirt, no = nocc, ne = noccEOS, ve = nvirtEOS, nb = NBA;
-  DevBuf dC, deo, dev, dUoE, dUvT, dUoT, dUvE, Po, Pv, C1, C2, D1, Ct, Ep, Et, wk;
+  DevBuf dC, deo, dev, dUoE, dUvT, dUoT, dUvE, Ep, Et, wk, C2[2], Ct[2];
   RIMP2_TRY(h2d(dC, Calpha, nb * nv * no, s));
   RIMP2_TRY(h2d(deo, EVocc, no, s));
   RIMP2_TRY(h2d(dev, EVvirt, nv, s));
@@ -883,63 +878,86 @@ int rimp2_energy_eos(const int *nvirt_, const int *nocc_, const int *noccEOS_,
   RIMP2_TRY(h2d(dUvT, UvirtT, nv * nv, s));
   RIMP2_TRY(h2d(dUoT, UoccT, no * no, s));
   RIMP2_TRY(h2d(dUvE, UvirtEOST, nv * ve, s));
-  const int kmax = std::max(noccEOS, nocc), vmax = std::max(nvirtEOS, nvirt);
-  RIMP2_TRY(dalloc(Po, no * no, s));
-  RIMP2_TRY(dalloc(Pv, nv * nv, s));
-  RIMP2_TRY(dalloc(C1, nb * nv * (size_t)kmax, s));
-  RIMP2_TRY(dalloc(C2, nb * nv * no, s));
-  RIMP2_TRY(dalloc(D1, nb * (size_t)vmax * no, s));
-  RIMP2_TRY(dalloc(Ct, nb * nv * no, s));
   RIMP2_TRY(dalloc(Ep, no * no, s));
   RIMP2_TRY(dalloc(Et, 2, s));
-  RIMP2_TRY(dalloc(wk, 1, s));
+  RIMP2_TRY(dalloc(wk, 4, s));
   const double *Uo[2] = {dUoE.as<double>(), dUoT.as<double>()};
   const double *Uv[2] = {dUvT.as<double>(), dUvE.as<double>()};
   const int ko[2] = {noccEOS, nocc}, kv[2] = {nvirt, nvirtEOS};
   const long long MV = (long long)NBA * nvirt;
+  // projectors of more than half rank: the identity (orthogonal U) is left
+  // out; all of them are looked at before the host waits once
+  DevBuf Po[2], Pv[2];
+  bool ido[2] = {false, false}, idv[2] = {false, false};
+  {
+    double dev4[4] = {1.0, 1.0, 1.0, 1.0};
+    RIMP2_CK(cudaMemsetAsync(wk.p, 0, 4 * sizeof(double), s));
+    for (int part = 0; part < 2; ++part) {
+      if (2 * ko[part] > nocc) {
+        RIMP2_TRY(dalloc(Po[part], no * no, s));
+        RIMP2_TRY(dev_dgemm('N', 'T', nocc, nocc, ko[part], 1.0, Uo[part], nocc, Uo[part], nocc, 0.0,
+                            Po[part].as<double>(), nocc, s));
+        RIMP2_TRY(identity_deviation(Po[part].as<double>(), nocc, wk.as<double>() + 2 * part, s));
+      }
+      if (2 * kv[part] > nvirt) {
+        RIMP2_TRY(dalloc(Pv[part], nv * nv, s));
+        RIMP2_TRY(dev_dgemm('N', 'T', nvirt, nvirt, kv[part], 1.0, Uv[part], nvirt, Uv[part], nvirt,
+                            0.0, Pv[part].as<double>(), nvirt, s));
+        RIMP2_TRY(identity_deviation(Pv[part].as<double>(), nvirt, wk.as<double>() + 2 * part + 1, s));
+      }
+    }
+    RIMP2_CK(cudaMemcpyAsync(dev4, wk.p, sizeof dev4, cudaMemcpyDeviceToHost, s));
+    RIMP2_CK(cudaStreamSynchronize(s));
+    for (int part = 0; part < 2; ++part) {
+      ido[part] = Po[part].p && dev4[2 * part] <= 1e-13;
+      idv[part] = Pv[part].p && dev4[2 * part + 1] <= 1e-13;
+    }
+  }
+  const double *ct[2];
   for (int part = 0; part < 2; ++part) {
     // occupied side: C2(:,c,i) = sum_k Calpha(:,c,k) Po(k,i), Po = Uo Uo^T
-    const double *c2 = C2.as<double>();
-    if (2 * ko[part] <= nocc) {  // low rank: (Calpha Uo) Uo^T
+    const double *c2 = dC.as<double>();
+    if (!Po[part].p) {  // low rank: (Calpha Uo) Uo^T
+      DevBuf C1;
+      RIMP2_TRY(dalloc(C1, nb * nv * (size_t)ko[part], s));
+      RIMP2_TRY(dalloc(C2[part], nb * nv * no, s));
       RIMP2_TRY(dev_dgemm('N', 'N', (int)MV, ko[part], nocc, 1.0, dC.as<double>(), (int)MV,
                           Uo[part], nocc, 0.0, C1.as<double>(), (int)MV, s));
       RIMP2_TRY(dev_dgemm('N', 'T', (int)MV, nocc, ko[part], 1.0, C1.as<double>(), (int)MV,
-                          Uo[part], nocc, 0.0, C2.as<double>(), (int)MV, s));
-    } else {
-      RIMP2_TRY(dev_dgemm('N', 'T', nocc, nocc, ko[part], 1.0, Uo[part], nocc, Uo[part], nocc, 0.0,
-                          Po.as<double>(), nocc, s));
-      bool id = false;
-      RIMP2_TRY(is_identity(Po.as<double>(), nocc, wk.as<double>(), &id, s));
-      if (id)
-        c2 = dC.as<double>();  // orthogonal Uo: Po = I
-      else
-        RIMP2_TRY(dev_dgemm('N', 'N', (int)MV, nocc, nocc, 1.0, dC.as<double>(), (int)MV,
-                            Po.as<double>(), nocc, 0.0, C2.as<double>(), (int)MV, s));
+                          Uo[part], nocc, 0.0, C2[part].as<double>(), (int)MV, s));
+      c2 = C2[part].as<double>();
+    } else if (!ido[part]) {
+      RIMP2_TRY(dalloc(C2[part], nb * nv * no, s));
+      RIMP2_TRY(dev_dgemm('N', 'N', (int)MV, nocc, nocc, 1.0, dC.as<double>(), (int)MV,
+                          Po[part].as<double>(), nocc, 0.0, C2[part].as<double>(), (int)MV, s));
+      c2 = C2[part].as<double>();
     }
     // virtual side: Ct(:,a,i) = sum_c Pv(c,a) C2(:,c,i), Pv = Uv Uv^T
-    const double *ct = Ct.as<double>();
-    if (2 * kv[part] <= nvirt) {  // low rank: Uv (Uv^T C2)
+    ct[part] = c2;
+    if (!Pv[part].p) {  // low rank: Uv (Uv^T C2)
+      DevBuf D1;
+      RIMP2_TRY(dalloc(D1, nb * (size_t)kv[part] * no, s));
+      RIMP2_TRY(dalloc(Ct[part], nb * nv * no, s));
       RIMP2_TRY(dev_transalpha2(nocc, nvirt, kv[part], NBA, Uv[part], c2, D1.as<double>(), s));
       RIMP2_TRY(dev_transalpha2_strided(nocc, kv[part], nvirt, NBA, Uv[part], nvirt, 1,
-                                        D1.as<double>(), Ct.as<double>(), s));
-    } else {
-      RIMP2_TRY(dev_dgemm('N', 'T', nvirt, nvirt, kv[part], 1.0, Uv[part], nvirt, Uv[part], nvirt,
-                          0.0, Pv.as<double>(), nvirt, s));
-      bool id = false;
-      RIMP2_TRY(is_identity(Pv.as<double>(), nvirt, wk.as<double>(), &id, s));
-      if (id)
-        ct = c2;  // orthogonal Uv: Pv = I
-      else
-        RIMP2_TRY(dev_transalpha2(nocc, nvirt, nvirt, NBA, Pv.as<double>(), c2, Ct.as<double>(),
-                                  s));
+                                        D1.as<double>(), Ct[part].as<double>(), s));
+      ct[part] = Ct[part].as<double>();
+      C2[part].release();
+    } else if (!idv[part]) {
+      RIMP2_TRY(dalloc(Ct[part], nb * nv * no, s));
+      RIMP2_TRY(dev_transalpha2(nocc, nvirt, nvirt, NBA, Pv[part].as<double>(), c2,
+                                Ct[part].as<double>(), s));
+      ct[part] = Ct[part].as<double>();
+      C2[part].release();
     }
-    const int ns = rimp2_split_nslices(nvirt, nocc, NBA);
-    if (*precision == RIMP2_PREC_SPLIT && ns > 0)
-      RIMP2_TRY(split_eos_energy(dC.as<double>(), ct, NBA, nvirt, nocc, deo.as<double>(),
-                                 dev.as<double>(), Ep.as<double>(), Et.as<double>() + part,
-                                 ns, s));
-    else
-      RIMP2_TRY(eos_energy_f64(dC.as<double>(), ct, NBA, nvirt, nocc, deo.as<double>(),
+  }
+  const int ns = rimp2_split_nslices(nvirt, nocc, NBA);
+  if (*precision == RIMP2_PREC_SPLIT && ns > 0) {
+    RIMP2_TRY(split_eos_energy(dC.as<double>(), ct, 2, NBA, nvirt, nocc, deo.as<double>(),
+                               dev.as<double>(), Ep.as<double>(), Et.as<double>(), ns, s));
+  } else {
+    for (int part = 0; part < 2; ++part)
+      RIMP2_TRY(eos_energy_f64(dC.as<double>(), ct[part], NBA, nvirt, nocc, deo.as<double>(),
                                dev.as<double>(), Ep.as<double>(), Et.as<double>() + part, s));
   }
   double h[2];

@@ -1371,14 +1371,15 @@ __global__ void build_pair_items_kernel(const FragDesc *__restrict__ fr, int nfr
 // Local-orbital fragment energy on the tensor cores (split form):
 //   sum_ij,ab g_ij^ab / D (2 gt_ij^ab - gt_ij^ba),
 // g from Calpha C, gt from its projected copy Ct (both sliced like Calpha).
+// Two residual slices run here, one residual slice on split_eos_pair_kernel.
 // Work item = (pair i<=j, tile pair A<=B, column half h): rows a in block A
 // (128), columns b in the h-th 64-column half of block B.  Four 128x64 tiles
 // per item: T1 = C_iA^T C_jB, T2 = C_jA^T C_iB, U1 = Ct_iA^T Ct_jB,
 // U2 = Ct_jA^T Ct_iB, each with L0/L1 accumulators: 8 x 64 = 512 TMEM columns.
 // Diagonal tile pairs compute T2/U2 too (no transpose), so each ordered (a,b)
 // of A x A is met once over the two halves; i = j reuses T1/U1.
-// Roles as in split_batch_kernel; the MMA issuer waits for the epilogue to
-// free all four tiles before the next item (no accumulator double-buffer).
+// Roles as in split_batch_kernel; a tile's accumulators are free for the next
+// item once the epilogue has read them.
 // --------------------------------------------------------------------------
 constexpr int HALF = 64;
 constexpr int HPANEL_BYTES = HALF * KSTEP * 2;  // 8 KB
@@ -1392,15 +1393,10 @@ struct EosParams {
   int *err;
   int nocc, nvirt, nvpad, nks, ntp, ncol;
   int rowC, rowCt;           // first slice row of C and of Ct (per plane)
-  const float *dcorr;        // one residual slice: per column sum_k R1 (V - S0 - R1)
 };
 
-// One residual slice adds the V plane (three products per element pair, as
-// in split_pair_kernel): a stage holds S0a, R1a (128 rows) and S0b, R1b, Vb
-// (64 rows).
-constexpr int eos_stage_bytes(int nsl) {
-  return nsl * PANEL_BYTES + (nsl + (nsl == 2 ? 1 : 0)) * HPANEL_BYTES;
-}
+// A stage holds S0a, R1a, R2a (128 rows) and S0b, R1b, R2b (64 rows).
+constexpr int eos_stage_bytes(int nsl) { return nsl * (PANEL_BYTES + HPANEL_BYTES); }
 
 __device__ __forceinline__ void eos_decode(const EosParams &P, long long id, int &i, int &j,
                                            int &tA, int &tB, int &h) {
@@ -1417,7 +1413,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
                      EosParams P) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  constexpr bool VP = (NSL == 2);  // V plane: R1a S0b + R1a R1b folded into R1a V
   constexpr int STAGE_BYTES = eos_stage_bytes(NSL);
   constexpr int NEPI = 8;
   uint8_t *stages = base;
@@ -1517,9 +1512,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
               tma_load_3d(dst + NSL * PANEL_BYTES + sl * HPANEL_BYTES, &tmB, fb, 0, rowk + colB,
                           sl);
             }
-            if (VP)
-              tma_load_3d(dst + NSL * PANEL_BYTES + NSL * HPANEL_BYTES, &tmB, fb, 0, rowk + colB,
-                          NSL);  // V
             if (++stage == NSTAGE) {
               stage = 0;
               phase ^= 1;
@@ -1588,10 +1580,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
               const uint32_t acc = (kc > 0 || k16 > 0) ? 1u : 0u;
               // [L0 | L1] += S0a x [S0b; R1b]: exact integer part and S0a R1b
               mma_f16_id(dL0, a0, b0, idesc2, acc);
-              if (VP) {  // R1a V (= R1a S0b + R1a R1b + R1a eps)
-                mma_f16_id(dL1, a1, smem_desc(sbB + NSL * HPANEL_BYTES + koff), idesc, 1u);
-                continue;
-              }
               mma_f16_id(dL1, a1, b0, idesc, 1u);   // R1a S0b
               mma_f16_id(dL1, a1, b1, idesc, 1u);   // R1a R1b
               if (NSL > 2) {
@@ -1661,12 +1649,6 @@ __global__ void __launch_bounds__(NTHREADS, 1)
       const float bw = dh0 - sh;
       const float dl0 = ((sh - (dh0 - bw)) + (-ea.x - bw)) + (sl - ea.y);
       // one tile's 32 columns of this thread into registers, then release it
-      // g_ii(a,a) and gt_ii(a,a) of the one-residual (V plane) form carry the
-      // same-column bias sum_k R1 (V - S0 - R1): its column among the
-      // thread's 32 (or -1) and the two corrections, removed as T1/U1 are read
-      const int cd = (VP && same && diag && a - b0 >= 0 && a - b0 < 32) ? a - b0 : -1;
-      const float cg = cd >= 0 ? P.dcorr[i * P.nvpad + a] : 0.0f;
-      const float cu = cd >= 0 ? P.dcorr[P.ncol + i * P.nvpad + a] : 0.0f;
       auto take = [&](int t, const float *sr, float srow, float (&v)[32]) -> bool {
         const bool w = mbar_wait(tfull0 + 8 * t, (par >> t) & 1, abort_flag, P.err, 4);
         if (epi_any(!w)) return false;
@@ -1679,10 +1661,7 @@ __global__ void __launch_bounds__(NTHREADS, 1)
           tmem_wait_ld();
 #pragma unroll
           for (int k = 0; k < 16; ++k) {
-            float x = l0[k] + l1[k];
-            if (t == 0 && c0 + k == cd) x -= cg;
-            if (t == 2 && c0 + k == cd) x -= cu;
-            v[c0 + k] = x * (srow * sr[b0 + c0 + k]);
+            v[c0 + k] = (l0[k] + l1[k]) * (srow * sr[b0 + c0 + k]);
           }
         }
         tc_fence_before();
@@ -1751,6 +1730,409 @@ __global__ void __launch_bounds__(NTHREADS, 1)
   if (warp == 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+  }
+}
+
+// --------------------------------------------------------------------------
+// One residual slice (three products): CTA pairs, both partitionings at once.
+// The one-CTA form above moves 14 KB into shared memory and reads 14 KB of it
+// per K16 step of 96 MMA cycles, more than the 128 bytes a clock that memory
+// gives, so half the tensor time is lost; and it contracts Calpha with itself
+// once per partitioning.  Here a pair of CTAs takes 256 rows (virtual blocks
+// 2R and 2R+1 of one occupied pair) by a 128-column block, the columns'
+// operand split between the two as in split_pair_kernel, and runs through the
+// tiles T1, T2 of Calpha and U1, U2 of each projected copy in two alternating
+// 256-column accumulators; g (T1, T2) waits in a thread-private stash (L2)
+// for the tiles of both partitionings.  Products, their order and the energy
+// terms are the one-CTA form's.  Row blocks beyond the column block (the pair
+// (2R+1, 2R)) are a dummy's: 14% of the tiles at six blocks, 3% at 24.
+// Measured (GB300, nvirt 741, nocc 59, NBA 2173, both partitionings): 33.8 ms,
+// against 57.4 ms in two launches of the one-CTA form with the V plane.
+// --------------------------------------------------------------------------
+struct EosPairParams {
+  const float *inv;      // inverse scales [set][ncol]: Calpha, then the projected copies
+  const float *dcorr;    // [set][ncol]
+  const float2 *eo2, *ev2;
+  long long nitems, npart;
+  unsigned int *queue;
+  double *part;          // [copy][pair * ntp + tile pair], npart values each
+  float *stash;          // per CTA [2][64][256]
+  int *err;
+  int nvpad, nks, nt, ntp, per, ncol, copies;
+  int row0[3];           // first slice row of each set
+};
+
+// item -> occupied pair, row block, column block
+__device__ __forceinline__ void eos_pair_decode(const EosPairParams &P, long long id, int &i, int &j,
+                                                int &R, int &tB) {
+  decode_pair((int)(id / P.per), i, j);
+  int r = (int)(id % P.per);
+  R = 0;
+  while (r >= P.nt - 2 * R) {
+    r -= P.nt - 2 * R;
+    ++R;
+  }
+  tB = 2 * R + r;
+}
+
+constexpr int EP_NSTAGE = 3;
+constexpr int EP_SMEM = EP_NSTAGE * PAIR_STAGE_BYTES + 1024 + 512;
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
+    split_eos_pair_kernel(const __grid_constant__ CUtensorMap tmA,
+                          const __grid_constant__ CUtensorMap tmB, EosPairParams P) {
+  constexpr int NSTAGE = EP_NSTAGE, STAGE_BYTES = PAIR_STAGE_BYTES, NEPI = 8;
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint8_t *stages = base;
+  uint64_t *bars = (uint64_t *)(base + NSTAGE * STAGE_BYTES);
+  // bars: full[NSTAGE], empty[NSTAGE], tfull[2], tempty[2], drain, item_full[IQ], item_empty[IQ]
+  constexpr int NB = 2 * NSTAGE + 5 + 2 * IQ;
+  uint32_t *tmem_slot = (uint32_t *)(bars + NB);
+  volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
+  volatile int *item_q = (volatile int *)(tmem_slot + 2);  // [IQ]
+  double *redd = (double *)(((uintptr_t)(tmem_slot + 2 + IQ) + 7) & ~(uintptr_t)7);  // [2][NEPI]
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  const bool leader = rank == 0;
+  const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[NSTAGE]);
+  const uint32_t tfull0 = smem_u32(&bars[2 * NSTAGE]), tempty0 = smem_u32(&bars[2 * NSTAGE + 2]);
+  const uint32_t drain = smem_u32(&bars[2 * NSTAGE + 4]);
+  const uint32_t ifull0 = smem_u32(&bars[2 * NSTAGE + 5]);
+  const uint32_t iempty0 = smem_u32(&bars[2 * NSTAGE + 5 + IQ]);
+  // the pair's shared barriers live in rank 0
+  const uint32_t full0_L = map_shared(full0, 0), tempty0_L = map_shared(tempty0, 0);
+  const uint32_t iempty0_L = map_shared(iempty0, 0);
+  const uint32_t abort_peer = map_shared(smem_u32((const void *)abort_flag), rank ^ 1u);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NSTAGE; ++s) {
+      mbar_init(full0 + 8 * s, 1);   // rank 0: its producer's arrive + both CTAs' bytes
+      mbar_init(empty0 + 8 * s, 1);  // multicast MMA commit
+    }
+    for (int u = 0; u < 2; ++u) {
+      mbar_init(tfull0 + 8 * u, 1);
+      mbar_init(tempty0 + 8 * u, 2 * NEPI);  // epilogue warps of both CTAs
+    }
+    mbar_init(drain, 1);
+    for (int s = 0; s < IQ; ++s) {
+      mbar_init(ifull0 + 8 * s, 1);
+      mbar_init(iempty0 + 8 * s, 2 + 2 * NEPI);  // MMA issuer, peer producer, all epilogue warps
+    }
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&tmA) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&tmB) : "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
+                     smem_u32(tmem_slot))
+                 : "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();  // both CTAs' barriers are initialised before any remote access
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  if (warp == 1)  // both CTAs hold their columns
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+
+  if (warp == 0) {
+    // --------------------- TMA producers (both CTAs) ---------------------
+    if (lane == 0) {
+      const uint32_t item_q_peer = map_shared(smem_u32((const void *)item_q), 1);
+      const uint32_t ifull0_peer = map_shared(ifull0, 1);
+      int stage = 0, islot = 0;
+      uint32_t phase = 0, iphase = 0, armed = 0, armed_par = 0;
+      bool ok = true;
+      while (ok) {
+        int qidx;
+        if (leader) {
+          if (!pair_wait(iempty0 + 8 * islot, iphase ^ 1, true, abort_flag, abort_peer, P.err, 35))
+            break;
+          const long long id = (long long)atomicAdd(P.queue, 1u);
+          qidx = id < P.nitems ? (int)id : -1;
+          item_q[islot] = qidx;
+          st_remote_u32(item_q_peer + 4 * islot, (uint32_t)qidx);
+          mbar_arrive(ifull0 + 8 * islot);
+          mbar_arrive_remote(ifull0_peer + 8 * islot);
+        } else {
+          if (!pair_wait(ifull0 + 8 * islot, iphase, true, abort_flag, abort_peer, P.err, 35)) break;
+          qidx = item_q[islot];
+          mbar_arrive_remote(iempty0_L + 8 * islot);
+        }
+        if (++islot == IQ) {
+          islot = 0;
+          iphase ^= 1;
+        }
+        if (qidx < 0) break;
+        int i, j, R, tB;
+        eos_pair_decode(P, qidx, i, j, R, tB);
+        const int tA = min(2 * R + (int)rank, tB);  // a dummy loads block tB's rows
+        for (int o = 0; o < 2 * (P.copies + 1) && ok; ++o) {
+          const int set = o >> 1, t = o & 1;
+          if (t && i == j) continue;  // T2 = T1, U2 = U1
+          const int colA = (t ? j : i) * P.nvpad + tA * TILE;
+          const int colB = (t ? i : j) * P.nvpad + tB * TILE;
+          const int colH = colB + BHALF * (int)rank;  // this rank's half of the V rows
+          for (int kc = 0; kc < P.nks; ++kc) {
+            if (!pair_wait(empty0 + 8 * stage, phase ^ 1, false, abort_flag, abort_peer, P.err, 31)) {
+              ok = false;
+              break;
+            }
+            if (leader) {
+              mbar_expect_tx(full0 + 8 * stage, 2 * STAGE_BYTES);
+              armed |= 1u << stage;
+              armed_par = (armed_par & ~(1u << stage)) | (phase << stage);
+            }
+            const uint32_t dst = smem_u32(stages + stage * STAGE_BYTES), fb = full0_L + 8 * stage;
+            const int rowk = P.row0[set] + kc * P.ncol;
+            tma_load_3d_pair(dst, &tmA, fb, 0, rowk + colA, 0);                            // S0a
+            tma_load_3d_pair(dst + PANEL_BYTES, &tmA, fb, 0, rowk + colA, 1);              // R1a
+            tma_load_3d_pair(dst + 2 * PANEL_BYTES, &tmA, fb, 0, rowk + colB, (int)rank);  // S0b / R1b
+            tma_load_3d_pair(dst + 3 * PANEL_BYTES, &tmB, fb, 0, rowk + colH, 2);          // half of Vb
+            if (++stage == NSTAGE) {
+              stage = 0;
+              phase ^= 1;
+            }
+          }
+        }
+      }
+      if (leader && (!ok || *abort_flag)) {  // copies in flight complete before the pair exits
+        for (int s = 0; s < NSTAGE; ++s) {
+          if (!((armed >> s) & 1u)) continue;
+          const long long t0 = clock64();
+          while (!mbar_test(full0 + 8 * s, (armed_par >> s) & 1u) && clock64() - t0 < WAIT_BUDGET) {
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // --------------------- MMA issuer (rank 0 only) ----------------------
+    if (lane == 0 && leader) {
+      int stage = 0, islot = 0;
+      uint32_t phase = 0, iphase = 0;
+      bool ok = true;
+      long long n = 0;  // tiles so far
+      while (ok) {
+        if (!pair_wait(ifull0 + 8 * islot, iphase, false, abort_flag, abort_peer, P.err, 36)) break;
+        const int qidx = item_q[islot];
+        mbar_arrive_remote(iempty0_L + 8 * islot);
+        if (++islot == IQ) {
+          islot = 0;
+          iphase ^= 1;
+        }
+        if (qidx < 0) break;
+        int i, j, R, tB;
+        eos_pair_decode(P, qidx, i, j, R, tB);
+        for (int o = 0; o < 2 * (P.copies + 1) && ok; ++o) {
+          if ((o & 1) && i == j) continue;
+          const int u = (int)(n & 1);
+          // both CTAs' epilogues have read this accumulator's previous tile
+          if (n >= 2 && !pair_wait(tempty0 + 8 * u, (uint32_t)(((n >> 1) - 1) & 1), true, abort_flag,
+                                   abort_peer, P.err, 32)) {
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t dL0 = tmem + (uint32_t)(u * 2 * TILE), dL1 = dL0 + TILE;
+          for (int kc = 0; kc < P.nks; ++kc) {
+            if (!pair_wait(full0 + 8 * stage, phase, false, abort_flag, abort_peer, P.err, 33)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint32_t sb = smem_u32(stages + stage * STAGE_BYTES);
+#pragma unroll
+            for (int k16 = 0; k16 < KSTEP / 16; ++k16) {
+              const uint32_t koff = k16 * 32;
+              const uint32_t acc = (kc > 0 || k16 > 0) ? 1u : 0u;
+              // [L0 | L1] += S0a x [S0b; R1b], then L1 += R1a V
+              mma_f16_pair(dL0, smem_desc(sb + koff), smem_desc(sb + 2 * PANEL_BYTES + koff),
+                           IDESC_PAIR_N256, acc);
+              mma_f16_pair(dL1, smem_desc(sb + PANEL_BYTES + koff),
+                           smem_desc(sb + 3 * PANEL_BYTES + koff), IDESC_PAIR, 1u);
+            }
+            mma_commit_pair(empty0 + 8 * stage);  // frees the stage in both CTAs
+            if (++stage == NSTAGE) {
+              stage = 0;
+              phase ^= 1;
+            }
+          }
+          if (!ok) break;
+          mma_commit_pair(tfull0 + 8 * u);
+          ++n;
+        }
+      }
+      mma_commit_pair(drain);  // both CTAs learn when the last MMA has completed
+    }
+  } else {
+    // --------------------- epilogue (both CTAs) ---------------------------
+    const int ew = warp - 2, quad = warp & 3;
+    const int cbase = (ew >> 2) * 64;  // 64 of the tile's 128 columns
+    const int row = quad * 32 + lane;
+    const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
+    float *st = P.stash + (size_t)blockIdx.x * (2 * 64 * 256) + (threadIdx.x - 64);
+    int islot = 0;
+    uint32_t iphase = 0;
+    long long n = 0;
+    bool ok = true;
+    while (ok) {
+      const bool w0 = pair_wait(ifull0 + 8 * islot, iphase, true, abort_flag, abort_peer, P.err, 37);
+      if (epi_any(!w0)) break;
+      const int qidx = item_q[islot];
+      __syncwarp();
+      if (lane == 0) mbar_arrive_remote(iempty0_L + 8 * islot);
+      if (++islot == IQ) {
+        islot = 0;
+        iphase ^= 1;
+      }
+      if (qidx < 0) break;
+      int i, j, R, tB;
+      eos_pair_decode(P, qidx, i, j, R, tB);
+      const int tA = 2 * R + (int)rank;
+      const bool dummy = tA > tB, same = i == j, diag = tA == tB;
+      const int a = min(tA, tB) * TILE + row, b0 = tB * TILE + cbase;
+      const float2 ea = P.ev2[a];
+      const float2 ei = P.eo2[i], ej = P.eo2[j];
+      const float sh = ei.x + ej.x;
+      const float bv = sh - ei.x;
+      const float sl = (ei.x - (sh - bv)) + (ej.x - bv) + ei.y + ej.y;
+      const float dh0 = sh - ea.x;
+      const float bw = dh0 - sh;
+      const float dl0 = ((sh - (dh0 - bw)) + (-ea.x - bw)) + (sl - ea.y);
+      auto rden = [&](int b) -> float {  // reciprocal denominator of (a, b)
+        const float2 eb = P.ev2[b];
+        const float dh = dh0 - eb.x;
+        const float bz = dh - dh0;
+        return rcp_denom(dh + (((dh0 - (dh - bz)) + (-eb.x - bz)) + (dl0 - eb.y)));
+      };
+      // g_ii(a,a) of each set carries the same-column bias sum_k R1 (V - S0 - R1)
+      const int cd = (same && diag && a - b0 >= 0 && a - b0 < 64) ? a - b0 : -1;
+      // this thread's 16 values of the current tile from column c0 on
+      auto read = [&](int set, int t, uint32_t tb, float corr, int c0, float (&v)[16]) {
+        const float *sc = P.inv + (size_t)set * P.ncol;
+        const float srow = sc[(t ? j : i) * P.nvpad + a];
+        const float *scol = sc + (t ? i : j) * P.nvpad + b0 + c0;
+        float l0[16], l1[16];
+        tmem_ld16(tb + c0, l0);
+        tmem_ld16(tb + TILE + c0, l1);
+        tmem_wait_ld();
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          float x = l0[k] + l1[k];
+          if (c0 + k == cd && t == 0) x -= corr;
+          v[k] = x * (srow * scol[k]);
+        }
+      };
+      double eacc[2] = {0.0, 0.0};
+      float u1[64];
+      for (int o = 0; o < 2 * (P.copies + 1); ++o) {
+        const int set = o >> 1, t = o & 1;
+        if (t && same) continue;
+        const int u = (int)(n & 1);
+        const bool w = pair_wait(tfull0 + 8 * u, (uint32_t)((n >> 1) & 1), false, abort_flag,
+                                 abort_peer, P.err, 34);
+        if (epi_any(!w)) {
+          ok = false;
+          break;
+        }
+        ++n;
+        tc_fence_after();
+        const uint32_t tb = tmem + lane_off + (uint32_t)(u * 2 * TILE + cbase);
+        const float corr = cd >= 0 ? P.dcorr[(size_t)set * P.ncol + i * P.nvpad + a] : 0.0f;
+        double e = 0.0;
+        if (dummy) {
+        } else if (set == 0) {  // g: kept for the projected sets
+#pragma unroll 1
+          for (int c0 = 0; c0 < 64; c0 += 16) {
+            float v[16];
+            read(0, t, tb, corr, c0, v);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) __stcg(st + (size_t)(t * 64 + c0 + k) * 256, v[k]);
+          }
+        } else if (t == 0) {
+#pragma unroll
+          for (int c0 = 0; c0 < 64; c0 += 16) {
+            float v[16];
+            read(set, 0, tb, corr, c0, v);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) u1[c0 + k] = v[k];
+          }
+          if (same) {  // g2 = g1, u2 = u1: diagonal g1 u1, otherwise 2 g1 u1
+#pragma unroll
+            for (int c0 = 0; c0 < 64; c0 += 32) {
+              float ef = 0.0f;
+#pragma unroll
+              for (int k = 0; k < 32; ++k)
+                ef = fmaf((diag ? 1.0f : 2.0f) * __ldcg(st + (size_t)(c0 + k) * 256) * u1[c0 + k],
+                          rden(b0 + c0 + k), ef);
+              e += (double)ef;
+            }
+          }
+        } else {
+#pragma unroll
+          for (int c0 = 0; c0 < 64; c0 += 16) {
+            float u2[16];
+            read(set, 1, tb, corr, c0, u2);
+            float ef = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 16; ++k) {
+              const float g1 = __ldcg(st + (size_t)(c0 + k) * 256);
+              const float g2 = __ldcg(st + (size_t)(64 + c0 + k) * 256);
+              float num = g1 * fmaf(2.0f, u1[c0 + k], -u2[k]);
+              if (!diag) num = fmaf(g2, fmaf(2.0f, u2[k], -u1[c0 + k]), num);
+              ef = fmaf(num, rden(b0 + c0 + k), ef);
+            }
+            e += (double)ef;
+          }
+        }
+        if (set == 1) eacc[0] += e;
+        if (set == 2) eacc[1] += e;
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_remote(tempty0_L + 8 * u);
+      }
+      if (!ok) break;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        double e = eacc[c];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+        if (lane == 0) redd[c * NEPI + ew] = e;
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (ew == 0 && lane < P.copies && !dummy) {
+        double tot = 0.0;
+#pragma unroll
+        for (int w = 0; w < NEPI; ++w) tot += redd[lane * NEPI + w];
+        const long long p = (long long)j * (j + 1) / 2 + i;
+        P.part[lane * P.npart + p * P.ntp + tB * (tB + 1) / 2 + tA] = tot;
+      }
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+    }
+  }
+  __syncthreads();
+  if (warp == 1 && lane == 0) {
+    // the last MMA of the pair has completed (it may write this CTA's TMEM)
+    const long long t0 = clock64();
+    while (!mbar_test(drain, 0) && clock64() - t0 < WAIT_BUDGET) {
+    }
+  }
+  if (*abort_flag) {
+    // after an abort the peer may still have copies in flight into its own
+    // shared memory (their completion is counted in rank 0): give them time
+    const long long t0 = clock64();
+    while (clock64() - t0 < 4000000LL) {
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync_all();
+  if (warp == 1) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
   }
 }
 
@@ -3904,30 +4286,50 @@ int ao_half_fused(const double *ao, int NBA, int nbas, const double *Cmo, int no
 // Local-orbital fragment energy in the split form: slices of Calpha and of its
 // projected copy Ct in one buffer, one persistent split_eos_kernel launch,
 // compensated FP64 pair and total reductions.
-int split_eos_energy(const double *Ca, const double *Ct, int NBA, int nvirt, int nocc,
-                     const double *eo, const double *ev, double *Epair, double *Etot,
+// Fragment energies of one or two projected copies of Calpha: Etot[c] from
+// copy Ct[c].
+int split_eos_energy(const double *Ca, const double *const *Ct, int copies, int NBA, int nvirt,
+                     int nocc, const double *eo, const double *ev, double *Epair, double *Etot,
                      int nslices, cudaStream_t s) {
   const int nsl = nslices + 1;
+  if (nsl > 2 && copies > 1) {  // the one-CTA kernel takes one copy
+    for (int c = 0; c < copies; ++c)
+      RIMP2_TRY(split_eos_energy(Ca, Ct + c, 1, NBA, nvirt, nocc, eo, ev, Epair, Etot + c, nslices, s));
+    return RIMP2_OK;
+  }
   auto encode = get_encode();
   if (!encode) {
     set_error("cuTensorMapEncodeTiled entry point unavailable");
     return RIMP2_ERR_UNSUPPORTED;
   }
-  FragDesc fh[2];
+  const int sets = copies + 1;
+  FragDesc fh[3];
   memset(fh, 0, sizeof fh);
   const int nvpad = (nvirt + TILE - 1) / TILE * TILE;
   const int nks = (NBA + KSTEP - 1) / KSTEP;
   const int nt = nvpad / TILE;
   const int ntp = nt * (nt + 1) / 2;
   const long long ncol = (long long)nocc * nvpad;
-  const long long R = 2LL * nks * ncol;
+  const long long R = (long long)sets * nks * ncol;
   const int npairs = nocc * (nocc + 1) / 2;
-  const long long nitems = (long long)npairs * ntp * 2;
+  const bool pair = nsl == 2;
+  int per = 2 * ntp;  // items of an occupied pair
+  if (pair) {
+    per = 0;
+    for (int r = 0; 2 * r < nt; ++r) per += nt - 2 * r;
+  }
+  const int nper = pair ? ntp : 2 * ntp;  // partial energies of an occupied pair
+  const long long nitems = (long long)npairs * per, npart = (long long)npairs * nper;
+  if (R > 2147483647LL - TILE && copies > 1) {  // too many rows for one tensor map: one copy at a time
+    for (int c = 0; c < copies; ++c)
+      RIMP2_TRY(split_eos_energy(Ca, Ct + c, 1, NBA, nvirt, nocc, eo, ev, Epair, Etot + c, nslices, s));
+    return RIMP2_OK;
+  }
   if (R > 2147483647LL - TILE || nitems > 2147483647LL || ncol > 2147483647LL) {
     set_error("split local-orbital energy: fragment too large (rows=%lld, items=%lld)", R, nitems);
     return RIMP2_ERR_ARG;
   }
-  for (int f = 0; f < 2; ++f) {
+  for (int f = 0; f < sets; ++f) {
     FragDesc &F = fh[f];
     F.nocc = nocc;
     F.nvirt = nvirt;
@@ -3938,26 +4340,48 @@ int split_eos_energy(const double *Ca, const double *Ct, int NBA, int nvirt, int
     F.ncol = (int)ncol;
     F.row_base = (long long)f * nks * ncol;
     F.col_base = (long long)f * ncol;
-    F.Ca = f ? Ct : Ca;
+    F.Ca = f ? Ct[f - 1] : Ca;
     F.eo = eo;
     F.ev = ev;
   }
-  const int vplane = nsl == 2 ? 1 : 0;  // one residual slice: V plane, three products
-  const int planes = nsl + vplane;
-  DevBuf frags, slices, inv, eo2, ev2, part, queue, pairs, dcorr;
-  RIMP2_TRY(frags.alloc(sizeof fh, s));
-  RIMP2_TRY(slices.alloc(sizeof(__half) * (size_t)planes * R * 64, s));
-  RIMP2_TRY(inv.alloc(sizeof(float) * 2 * (size_t)ncol, s));
-  if (vplane) RIMP2_TRY(dcorr.alloc(sizeof(float) * 2 * (size_t)ncol, s));
-  RIMP2_TRY(eo2.alloc(sizeof(float2) * nocc, s));
-  RIMP2_TRY(ev2.alloc(sizeof(float2) * nvpad, s));
-  RIMP2_TRY(part.alloc(sizeof(double) * (size_t)nitems, s));
-  RIMP2_TRY(queue.alloc(sizeof(unsigned int), s));
-  RIMP2_TRY(pairs.alloc(sizeof(int) * 2 * (size_t)npairs, s));
+  int dev = 0, nsm = 0;
+  RIMP2_CK(cudaGetDevice(&dev));
+  RIMP2_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const int planes = nsl + (pair ? 1 : 0);  // one residual slice: V plane, three products
+  DevBuf arena, frags, slices, inv, eo2, ev2, part, queue, pairs, dcorr, stash;
+  {
+    DevBuf *buf[] = {&slices, &frags, &inv, &dcorr, &eo2, &ev2, &part, &queue, &pairs, &stash};
+    const size_t bytes[] = {sizeof(__half) * (size_t)planes * R * 64,
+                            sizeof fh,
+                            sizeof(float) * sets * (size_t)ncol,
+                            pair ? sizeof(float) * sets * (size_t)ncol : 16,
+                            sizeof(float2) * nocc,
+                            sizeof(float2) * nvpad,
+                            sizeof(double) * copies * (size_t)npart,
+                            sizeof(unsigned int),
+                            sizeof(int) * 2 * (size_t)npairs,
+                            pair ? sizeof(float) * 2 * 64 * 256 * (size_t)nsm : 16};
+    size_t total = 0;
+    for (size_t n : bytes) total += (n + 255) / 256 * 256;
+    const int rc = arena.alloc(total, s);
+    if (rc != RIMP2_OK && copies > 1) {  // no room for both copies at once
+      (void)cudaGetLastError();
+      clear_error();
+      for (int c = 0; c < copies; ++c)
+        RIMP2_TRY(split_eos_energy(Ca, Ct + c, 1, NBA, nvirt, nocc, eo, ev, Epair, Etot + c, nslices, s));
+      return RIMP2_OK;
+    }
+    RIMP2_TRY(rc);
+    char *at = arena.as<char>();
+    for (int k = 0; k < 10; ++k) {
+      buf[k]->alias(at, bytes[k], s);
+      at += (bytes[k] + 255) / 256 * 256;
+    }
+  }
   RIMP2_CK(cudaMemcpyAsync(frags.p, fh, sizeof fh, cudaMemcpyHostToDevice, s));
   const FragDesc *fr = frags.as<FragDesc>();
-  slice_batch_kernel<<<dim3((unsigned)((ncol * 32 + 255) / 256), 2), 256, 0, s>>>(
-      fr, nsl, R * 64, slices.as<__half>(), inv.as<float>(), 0, 0x7fffffff, vplane,
+  slice_batch_kernel<<<dim3((unsigned)((ncol * 32 + 255) / 256), (unsigned)sets), 256, 0, s>>>(
+      fr, nsl, R * 64, slices.as<__half>(), inv.as<float>(), 0, 0x7fffffff, pair ? 1 : 0,
       dcorr.as<float>());
   eps_batch_kernel<<<dim3((unsigned)((std::max(nvpad, nocc) + 255) / 256), 1), 256, 0, s>>>(
       fr, eo2.as<float2>(), ev2.as<float2>());
@@ -3978,49 +4402,67 @@ int split_eos_energy(const double *Ca, const double *Ct, int NBA, int nvirt, int
     set_error("cuTensorMapEncodeTiled failed (%d)", (int)cr);
     return RIMP2_ERR_CUDA;
   }
-  EosParams P;
-  P.inv = inv.as<float>();
-  P.eo2 = eo2.as<float2>();
-  P.ev2 = ev2.as<float2>();
-  P.nitems = nitems;
-  P.queue = queue.as<unsigned int>();
-  P.part = part.as<double>();
-  P.err = device_error_word();
-  P.nocc = nocc;
-  P.nvirt = nvirt;
-  P.nvpad = nvpad;
-  P.nks = nks;
-  P.ntp = ntp;
-  P.ncol = (int)ncol;
-  P.rowC = 0;
-  P.rowCt = (int)((long long)nks * ncol);
-  P.dcorr = dcorr.as<float>();
-  int dev = 0, nsm = 0;
-  RIMP2_CK(cudaGetDevice(&dev));
-  RIMP2_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const int grid = (int)std::min<long long>(nitems, nsm);
   RIMP2_CK(cudaMemsetAsync(queue.p, 0, sizeof(unsigned int), s));
   if (inject_fault("launch")) {
     set_error("injected launch failure (RIMP2_FAULT_INJECT=launch)");
     return RIMP2_ERR_CUDA;
   }
-  if (nsl == 2) {
-    RIMP2_CK(cudaFuncSetAttribute(split_eos_kernel<2, 4>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, eos_smem_bytes(2, 4)));
-    split_eos_kernel<2, 4><<<grid, NTHREADS, eos_smem_bytes(2, 4), s>>>(tmA, tmB, P);
+  if (pair) {
+    EosPairParams P;
+    P.inv = inv.as<float>();
+    P.dcorr = dcorr.as<float>();
+    P.eo2 = eo2.as<float2>();
+    P.ev2 = ev2.as<float2>();
+    P.nitems = nitems;
+    P.npart = npart;
+    P.queue = queue.as<unsigned int>();
+    P.part = part.as<double>();
+    P.stash = stash.as<float>();
+    P.err = device_error_word();
+    P.nvpad = nvpad;
+    P.nks = nks;
+    P.nt = nt;
+    P.ntp = ntp;
+    P.per = per;
+    P.ncol = (int)ncol;
+    P.copies = copies;
+    for (int f = 0; f < 3; ++f) P.row0[f] = (int)((long long)f * nks * ncol);
+    RIMP2_CK(cudaFuncSetAttribute(split_eos_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  EP_SMEM));
+    const int npair = (int)std::min<long long>(nitems, std::max(1, nsm / 2));
+    RIMP2_CK(launch_hi(split_eos_pair_kernel, 2 * npair, NTHREADS, EP_SMEM, s, tmA, tmB, P));
   } else {
-    RIMP2_CK(cudaFuncSetAttribute(split_eos_kernel<3, 3>,
-                                  cudaFuncAttributeMaxDynamicSharedMemorySize, eos_smem_bytes(3, 3)));
+    EosParams P;
+    P.inv = inv.as<float>();
+    P.eo2 = eo2.as<float2>();
+    P.ev2 = ev2.as<float2>();
+    P.nitems = nitems;
+    P.queue = queue.as<unsigned int>();
+    P.part = part.as<double>();
+    P.err = device_error_word();
+    P.nocc = nocc;
+    P.nvirt = nvirt;
+    P.nvpad = nvpad;
+    P.nks = nks;
+    P.ntp = ntp;
+    P.ncol = (int)ncol;
+    P.rowC = 0;
+    P.rowCt = (int)((long long)nks * ncol);
+    RIMP2_CK(cudaFuncSetAttribute(split_eos_kernel<3, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  eos_smem_bytes(3, 3)));
+    const int grid = (int)std::min<long long>(nitems, nsm);
     split_eos_kernel<3, 3><<<grid, NTHREADS, eos_smem_bytes(3, 3), s>>>(tmA, tmB, P);
   }
   count_launch(1);
   RIMP2_CK(cudaGetLastError());
   make_pairs_kernel<<<(npairs + 255) / 256, 256, 0, s>>>(nocc, pairs.as<int>());
-  RIMP2_CK(cudaMemsetAsync(Epair, 0, sizeof(double) * (size_t)nocc * nocc, s));
-  pair_reduce_kernel<<<(npairs + 7) / 8, 256, 0, s>>>(part.as<double>(), 2 * ntp, pairs.as<int>(),
-                                                     npairs, nocc, Epair);
-  total_reduce_kernel<<<1, total_threads(nocc), 0, s>>>(Epair, nocc, Etot);
-  count_launch(3);
+  count_launch(1);
+  for (int c = 0; c < copies; ++c) {
+    pair_reduce_kernel<<<(npairs + 7) / 8, 256, 0, s>>>(part.as<double>() + c * npart, nper,
+                                                       pairs.as<int>(), npairs, nocc, Epair);
+    total_reduce_kernel<<<1, total_threads(nocc), 0, s>>>(Epair, nocc, Etot + c);
+    count_launch(2);
+  }
   RIMP2_CK(cudaGetLastError());
   return RIMP2_OK;
 }

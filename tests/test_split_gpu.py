@@ -125,6 +125,33 @@ def test_split_eos_energy_vs_fp64(nocc, nvirt, NBA, noE, nvE):
         assert abs(g - r) <= 1e-7 * abs(r), (g, r)
 
 
+@pytest.mark.parametrize("nocc,nvirt,NBA,noE,nvE", [
+    (1, 128, 65, 1, 3),      # one pair, one block: the pair's second CTA is a dummy
+    (3, 257, 64, 1, 30),     # three blocks: half a row block
+    (2, 385, 130, 2, 385),   # four blocks, full-rank projectors
+    (7, 129, 700, 7, 129),   # one virtual past a block
+    (5, 520, 200, 2, 40),    # five blocks
+])
+def test_split_eos_pair_kernel(nocc, nvirt, NBA, noE, nvE):
+    """Local-orbital energies on CTA pairs (one residual slice): edges of the
+    row and column blocks, both partitionings against the FP64 form; the last
+    local blocks are not orthonormal, so neither projector is the identity."""
+    from rimp2_gpu_gb300 import api
+    assert api.split_nslices(nvirt, nocc, NBA) == 1
+    Ca, eo, ev = O.gen_fragment(60 + nvirt, nocc, nvirt, NBA)
+
+    def u(m, k, s, orth):
+        g = O.gen_matrix(60 + nvirt, s, m, m) / np.sqrt(m)
+        return np.asfortranarray((np.linalg.qr(g)[0] if orth else g)[:, :k])
+    for orth in (True, False):
+        U = (u(nocc, noE, 1, orth), u(nvirt, nvirt, 2, orth), u(nocc, nocc, 3, orth),
+             u(nvirt, nvE, 4, orth))
+        ref = api.energy_eos(nvirt, nocc, noE, nvE, NBA, Ca, eo, ev, *U, precision=api.PREC_FP64)
+        got = api.energy_eos(nvirt, nocc, noE, nvE, NBA, Ca, eo, ev, *U, precision=api.PREC_SPLIT)
+        for r, g in zip(ref, got):
+            assert abs(g - r) <= 1e-7 * abs(r), (g, r)
+
+
 def test_split_eos_identity_is_canonical():
     from oracle import oracle as O
     from rimp2_gpu_gb300 import api
