@@ -72,89 +72,172 @@ __device__ void tri_inverse(double (*A)[DP], double (*X)[DP], double *part, doub
   }
 }
 
+constexpr int PS = NB + 4;  // padded row (doubles): DMMA operands from two rows of banks
+__device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+               : "+d"(d0), "+d"(d1)
+               : "d"(a), "d"(b));
+}
+
 // In-place Cholesky of the b x b diagonal block at (k0,k0) of V (ld n); *bad =
-// pivot+1 on a non-positive pivot.  One CTA, so its FP64 pipe (two FMAs a
-// clock) and the chain of 64 pivots bound it: the block lives in registers
-// (lane = row, a warp holds every fourth column of 32 rows, so that a finished
-// column costs whole warps nothing), column k passes through shared memory
-// with one barrier a step, and the chain is kept short by eliminating with
-// column k over d_k (a reciprocal; the columns get their 1/sqrt(d_k) at the end,
-// all at once).
+// pivot+1 on a non-positive pivot.  One CTA: the chain of 64 pivots and its
+// FP64 pipe (two FMAs a clock, so every idle lane of a warp counts) bound it.
+// Sixteen columns at a time: their diagonal block in one warp's registers
+// (lane = row; columns over their pivot, the square roots at the end), the rows
+// below by substitution, a row per thread, the rest with DMMA.  143 us as a
+// rank-one update per column with the inverse, 69 us with the block in
+// registers and a barrier per column.
 __global__ void __launch_bounds__(256) potrf_block_kernel(double *V, int n, int k0, int b, int *bad) {
-  __shared__ double col[2][NB];  // column k, not yet scaled
-  __shared__ double piv[NB];     // 1 / sqrt(d_k)
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, q = w & 3, half = w >> 2;
-  const int r = 32 * half + lane;
-  double a[NB / 4];
+  __shared__ double A[NB][PS];
+  __shared__ double rd[NB];  // 1 / L(k, k)
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
 #pragma unroll
-  for (int x = 0; x < NB / 4; ++x) {
-    const int c = 4 * x + q;
-    a[x] = r < b && c < b ? V[(size_t)(k0 + (r > c ? r : c)) + (size_t)n * (k0 + (r > c ? c : r))]
-                          : (r == c ? 1.0 : 0.0);
+  for (int x = 0; x < NB * NB / 256; ++x) {
+    const int t = threadIdx.x + 256 * x, r = t & (NB - 1), c = t >> 6;
+    A[r][c] = r < b && c <= r ? V[(size_t)(k0 + r) + (size_t)n * (k0 + c)] : (r == c ? 1.0 : 0.0);
   }
-  if (q == 0) col[0][r] = a[0];
   __syncthreads();
 #pragma unroll 1
-  for (int k = 0; k < NB; ++k) {
-    const double *ck = col[k & 1];
-    const double d = ck[k];
-    const bool ok = d > 0.0;
-    if (!ok && threadIdx.x == 0) atomicCAS(bad, 0, k0 + k + 1);
-    if (threadIdx.x == 0) piv[k] = ok ? d : 1.0;
-    const double f = -(ok ? recip_f64(d) : 1.0) * ck[r];
+  for (int o = 0; o < NB; o += 16) {
+    if (w == 0) {
+      const int r = lane & 15;
+      double a[16], dmine = 1.0;
 #pragma unroll
-    for (int x = 0; x < NB / 4; ++x) {
-      const int c = 4 * x + q;
-      if (c <= k || (half == 0 && c >= 32)) continue;  // uniform over the warp
-      a[x] = fma(f, ck[c], a[x]);
-      if (c == k + 1) col[(k + 1) & 1][r] = a[x];
+      for (int c = 0; c < 16; ++c) a[c] = r >= c ? A[o + r][o + c] : A[o + c][o + r];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const double d = __shfl_sync(0xffffffffu, a[k], k);
+        const bool ok = d > 0.0;
+        if (!ok && lane == 0) atomicCAS(bad, 0, k0 + o + k + 1);
+        if (r == k) dmine = ok ? d : 1.0;
+        const double f = -(ok ? recip_f64(d) : 1.0) * a[k];
+#pragma unroll
+        for (int c = k + 1; c < 16; ++c) a[c] = fma(f, __shfl_sync(0xffffffffu, a[k], c), a[c]);
+      }
+      const double s = 1.0 / sqrt(dmine);
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {
+        const double v = a[k] * __shfl_sync(0xffffffffu, s, k);
+        if (lane < 16 && r >= k) A[o + r][o + k] = v;
+      }
+      if (lane < 16) rd[o + r] = s;
     }
-    // rows 0..31 of column k+1 >= 32 lie above the diagonal: not needed
+    __syncthreads();
+    const int row = o + 16 + threadIdx.x;
+    if (row < NB) {
+      double x[16];
+#pragma unroll
+      for (int c = 0; c < 16; ++c) x[c] = A[row][o + c];
+#pragma unroll
+      for (int c = 0; c < 16; ++c) {
+        x[c] *= rd[o + c];
+#pragma unroll
+        for (int j = c + 1; j < 16; ++j) x[j] = fma(-A[o + j][o + c], x[c], x[j]);
+      }
+#pragma unroll
+      for (int c = 0; c < 16; ++c) A[row][o + c] = x[c];
+    }
+    __syncthreads();
+    const int n8 = (NB - 16 - o) / 8;
+    for (int t = w; t < n8 * (n8 + 1) / 2; t += 8) {  // 8 x 8 tiles of the lower triangle
+      int ti = 0;
+      while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
+      const int r0 = o + 16 + 8 * ti, c0 = o + 16 + 8 * (t - ti * (ti + 1) / 2);
+      double d0 = A[r0 + gid][c0 + 2 * tig], d1 = A[r0 + gid][c0 + 2 * tig + 1];
+#pragma unroll
+      for (int k = 0; k < 16; k += 4) dmma(d0, d1, -A[r0 + gid][o + k + tig], A[c0 + gid][o + k + tig]);
+      A[r0 + gid][c0 + 2 * tig] = d0;
+      A[r0 + gid][c0 + 2 * tig + 1] = d1;
+    }
     __syncthreads();
   }
-  if (threadIdx.x < NB) piv[threadIdx.x] = 1.0 / sqrt(piv[threadIdx.x]);
-  __syncthreads();
 #pragma unroll
-  for (int x = 0; x < NB / 4; ++x) {
-    const int c = 4 * x + q;
-    if (r < b && c < b) V[(size_t)(k0 + r) + (size_t)n * (k0 + c)] = r >= c ? a[x] * piv[c] : 0.0;
+  for (int x = 0; x < NB * NB / 256; ++x) {
+    const int t = threadIdx.x + 256 * x, r = t & (NB - 1), c = t >> 6;
+    if (r < b && c < b) V[(size_t)(k0 + r) + (size_t)n * (k0 + c)] = r >= c ? A[r][c] : 0.0;
   }
 }
 
 // X := X L^{-T} for the rows [k0+64, n) of the block column at k0, L its
-// factored diagonal block: eight rows per CTA (136 CTAs at n = 1152), 16
-// threads a row with four columns each, one barrier-free chain of 64 columns
-// within each row's half warp.  (As a product with L^{-1} the inverse sat on
-// the critical path: 70 of 143 us.)
+// factored diagonal block: eight rows per CTA (136 CTAs at n = 1152), warp j
+// holds their columns 16 j .. 16 j + 15.  Sixteen columns at a time: warp l
+// multiplies by the inverse of L_ll (formed by that warp beforehand), the warps
+// after it subtract X_l L_jl^T, both with DMMA m8n8k4: 80 of those, 5 us of
+// the SM's FP64 pipe.  (Column by column, with one chain of 64 dependent
+// steps, it took 34 us; as a product with L^{-1} of 64 x 64 the inverse sat on
+// the critical path.)
 __global__ void __launch_bounds__(128) panel_solve_kernel(double *V, int n, int k0) {
-  __shared__ double Ls[NB][NB + 1];  // Ls[c][j] = L(j, c) below, 1 / L(c, c) on the diagonal
-  for (int t = threadIdx.x; t < NB * NB; t += 128) {
-    const int j = t & (NB - 1), c = t >> 6;
-    const double l = V[(size_t)(k0 + j) + (size_t)n * (k0 + c)];
-    Ls[c][j] = j == c ? 1.0 / l : l;
+  __shared__ double Ls[NB][PS];     // L(j, c)
+  __shared__ double Inv[4][16][17];  // inverses of the 16 x 16 diagonal blocks
+  __shared__ double Xs[8][PS];      // the rows
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
+  const int row0 = k0 + NB + blockIdx.x * 8;
+#pragma unroll 16
+  for (int x = 0; x < NB * NB / 128; ++x) {
+    const int t = threadIdx.x + 128 * x, j = t & (NB - 1), c = t >> 6;
+    Ls[j][c] = V[(size_t)(k0 + j) + (size_t)n * (k0 + c)];
   }
-  const int row = k0 + NB + blockIdx.x * 8 + (threadIdx.x >> 4), g = threadIdx.x & 15;
-  double x[4];
 #pragma unroll
-  for (int u = 0; u < 4; ++u) x[u] = row < n ? V[(size_t)row + (size_t)n * (k0 + g + 16 * u)] : 0.0;
+  for (int x = 0; x < 8 * NB / 128; ++x) {
+    const int t = threadIdx.x + 128 * x, r = t & 7, c = t >> 3;
+    Xs[r][c] = row0 + r < n ? V[(size_t)(row0 + r) + (size_t)n * (k0 + c)] : 0.0;
+  }
   __syncthreads();
+  if (lane < 16) {  // column `lane` of the inverse of L_ww by forward substitution
+    const int o = 16 * w;
+    double x[16];
 #pragma unroll
-  for (int u = 0; u < 4; ++u)  // columns 16 u + v, owned by thread v
-#pragma unroll 4
-    for (int v = 0; v < 16; ++v) {
-      const int c = 16 * u + v;
-      const double y = __shfl_sync(0xffffffffu, x[u], v, 16) * Ls[c][c];
-      if (g == v) x[u] = y;
+    for (int r = 0; r < 16; ++r) x[r] = r == lane ? 1.0 : 0.0;
 #pragma unroll
-      for (int s = 0; s < 4; ++s) {
-        if (s < u) continue;
-        const int j = g + 16 * s;
-        if (s > u || g > v) x[s] = fma(-y, Ls[c][j], x[s]);
-      }
+    for (int r = 0; r < 16; ++r) {
+      x[r] *= recip_f64(Ls[o + r][o + r]);
+#pragma unroll
+      for (int p = r + 1; p < 16; ++p) x[p] = fma(-Ls[o + p][o + r], x[r], x[p]);
     }
 #pragma unroll
-  for (int u = 0; u < 4; ++u)
-    if (row < n) V[(size_t)row + (size_t)n * (k0 + g + 16 * u)] = x[u];
+    for (int r = 0; r < 16; ++r) Inv[w][r][lane] = x[r];
+  }
+  __syncwarp();
+  double acc[2][2];  // rows gid, columns 16 w + 8 y + 2 tig + {0, 1}
+#pragma unroll
+  for (int y = 0; y < 2; ++y)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) acc[y][h] = Xs[gid][16 * w + 8 * y + 2 * tig + h];
+#pragma unroll 1
+  for (int l = 0; l < 4; ++l) {
+    if (w == l) {
+      if (l) {  // the rows' columns after the updates, as the left operand
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) Xs[gid][16 * w + 8 * y + 2 * tig + h] = acc[y][h];
+        __syncwarp();
+      }
+      double x[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+      for (int k = 0; k < 16; k += 4)
+#pragma unroll
+        for (int y = 0; y < 2; ++y)  // X(r, c) = sum_k P(r, k) Inv(c, k)
+          dmma(x[y][0], x[y][1], Xs[gid][16 * w + k + tig], Inv[w][8 * y + gid][k + tig]);
+      __syncwarp();
+#pragma unroll
+      for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) Xs[gid][16 * w + 8 * y + 2 * tig + h] = x[y][h];
+    }
+    __syncthreads();
+    if (w > l) {
+#pragma unroll
+      for (int k = 0; k < 16; k += 4)
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+          dmma(acc[y][0], acc[y][1], -Xs[gid][16 * l + k + tig], Ls[16 * w + 8 * y + gid][16 * l + k + tig]);
+    }
+  }
+  for (int t = threadIdx.x; t < 8 * NB; t += 128) {
+    const int r = t & 7, c = t >> 3;
+    if (row0 + r < n) V[(size_t)(row0 + r) + (size_t)n * (k0 + c)] = Xs[r][c];
+  }
 }
 
 __global__ void zero_upper_kernel(double *V, int n) {
