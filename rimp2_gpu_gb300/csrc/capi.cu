@@ -21,7 +21,16 @@ static cudaStream_t g_user_stream = nullptr;
 static cudaStream_t g_lib_stream = nullptr;
 static std::mutex g_mu;
 static int g_dev_ok = -1;  // -1 unknown, 0 no, 1 yes
-static int *g_dev_err = nullptr;
+// the error word lives in page-locked host memory that kernels can write (only a
+// kernel that gives up does): reading it after a synchronisation costs nothing,
+// as a device word its copy took 10 us of every host call
+static int *g_dev_err = nullptr;   // its device address
+static int *g_host_err = nullptr;
+// behind it, room for a call's small results (one asynchronous copy instead of
+// two blocking ones of 10 us each); one call at a time, others copy directly
+static double *g_stage = nullptr;
+static std::mutex g_stage_mu;
+constexpr size_t kStage = 32768;  // doubles
 static bool g_timing = false;
 static float g_times[4] = {0, 0, 0, 0};
 
@@ -33,10 +42,9 @@ void record_timing(int slot, float ms) {
 
 int collect_device_error(cudaStream_t s) {
   RIMP2_CK(cudaStreamSynchronize(s));
-  int h = 0;
-  RIMP2_CK(cudaMemcpy(&h, g_dev_err, sizeof(int), cudaMemcpyDeviceToHost));
+  const int h = *(volatile int *)g_host_err;
   if (h != 0) {
-    RIMP2_CK(cudaMemset(g_dev_err, 0, sizeof(int)));
+    *(volatile int *)g_host_err = 0;
     set_error("a device-side bounded wait expired (code %d); the kernel returned early", h);
     return RIMP2_ERR_TIMEOUT;
   }
@@ -108,11 +116,17 @@ int ensure_device() {
     }
   }
   if (!g_dev_err) {
-    if (cudaMalloc(&g_dev_err, sizeof(int)) != cudaSuccess ||
-        cudaMemset(g_dev_err, 0, sizeof(int)) != cudaSuccess) {
+    void *h = nullptr, *d = nullptr;
+    if (cudaHostAlloc(&h, 256 + kStage * sizeof(double), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer(&d, h, 0) != cudaSuccess) {
       set_error("error-word allocation failed");
+      if (h) cudaFreeHost(h);
       return RIMP2_ERR_NOMEM;
     }
+    memset(h, 0, 256);
+    g_host_err = (int *)h;
+    g_stage = (double *)((char *)h + 256);
+    g_dev_err = (int *)d;
   }
   // keep freed stream-ordered scratch in the pool between calls instead of
   // returning it to the driver at every synchronisation
@@ -159,6 +173,21 @@ int h2d(DevBuf &b, const double *h, size_t n, cudaStream_t s) {
 int dalloc(DevBuf &b, size_t n, cudaStream_t s) { return b.alloc(n * sizeof(double), s); }
 int d2h(double *h, const DevBuf &b, size_t n, cudaStream_t s) {
   RIMP2_CK(cudaMemcpyAsync(h, b.p, n * sizeof(double), cudaMemcpyDeviceToHost, s));
+  return RIMP2_OK;
+}
+// ne + 1 doubles at dE: pair energies, then the total; ends the call on s
+int finish(cudaStream_t s);
+int finish_energies(double *Epair, double *Etot, const double *dE, size_t ne, cudaStream_t s) {
+  std::unique_lock<std::mutex> lk(g_stage_mu, std::try_to_lock);
+  if (!lk.owns_lock() || ne + 1 > kStage) {
+    RIMP2_CK(cudaMemcpyAsync(Epair, dE, ne * sizeof(double), cudaMemcpyDeviceToHost, s));
+    RIMP2_CK(cudaMemcpyAsync(Etot, dE + ne, sizeof(double), cudaMemcpyDeviceToHost, s));
+    return finish(s);
+  }
+  RIMP2_CK(cudaMemcpyAsync(g_stage, dE, (ne + 1) * sizeof(double), cudaMemcpyDeviceToHost, s));
+  RIMP2_TRY(finish(s));
+  memcpy(Epair, g_stage, ne * sizeof(double));
+  *Etot = g_stage[ne];
   return RIMP2_OK;
 }
 int finish(cudaStream_t s) {
@@ -1205,7 +1234,7 @@ int rimp2_energy(const int *nvirt, const int *nocc, const int *NBA, const double
   RIMP2_TRY(ensure_device());
   cudaStream_t s = current_stream();
   const size_t nv = *nvirt, no = *nocc, nb = *NBA;
-  DevBuf dC, deo, dev, dE, dT, dA;
+  DevBuf dC, deo, dev, dE, dA;
   // the bucket table sends tiny fragments to the FP64 kernel
   if (*precision == RIMP2_PREC_SPLIT && rimp2_split_nslices(*nvirt, *nocc, *NBA) > 0) {
     // copy Calpha in occupied-index chunks overlapped with the energy work
@@ -1214,8 +1243,7 @@ int rimp2_energy(const int *nvirt, const int *nocc, const int *NBA, const double
     RIMP2_TRY(dalloc(dC, nb * nv * no, s));
     RIMP2_TRY(h2d(deo, EVocc, no, s));
     RIMP2_TRY(h2d(dev, EVvirt, nv, s));
-    RIMP2_TRY(dalloc(dE, no * no, s));
-    RIMP2_TRY(dalloc(dT, 1, s));
+    RIMP2_TRY(dalloc(dE, no * no + 1, s));  // pair energies, total
     // the copy stream must see dC allocated before it writes into it
     cudaEvent_t ready;
     RIMP2_CK(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming));
@@ -1230,28 +1258,23 @@ int rimp2_energy(const int *nvirt, const int *nocc, const int *NBA, const double
     a.eo = deo.as<double>();
     a.ev = dev.as<double>();
     a.Epair = dE.as<double>();
-    a.Etot = dT.as<double>();
+    a.Etot = dE.as<double>() + no * no;
     a.nslices = rimp2_split_nslices(*nvirt, *nocc, *NBA);
     const int chunk = std::max(1, std::min(16, (*nocc + 7) / 8));
     RIMP2_TRY(split_energy_streamed(Calpha, dC.as<double>(), a, s, cs, chunk));
-    RIMP2_TRY(d2h(Epair, dE, no * no, s));
-    RIMP2_TRY(d2h(Etot, dT, 1, s));
     RIMP2_CK(cudaStreamSynchronize(cs));
-    return finish(s);
+    return finish_energies(Epair, Etot, dE.as<double>(), no * no, s);
   }
   RIMP2_TRY(h2d(dC, Calpha, nb * nv * no, s));
   RIMP2_TRY(h2d(deo, EVocc, no, s));
   RIMP2_TRY(h2d(dev, EVvirt, nv, s));
-  RIMP2_TRY(dalloc(dE, no * no, s));
-  RIMP2_TRY(dalloc(dT, 1, s));
+  RIMP2_TRY(dalloc(dE, no * no + 1, s));  // pair energies, total
   if (tamp) RIMP2_TRY(dalloc(dA, nv * no * nv * no, s));
   RIMP2_TRY(rimp2_energy_dev(*nvirt, *nocc, *NBA, dC.as<double>(), deo.as<double>(),
-                             dev.as<double>(), dE.as<double>(), dT.as<double>(),
+                             dev.as<double>(), dE.as<double>(), dE.as<double>() + no * no,
                              tamp ? dA.as<double>() : nullptr, *precision, s));
-  RIMP2_TRY(d2h(Epair, dE, no * no, s));
-  RIMP2_TRY(d2h(Etot, dT, 1, s));
   if (tamp) RIMP2_TRY(d2h(tamp, dA, nv * no * nv * no, s));
-  return finish(s);
+  return finish_energies(Epair, Etot, dE.as<double>(), no * no, s);
 }
 
 int rimp2_energy_batched(const int *nfrag, const int *nocc, const int *nvirt, const int *NBA,

@@ -886,14 +886,17 @@ static int g_energy(const PlainEnergyArgs &a, cudaStream_t s, bool *handled) {
     (void)cudaGetLastError();
     return RIMP2_OK;  // a captured call keeps to the fused kernel (mod_gemm.cu)
   }
-  DevBuf G, pairs, part;
-  RIMP2_TRY(pairs.alloc(sizeof(int) * 2 * (size_t)npairs, s));
-  RIMP2_TRY(part.alloc(sizeof(double) * (size_t)nitems, s));
+  DevBuf arena, G, pairs, part;
   const long long ld = (long long)bo * a.nvirt;
-  if (G.alloc(sizeof(double) * (size_t)ld * ld, s) != RIMP2_OK) {
-    (void)cudaGetLastError();  // no room: the fused kernel needs none
-    clear_error();
-    return RIMP2_OK;
+  {
+    DevBuf *const buf[] = {&G, &pairs, &part};
+    const size_t bytes[] = {sizeof(double) * (size_t)ld * ld, sizeof(int) * 2 * (size_t)npairs,
+                            sizeof(double) * (size_t)nitems};
+    if (alloc_parts(arena, buf, bytes, s) != RIMP2_OK) {
+      (void)cudaGetLastError();  // no room: the fused kernel needs little
+      clear_error();
+      return RIMP2_OK;
+    }
   }
   if (inject_fault("launch")) {
     set_error("injected launch failure (RIMP2_FAULT_INJECT=launch)");

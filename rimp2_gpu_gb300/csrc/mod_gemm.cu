@@ -304,10 +304,13 @@ __device__ __forceinline__ void residues8(const double (&v)[8], int e, bool live
 }
 
 // out[(p * nkc + kc) * rows + row][64]; a block takes 32 rows of one K chunk.
-// A: the rows' operand, B: the columns'.
+// A: the rows' operand, B: the columns'.  SCALE: the rows are one chunk long,
+// the eight threads of a row find its scale themselves (no row_scale launch).
+template <bool SCALE>
 __global__ void __launch_bounds__(256) residue_kernel(const __grid_constant__ OpArgs A,
-                                                      const __grid_constant__ OpArgs B) {
+                                                      const __grid_constant__ OpArgs B, unsigned *list) {
   __shared__ double sh[64][33];
+  if (SCALE && blockIdx.x == 0 && threadIdx.x == 0) *list = 0;  // the count of tiles left to FP64
   const bool second = (int)blockIdx.x >= A.blocks;
   const OpArgs &P = second ? B : A;
   const RowMap &M = P.M;
@@ -342,12 +345,36 @@ __global__ void __launch_bounds__(256) residue_kernel(const __grid_constant__ Op
 #pragma unroll
     for (int u = 0; u < 8; ++u) v[u] = sh[kq * 8 + u][rr];
   }
-  const bool live = !(P.flag[r] & MG_ROW_FP64);
+  int e;
+  unsigned char flag;
+  if (SCALE) {
+    RowStat s{0, 0.0f, MG_NO_LSB, 0};
+#pragma unroll
+    for (int u = 0; u < 8; ++u) stat_add(s, v[u]);
+    const unsigned group = 0xFFu << (threadIdx.x & 24);  // rows leave by groups of eight
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      const int e2 = __shfl_xor_sync(group, s.e, o);
+      const float s2 = __shfl_xor_sync(group, s.ss, o);
+      const int l2 = __shfl_xor_sync(group, s.lsb, o);
+      const int b2 = __shfl_xor_sync(group, s.bad, o);
+      stat_merge(s, e2, s2, l2, b2);
+    }
+    stat_store(s, &e, &flag);
+    if (kq == 0) {
+      P.e[r] = e;
+      P.flag[r] = flag;
+    }
+  } else {
+    e = P.e[r];
+    flag = P.flag[r];
+  }
+  const bool live = !(flag & MG_ROW_FP64);
   __half *out = P.out + ((size_t)kc * P.rows + r) * 64 + kq * 8;
   if (second)
-    residues8<true>(v, P.e[r], live, out, P.plane);
+    residues8<true>(v, e, live, out, P.plane);
   else
-    residues8<false>(v, P.e[r], live, out, P.plane);
+    residues8<false>(v, e, live, out, P.plane);
 }
 
 // --------------------------------------------------------------------------
@@ -356,8 +383,8 @@ __global__ void __launch_bounds__(256) residue_kernel(const __grid_constant__ Op
 // Work item = (plane, 256 columns n x TQ rows m of C): the columns' operand
 // lies on the TMEM lanes (M = 256 over the pair), the rows' operand on the
 // accumulator columns (N = TQ, half of it in each CTA), so that a thread
-// stores runs of bytes along m.  Two TQ-column accumulators per CTA: the
-// MMAs of one item run while the epilogue reduces the other.  Sums longer
+// stores runs of bytes along m.  Two (four) TQ-column accumulators per CTA: the
+// MMAs of one item run while the epilogue reduces another.  Sums longer
 // than 1024 are cut there (exactness) and joined modulo p in the epilogue's
 // registers.  A 64-deep stage is 32 KB per CTA (TQ = 256), six stages.
 // TQ, the rows of C in a tile, is 128 or 64 where 256 would mostly be padding
@@ -367,6 +394,7 @@ constexpr int MG_THREADS = 320;
 constexpr int MG_SEG = 16;  // most K chunks of an exact sum
 constexpr int mg_stage(int tq) { return PANEL_BYTES + tq / 2 * KSTEP * 2; }
 constexpr int mg_nst(int tq) { return tq == 256 ? 6 : 8; }
+constexpr int mg_nacc(int tq) { return tq == 256 ? 2 : 4; }  // accumulators: short sums need more in flight
 constexpr int mg_smem(int tq) { return mg_nst(tq) * mg_stage(tq) + 1024 + 256; }
 
 struct MgParams {
@@ -409,19 +437,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
     mod_gemm_kernel(const __grid_constant__ CUtensorMap tmL, const __grid_constant__ CUtensorMap tmQ,
                     MgParams P) {
   constexpr int NST = mg_nst(TQ), STAGE = mg_stage(TQ);
+  constexpr int NACC = mg_nacc(TQ);
   constexpr int NG = TQ / 32;  // groups of 16 accumulator columns per epilogue warp
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  // bars: full[NST], empty[NST], tfull[2], tempty[2], drain
+  // bars: full[NST], empty[NST], tfull[NACC], tempty[NACC], drain
   uint64_t *bars = (uint64_t *)(base + NST * STAGE);
-  uint32_t *tmem_slot = (uint32_t *)(bars + 2 * NST + 5);
+  uint32_t *tmem_slot = (uint32_t *)(bars + 2 * NST + 2 * NACC + 1);
   volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
   const bool leader = rank == 0;
   const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[NST]);
-  const uint32_t tfull0 = smem_u32(&bars[2 * NST]), tempty0 = smem_u32(&bars[2 * NST + 2]);
-  const uint32_t drain = smem_u32(&bars[2 * NST + 4]);
+  const uint32_t tfull0 = smem_u32(&bars[2 * NST]), tempty0 = smem_u32(&bars[2 * NST + NACC]);
+  const uint32_t drain = smem_u32(&bars[2 * NST + 2 * NACC]);
   const uint32_t full0_L = map_shared(full0, 0), tempty0_L = map_shared(tempty0, 0);
   const uint32_t abort_peer = map_shared(smem_u32((const void *)abort_flag), rank ^ 1u);
   const long long nitems = (long long)MG_PLANES * mg_tiles(P);
@@ -432,7 +461,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
       mbar_init(full0 + 8 * s, 1);   // rank 0: its producer's arrive + both CTAs' bytes
       mbar_init(empty0 + 8 * s, 1);  // multicast MMA commit
     }
-    for (int u = 0; u < 2; ++u) {
+    for (int u = 0; u < NACC; ++u) {
       mbar_init(tfull0 + 8 * u, 1);
       mbar_init(tempty0 + 8 * u, 16);  // the epilogue warps of both CTAs
     }
@@ -499,13 +528,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      long long t = 0;  // sums so far
+      unsigned t = 0;  // sums so far
       for (long long item = pair; item < nitems && ok; item += npair) {
         int p, tl, tq;
         mg_item(P, item, p, tl, tq);
         for (int s0 = 0; s0 < P.nkc && ok; s0 += P.seg, ++t) {
-          const int u = (int)(t & 1);
-          if (t >= 2 && !pair_wait(tempty0 + 8 * u, (uint32_t)(((t >> 1) - 1) & 1), true, abort_flag,
+          const int u = (int)(t % NACC);
+          if (t >= NACC && !pair_wait(tempty0 + 8 * u, (uint32_t)((t / NACC - 1) & 1), true, abort_flag,
                                    abort_peer, P.err, 22)) {
             ok = false;
             break;
@@ -541,7 +570,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
     const int quad = warp & 3, half = (warp - 2) >> 2;
     const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
     const int nl = P.rows_l;
-    long long t = 0;
+    unsigned t = 0;
     bool ok = true;
     for (long long item = pair; item < nitems && ok; item += npair) {
       int p, tl, tq;
@@ -551,8 +580,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
       const float pf = mag ? 1.0f : DT.p[p], inv = mag ? 1.0f : DT.inv[p];
       uint32_t pk[NG][4];
       for (int s0 = 0; s0 < P.nkc; s0 += P.seg, ++t) {
-        const int u = (int)(t & 1);
-        ok = pair_wait(tfull0 + 8 * u, (uint32_t)((t >> 1) & 1), false, abort_flag, abort_peer, P.err, 24);
+        const int u = (int)(t % NACC);
+        ok = pair_wait(tfull0 + 8 * u, (uint32_t)((t / NACC) & 1), false, abort_flag, abort_peer, P.err, 24);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
         tc_fence_after();
@@ -955,30 +984,11 @@ int encode_planes(CUtensorMap &tm, const ModOperand &op, int boxrows) {
   return RIMP2_OK;
 }
 
-// Stream-ordered allocation that leaves no error behind: the caller has
-// another way to compute the product.
-int try_alloc(DevBuf &b, size_t bytes, cudaStream_t s) {
-  const int rc = b.alloc(bytes, s);
-  if (rc != RIMP2_OK) {
-    (void)cudaGetLastError();
-    clear_error();
-  }
-  return rc;
-}
-
 }  // namespace
 
 size_t mod_operand_bytes(int rows, int K) {
   const size_t nkc = (K + 63) / 64;
   return (size_t)MG_PLANES * nkc * rows * 128;
-}
-
-int mod_operand_alloc(ModOperand &op, int rows, int K, cudaStream_t s) {
-  op.rows = rows;
-  op.nkc = (K + 63) / 64;
-  if (try_alloc(op.planes, mod_operand_bytes(rows, K), s) != RIMP2_OK) return RIMP2_ERR_NOMEM;
-  if (try_alloc(op.e, sizeof(int) * (size_t)rows, s) != RIMP2_OK) return RIMP2_ERR_NOMEM;
-  return try_alloc(op.flag, (size_t)rows, s);
 }
 
 namespace {
@@ -1002,12 +1012,18 @@ OpArgs op_args(ModOperand &op, const RowMap &M, int row0, bool used) {
 int fill_operands(ModOperand &Q, const RowMap &A, int r0, bool rows, ModOperand &L, const RowMap &B,
                   int c0, bool cols, unsigned *list, cudaStream_t s) {
   OpArgs a = op_args(Q, A, r0, rows), b = op_args(L, B, c0, cols);
-  row_scale_kernel<<<(unsigned)std::max(1, a.blocks + b.blocks), 256, 0, s>>>(a, b, list);
-  count_launch(1);
+  const bool one = a.nkc == 1 && a.blocks + b.blocks > 0;
+  if (!one) {
+    row_scale_kernel<<<(unsigned)std::max(1, a.blocks + b.blocks), 256, 0, s>>>(a, b, list);
+    count_launch(1);
+  }
   a.blocks = rows ? a.nkc * ((a.rows + 31) / 32) : 0;
   b.blocks = cols ? b.nkc * ((b.rows + 31) / 32) : 0;
   if (a.blocks + b.blocks > 0) {
-    residue_kernel<<<(unsigned)(a.blocks + b.blocks), 256, 0, s>>>(a, b);
+    if (one)
+      residue_kernel<true><<<(unsigned)(a.blocks + b.blocks), 256, 0, s>>>(a, b, list);
+    else
+      residue_kernel<false><<<(unsigned)(a.blocks + b.blocks), 256, 0, s>>>(a, b, list);
     count_launch(1);
   }
   RIMP2_CK(cudaGetLastError());
@@ -1165,11 +1181,26 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
   if ((rb + 63) / 64 > 65535) return RIMP2_OK;
   const long long tiles_m = (ra + 63) / 64, tiles_n = (rb + 63) / 64;
   ModOperand Q, L;
-  DevBuf res, list;
-  if (mod_operand_alloc(Q, ra, g.K, s) != RIMP2_OK || mod_operand_alloc(L, rb, g.K, s) != RIMP2_OK ||
-      try_alloc(res, (size_t)MG_PLANES * rb * ldm, s) != RIMP2_OK ||
-      try_alloc(list, sizeof(unsigned) * (size_t)(tiles_m * tiles_n + 1), s) != RIMP2_OK)
-    return RIMP2_OK;  // no room: the FP64 kernel needs none
+  Q.rows = ra;
+  L.rows = rb;
+  Q.nkc = L.nkc = (g.K + 63) / 64;
+  DevBuf arena, res, list;
+  {
+    DevBuf *const buf[] = {&Q.planes, &L.planes, &res, &Q.e, &L.e, &Q.flag, &L.flag, &list};
+    const size_t bytes[] = {mod_operand_bytes(ra, g.K),
+                            mod_operand_bytes(rb, g.K),
+                            (size_t)MG_PLANES * rb * ldm,
+                            sizeof(int) * (size_t)ra,
+                            sizeof(int) * (size_t)rb,
+                            (size_t)ra,
+                            (size_t)rb,
+                            sizeof(unsigned) * (size_t)(tiles_m * tiles_n + 1)};
+    if (alloc_parts(arena, buf, bytes, s) != RIMP2_OK) {
+      (void)cudaGetLastError();  // no room: the FP64 kernel needs none
+      clear_error();
+      return RIMP2_OK;
+    }
+  }
   ModOrder order(s);
   RIMP2_TRY(order.begin());
   CrtParams P;

@@ -116,7 +116,6 @@ struct ModOperand {
 };
 
 size_t mod_operand_bytes(int rows, int K);
-int mod_operand_alloc(ModOperand &op, int rows, int K, cudaStream_t s);
 // out[plane][n][ldm] = residues of sum_k Q(m,k) L(n,k)
 int mod_product(const ModOperand &L, const ModOperand &Q, signed char *out, long long ldm, bool lower,
                 cudaStream_t s);

@@ -2464,14 +2464,7 @@ int build_group(Group &g, cudaStream_t s, bool single = false) {
                             sizeof(float2) * (size_t)ev,
                             sizeof(double) * (size_t)g.nitems,
                             2 * sizeof(unsigned int)};
-    size_t total = 0;
-    for (size_t n : bytes) total += (n + 255) / 256 * 256;
-    RIMP2_TRY(g.arena.alloc(total, s));
-    char *at = g.arena.as<char>();
-    for (int k = 0; k < 10; ++k) {
-      buf[k]->alias(at, bytes[k], s);
-      at += (bytes[k] + 255) / 256 * 256;
-    }
+    RIMP2_TRY(alloc_parts(g.arena, buf, bytes, s));
   }
   if (!single) {
     RIMP2_CK(cudaMemcpyAsync(g.frags.p, g.fh.data(), sizeof(FragDesc) * g.nfrag,
@@ -4361,9 +4354,7 @@ int split_eos_energy(const double *Ca, const double *const *Ct, int copies, int 
                             sizeof(unsigned int),
                             sizeof(int) * 2 * (size_t)npairs,
                             pair ? sizeof(float) * 2 * 64 * 256 * (size_t)nsm : 16};
-    size_t total = 0;
-    for (size_t n : bytes) total += (n + 255) / 256 * 256;
-    const int rc = arena.alloc(total, s);
+    const int rc = alloc_parts(arena, buf, bytes, s);
     if (rc != RIMP2_OK && copies > 1) {  // no room for both copies at once
       (void)cudaGetLastError();
       clear_error();
@@ -4372,11 +4363,6 @@ int split_eos_energy(const double *Ca, const double *const *Ct, int copies, int 
       return RIMP2_OK;
     }
     RIMP2_TRY(rc);
-    char *at = arena.as<char>();
-    for (int k = 0; k < 10; ++k) {
-      buf[k]->alias(at, bytes[k], s);
-      at += (bytes[k] + 255) / 256 * 256;
-    }
   }
   RIMP2_CK(cudaMemcpyAsync(frags.p, fh, sizeof fh, cudaMemcpyHostToDevice, s));
   const FragDesc *fr = frags.as<FragDesc>();
