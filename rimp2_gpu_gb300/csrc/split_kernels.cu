@@ -2889,49 +2889,59 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 // page (the last index is 8 NBA nbas bytes apart: a chunk would touch 64).
 // GEMM rows are (alpha, mu) -- 16 alpha x 8 mu per CTA tile, row r = a + 16 m
 // -- K = nu in chunks of 64, N = the occupied orbitals (NT <= 80, padded to
-// a multiple of 16).  The AO tensor is read once -- per row group (the 32
-// rows of 16 alpha x 2 mu) one 16 alpha x 64 nu x 2 mu TMA box per chunk
-// (even NBA, 16-byte aligned tensor), or per-thread 8-byte cp.async copies
-// otherwise -- and sliced by the converter warps (an FP32-arithmetic split,
-// split_f32) with a power-of-two scale per (row, K chunk):
+// a multiple of 16).  The AO tensor is read once, in 64-nu chunks of the 32 rows
+// (16 alpha x 2 mu) of a row group by TMA (rows that do not start on 16-byte
+// boundaries in four boxes by parity: 1.35 ms at nbas = 509 of the transform,
+// 1.35 at 510, where per-thread 8-byte copies took 1.94 against 1.65) and sliced
+// by the converter warps (split_chunk) with a power-of-two scale per (row, K chunk):
 // |x 2^e| <= 511.5, so S0 is a 10-bit integer, and with the occupied MO
 // block sliced the same way (per column and chunk, precomputed) every
 // partial sum of S0a S0b over a chunk is below 64 * 511^2 < 2^24: the integer
 // part of each chunk's product is exact in FP32.  Products per element pair:
 // S0 S0 (L0), S0 R1 + R1 S0 + R1 R1 + S0 R2 + R2 S0 (L1).  Each chunk's L0/L1
-// go to one of two TMEM buffers; the epilogue scales them by the row and
-// column scales of that chunk (powers of two: exact) and adds them into a
-// double-float (FP32 hi + lo, two-sum) running total kept in TMEM, so the
-// result carries ~2^-40 of the chunk products' magnitude.  At the end of
-// the tile the totals are converted to FP64 (bits moved, one FP64 add: the
-// FP64 pipe is slow on GB300), staged in shared memory and written as
-// 64-byte runs of 8 mu per (i, alpha).
-// Roles: warps 0-15 converters (row r = 32 (w & 3) + lane, K quarter w >> 2
-// of each chunk: 16 values a thread), warp 16 MMA issuer and TMEM owner.
-// The converter warps are also the epilogue: each is bound to the TMEM lane
-// quadrant of its rows and takes a quarter of the NT columns; in iteration
-// c they slice chunk c and then fold chunk c-1's accumulators into the
-// running totals, while the tensor core runs chunk c.  The four warps of a
-// row group synchronise among themselves only (the chunk maxima exchange),
-// so the groups' latency-bound phases interleave; a group's next box is
-// requested as soon as its warps hold their values (the cp.async form
-// copies after the chunk is handed to the tensor core and prefetches the
-// chunk after that into L2).  The converter warps bound the kernel (issue
-// about 44% active; 3.11 ms at nbas=680, 6.45 ms with all 16 warps in
-// lockstep, a 64-bit integer split, cp.async copies and FP64-pipe
-// conversions).  Every wait is bounded; on expiry the CTA records an error
-// code, drains its copies and MMAs and returns.
+// go to one of two TMEM buffers; the fold scales them by the row and column
+// scales of that chunk (powers of two: exact) and adds them into a double-float
+// (FP32 hi + lo, two-sum) running total in registers, so the result carries
+// ~2^-40 of the chunk products' magnitude.  A tile's last fold writes the totals
+// as FP64 (bits moved, one FP64 add: the FP64 pipe is slow on GB300).
+// Roles: warps 0-15 converters, warp 16 MMA issuer and TMEM owner.  As slicer a
+// converter warp takes a K quarter of one row group, 16 values a thread; the
+// four warps of a group, which exchange the chunk's maxima, sit on the four
+// schedulers, so that each scheduler holds one warp of every group and a group's
+// waits are filled by the others.  In the folds a warp is bound to the TMEM
+// lanes of its quadrant and takes a quarter of the NT columns: in iteration n it
+// slices chunk n and then folds chunk n - 1 while the tensor core runs chunk n.
+// A CTA per SM walks over its tiles without a break between them (the first
+// chunk of a tile is on its way while the last one of the tile before is
+// folded).  Bound by the converter warps (issue 54% active; 52 instructions a
+// value): 1.05 ms of the 1.32 at nbas = 509 (3.0 TB/s; the tensor's bytes alone
+// take 0.48).  Steps at that size, transform: 1.91 ms; totals in registers, boxes
+// by parity and groups across schedulers 1.53; fewer operations to split a value,
+// one arrival a warp 1.46; one CTA per SM over its tiles 1.34; column scales
+// loaded before the wait 1.32.  Prefetching the boxes of a further chunk into L2:
+// 1.43.  Every wait is bounded; on expiry the CTA records an error code, drains
+// its copies and MMAs and returns.
 // --------------------------------------------------------------------------
 constexpr int AH_TA = 16, AH_TM = 8;  // alpha x mu rows of a tile (16 x 8 = 128)
 constexpr int AH_CONV = 16;
 constexpr int AH_THREADS = 32 * (AH_CONV + 1);
 constexpr int AH_NT_MAX = 80;
-constexpr int AH_STG = AH_TA * 9;  // staged output doubles per column
+
+// How an AO chunk reaches shared memory.
+enum : int {
+  AH_COPY,  // per-thread 8-byte copies
+  AH_BOX,   // a TMA box of 16 alpha x 64 k x 2 mu per row group
+  AH_BOX4   // four boxes of 18 alpha x 32 k, one per parity of k and mu
+};
+struct AoMaps {
+  CUtensorMap m[4];
+};
 
 struct AoHalfParams {
   const double *ao;   // (alpha|mu nu), alpha fastest: ao[alpha + NBA (mu + nbas nu)]
-  int NBA, nbas, nocc, NT, nks;
-  int ta_tiles;       // alpha tiles (of 16)
+  int NBA, nbas, nocc, nks;
+  int ta_tiles, tiles;  // alpha tiles (of 16), tiles
+  unsigned shift;     // AH_BOX4: bit 2 (parity of k) + (parity of mu): its box starts 8 bytes early
   const float *sb;    // [chunk][NT] column scales of the sliced occupied MO block
   double *half;       // H[i][alpha][mu]
   uint32_t idesc;
@@ -2940,10 +2950,12 @@ struct AoHalfParams {
 
 constexpr int ah_b_plane(int NT) { return NT * 128; }  // bytes of one B plane (NT rows x 64 FP16)
 constexpr int ah_stage_bytes(int NT) { return 3 * PANEL_BYTES + 3 * ah_b_plane(NT); }
-constexpr int AH_SLOT_BYTES = KSTEP * 128 * 8;  // one FP64 chunk of the tile (64 KB)
-constexpr int ah_smem_bytes(int NT) {
-  return 1024 + 2 * ah_stage_bytes(NT) + AH_SLOT_BYTES + 2 * 4 * 128 * 4 /*row max exchange*/ +
-         2 * 128 * 4 /*row scales*/ + 256 /*barriers, slot*/;
+// one FP64 chunk of the tile: 64 k of 128 rows, in runs of 16 alpha (18 in the
+// form of four boxes)
+constexpr int ah_slot_bytes(int form) { return KSTEP * AH_TM * (form == AH_BOX4 ? 18 : 16) * 8; }
+constexpr int ah_smem_bytes(int form, int NT) {
+  return 1024 + 2 * ah_stage_bytes(NT) + ah_slot_bytes(form) + 2 * 4 * 128 * 4 /*row max exchange*/ +
+         4 * 128 /*row exponents*/ + 256 /*barriers, slot*/;
 }
 
 // 8-byte asynchronous global -> shared copy; src_bytes = 0 fills zeros and
@@ -2953,7 +2965,7 @@ __device__ __forceinline__ void cp_async8_zfill(uint32_t dst, const void *src, u
                : "memory");
 }
 
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float *v) {
   uint32_t r[4];
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
@@ -2962,96 +2974,44 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float (&v)[4]) {
   for (int k = 0; k < 4; ++k) v[k] = __uint_as_float(r[k]);
 }
 
-__device__ __forceinline__ void tmem_st4(uint32_t taddr, const float (&v)[4]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};" ::"r"(taddr),
-               "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
-               "r"(__float_as_uint(v[3]))
-               : "memory");
-}
-
-__device__ __forceinline__ void tmem_wait_st() {
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
-  uint32_t r[8];
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]),
-                 "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-#pragma unroll
-  for (int k = 0; k < 8; ++k) v[k] = __uint_as_float(r[k]);
-}
-
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const float (&v)[8]) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr),
-               "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
-               "r"(__float_as_uint(v[3])), "r"(__float_as_uint(v[4])), "r"(__float_as_uint(v[5])),
-               "r"(__float_as_uint(v[6])), "r"(__float_as_uint(v[7]))
-               : "memory");
-}
-
-// Fold of W columns (4 or 8) of one AO chunk's products into the running
+// Fold of this thread's NC columns of one AO chunk's products into the running
 // double-float totals: L0 and L1 scaled by the row and column powers of two
 // (exact), added to hi/lo with a two-sum of the high parts (first chunk:
-// assigned), written back to TMEM -- or, on the last chunk, turned into
-// FP64 in the staging area ([column][alpha][mu], 9-double pitch per alpha).
-template <int W>
-__device__ __forceinline__ void ah_fold(uint32_t tL0, int NT, uint32_t rs_hi, uint32_t rs_lo,
-                                        int col, float sa, const float *sbc, bool first,
-                                        bool last, double *stg, int a_l, int m_l) {
-  float l0[W], l1[W], hi[W], lo[W], sbk[W];
+// assigned).
+template <int NC>
+__device__ __forceinline__ void ah_fold(uint32_t tL0, uint32_t tL1, float sa,
+                                        const float4 (&sb)[NC / 4], bool first, float (&hi)[NC], float (&lo)[NC]) {
+  constexpr int G = NC <= 16 ? NC : 8;  // columns read at a time (96 registers a thread)
 #pragma unroll
-  for (int q = 0; q < W; q += 4) {  // 16-byte loads (NT and col are multiples of 4)
-    const float4 sb4 = *reinterpret_cast<const float4 *>(sbc + col + q);
-    sbk[q] = sb4.x;
-    sbk[q + 1] = sb4.y;
-    sbk[q + 2] = sb4.z;
-    sbk[q + 3] = sb4.w;
-  }
-  if constexpr (W == 8) {
-    tmem_ld8(tL0 + col, l0);
-    tmem_ld8(tL0 + NT + col, l1);
-    if (!first) {
-      tmem_ld8(rs_hi + col, hi);
-      tmem_ld8(rs_lo + col, lo);
-    }
-  } else {
-    tmem_ld4(tL0 + col, l0);
-    tmem_ld4(tL0 + NT + col, l1);
-    if (!first) {
-      tmem_ld4(rs_hi + col, hi);
-      tmem_ld4(rs_lo + col, lo);
-    }
-  }
-  tmem_wait_ld();
+  for (int g = 0; g < NC; g += G) {
+    float l0[G], l1[G];
 #pragma unroll
-  for (int k = 0; k < W; ++k) {
-    const float sc = sa * sbk[k];  // power of two: the products below are exact
-    const float xh = l0[k] * sc, xl = l1[k] * sc;
-    if (first) {
-      hi[k] = xh;
-      lo[k] = xl;
-    } else {  // two-sum of the high parts, low parts added
-      const float s = hi[k] + xh;
-      const float bv = s - hi[k];
-      const float err = (hi[k] - (s - bv)) + (xh - bv);
-      lo[k] = lo[k] + xl + err;
-      hi[k] = s;
+    for (int q = 0; q < G && g + q < NC; q += 4) {
+      tmem_ld4(tL0 + g + q, l0 + q);
+      tmem_ld4(tL1 + g + q, l1 + q);
     }
-  }
-  if (!last) {
-    if constexpr (W == 8) {
-      tmem_st8(rs_hi + col, hi);
-      tmem_st8(rs_lo + col, lo);
-    } else {
-      tmem_st4(rs_hi + col, hi);
-      tmem_st4(rs_lo + col, lo);
-    }
-  } else {
+    tmem_wait_ld();
 #pragma unroll
-    for (int k = 0; k < W; ++k)  // one FP64 add per output (bit-moved conversions)
-      stg[(col + k) * AH_STG + a_l * 9 + m_l] = f2d_bits(hi[k]) + f2d_bits(lo[k]);
+    for (int q = 0; q < G && g + q < NC; q += 4) {
+      const float4 sb4 = sb[(g + q) / 4];
+      const float sbk[4] = {sb4.x, sb4.y, sb4.z, sb4.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float sc = sa * sbk[k];  // power of two: the products below are exact
+        const float xh = l0[q + k] * sc, xl = l1[q + k] * sc;
+        float &h = hi[g + q + k], &l = lo[g + q + k];
+        if (first) {
+          h = xh;
+          l = xl;
+        } else {  // two-sum of the high parts, low parts added
+          const float t = h + xh;
+          const float bv = t - h;
+          const float err = (h - (t - bv)) + (xh - bv);
+          l = l + xl + err;
+          h = t;
+        }
+      }
+    }
   }
 }
 
@@ -3072,18 +3032,22 @@ __device__ __forceinline__ int chunk_exponent_511(uint32_t key) {
   return max(-126, min(126, e));
 }
 
-// Bounded vote over the converter threads (named barrier 2).
-__device__ __forceinline__ bool conv_any(bool p) {
-  uint32_t r;
-  asm volatile(
-      "{\n\t.reg .pred q, o;\n\t"
-      "setp.ne.u32 q, %1, 0;\n\t"
-      "bar.red.or.pred o, 2, %2, q;\n\t"
-      "selp.u32 %0, 1, 0, o;\n\t}"
-      : "=r"(r)
-      : "r"((uint32_t)p), "r"(32 * AH_CONV)
-      : "memory");
-  return r != 0;
+// split_f32 for the values of a row chunk with exponent e, in fewer
+// operations: shift = (e - 896) << 23 moves the exponent field along with the
+// fraction bits (its value is at most 254: no carry into the sign), and least =
+// (963 - e) << 20 holds |x| 2^e at 2^-60 or above, so that no case needs a
+// select: below 2^-40, zeros and subnormals leave q = 0 and an r whose FP16
+// parts are zero.  q and r are split_f32's otherwise.
+__device__ __forceinline__ void split_chunk(double x, uint32_t least, uint32_t shift, float &q,
+                                            float &r) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t h = max(hi & 0x7FFFFFFFu, least);
+  const uint32_t f = (__funnelshift_l(lo, h, 3) + shift) | (hi & 0x80000000u);
+  const float v = __uint_as_float(f);                // x 2^e to 24 bits
+  const float p = __uint_as_float(f & 0xFF800000u);  // its sign and power of two
+  const float l = fmaf(__uint_as_float(0x4B000000u | ((lo >> 6) & 0x7FFFFFu)), 0x1p-46f, -0x1p-23f);
+  q = (v + 12582912.0f) - 12582912.0f;
+  r = fmaf(l, p, v - q);
 }
 
 // Bounded vote over the 128 converter threads of row group g (the four warps
@@ -3101,22 +3065,25 @@ __device__ __forceinline__ bool group_any(bool p, int g) {
   return r != 0;
 }
 
-template <bool AO_TMA>
+// 17 warps: one scheduler holds five, whose registers allow 96 a thread.
+template <int FORM, int NT>
 __global__ void __maxnreg__(96)
-    ao_half_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmAO,
+    ao_half_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ AoMaps tmAO,
                    AoHalfParams P) {
+  constexpr int NC = NT / 4;  // columns of a converter thread's totals
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *base = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int NT = P.NT;
-  const int BPL = ah_b_plane(NT);
-  const int STAGE = 3 * PANEL_BYTES + 3 * BPL;
+  constexpr int BPL = ah_b_plane(NT);
+  constexpr int STAGE = 3 * PANEL_BYTES + 3 * BPL;
   uint8_t *stages = base;
-  double *slot = (double *)(base + 2 * STAGE);                     // [64 k][128 rows] FP64
-  uint32_t *smx = (uint32_t *)(base + 2 * STAGE + AH_SLOT_BYTES);  // [2 parity][4 quarter][128]
-  float *sscale = (float *)(smx + 2 * 4 * 128);                    // [2][128]
-  uint64_t *bars = (uint64_t *)(sscale + 2 * 128);
+  double *slot = (double *)(base + 2 * STAGE);  // the chunk's FP64 values
+  uint32_t *smx = (uint32_t *)(base + 2 * STAGE + ah_slot_bytes(FORM));  // [2 parity][4 quarter][128]
+  // [4][128]: a group may be two chunks ahead of another warp's fold, not four
+  // (it waits for the MMAs of two chunks before, which waited for every warp)
+  signed char *sexp = (signed char *)(smx + 2 * 4 * 128);
+  uint64_t *bars = (uint64_t *)(sexp + 4 * 128);
   // bars: stage_full[2], stage_empty[2], acc_full[2], acc_empty[2], drain,
-  //       ao_full[4] (the AO chunk of each row group, TMA form)
+  //       ao_full[4] (the AO chunk of each row group, box forms)
   uint32_t *tmem_slot = (uint32_t *)(bars + 13);
   volatile int *abort_flag = (volatile int *)(tmem_slot + 1);
   const uint32_t sfull0 = smem_u32(&bars[0]), sempty0 = smem_u32(&bars[2]);
@@ -3124,13 +3091,14 @@ __global__ void __maxnreg__(96)
   const uint32_t drain = smem_u32(&bars[8]);
   const uint32_t aofull0 = smem_u32(&bars[9]);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int ta = blockIdx.x % P.ta_tiles, tm = blockIdx.x / P.ta_tiles;
-  const int alpha0 = ta * AH_TA, mu0 = tm * AH_TM;
+  // this CTA's tiles: blockIdx.x and every gridDim.x-th after it; its chunks in
+  // one sequence n = 0 ... total - 1
   const int nks = P.nks;
+  const int total = (P.tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x * nks;
 
   if (threadIdx.x == 0) {
     for (int b = 0; b < 2; ++b) {
-      mbar_init(sfull0 + 8 * b, 32 * AH_CONV);  // every converter thread (one with the B bytes)
+      mbar_init(sfull0 + 8 * b, AH_CONV);       // converter warps (one with the B bytes)
       mbar_init(sempty0 + 8 * b, 1);            // MMA commit
       mbar_init(afull0 + 8 * b, 1);             // MMA commit
       mbar_init(aempty0 + 8 * b, AH_CONV);      // converter warps, after reading the chunk
@@ -3140,7 +3108,8 @@ __global__ void __maxnreg__(96)
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&tmB) : "memory");
-    if (AO_TMA) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&tmAO) : "memory");
+    if (FORM != AH_COPY)
+      asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&tmAO.m[0]) : "memory");
   }
   if (warp == AH_CONV) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
@@ -3154,118 +3123,147 @@ __global__ void __maxnreg__(96)
   const uint32_t tmem = *tmem_slot;
 
   if (warp < AH_CONV) {
-    // ------------------------- converters and epilogue ------------------------
-    const int r = 32 * (warp & 3) + lane;  // tile row = TMEM lane of this thread
-    const int kq = warp >> 2;              // K quarter of each chunk; column quarter of N
+    // --------------------------- slicers and folds ----------------------------
+    // as a slicer: tile row r of row group rg, K quarter kq of each chunk
+    const int rg = warp >> 2, kq = warp & 3;
+    const int r = 32 * rg + lane;
     const int a_l = r % AH_TA, m_l = r / AH_TA;
-    const int alpha = alpha0 + a_l, mu = mu0 + m_l;
-    const bool live = alpha < P.NBA && mu < P.nbas;
+    // in the folds: tile row (TMEM lane) re, columns col0 .. col0 + NC
+    const int re = 32 * (warp & 3) + lane, col0 = (warp >> 2) * NC;
+    const uint32_t te = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col0;
     // row (alpha, mu) contracted over the middle index: (alpha|nu mu) =
     // (alpha|mu nu), and the middle index is 8 NBA bytes apart, so a chunk of
     // 64 values stays inside one memory page (the last index: 64 pages)
-    const long long kstride = P.NBA;
-    const double *src = P.ao + (live ? (long long)alpha + (long long)P.NBA * P.nbas * mu : 0);
     const int within = r & 7;
     int armed = -1;  // thread 0: parity of the last stage it armed for the B copy
     int armed_b = 0;
-    // this thread's 16 values of a chunk in the FP64 slot: k = 16 kq + j.
-    // cp.async form: [k][row]; TMA form: one 16 KB box per row group g
-    // (16 alpha x 64 k x 2 mu, alpha fastest), value (a_l, k, m_l) at
-    // g * 2048 + ((m_l & 1) * 64 + k) * 16 + a_l
-    const int rg = warp & 3;
-    double *myslot = AO_TMA ? slot + rg * 2048 + ((m_l & 1) * 64 + 16 * kq) * 16 + a_l
-                            : slot + (16 * kq) * 128 + r;
-    const int jstride = AO_TMA ? 16 : 128;
-    const uint32_t myslot_s = smem_u32(myslot);
+    // this thread's 16 values of a chunk, k = 16 kq + j, in the FP64 slot: even j
+    // at even + (j / 2) pitch, odd j at odd + (j / 2) pitch
+    constexpr int pitch = FORM == AH_COPY ? 256 : FORM == AH_BOX ? 32 : 18;
+    const double *even, *odd;
+    if constexpr (FORM == AH_COPY) {  // [k][row]
+      even = slot + (16 * kq) * 128 + r;
+      odd = even + 128;
+    } else if constexpr (FORM == AH_BOX) {  // [group][mu][k][alpha]
+      even = slot + rg * 2048 + ((m_l & 1) * 64 + 16 * kq) * 16 + a_l;
+      odd = even + 16;
+    } else {  // [group][parity of k][parity of mu][k / 2][alpha + shift]
+      const int mp = m_l & 1;
+      even = slot + rg * 2304 + mp * 576 + 8 * kq * 18 + a_l + (P.shift >> mp & 1);
+      odd = slot + rg * 2304 + (2 + mp) * 576 + 8 * kq * 18 + a_l + (P.shift >> (2 + mp) & 1);
+    }
     const uint32_t aofull = aofull0 + 8 * rg;
-    // TMA form: lane 0 of the group's K-quarter-0 warp issues the group's box
-    const bool ao_issuer = AO_TMA && kq == 0 && lane == 0;
-    int ao_pending = -1;  // parity of a box in flight (issuer)
-    auto issue_box = [&](int c) {
-      mbar_expect_tx(aofull, AH_TA * KSTEP * 2 * 8);
-      asm volatile(
-          "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
-          " [%0], [%1, {%3, %4, %5}], [%2];" ::"r"(smem_u32(slot + rg * 2048)),
-          "l"((uint64_t)&tmAO), "r"(aofull), "r"(alpha0), "r"(c * KSTEP), "r"(mu0 + 2 * rg)
-          : "memory");
-      ao_pending = c & 1;
+    // box forms: lane 0 of the group's K-quarter-0 warp issues the group's boxes
+    const bool ao_issuer = FORM != AH_COPY && kq == 0 && lane == 0;
+    int ao_pending = -1;  // parity of a chunk in flight (issuer)
+    auto issue_box = [&](int n, int tile, int c) {
+      const int alpha0 = tile % P.ta_tiles * AH_TA, mu0 = tile / P.ta_tiles * AH_TM;
+      if constexpr (FORM == AH_BOX) {
+        mbar_expect_tx(aofull, AH_TA * KSTEP * 2 * 8);
+        tma_load_3d(smem_u32(slot + rg * 2048), &tmAO.m[0], aofull, alpha0, c * KSTEP, mu0 + 2 * rg);
+      } else {
+        mbar_expect_tx(aofull, 4 * 576 * 8);
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          tma_load_3d(smem_u32(slot + rg * 2304 + q * 576), &tmAO.m[q], aofull, alpha0,
+                      c * (KSTEP / 2), mu0 / 2 + rg);
+      }
+      ao_pending = n & 1;
     };
     // L2 prefetch of a later chunk: thread t covers the 16-alpha run (128
     // bytes, at most two lines) of k = t / 8 and mu = mu0 + t % 8, so that
     // the chunk's cp.async copies find their data in L2; with one chunk in
     // flight per CTA the copies would otherwise wait out the slowest DRAM
     // access of each chunk
-    const int pf_k = threadIdx.x >> 3, pf_m = mu0 + (threadIdx.x & 7);
-    const int pf_a = min(AH_TA, P.NBA - alpha0);  // alpha values of the tile
-    auto prefetch_chunk = [&](int c) {
-      const int k = c * KSTEP + pf_k;
-      if (k < P.nbas && pf_m < P.nbas) {
-        const double *p = P.ao + alpha0 + (long long)P.NBA * k + (long long)P.NBA * P.nbas * pf_m;
+    auto prefetch_chunk = [&](int tile, int c) {
+      const int alpha0 = tile % P.ta_tiles * AH_TA;
+      const int k = c * KSTEP + (threadIdx.x >> 3);
+      const int mu = tile / P.ta_tiles * AH_TM + (threadIdx.x & 7);
+      if (k < P.nbas && mu < P.nbas) {
+        const double *p = P.ao + alpha0 + (long long)P.NBA * k + (long long)P.NBA * P.nbas * mu;
         asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(p + (pf_a - 1)));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p + (min(AH_TA, P.NBA - alpha0) - 1)));
       }
     };
-    auto issue_chunk = [&](int c) {
+    const uint32_t myslot_s = smem_u32(even);
+    auto issue_chunk = [&](int tile, int c) {
+      const int alpha = tile % P.ta_tiles * AH_TA + a_l, mu = tile / P.ta_tiles * AH_TM + m_l;
+      const bool live = alpha < P.NBA && mu < P.nbas;
       const int k0 = c * KSTEP + 16 * kq;
       const int lim = live ? min(16, P.nbas - k0) : 0;  // values that exist
-      const double *p = src + kstride * k0;
+      const double *p =
+          P.ao + (live ? alpha + (long long)P.NBA * P.nbas * mu : 0) + (long long)P.NBA * k0;
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         cp_async8_zfill(myslot_s + j * 128 * 8, j < lim ? (const void *)p : (const void *)P.ao,
                         j < lim ? 8u : 0u);
-        p += kstride;
+        p += P.NBA;
       }
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    // epilogue of chunk ce: its L0/L1 scaled by the row and column scales of
-    // the chunk and added to the running double-float totals (TMEM), or on
-    // the last chunk turned into FP64 in the staging area
-    const int ncol = NT / 4, col0 = kq * ncol;
-    const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t rs_hi = tmem + lane_off + (uint32_t)(4 * NT);
-    const uint32_t rs_lo = rs_hi + (uint32_t)NT;
-    auto epilogue = [&](int ce) -> bool {
-      const int b = ce & 1;
-      if (!mbar_wait(afull0 + 8 * b, (uint32_t)((ce >> 1) & 1), abort_flag, P.err, 25)) return false;
+    // fold of the n-th chunk (chunk c of the tile) into this thread's totals; the
+    // tile's last one writes them: 16-byte runs of two mu, which the four groups'
+    // stores complete to 64 bytes in L2 (one FP64 add per output, bit-moved
+    // conversions)
+    float hi[NC], lo[NC];
+    auto fold = [&](int n, int tile, int c) -> bool {
+      const int b = n & 1;
+      float4 sb[NC / 4];  // 16-byte loads, before the wait: offsets are multiples of 4
+#pragma unroll
+      for (int q = 0; q < NC / 4; ++q)
+        sb[q] = __ldg(reinterpret_cast<const float4 *>(P.sb + (size_t)c * NT + col0) + q);
+      if (!mbar_wait(afull0 + 8 * b, (uint32_t)((n >> 1) & 1), abort_flag, P.err, 25)) return false;
       tc_fence_after();
-      const float sa = sscale[b * 128 + r];
-      const uint32_t tL0 = tmem + lane_off + (uint32_t)(b * 2 * NT);
-      const float *sbc = P.sb + (size_t)ce * NT;
-      const bool last = ce + 1 == nks;
-      double *stg = reinterpret_cast<double *>(stages);
-      // eight columns per TMEM round trip, four for a remainder
-      int col = col0;
-      for (; col + 8 <= col0 + ncol; col += 8)
-        ah_fold<8>(tL0, NT, rs_hi, rs_lo, col, sa, sbc, ce == 0, last, stg, a_l, m_l);
-      if (col < col0 + ncol)
-        ah_fold<4>(tL0, NT, rs_hi, rs_lo, col, sa, sbc, ce == 0, last, stg, a_l, m_l);
-      if (!last) tmem_wait_st();
+      const uint32_t tL0 = te + (uint32_t)(b * 2 * NT);
+      const float sa = __int_as_float((127 - sexp[(n & 3) * 128 + re]) << 23);  // 2^-e
+      ah_fold<NC>(tL0, tL0 + NT, sa, sb, c == 0, hi, lo);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(aempty0 + 8 * b);
+      if (c + 1 == nks) {
+        const int alpha = tile % P.ta_tiles * AH_TA + re % AH_TA;
+        const int mu = tile / P.ta_tiles * AH_TM + re / AH_TA;
+        if (alpha < P.NBA && mu < P.nbas) {
+          double *o = P.half + ((long long)col0 * P.NBA + alpha) * P.nbas + mu;
+#pragma unroll
+          for (int k = 0; k < NC; ++k) {
+            if (col0 + k < P.nocc) *o = f2d_bits(hi[k]) + f2d_bits(lo[k]);
+            o += (long long)P.NBA * P.nbas;
+          }
+        }
+      }
       return true;
     };
-    bool ok_all = true;
-    if (AO_TMA) {
-      if (ao_issuer) issue_box(0);
+    bool ok_all = true, folded = true;
+    int tile = blockIdx.x, c = 0;
+    auto advance = [&](int &t, int &k) {
+      if (++k == nks) {
+        k = 0;
+        t += gridDim.x;
+      }
+    };
+    if (FORM != AH_COPY) {
+      if (ao_issuer) issue_box(0, tile, 0);
     } else {
-      if (nks > 1) prefetch_chunk(1);
-      issue_chunk(0);
+      issue_chunk(tile, 0);
     }
-    for (int c = 0; c < nks; ++c) {
-      const int b = c & 1;
+    int tp = tile, cp = 0;  // the chunk before
+    for (int n = 0; n < total; ++n) {
+      const int b = n & 1;
+      int tn = tile, cn = c;  // the chunk after
+      advance(tn, cn);
       bool landed = true;
-      if (AO_TMA) {
-        landed = mbar_wait(aofull, (uint32_t)(c & 1), abort_flag, P.err, 26);
+      if (FORM != AH_COPY) {
+        landed = mbar_wait(aofull, (uint32_t)(n & 1), abort_flag, P.err, 26);
         if (ao_issuer && landed) ao_pending = -1;
       } else {
-        if (c + 2 < nks) prefetch_chunk(c + 2);
-        // chunk c has landed (each thread reads only the values it copied)
+        if (n + 1 < total) prefetch_chunk(tn, cn);
+        // chunk n has landed (each thread reads only the values it copied)
         asm volatile("cp.async.wait_group 0;" ::: "memory");
       }
       double v[16];
 #pragma unroll
-      for (int j = 0; j < 16; ++j) v[j] = myslot[j * jstride];
+      for (int j = 0; j < 16; ++j) v[j] = (j & 1 ? odd : even)[(j >> 1) * pitch];
       uint32_t key = 0;
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
@@ -3274,25 +3272,27 @@ __global__ void __maxnreg__(96)
         key = kj > key ? kj : key;
       }
       smx[(b * 4 + kq) * 128 + r] = key;
-      bool ok = landed;
-      if (ok && c >= 2)
-        ok = mbar_wait(sempty0 + 8 * b, (uint32_t)(((c - 2) >> 1) & 1), abort_flag, P.err, 21);
+      bool ok = landed && folded;
+      if (ok && n >= 2)
+        ok = mbar_wait(sempty0 + 8 * b, (uint32_t)(((n - 2) >> 1) & 1), abort_flag, P.err, 21);
       // the four warps of a row group exchange their K quarters' maxima; the
-      // groups do not wait for one another, so their latency-bound phases
-      // (loads, slicing, TMEM round trips) interleave
-      if (group_any(!ok, warp & 3)) {
+      // groups do not wait for one another, and the four warps of a scheduler
+      // belong to four groups, so that their latency-bound phases (loads,
+      // slicing, TMEM round trips) interleave on it
+      if (group_any(!ok, rg)) {
         ok_all = false;
         break;
       }
       // every warp of the group has its values: the group's box is free
-      if (ao_issuer && c + 1 < nks) issue_box(c + 1);
+      if (ao_issuer && n + 1 < total) issue_box(n + 1, tn, cn);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const uint32_t o = smx[(b * 4 + q) * 128 + r];
         key = o > key ? o : key;
       }
       const int e = chunk_exponent_511(key);
-      if (kq == 0) sscale[b * 128 + r] = ldexpf(1.0f, -e);
+      if (kq == 0) sexp[(n & 3) * 128 + r] = (signed char)e;
+      const uint32_t least = (uint32_t)(963 - e) << 20, shift = (uint32_t)(e - 896) << 23;
       uint8_t *st = stages + b * STAGE;
 #pragma unroll
       for (int g = 0; g < 2; ++g) {
@@ -3300,8 +3300,8 @@ __global__ void __maxnreg__(96)
 #pragma unroll
         for (int q = 0; q < 4; ++q) {  // two values at a time, packed conversions
           float qa, ra, qb, rb;
-          split_f32(v[8 * g + 2 * q], e, qa, ra);
-          split_f32(v[8 * g + 2 * q + 1], e, qb, rb);
+          split_chunk(v[8 * g + 2 * q], least, shift, qa, ra);
+          split_chunk(v[8 * g + 2 * q + 1], least, shift, qb, rb);
           h0[q] = __floats2half2_rn(qa, qb);  // |q| <= 512: exact in FP16
           h1[q] = __floats2half2_rn(ra, rb);
           const float2 f1 = __half22float2(h1[q]);
@@ -3315,28 +3315,31 @@ __global__ void __maxnreg__(96)
       }
       // generic-proxy writes of the A panels become visible to the tensor core
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
       if (threadIdx.x == 0) {
         const uint32_t fb = sfull0 + 8 * b;
         mbar_expect_tx(fb, 3 * BPL);
-        armed = (int)((c >> 1) & 1);
+        armed = (int)((n >> 1) & 1);
         armed_b = b;
         const uint32_t dst = smem_u32(st + 3 * PANEL_BYTES);
 #pragma unroll
         for (int p = 0; p < 3; ++p) tma_load_3d(dst + p * BPL, &tmB, fb, 0, 0, 3 * c + p);
-      } else {
+      } else if (lane == 0) {
         mbar_arrive(sfull0 + 8 * b);
       }
-      // the next chunk's copies overlap the previous chunk's epilogue and
-      // the next iteration's start (the L2 prefetch keeps their latency short)
-      if (!AO_TMA && c + 1 < nks) issue_chunk(c + 1);
-      // the previous chunk's epilogue runs while this chunk's MMAs do
-      if (c >= 1 && group_any(!epilogue(c - 1), warp & 3)) {
-        ok_all = false;
-        break;
-      }
+      // the next chunk's copies overlap the previous chunk's fold and the
+      // next iteration's start (the L2 prefetch keeps their latency short)
+      if (FORM == AH_COPY && n + 1 < total) issue_chunk(tn, cn);
+      // the previous chunk is folded while this chunk's MMAs run; a failed
+      // wait is told to the group at its next exchange
+      if (n >= 1) folded = fold(n - 1, tp, cp);
+      tp = tile;
+      cp = c;
+      tile = tn;
+      c = cn;
     }
     // copies still in flight land before the CTA may exit
-    if (AO_TMA) {
+    if (FORM != AH_COPY) {
       if (ao_issuer && ao_pending >= 0) {
         const long long t0 = clock64();
         while (!mbar_test(aofull, (uint32_t)ao_pending) && clock64() - t0 < WAIT_BUDGET) {
@@ -3345,17 +3348,7 @@ __global__ void __maxnreg__(96)
     } else {
       asm volatile("cp.async.wait_all;" ::: "memory");
     }
-    const bool last_ok = ok_all && epilogue(nks - 1);
-    ok_all = !conv_any(!last_ok);  // every converter thread reaches this vote
-    if (ok_all) {
-      const double *stg = reinterpret_cast<const double *>(stages);
-      for (int idx = threadIdx.x; idx < P.nocc * AH_TA * AH_TM; idx += 32 * AH_CONV) {
-        const int ml = idx & 7, al = (idx >> 3) & 15, n = idx >> 7;
-        const int ga = alpha0 + al, gm = mu0 + ml;
-        if (ga < P.NBA && gm < P.nbas)
-          P.half[((long long)n * P.NBA + ga) * P.nbas + gm] = stg[n * AH_STG + al * 9 + ml];
-      }
-    }
+    if (ok_all && folded) fold(total - 1, tp, cp);
     if (threadIdx.x == 0 && armed >= 0 && *abort_flag) {
       // the last B copy completes before the CTA may exit
       const long long t0 = clock64();
@@ -3365,11 +3358,11 @@ __global__ void __maxnreg__(96)
   } else if (warp == AH_CONV) {
     // ------------------------------ MMA issuer -------------------------------
     if (lane == 0) {
-      for (int c = 0; c < nks; ++c) {
-        const int b = c & 1;
-        if (!mbar_wait(sfull0 + 8 * b, (uint32_t)((c >> 1) & 1), abort_flag, P.err, 23)) break;
-        if (c >= 2 &&
-            !mbar_wait(aempty0 + 8 * b, (uint32_t)(((c - 2) >> 1) & 1), abort_flag, P.err, 24))
+      for (int n = 0; n < total; ++n) {
+        const int b = n & 1;
+        if (!mbar_wait(sfull0 + 8 * b, (uint32_t)((n >> 1) & 1), abort_flag, P.err, 23)) break;
+        if (n >= 2 &&
+            !mbar_wait(aempty0 + 8 * b, (uint32_t)(((n - 2) >> 1) & 1), abort_flag, P.err, 24))
           break;
         tc_fence_after();
         const uint32_t sA = smem_u32(stages + b * STAGE);
@@ -4238,38 +4231,65 @@ int ao_half_fused(const double *ao, int NBA, int nbas, const double *Cmo, int no
   P.NBA = NBA;
   P.nbas = nbas;
   P.nocc = nocc;
-  P.NT = NT;
   P.nks = nks;
   P.ta_tiles = (NBA + AH_TA - 1) / AH_TA;
+  P.tiles = (int)ntiles;
   P.sb = sb.as<float>();
   P.half = half;
   P.idesc = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | ((uint32_t)(TILE >> 4) << 24);
   P.err = device_error_word();
-  // The AO chunks arrive by TMA (one 16 alpha x 64 nu x 2 mu box per row
-  // group) when the tensor's strides allow it (NBA even: 16-byte multiples)
-  // and its base is 16-byte aligned; otherwise by per-thread cp.async.
-  CUtensorMap tmAO;
+  // The AO chunks arrive by TMA: in one box per row group where the rows of
+  // the tensor start on 16-byte boundaries (even NBA, aligned base).
+  // Elsewhere every second row along k and every second one along mu are 16-byte
+  // multiples apart: four tensors, one per parity of k and of mu, each starting at
+  // the boundary at or before its first element, in boxes two alpha wider.
+  // Their chunk takes 72 KB instead of 64, which NT = 80 has no room for: it
+  // keeps the copies (nbas = 677: 4.05 ms, against 3.27 at 680 in one box).
+  int form = NBA % 2 == 0 && (uintptr_t)ao % 16 == 0 ? AH_BOX
+             : nbas > 1 && NT < AH_NT_MAX            ? AH_BOX4
+                                                     : AH_COPY;
+  AoMaps tmAO;
   memset(&tmAO, 0, sizeof tmAO);
-  const bool ao_tma = (NBA % 2 == 0) && ((uintptr_t)ao % 16 == 0);
-  if (ao_tma) {
-    cuuint64_t adims[3] = {(cuuint64_t)NBA, (cuuint64_t)nbas, (cuuint64_t)nbas};
-    cuuint64_t astr[2] = {(cuuint64_t)NBA * 8, (cuuint64_t)NBA * nbas * 8};
-    cuuint32_t abox[3] = {AH_TA, KSTEP, 2};
-    cr = encode(&tmAO, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double *>(ao), adims, astr,
-                abox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+  P.shift = 0;
+  for (int q = 0; q < (form == AH_COPY ? 0 : form == AH_BOX ? 1 : 4); ++q) {
+    const int kp = q >> 1, mp = q & 1, step = form == AH_BOX ? 1 : 2;
+    const double *first = ao + (size_t)kp * NBA + (size_t)mp * NBA * nbas;
+    const unsigned sh = (uintptr_t)first % 16 ? 1 : 0;
+    P.shift |= sh << q;
+    cuuint64_t adims[3] = {(cuuint64_t)NBA + sh, (cuuint64_t)((nbas - kp + step - 1) / step),
+                           (cuuint64_t)((nbas - mp + step - 1) / step)};
+    cuuint64_t astr[2] = {(cuuint64_t)step * NBA * 8, (cuuint64_t)step * NBA * nbas * 8};
+    cuuint32_t abox[3] = {(cuuint32_t)(form == AH_BOX ? AH_TA : AH_TA + 2),
+                          (cuuint32_t)(KSTEP / step), (cuuint32_t)(form == AH_BOX ? 2 : 1)};
+    cr = encode(&tmAO.m[q], CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3, const_cast<double *>(first - sh), adims,
+                astr, abox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (cr != CUDA_SUCCESS) {
       set_error("cuTensorMapEncodeTiled (AO tensor) failed (%d)", (int)cr);
       return RIMP2_ERR_CUDA;
     }
   }
-  auto kern = ao_tma ? ao_half_kernel<true> : ao_half_kernel<false>;
-  const int smem = ah_smem_bytes(NT);
+  void (*kern)(CUtensorMap, AoMaps, AoHalfParams) = nullptr;
+  switch (NT) {
+    case 16:
+      kern = form == AH_BOX    ? ao_half_kernel<AH_BOX, 16>
+             : form == AH_BOX4 ? ao_half_kernel<AH_BOX4, 16>
+                               : ao_half_kernel<AH_COPY, 16>;  // one function
+      break;
+    case 32: kern = form == AH_BOX ? ao_half_kernel<AH_BOX, 32> : ao_half_kernel<AH_BOX4, 32>; break;
+    case 48: kern = form == AH_BOX ? ao_half_kernel<AH_BOX, 48> : ao_half_kernel<AH_BOX4, 48>; break;
+    case 64: kern = form == AH_BOX ? ao_half_kernel<AH_BOX, 64> : ao_half_kernel<AH_BOX4, 64>; break;
+    default: kern = form == AH_BOX ? ao_half_kernel<AH_BOX, 80> : ao_half_kernel<AH_COPY, 80>;
+  }
+  const int smem = ah_smem_bytes(form, NT);
   RIMP2_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   int resident = 0;
   RIMP2_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kern, AH_THREADS, smem));
   if (resident < 1) return RIMP2_OK;  // cannot be resident here: the sliced path runs
-  kern<<<(unsigned)ntiles, AH_THREADS, smem, s>>>(tm, tmAO, P);
+  int dev = 0, nsm = 0;
+  RIMP2_CK(cudaGetDevice(&dev));
+  RIMP2_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  kern<<<(unsigned)std::min<long long>(ntiles, nsm), AH_THREADS, smem, s>>>(tm, tmAO, P);
   count_launch(1);
   RIMP2_CK(cudaGetLastError());
   *handled = true;

@@ -171,3 +171,69 @@ def test_split_ao2mo_sliced_first_half(monkeypatch, NBA, nbas, nocc):
     api.sync_status()
     a, b = osp.cpu().numpy(), o64.cpu().numpy()
     assert np.abs(a - b).max() / np.abs(b).max() <= 1e-8
+
+
+@pytest.mark.parametrize("NBA,nbas,nocc", [(17, 2, 1), (16, 65, 16), (33, 64, 17), (75, 129, 33),
+                                           (48, 130, 64), (31, 83, 65), (47, 101, 80), (335, 131, 20)])
+def test_split_ao2mo_tensor_alignment(monkeypatch, NBA, nbas, nocc):
+    """The fused first half reads the AO tensor in one box per chunk where its
+    rows start on 16-byte boundaries, in four boxes by the parities of the two
+    AO indices elsewhere (odd NBA, a base 8 bytes off), by copies for 65 to 80
+    orbitals.  Every output element depends on its own row alone, and the same
+    operations follow: equal bits, whatever the way in."""
+    import torch
+    from rimp2_gpu_gb300 import api
+    nvirt = nbas - nocc
+    even = NBA + NBA % 2
+    full = np.asfortranarray(np.random.default_rng(NBA).standard_normal((even, nbas, nbas)))
+    full = np.asfortranarray(full + full.transpose(0, 2, 1))
+    dC = t(O.gen_mo(19, nbas))
+
+    def run(n, offset):
+        buf = torch.full((n * nbas * nbas + 8,), float("nan"), dtype=torch.float64, device="cuda")
+        buf[offset:offset + n * nbas * nbas] = t(full[:n])
+        out = torch.zeros(n * nvirt * nocc, dtype=torch.float64, device="cuda")
+        before = api.kernel_launch_count()
+        api.ao2mo_dev(n, nbas, nocc, nvirt, buf.data_ptr() + 8 * offset, dC.data_ptr(),
+                      out.data_ptr(), split=True)
+        launches.append(api.kernel_launch_count() - before)
+        torch.cuda.synchronize()
+        api.sync_status()
+        return out.cpu().numpy().reshape(nocc * nvirt, n)[:, :NBA]
+
+    launches = []
+    with monkeypatch.context() as m:
+        m.setenv("RIMP2_AO_FUSED", "0")
+        run(even, 0)
+    sliced = launches.pop()
+    want = run(even, 0)
+    assert np.isfinite(want).all() and np.abs(want).max() > 0
+    for n, offset in ((even, 1), (NBA, 0), (NBA, 1)):
+        assert np.array_equal(run(n, offset), want), (n, offset)
+    assert max(launches) < sliced  # every call took the fused kernel
+
+
+@pytest.mark.parametrize("NBA,nbas,nocc", [(33, 70, 9), (32, 129, 40)])
+def test_split_ao2mo_wide_range(NBA, nbas, nocc):
+    """AO values over 90 powers of two within a row, zeros, a subnormal and rows of
+    zeros: 1e-8 of the largest element against the FP64 form, zeros for the
+    rows of zeros."""
+    import torch
+    from rimp2_gpu_gb300 import api
+    nvirt = nbas - nocc
+    rng = np.random.default_rng(nbas)
+    x = rng.standard_normal((NBA, nbas, nbas)) * 2.0 ** -rng.integers(0, 90, (NBA, nbas, nbas))
+    x[rng.random(x.shape) < 0.1] = 0.0
+    x[3, 1, 2] = 5e-324
+    x[5] = 0.0
+    dao = t(np.asfortranarray(x + x.transpose(0, 2, 1)))
+    dC = t(O.gen_mo(23, nbas))
+    out = []
+    for split in (False, True):
+        o = torch.zeros(NBA * nvirt * nocc, dtype=torch.float64, device="cuda")
+        api.ao2mo_dev(NBA, nbas, nocc, nvirt, dao.data_ptr(), dC.data_ptr(), o.data_ptr(), split=split)
+        torch.cuda.synchronize()
+        api.sync_status()
+        out.append(o.cpu().numpy().reshape(-1, NBA))
+    assert np.abs(out[1] - out[0]).max() <= 1e-8 * np.abs(out[0]).max()
+    assert (out[1][:, 5] == 0).all()
