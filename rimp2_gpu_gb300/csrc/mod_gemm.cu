@@ -413,10 +413,10 @@ __host__ __device__ inline int mg_tiles(const MgParams &P) {
   return P.lower ? P.tiles_q * (P.tiles_q + 1) / 2 : P.tiles_l * P.tiles_q;
 }
 
-__device__ __forceinline__ void mg_item(const MgParams &P, long long item, int &plane, int &tl, int &tq) {
+__device__ __forceinline__ void mg_item(const MgParams &P, int item, int &plane, int &tl, int &tq) {
   const int tiles = mg_tiles(P);
-  plane = (int)(item / tiles);
-  const int t = (int)(item % tiles);
+  plane = item / tiles;
+  const int t = item % tiles;
   if (P.lower) {
     int q = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
     while ((q + 1) * (q + 2) / 2 <= t) ++q;
@@ -453,7 +453,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
   const uint32_t drain = smem_u32(&bars[2 * NST + 2 * NACC]);
   const uint32_t full0_L = map_shared(full0, 0), tempty0_L = map_shared(tempty0, 0);
   const uint32_t abort_peer = map_shared(smem_u32((const void *)abort_flag), rank ^ 1u);
-  const long long nitems = (long long)MG_PLANES * mg_tiles(P);
+  const int nitems = MG_PLANES * mg_tiles(P);
   const int pair = blockIdx.x >> 1, npair = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
@@ -490,7 +490,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
       int stage = 0;
       uint32_t phase = 0, armed = 0, armed_par = 0;
       bool ok = true;
-      for (long long item = pair; item < nitems && ok; item += npair) {
+      for (int item = pair; item < nitems && ok; item += npair) {
         int p, tl, tq;
         mg_item(P, item, p, tl, tq);
         const int rl = tl * 256 + 128 * (int)rank, rq = tq * TQ + TQ / 2 * (int)rank;
@@ -529,7 +529,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
       uint32_t phase = 0;
       bool ok = true;
       unsigned t = 0;  // sums so far
-      for (long long item = pair; item < nitems && ok; item += npair) {
+      for (int item = pair; item < nitems && ok; item += npair) {
         int p, tl, tq;
         mg_item(P, item, p, tl, tq);
         for (int s0 = 0; s0 < P.nkc && ok; s0 += P.seg, ++t) {
@@ -572,7 +572,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
     const int nl = P.rows_l;
     unsigned t = 0;
     bool ok = true;
-    for (long long item = pair; item < nitems && ok; item += npair) {
+    for (int item = pair; item < nitems && ok; item += npair) {
       int p, tl, tq;
       mg_item(P, item, p, tl, tq);
       const int n = tl * 256 + 128 * (int)rank + quad * 32 + lane;
@@ -619,7 +619,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive_remote(tempty0_L + 8 * u);
+        if (lane == 0) mbar_arrive_relaxed(tempty0_L + 8 * u);
       }
       if (ok && n < nl) {
         signed char *o = P.out + ((long long)p * nl + n) * P.ldm + tq * TQ + half * (TQ / 2);
@@ -755,34 +755,44 @@ __device__ __forceinline__ bool needs_fp64(unsigned f, unsigned fn, unsigned mea
          (!((f | fn) & MG_ROW_ZERO) && !(f & fn & MG_ROW_EXACT) && !measured);
 }
 
+// What becomes of the products: every FP64 operation, a comparison or one
+// whose result is not used too, takes half a clock of the SM an element, so that
+// the common forms are instances of their own.
+enum : int { CRT_ANY, CRT_PLAIN /* C = v */, CRT_MINUS /* C -= v */, CRT_QUOTIENT /* C = v / d */ };
+
 // What a row or column of C brings to its elements.
 struct Side {
   long long off;   // in C
   double eo, ev;   // orbital energies of its indices
 };
+template <int MODE>
 __device__ __forceinline__ Side side(const CrtParams &P, const RowMap &M, int r) {
   Side s;
   s.off = c_off(M, r);
-  s.eo = P.denom ? P.eo[role_index(M, r, 1)] : 0.0;
-  s.ev = P.denom ? P.ev[role_index(M, r, 0)] : 0.0;
+  s.eo = s.ev = 0.0;
+  if (MODE == CRT_QUOTIENT || (MODE == CRT_ANY && P.denom)) {
+    s.eo = P.eo[role_index(M, r, 1)];
+    s.ev = P.ev[role_index(M, r, 0)];
+  }
   return s;
 }
 
 // A block takes 64 rows x 64 columns of C; a thread four consecutive rows of
-// four columns.  It reads 17 bytes and writes 8 per element; about 150
+// two columns.  It reads 17 bytes and writes 8 per element; about 150
 // instructions an element bound it, so what only depends on the row or the
 // column (offsets, orbital energies) is formed once.  A symmetric product (g
 // of one set of vectors with itself) has only the tiles m >= n: C(n,m) is
 // written along with C(m,n) through shared memory, with the same denominator
 // (the reference subtracts the two virtual energies in the other order there).
-__global__ void __launch_bounds__(256) crt_epilogue_kernel(const __grid_constant__ CrtParams P) {
+template <int MODE>
+__global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_constant__ CrtParams P) {
   __shared__ int count;
   __shared__ long long rows[64], cols[64];  // symmetric: offsets of the mirror's columns
   extern __shared__ double S[];             // symmetric: [64][65]
   const int tm = blockIdx.x, tn = blockIdx.y;
   if ((P.lower || P.sym) && tm < tn) return;
   const int t0 = threadIdx.x & 15, t1 = threadIdx.x >> 4;
-  const int mq = (P.nfast ? t1 : t0) * 4, nq = P.nfast ? t0 : t1;
+  const int mq = (P.nfast ? t1 & 15 : t0) * 4, nq = P.nfast ? t0 + (t1 & 16) : t1;
   const int m0 = tm * 64 + mq, n0 = tn * 64 + nq;
   const long long plane = (long long)P.nn * P.ldm;
   const bool mirror = P.sym && tm != tn;
@@ -798,8 +808,8 @@ __global__ void __launch_bounds__(256) crt_epilogue_kernel(const __grid_constant
 #pragma unroll
   for (int k = 0; k < 4; ++k) fm |= (unsigned)(m0 + k < P.nm ? P.fa[m0 + k] : (unsigned)MG_ROW_ZERO) << (8 * k);
 #pragma unroll
-  for (int y = 0; y < 4; ++y) {
-    const int n = n0 + 16 * y;
+  for (int y = 0; y < 2; ++y) {
+    const int n = n0 + 32 * y;
     if (n >= P.nn) continue;
     const unsigned g = *reinterpret_cast<const unsigned *>(P.res + MG_P * plane + n * P.ldm + m0);
     const unsigned fn = P.fb[n];
@@ -819,27 +829,29 @@ __global__ void __launch_bounds__(256) crt_epilogue_kernel(const __grid_constant
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     ea[k] = m0 + k < P.nm ? P.ea[m0 + k] : 0;
-    if (m0 + k < P.nm) sm[k] = side(P, P.A, P.row0 + m0 + k);
+    if (m0 + k < P.nm) sm[k] = side<MODE>(P, P.A, P.row0 + m0 + k);
   }
   auto put = [&](const Side &a, const Side &b, int k, int y, double v) {
-    if (P.denom) v = div_f64(v, a.eo + b.eo - b.ev - a.ev);  // RIMP2.F90:403-404
-    if (P.alpha != 1.0) v *= P.alpha;
-    if (mirror) S[(mq + k) * 65 + nq + 16 * y] = v;
+    if (MODE == CRT_QUOTIENT || (MODE == CRT_ANY && P.denom))
+      v = div_f64(v, a.eo + b.eo - b.ev - a.ev);  // RIMP2.F90:403-404
+    if (MODE == CRT_ANY && P.alpha != 1.0) v *= P.alpha;
+    if (mirror) S[(mq + k) * 65 + nq + 32 * y] = v;
     double *c = P.C + a.off + b.off;
-    if (P.beta != 0.0) v += P.beta * *c;
+    if (MODE == CRT_MINUS) v = *c - v;
+    if (MODE == CRT_ANY && P.beta != 0.0) v += P.beta * *c;
     *c = v;
   };
   unsigned small = 0;
 #pragma unroll 1
-  for (int y = 0; y < 4; ++y) {
-    const int n = n0 + 16 * y;
+  for (int y = 0; y < 2; ++y) {
+    const int n = n0 + 32 * y;
     if (n < P.nn) {
       unsigned w[MG_P];
       const signed char *src = P.res + n * P.ldm + m0;
 #pragma unroll
       for (int p = 0; p < MG_P; ++p) w[p] = *reinterpret_cast<const unsigned *>(src + p * plane);
       const int eb = P.eb[n];
-      const Side sn = side(P, P.B, P.col0 + n);
+      const Side sn = side<MODE>(P, P.B, P.col0 + n);
       // 4 x 4 byte transposes: r[k][q] holds planes 4q .. 4q+3 of row m0 + k
       unsigned r[4][4];
 #pragma unroll
@@ -865,10 +877,10 @@ __global__ void __launch_bounds__(256) crt_epilogue_kernel(const __grid_constant
   // the few others: exact integers, or a sum in FP64 by one warp
   if (__any_sync(0xffffffffu, small | todo)) {
 #pragma unroll 1
-    for (int x = 0; x < 16; ++x) {
-      const int k = x & 3, y = x >> 2, n = n0 + 16 * y;
+    for (int x = 0; x < 8; ++x) {
+      const int k = x & 3, y = x >> 2, n = n0 + 32 * y;
       if ((small >> x) & 1u)
-        put(side(P, P.A, P.row0 + m0 + k), side(P, P.B, P.col0 + n), k, y,
+        put(side<MODE>(P, P.A, P.row0 + m0 + k), side<MODE>(P, P.B, P.col0 + n), k, y,
             crt_small(P.res + n * P.ldm + m0 + k, plane, P.ea[m0 + k] + P.eb[n]));
       unsigned mask = __ballot_sync(0xffffffffu, (todo >> x) & 1u);
       while (mask) {
@@ -881,7 +893,7 @@ __global__ void __launch_bounds__(256) crt_epilogue_kernel(const __grid_constant
         for (int q = lane; q < P.A.K; q += 32) s = fma(a[q * P.A.sk], b[q * P.B.sk], s);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == src) put(side(P, P.A, m), side(P, P.B, nn), k, y, s);
+        if (lane == src) put(side<MODE>(P, P.A, m), side<MODE>(P, P.B, nn), k, y, s);
       }
     }
   }
@@ -890,7 +902,7 @@ __global__ void __launch_bounds__(256) crt_epilogue_kernel(const __grid_constant
   // C(n, m): rows along n are the fast direction here
   const int c = threadIdx.x & 63;
   if (tn * 64 + c < P.nn)
-    for (int r = threadIdx.x >> 6; r < 64 && tm * 64 + r < P.nm; r += 4)
+    for (int r = threadIdx.x >> 6; r < 64 && tm * 64 + r < P.nm; r += 8)
       P.C[cols[c] + rows[r]] = S[r * 65 + c];
 }
 
@@ -1222,6 +1234,10 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
           memcmp(A.ext, B.ext, sizeof A.ext) == 0 && memcmp(A.st, B.st, sizeof A.st) == 0 &&
           memcmp(A.role, B.role, sizeof A.role) == 0;
   constexpr int mirror_smem = 64 * 65 * (int)sizeof(double);
+  const bool plain = g.alpha == 1.0 && g.beta == 0.0;
+  auto *crt = plain ? (g.denom ? crt_epilogue_kernel<CRT_QUOTIENT> : crt_epilogue_kernel<CRT_PLAIN>)
+              : !g.denom && g.alpha == -1.0 && g.beta == 1.0 ? crt_epilogue_kernel<CRT_MINUS>
+                                                             : crt_epilogue_kernel<CRT_ANY>;
   P.list = list.as<unsigned>();
   P.ea = Q.e.as<int>();
   P.fa = Q.flag.as<unsigned char>();
@@ -1241,7 +1257,7 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
       P.ldm = ((long long)Q.rows + 255) / 256 * 256;
       RIMP2_TRY(mod_product(L, Q, res.as<signed char>(), P.ldm, g.lower || P.sym, s));
       dim3 grid((unsigned)((P.nm + 63) / 64), (unsigned)((P.nn + 63) / 64));
-      crt_epilogue_kernel<<<grid, 256, P.sym ? mirror_smem : 0, s>>>(P);
+      crt<<<grid, 512, P.sym ? mirror_smem : 0, s>>>(P);
       const long long nt = (long long)grid.x * grid.y;
       dmma_tiles_kernel<<<(unsigned)std::min<long long>(nt, 304), 256, 0, s>>>(P, (int)grid.x);
       count_launch(2);

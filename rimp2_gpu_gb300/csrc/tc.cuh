@@ -185,6 +185,14 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
                : "memory");
 }
 
+// The same without the release: it does not wait for the thread's stores to global
+// memory.  For an arrival that only says that TMEM has been read (the loads are
+// complete, tcgen05.fence::before_thread_sync precedes it).
+__device__ __forceinline__ void mbar_arrive_relaxed(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr)
+               : "memory");
+}
+
 __device__ __forceinline__ bool mbar_test_cl(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
