@@ -15,7 +15,8 @@
 //   3. residues are at most 128 in magnitude, exact in FP16, and 1024 of their
 //      products sum to at most 2^24: the FP32 accumulation of the tensor core
 //      is exact, whatever its internal rounding;
-//   4. the fraction X/P = sum_p r_p / p mod 1 is summed in 96-bit fixed point,
+//   4. the fraction X/P = sum_p r_p w_p / p mod 1, w_p = (P/p)^-1 mod p (Chinese
+//      remainder theorem), is summed in 96-bit fixed point,
 //      multiplied by P and rounded once to FP64 (a fraction below 2^-28 is
 //      redone in exact integers): a sum that FP64 can hold comes out exact.
 // Everything between the rounding to 62-bit integers and the final rounding
@@ -60,9 +61,9 @@ typedef unsigned __int128 u128;
 // itself).
 struct ModTables {
   float p[MG_P], inv[MG_P];
-  float ca[MG_P][5];      // 2^(13 l) mod p, symmetric: A's limbs
-  float cb[MG_P][5];      // the same times (P/p)^-1 mod p: B's limbs
-  unsigned phi[4][12];    // byte b of round(2^96 / p) for p = 4q .. 4q+3
+  float limb[MG_P][5];    // 2^(13 l) mod p, symmetric
+  int w[MG_P];            // (P/p)^-1 mod p, symmetric
+  unsigned phi[4][12];    // byte b of round(2^96 (w / p mod 1)) for p = 4q .. 4q+3
   unsigned long long pm;  // P 2^-62
   unsigned long long plo, phi64;         // P
   unsigned long long wlo[MG_P], whi[MG_P];  // P / p
@@ -89,12 +90,11 @@ constexpr ModTables make_tables() {
       if ((long long)x * q % p == 1) inv = x;
     long long w = 1;
     for (int l = 0; l < 5; ++l) {
-      t.ca[i][l] = (float)sym(w, p);
-      t.cb[i][l] = (float)sym(w * inv, p);
+      t.limb[i][l] = (float)sym(w, p);
       w = w * 8192 % p;
     }
-    const u128 one = (u128)1 << 96;
-    const u128 phi = (one + (u128)(p / 2)) / (u128)p;
+    t.w[i] = sym(inv, p);
+    const u128 phi = (((u128)inv << 96) + (u128)(p / 2)) / (u128)p;  // inv < p: below 2^96
     for (int b = 0; b < 12; ++b)
       t.phi[i >> 2][b] |= (unsigned)((phi >> (8 * b)) & 0xFF) << (8 * (i & 3));
     const u128 w128 = P / (u128)p;
@@ -257,7 +257,6 @@ __device__ __forceinline__ unsigned long long to_int(double x, int e) {
 // Five 13-bit limbs times the residues of 2^(13 l), summed in FP32 (exact:
 // below 2^23), reduced once, packed to FP16 with the value's sign.  FP32
 // arithmetic bounds it: 9 operations per value and modulus.
-template <bool COL>
 __device__ __forceinline__ void residues8(const double (&v)[8], int e, bool live,
                                           __half *__restrict__ out, size_t plane) {
   float l[5][8];
@@ -289,10 +288,10 @@ __device__ __forceinline__ void residues8(const double (&v)[8], int e, bool live
       float r[2];
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        float y = l[0][u + h] * (COL ? DT.cb[p][0] : DT.ca[p][0]);
+        float y = l[0][u + h] * DT.limb[p][0];
 #pragma unroll
         for (int q = 1; q < 5; ++q)
-          y = fmaf(l[q][u + h], (COL ? DT.cb[p][q] : DT.ca[p][q]), y);
+          y = fmaf(l[q][u + h], DT.limb[p][q], y);
         const float q = fmaf(y, inv, MAGIC) - MAGIC;
         r[h] = fmaf(-q, pf, y);
       }
@@ -371,10 +370,7 @@ __global__ void __launch_bounds__(256) residue_kernel(const __grid_constant__ Op
   }
   const bool live = !(flag & MG_ROW_FP64);
   __half *out = P.out + ((size_t)kc * P.rows + r) * 64 + kq * 8;
-  if (second)
-    residues8<true>(v, e, live, out, P.plane);
-  else
-    residues8<false>(v, e, live, out, P.plane);
+  residues8(v, e, live, out, P.plane);
 }
 
 // --------------------------------------------------------------------------
@@ -668,8 +664,8 @@ __device__ __forceinline__ double assemble(unsigned long long m, int x, bool neg
   return __longlong_as_double((long long)(bits | (neg ? 0x8000000000000000ull : 0ull)));
 }
 
-// X 2^-eab where |X / P| < 2^-28: X = sum_p r_p P/p - k P in 128-bit integers
-// (wrapping), k the whole part of sum_p r_p / p.  Sums that cancel exactly,
+// X 2^-eab where |X / P| < 2^-28: X = sum_p v_p P/p - k P in 128-bit integers
+// (wrapping), v_p = r_p w_p mod p, k the whole part of sum_p v_p / p.  Sums that cancel exactly,
 // or nearly, come here: the fraction's 96 bits would leave them too few.
 // src: the element's residues, one byte per plane.
 __device__ __forceinline__ double crt_small(const signed char *src, long long plane, int eab) {
@@ -677,7 +673,8 @@ __device__ __forceinline__ double crt_small(const signed char *src, long long pl
   float ks = 0.0f;
 #pragma unroll 4
   for (int p = 0; p < MG_P; ++p) {
-    const long long v = src[p * plane];
+    const int rw = src[p * plane] * DT.w[p];
+    const long long v = rw - (int)rintf((float)rw * DT.inv[p]) * (int)DT.p[p];
     ks = fmaf((float)v, DT.inv[p], ks);
     const unsigned long long w = DT.wlo[p], q = lo + w * (unsigned long long)v;
     hi += DT.whi[p] * (unsigned long long)v + (unsigned long long)__mul64hi((long long)w, v) +
@@ -1196,11 +1193,14 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
   Q.rows = ra;
   L.rows = rb;
   Q.nkc = L.nkc = (g.K + 63) / 64;
+  // a product of one set of vectors with itself needs their residues once
+  const bool same = ra == A.rows && rb == B.rows && A.rows == B.rows && A.base == B.base && A.sk == B.sk &&
+                    memcmp(A.ext, B.ext, sizeof A.ext) == 0 && memcmp(A.st, B.st, sizeof A.st) == 0;
   DevBuf arena, res, list;
   {
     DevBuf *const buf[] = {&Q.planes, &L.planes, &res, &Q.e, &L.e, &Q.flag, &L.flag, &list};
     const size_t bytes[] = {mod_operand_bytes(ra, g.K),
-                            mod_operand_bytes(rb, g.K),
+                            same ? 0 : mod_operand_bytes(rb, g.K),
                             (size_t)MG_PLANES * rb * ldm,
                             sizeof(int) * (size_t)ra,
                             sizeof(int) * (size_t)rb,
@@ -1212,6 +1212,11 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
       clear_error();
       return RIMP2_OK;
     }
+  }
+  if (same) {
+    L.planes.alias(Q.planes.p, Q.planes.n, s);
+    L.e.alias(Q.e.p, Q.e.n, s);
+    L.flag.alias(Q.flag.p, Q.flag.n, s);
   }
   ModOrder order(s);
   RIMP2_TRY(order.begin());
@@ -1228,11 +1233,7 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
   P.denom = g.denom;
   P.lower = g.lower;
   P.nfast = B.cst[0] < A.cst[0];
-  // the product of a set of vectors with itself
-  P.sym = !g.lower && g.beta == 0.0 && ra == A.rows && rb == B.rows && A.rows == B.rows && A.rows > 256 &&
-          A.base == B.base && A.sk == B.sk &&
-          memcmp(A.ext, B.ext, sizeof A.ext) == 0 && memcmp(A.st, B.st, sizeof A.st) == 0 &&
-          memcmp(A.role, B.role, sizeof A.role) == 0;
+  P.sym = same && !g.lower && g.beta == 0.0 && A.rows > 256 && memcmp(A.role, B.role, sizeof A.role) == 0;
   constexpr int mirror_smem = 64 * 65 * (int)sizeof(double);
   const bool plain = g.alpha == 1.0 && g.beta == 0.0;
   auto *crt = plain ? (g.denom ? crt_epilogue_kernel<CRT_QUOTIENT> : crt_epilogue_kernel<CRT_PLAIN>)
@@ -1247,8 +1248,8 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
     Q.rows = std::min(ra, A.rows - r0);
     for (int c0 = 0; c0 < B.rows; c0 += rb) {
       const int nc = std::min(rb, B.rows - c0);
-      const bool cols = r0 == 0 || rb < B.rows;
-      if (cols) L.rows = nc;
+      const bool cols = !same && (r0 == 0 || rb < B.rows);
+      if (cols || same) L.rows = nc;
       RIMP2_TRY(fill_operands(Q, A, r0, c0 == 0, L, B, c0, cols, list.as<unsigned>(), s));
       P.row0 = r0;
       P.col0 = c0;
