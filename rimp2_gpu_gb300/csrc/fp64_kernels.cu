@@ -438,7 +438,20 @@ __global__ void __launch_bounds__(NTHR) g_energy_kernel(GEnergyArgs P) {
   const double eij = P.eo[i] + P.eo[j];
   const int b = b0 + r;
   double e = 0.0;
-  if (b < nv) {
+  if (!diag && !same && !P.tamp) {
+    // most tiles, by themselves: a predicated FP64 operation takes its half clock too
+    if (b < nv) {
+      const double eb = P.ev[b];
+#pragma unroll 8
+      for (int c = c0; c < T; c += NTHR / T) {
+        const int a = a0 + c;
+        if (a >= nv) break;
+        const double g1 = gi[b + P.ld * a], g2 = S[r * (T + 1) + c];
+        const double d = eij - eb - P.ev[a];  // RIMP2.F90:403 order
+        e = fma(fma(g1, g1 - g2, g2 * g2), recip_f64(d), e);  // doubled below
+      }
+    }
+  } else if (b < nv) {
     const double eb = P.ev[b];
 #pragma unroll 8
     for (int c = c0; c < T; c += NTHR / T) {

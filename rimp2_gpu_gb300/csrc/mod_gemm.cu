@@ -775,15 +775,16 @@ __device__ __forceinline__ Side side(const CrtParams &P, const RowMap &M, int r)
 }
 
 // A block takes 64 rows x 64 columns of C; a thread four consecutive rows of
-// two columns.  It reads 17 bytes and writes 8 per element; about 150
-// instructions an element bound it, so what only depends on the row or the
-// column (offsets, orbital energies) is formed once.  A symmetric product (g
+// two columns.  It reads 17 bytes and writes 8 per element; its instructions
+// (some 170 an element) bound it, so what only depends on the row or the column
+// (offsets with their divisions, orbital energies) is formed once a block.  A symmetric product (g
 // of one set of vectors with itself) has only the tiles m >= n: C(n,m) is
 // written along with C(m,n) through shared memory, with the same denominator
 // (the reference subtracts the two virtual energies in the other order there).
 template <int MODE>
 __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_constant__ CrtParams P) {
   __shared__ int count;
+  __shared__ Side sr[64], sc[64];           // the tile's rows and columns
   __shared__ long long rows[64], cols[64];  // symmetric: offsets of the mirror's columns
   extern __shared__ double S[];             // symmetric: [64][65]
   const int tm = blockIdx.x, tn = blockIdx.y;
@@ -794,6 +795,10 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
   const long long plane = (long long)P.nn * P.ldm;
   const bool mirror = P.sym && tm != tn;
   if (threadIdx.x == 0) count = 0;
+  if (threadIdx.x < 64 && tm * 64 + threadIdx.x < P.nm)
+    sr[threadIdx.x] = side<MODE>(P, P.A, P.row0 + tm * 64 + threadIdx.x);
+  else if (threadIdx.x >= 64 && threadIdx.x < 128 && tn * 64 + threadIdx.x - 64 < P.nn)
+    sc[threadIdx.x - 64] = side<MODE>(P, P.B, P.col0 + tn * 64 + threadIdx.x - 64);
   if (mirror && threadIdx.x < 64) {
     if (tm * 64 + threadIdx.x < P.nm) rows[threadIdx.x] = c_off(P.B, tm * 64 + threadIdx.x);
     if (tn * 64 + threadIdx.x < P.nn) cols[threadIdx.x] = c_off(P.A, tn * 64 + threadIdx.x);
@@ -822,13 +827,10 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
   }
   const int lane = threadIdx.x & 31;
   int ea[4];
-  Side sm[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    ea[k] = m0 + k < P.nm ? P.ea[m0 + k] : 0;
-    if (m0 + k < P.nm) sm[k] = side<MODE>(P, P.A, P.row0 + m0 + k);
-  }
-  auto put = [&](const Side &a, const Side &b, int k, int y, double v) {
+  for (int k = 0; k < 4; ++k) ea[k] = m0 + k < P.nm ? P.ea[m0 + k] : 0;
+  auto put = [&](int k, int y, double v) {
+    const Side &a = sr[mq + k], &b = sc[nq + 32 * y];
     if (MODE == CRT_QUOTIENT || (MODE == CRT_ANY && P.denom))
       v = div_f64(v, a.eo + b.eo - b.ev - a.ev);  // RIMP2.F90:403-404
     if (MODE == CRT_ANY && P.alpha != 1.0) v *= P.alpha;
@@ -848,7 +850,6 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
 #pragma unroll
       for (int p = 0; p < MG_P; ++p) w[p] = *reinterpret_cast<const unsigned *>(src + p * plane);
       const int eb = P.eb[n];
-      const Side sn = side<MODE>(P, P.B, P.col0 + n);
       // 4 x 4 byte transposes: r[k][q] holds planes 4q .. 4q+3 of row m0 + k
       unsigned r[4][4];
 #pragma unroll
@@ -865,7 +866,7 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
         double v;
         if (m0 + k >= P.nm || ((todo >> (4 * y + k)) & 1u)) continue;
         if (crt_value(r[k], ea[k] + eb, v))
-          put(sm[k], sn, k, y, v);
+          put(k, y, v);
         else
           small |= 1u << (4 * y + k);
       }
@@ -877,8 +878,7 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
     for (int x = 0; x < 8; ++x) {
       const int k = x & 3, y = x >> 2, n = n0 + 32 * y;
       if ((small >> x) & 1u)
-        put(side<MODE>(P, P.A, P.row0 + m0 + k), side<MODE>(P, P.B, P.col0 + n), k, y,
-            crt_small(P.res + n * P.ldm + m0 + k, plane, P.ea[m0 + k] + P.eb[n]));
+        put(k, y, crt_small(P.res + n * P.ldm + m0 + k, plane, P.ea[m0 + k] + P.eb[n]));
       unsigned mask = __ballot_sync(0xffffffffu, (todo >> x) & 1u);
       while (mask) {
         const int src = __ffs(mask) - 1;
@@ -890,7 +890,7 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
         for (int q = lane; q < P.A.K; q += 32) s = fma(a[q * P.A.sk], b[q * P.B.sk], s);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == src) put(side<MODE>(P, P.A, m), side<MODE>(P, P.B, nn), k, y, s);
+        if (lane == src) put(k, y, s);
       }
     }
   }
