@@ -79,65 +79,155 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
                : "d"(a), "d"(b));
 }
 
+// 1/d for a positive normal d: the FP32 reciprocal of its significand, its
+// exponent put back, refined by a third-order Newton step (Householder's method)
+// to about an ulp.  No branch, so that the steps around it can overlap; odd: d is
+// too near the ends of the range.
+__device__ __forceinline__ double recip_pos(double d, bool &odd) {
+  const int hi = __double2hiint(d), ed = (hi >> 20) & 0x7FF;
+  odd |= ed < 2 || ed > 2040;
+  const float f = __int_as_float(0x3F800000 | ((hi & 0xFFFFF) << 3) | ((unsigned)__double2loint(d) >> 29));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f));
+  const int b = __float_as_int(r);  // 0.5 .. 1
+  const double r0 = __hiloint2double((((b >> 23) + 1919 - ed) << 20) | ((b >> 3) & 0xFFFFF), b << 29);
+  const double e = fma(-d, r0, 1.0);
+  return fma(r0, fma(e, e, e), r0);
+}
+
+// 1/sqrt(d) likewise: FP32 seed for the significand in [1, 4), third-order step.
+__device__ __forceinline__ double rsqrt_pos(double d, bool &odd) {
+  const int hi = __double2hiint(d), ed = (hi >> 20) & 0x7FF;
+  odd |= ed < 2 || ed > 2040;
+  const int up = (ed & 1) ^ 1;  // exponent ed - 1023 = 2 half + up
+  const float f = __int_as_float(((127 + up) << 23) | ((hi & 0xFFFFF) << 3) | ((unsigned)__double2loint(d) >> 29));
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f));
+  const int b = __float_as_int(r), half = (ed - 1023 - up) / 2;
+  const double y = __hiloint2double((((b >> 23) + 896 - half) << 20) | ((b >> 3) & 0xFFFFF), b << 29);
+  const double e = fma(-d * y, y, 1.0);
+  return fma(y, e * fma(0.375, e, 0.5), y);
+}
+
+// Sixteen columns of L D L^T in a warp: lane (r, h) holds row r's columns 2 j + h
+// (the upper triangle comes along), left over their pivots.  first: the first
+// pivot that is not positive (16: none); dmine: pivot r.  True if a reciprocal
+// was out of range: then SLOW with the block's values again.
+template <bool SLOW>
+__device__ __forceinline__ bool factor16(double (&a)[8], int lane, double &dmine, int &first) {
+  const int r = lane & 15, h = lane >> 4;
+  bool odd = false;
+  dmine = 1.0;
+  first = 16;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    const double d = __shfl_sync(0xffffffffu, a[k >> 1], k + 16 * (k & 1));
+    const double ark = __shfl_sync(0xffffffffu, a[k >> 1], r + 16 * (k & 1));
+    const long long bits = __double_as_longlong(d);
+    const bool ok = bits > 0 && bits <= 0x7FF0000000000000ll;  // d > 0
+    first = !ok && first == 16 ? k : first;
+    dmine = r == k && ok ? d : dmine;
+    const double q = ok ? (SLOW ? 1.0 / d : recip_pos(d, odd)) : 1.0;
+    const double f = -q * ark;
+#pragma unroll
+    for (int j = (k + 1) >> 1; j < 8; ++j) {  // columns past k: of j = k / 2 only the odd one
+      double t = __shfl_sync(0xffffffffu, ark, 2 * j + h);
+      if (2 * j == k) t = h ? t : 0.0;
+      a[j] = fma(f, t, a[j]);
+    }
+  }
+  return odd;
+}
+
 // In-place Cholesky of the b x b diagonal block at (k0,k0) of V (ld n); *bad =
-// pivot+1 on a non-positive pivot.  One CTA: the chain of 64 pivots and its
-// FP64 pipe (two FMAs a clock, so every idle lane of a warp counts) bound it.
-// Sixteen columns at a time: their diagonal block in one warp's registers
-// (lane = row; columns over their pivot, the square roots at the end), the rows
-// below by substitution, a row per thread, the rest with DMMA.  143 us as a
-// rank-one update per column with the inverse, 69 us with the block in
-// registers and a barrier per column.
-__global__ void __launch_bounds__(256) potrf_block_kernel(double *V, int n, int k0, int b, int *bad) {
+// pivot+1 on a non-positive pivot; Dinv: the inverses of the first three of its
+// four 16 x 16 diagonal blocks.  One CTA: the chain of 64 pivots bounds it, and in
+// it the FP64 instructions of a warp, one in 64 clocks (each scheduler's unit does
+// half an FMA a clock, idle lanes count): two lanes share a row.
+// Sixteen columns at a time: their diagonal block in warp 0, columns over
+// their pivot, the square roots at the end; the rows below by substitution
+// (warps 1 to 3); the rest with DMMA (eight warps); a warp of its own forms the
+// block's inverse beside the next block.  In us: 143 as a rank-one update per
+// column with the inverse, 69 with the block in registers and a barrier per
+// column, 71 as here with a lane per row (11 of them a block, 5.3 a
+// substitution), 82 with the rows below in the lanes of the block's warp.
+constexpr int PT = 384;
+__global__ void __launch_bounds__(PT) potrf_block_kernel(double *V, int n, int k0, int b, int *bad,
+                                                         double *Dinv) {
   __shared__ double A[NB][PS];
   __shared__ double rd[NB];  // 1 / L(k, k)
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
+  const int r = lane & 15, h = lane >> 4;
 #pragma unroll
-  for (int x = 0; x < NB * NB / 256; ++x) {
-    const int t = threadIdx.x + 256 * x, r = t & (NB - 1), c = t >> 6;
-    A[r][c] = r < b && c <= r ? V[(size_t)(k0 + r) + (size_t)n * (k0 + c)] : (r == c ? 1.0 : 0.0);
+  for (int t = threadIdx.x; t < NB * NB; t += PT) {
+    const int i = t & (NB - 1), c = t >> 6;
+    A[i][c] = i < b && c <= i ? V[(size_t)(k0 + i) + (size_t)n * (k0 + c)] : (i == c ? 1.0 : 0.0);
   }
   __syncthreads();
+  if (w >= 8) {  // inverse of block w - 9: column `lane` by forward substitution
+    if (w == 8) return;
+    asm volatile("bar.sync %0, 288;" ::"r"(w - 7) : "memory");
+    const int o = 16 * (w - 9);
+    double x[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) x[i] = i == lane ? 1.0 : 0.0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      x[i] *= rd[o + i];
+#pragma unroll
+      for (int p = i + 1; p < 16; ++p) x[p] = fma(-A[o + p][o + i], x[i], x[p]);
+    }
+    if (lane < 16)
+#pragma unroll
+      for (int i = 0; i < 16; ++i) Dinv[(w - 9) * 256 + i * 16 + lane] = x[i];
+    return;
+  }
 #pragma unroll 1
   for (int o = 0; o < NB; o += 16) {
     if (w == 0) {
-      const int r = lane & 15;
-      double a[16], dmine = 1.0;
+      double a[8], dmine;
+      int first;
 #pragma unroll
-      for (int c = 0; c < 16; ++c) a[c] = r >= c ? A[o + r][o + c] : A[o + c][o + r];
+      for (int j = 0; j < 8; ++j) a[j] = r >= 2 * j + h ? A[o + r][o + 2 * j + h] : A[o + 2 * j + h][o + r];
+      bool odd = factor16<false>(a, lane, dmine, first);
+      double s = rsqrt_pos(dmine, odd);
+      if (__any_sync(0xffffffffu, odd)) {
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        const double d = __shfl_sync(0xffffffffu, a[k], k);
-        const bool ok = d > 0.0;
-        if (!ok && lane == 0) atomicCAS(bad, 0, k0 + o + k + 1);
-        if (r == k) dmine = ok ? d : 1.0;
-        const double f = -(ok ? recip_f64(d) : 1.0) * a[k];
-#pragma unroll
-        for (int c = k + 1; c < 16; ++c) a[c] = fma(f, __shfl_sync(0xffffffffu, a[k], c), a[c]);
+        for (int j = 0; j < 8; ++j) a[j] = r >= 2 * j + h ? A[o + r][o + 2 * j + h] : A[o + 2 * j + h][o + r];
+        factor16<true>(a, lane, dmine, first);
+        s = 1.0 / sqrt(dmine);
       }
-      const double s = 1.0 / sqrt(dmine);
+      if (lane == 0 && first < 16) atomicCAS(bad, 0, k0 + o + first + 1);
+      __syncwarp();
 #pragma unroll
-      for (int k = 0; k < 16; ++k) {
-        const double v = a[k] * __shfl_sync(0xffffffffu, s, k);
-        if (lane < 16 && r >= k) A[o + r][o + k] = v;
+      for (int j = 0; j < 8; ++j) {
+        const double v = a[j] * __shfl_sync(0xffffffffu, s, 2 * j + h);
+        if (r >= 2 * j + h) A[o + r][o + 2 * j + h] = v;
       }
       if (lane < 16) rd[o + r] = s;
     }
-    __syncthreads();
-    const int row = o + 16 + threadIdx.x;
-    if (row < NB) {
-      double x[16];
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    if (o < 48) asm volatile("bar.arrive %0, 288;" ::"r"(2 + o / 16) : "memory");
+    const int row = o + 16 * w + r;
+    if (w >= 1 && w <= 3 && row < NB) {  // lane (r, h): its row's columns 2 j + h
+      double x[8];
 #pragma unroll
-      for (int c = 0; c < 16; ++c) x[c] = A[row][o + c];
+      for (int j = 0; j < 8; ++j) x[j] = A[row][o + 2 * j + h];
 #pragma unroll
       for (int c = 0; c < 16; ++c) {
-        x[c] *= rd[o + c];
+        const double xc = __shfl_sync(0xffffffffu, x[c >> 1] * rd[o + c], r + 16 * (c & 1));
+        if (h == (c & 1)) x[c >> 1] = xc;
 #pragma unroll
-        for (int j = c + 1; j < 16; ++j) x[j] = fma(-A[o + j][o + c], x[c], x[j]);
+        for (int j = (c + 1) >> 1; j < 8; ++j) {
+          double l = A[o + 2 * j + h][o + c];
+          if (2 * j == c) l = h ? l : 0.0;
+          x[j] = fma(-l, xc, x[j]);
+        }
       }
 #pragma unroll
-      for (int c = 0; c < 16; ++c) A[row][o + c] = x[c];
+      for (int j = 0; j < 8; ++j) A[row][o + 2 * j + h] = x[j];
     }
-    __syncthreads();
+    asm volatile("bar.sync 1, 256;" ::: "memory");
     const int n8 = (NB - 16 - o) / 8;
     for (int t = w; t < n8 * (n8 + 1) / 2; t += 8) {  // 8 x 8 tiles of the lower triangle
       int ti = 0;
@@ -149,55 +239,67 @@ __global__ void __launch_bounds__(256) potrf_block_kernel(double *V, int n, int 
       A[r0 + gid][c0 + 2 * tig] = d0;
       A[r0 + gid][c0 + 2 * tig + 1] = d1;
     }
-    __syncthreads();
+    asm volatile("bar.sync 1, 256;" ::: "memory");
   }
-#pragma unroll
+#pragma unroll 8
   for (int x = 0; x < NB * NB / 256; ++x) {
-    const int t = threadIdx.x + 256 * x, r = t & (NB - 1), c = t >> 6;
-    if (r < b && c < b) V[(size_t)(k0 + r) + (size_t)n * (k0 + c)] = r >= c ? A[r][c] : 0.0;
+    const int t = threadIdx.x + 256 * x, i = t & (NB - 1), c = t >> 6;
+    if (i < b && c < b) V[(size_t)(k0 + i) + (size_t)n * (k0 + c)] = i >= c ? A[i][c] : 0.0;
   }
 }
 
 // X := X L^{-T} for the rows [k0+64, n) of the block column at k0, L its
-// factored diagonal block: eight rows per CTA (136 CTAs at n = 1152), warp j
+// factored diagonal block: eight rows per CTA (136 CTAs at n = 1152), warp j < 4
 // holds their columns 16 j .. 16 j + 15.  Sixteen columns at a time: warp l
-// multiplies by the inverse of L_ll (formed by that warp beforehand), the warps
-// after it subtract X_l L_jl^T, both with DMMA m8n8k4: 80 of those, 5 us of
-// the SM's FP64 pipe.  (Column by column, with one chain of 64 dependent
-// steps, it took 34 us; as a product with L^{-1} of 64 x 64 the inverse sat on
-// the critical path.)
-__global__ void __launch_bounds__(128) panel_solve_kernel(double *V, int n, int k0) {
+// multiplies by the inverse of L_ll (Dinv; the last one is formed here by warp 4
+// meanwhile), the warps after it subtract X_l L_jl^T, both with DMMA m8n8k4 in two
+// chains each: 80 of those, 5 us of the SM's FP64 pipe, but their latency (576
+// clocks) bounds it.  (In us: 34 column by column, with one chain of 64 dependent
+// steps; 28 with all inverses formed here first and one chain a product.)
+__global__ void __launch_bounds__(160) panel_solve_kernel(double *V, int n, int k0, const double *Dinv) {
   __shared__ double Ls[NB][PS];     // L(j, c)
   __shared__ double Inv[4][16][17];  // inverses of the 16 x 16 diagonal blocks
   __shared__ double Xs[8][PS];      // the rows
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
   const int row0 = k0 + NB + blockIdx.x * 8;
+  if (w < 4) {
 #pragma unroll 16
-  for (int x = 0; x < NB * NB / 128; ++x) {
-    const int t = threadIdx.x + 128 * x, j = t & (NB - 1), c = t >> 6;
-    Ls[j][c] = V[(size_t)(k0 + j) + (size_t)n * (k0 + c)];
-  }
+    for (int x = 0; x < NB * NB / 128; ++x) {
+      const int t = threadIdx.x + 128 * x, j = t & (NB - 1), c = t >> 6;
+      Ls[j][c] = V[(size_t)(k0 + j) + (size_t)n * (k0 + c)];
+    }
 #pragma unroll
-  for (int x = 0; x < 8 * NB / 128; ++x) {
-    const int t = threadIdx.x + 128 * x, r = t & 7, c = t >> 3;
-    Xs[r][c] = row0 + r < n ? V[(size_t)(row0 + r) + (size_t)n * (k0 + c)] : 0.0;
+    for (int x = 0; x < 8 * NB / 128; ++x) {
+      const int t = threadIdx.x + 128 * x, r = t & 7, c = t >> 3;
+      Xs[r][c] = row0 + r < n ? V[(size_t)(row0 + r) + (size_t)n * (k0 + c)] : 0.0;
+    }
+#pragma unroll
+    for (int x = 0; x < 6; ++x) {
+      const int t = threadIdx.x + 128 * x;
+      Inv[t >> 8][(t >> 4) & 15][t & 15] = Dinv[t];
+    }
   }
   __syncthreads();
-  if (lane < 16) {  // column `lane` of the inverse of L_ww by forward substitution
-    const int o = 16 * w;
-    double x[16];
-#pragma unroll
-    for (int r = 0; r < 16; ++r) x[r] = r == lane ? 1.0 : 0.0;
+  if (w == 4) {  // column `lane` of the inverse of L_33 by forward substitution
+    constexpr int o = 48;
+    double x[16], q[16];
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
-      x[r] *= recip_f64(Ls[o + r][o + r]);
+      x[r] = r == lane ? 1.0 : 0.0;
+      q[r] = recip_f64(Ls[o + r][o + r]);
+    }
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      x[r] *= q[r];
 #pragma unroll
       for (int p = r + 1; p < 16; ++p) x[p] = fma(-Ls[o + p][o + r], x[r], x[p]);
     }
+    if (lane < 16)
 #pragma unroll
-    for (int r = 0; r < 16; ++r) Inv[w][r][lane] = x[r];
+      for (int r = 0; r < 16; ++r) Inv[3][r][lane] = x[r];
+    asm volatile("bar.arrive 2, 160;" ::: "memory");
+    return;
   }
-  __syncwarp();
   double acc[2][2];  // rows gid, columns 16 w + 8 y + 2 tig + {0, 1}
 #pragma unroll
   for (int y = 0; y < 2; ++y)
@@ -205,6 +307,7 @@ __global__ void __launch_bounds__(128) panel_solve_kernel(double *V, int n, int 
     for (int h = 0; h < 2; ++h) acc[y][h] = Xs[gid][16 * w + 8 * y + 2 * tig + h];
 #pragma unroll 1
   for (int l = 0; l < 4; ++l) {
+    if (l == 3) asm volatile("bar.sync 2, 160;" ::: "memory");
     if (w == l) {
       if (l) {  // the rows' columns after the updates, as the left operand
 #pragma unroll
@@ -213,25 +316,34 @@ __global__ void __launch_bounds__(128) panel_solve_kernel(double *V, int n, int 
           for (int h = 0; h < 2; ++h) Xs[gid][16 * w + 8 * y + 2 * tig + h] = acc[y][h];
         __syncwarp();
       }
-      double x[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+      double x[2][2][2] = {};
 #pragma unroll
-      for (int k = 0; k < 16; k += 4)
+      for (int k = 0; k < 8; k += 4)
 #pragma unroll
         for (int y = 0; y < 2; ++y)  // X(r, c) = sum_k P(r, k) Inv(c, k)
-          dmma(x[y][0], x[y][1], Xs[gid][16 * w + k + tig], Inv[w][8 * y + gid][k + tig]);
+#pragma unroll
+          for (int z = 0; z < 2; ++z)
+            dmma(x[z][y][0], x[z][y][1], Xs[gid][16 * w + 8 * z + k + tig], Inv[w][8 * y + gid][8 * z + k + tig]);
       __syncwarp();
 #pragma unroll
       for (int y = 0; y < 2; ++y)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) Xs[gid][16 * w + 8 * y + 2 * tig + h] = x[y][h];
+        for (int h = 0; h < 2; ++h) Xs[gid][16 * w + 8 * y + 2 * tig + h] = x[0][y][h] + x[1][y][h];
     }
-    __syncthreads();
+    asm volatile("bar.sync 1, 128;" ::: "memory");
     if (w > l) {
+      double u[2][2] = {};
 #pragma unroll
-      for (int k = 0; k < 16; k += 4)
+      for (int k = 0; k < 8; k += 4)
 #pragma unroll
-        for (int y = 0; y < 2; ++y)
+        for (int y = 0; y < 2; ++y) {
           dmma(acc[y][0], acc[y][1], -Xs[gid][16 * l + k + tig], Ls[16 * w + 8 * y + gid][16 * l + k + tig]);
+          dmma(u[y][0], u[y][1], -Xs[gid][16 * l + 8 + k + tig], Ls[16 * w + 8 * y + gid][16 * l + 8 + k + tig]);
+        }
+#pragma unroll
+      for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) acc[y][h] += u[y][h];
     }
   }
   for (int t = threadIdx.x; t < 8 * NB; t += 128) {
@@ -289,8 +401,9 @@ int diag_kernels_init() {
 // whole width (a product of 256 terms a sum, which the residue form takes).
 constexpr int CH_PANEL = 256;
 int dev_cholesky(int n, double *V, cudaStream_t s) {
-  DevBuf bad;
+  DevBuf bad, dinv;  // dinv: inverses of a diagonal block's 16 x 16 blocks
   RIMP2_TRY(bad.alloc(sizeof(int), s));
+  RIMP2_TRY(dinv.alloc(sizeof(double) * 3 * 256, s));
   RIMP2_CK(cudaMemsetAsync(bad.p, 0, sizeof(int), s));
   // C(r0.., c0 .. c0+nc) -= P(r0..) P(c0 .. c0+nc)^T, P the columns [k0, k0 + K)
   auto update = [&](int r0, int c0, int nc, int k0, int K, bool lower) -> int {
@@ -316,11 +429,11 @@ int dev_cholesky(int n, double *V, cudaStream_t s) {
     const int p1 = n - p0 < CH_PANEL ? n : p0 + CH_PANEL;
     for (int k0 = p0; k0 < p1; k0 += NB) {
       const int b = n - k0 < NB ? n - k0 : NB;
-      potrf_block_kernel<<<1, 256, 0, s>>>(V, n, k0, b, bad.as<int>());
+      potrf_block_kernel<<<1, PT, 0, s>>>(V, n, k0, b, bad.as<int>(), dinv.as<double>());
       count_launch(1);
       const int r0 = k0 + b;
       if (r0 >= n) break;
-      panel_solve_kernel<<<(n - r0 + 7) / 8, 128, 0, s>>>(V, n, k0);
+      panel_solve_kernel<<<(n - r0 + 7) / 8, 160, 0, s>>>(V, n, k0, dinv.as<double>());
       count_launch(1);
       if (r0 < p1) RIMP2_TRY(update(r0, r0, p1 - r0, k0, NB, false));
     }
