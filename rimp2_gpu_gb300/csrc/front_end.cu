@@ -146,11 +146,13 @@ __device__ __forceinline__ bool factor16(double (&a)[8], int lane, double &dmine
 // half an FMA a clock, idle lanes count): two lanes share a row.
 // Sixteen columns at a time: their diagonal block in warp 0, columns over
 // their pivot, the square roots at the end; the rows below by substitution
-// (warps 1 to 3); the rest with DMMA (eight warps); a warp of its own forms the
-// block's inverse beside the next block.  In us: 143 as a rank-one update per
+// (warps 1 to 3); then the next diagonal block with DMMA, the rest beside that
+// block's factorisation on the other schedulers, as a warp of its own forms the
+// block's inverse.  In us: 143 as a rank-one update per
 // column with the inverse, 69 with the block in registers and a barrier per
 // column, 71 as here with a lane per row (11 of them a block, 5.3 a
-// substitution), 82 with the rows below in the lanes of the block's warp.
+// substitution), 82 with the rows below in the lanes of the block's warp, 52 with
+// the rest updated before the next block.
 constexpr int PT = 384;
 __global__ void __launch_bounds__(PT) potrf_block_kernel(double *V, int n, int k0, int b, int *bad,
                                                          double *Dinv) {
@@ -182,8 +184,23 @@ __global__ void __launch_bounds__(PT) potrf_block_kernel(double *V, int n, int k
       for (int i = 0; i < 16; ++i) Dinv[(w - 9) * 256 + i * 16 + lane] = x[i];
     return;
   }
+  // 8 x 8 tile t of the lower triangle right of and below the 16 columns at o
+  auto update = [&](int o, int t) {
+    int ti = 0;
+    while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
+    const int r0 = o + 16 + 8 * ti, c0 = o + 16 + 8 * (t - ti * (ti + 1) / 2);
+    double d0 = A[r0 + gid][c0 + 2 * tig], d1 = A[r0 + gid][c0 + 2 * tig + 1];
+#pragma unroll
+    for (int k = 0; k < 16; k += 4) dmma(d0, d1, -A[r0 + gid][o + k + tig], A[c0 + gid][o + k + tig]);
+    A[r0 + gid][c0 + 2 * tig] = d0;
+    A[r0 + gid][c0 + 2 * tig + 1] = d1;
+  };
 #pragma unroll 1
   for (int o = 0; o < NB; o += 16) {
+    if (o > 0 && (w & 3) != 0) {  // the other tiles of the columns before
+      const int n8 = (NB - o) / 8;
+      for (int t = 3 + (w & 3) - 1 + 3 * (w >> 2); t < n8 * (n8 + 1) / 2; t += 6) update(o - 16, t);
+    }
     if (w == 0) {
       double a[8], dmine;
       int first;
@@ -228,17 +245,8 @@ __global__ void __launch_bounds__(PT) potrf_block_kernel(double *V, int n, int k
       for (int j = 0; j < 8; ++j) A[row][o + 2 * j + h] = x[j];
     }
     asm volatile("bar.sync 1, 256;" ::: "memory");
-    const int n8 = (NB - 16 - o) / 8;
-    for (int t = w; t < n8 * (n8 + 1) / 2; t += 8) {  // 8 x 8 tiles of the lower triangle
-      int ti = 0;
-      while ((ti + 1) * (ti + 2) / 2 <= t) ++ti;
-      const int r0 = o + 16 + 8 * ti, c0 = o + 16 + 8 * (t - ti * (ti + 1) / 2);
-      double d0 = A[r0 + gid][c0 + 2 * tig], d1 = A[r0 + gid][c0 + 2 * tig + 1];
-#pragma unroll
-      for (int k = 0; k < 16; k += 4) dmma(d0, d1, -A[r0 + gid][o + k + tig], A[c0 + gid][o + k + tig]);
-      A[r0 + gid][c0 + 2 * tig] = d0;
-      A[r0 + gid][c0 + 2 * tig + 1] = d1;
-    }
+    // the next diagonal block's three tiles
+    if (o < 48 && w >= 1 && w <= 3) update(o, w - 1);
     asm volatile("bar.sync 1, 256;" ::: "memory");
   }
 #pragma unroll 8
@@ -249,106 +257,89 @@ __global__ void __launch_bounds__(PT) potrf_block_kernel(double *V, int n, int k
 }
 
 // X := X L^{-T} for the rows [k0+64, n) of the block column at k0, L its
-// factored diagonal block: eight rows per CTA (136 CTAs at n = 1152), warp j < 4
-// holds their columns 16 j .. 16 j + 15.  Sixteen columns at a time: warp l
-// multiplies by the inverse of L_ll (Dinv; the last one is formed here by warp 4
-// meanwhile), the warps after it subtract X_l L_jl^T, both with DMMA m8n8k4 in two
-// chains each: 80 of those, 5 us of the SM's FP64 pipe, but their latency (576
-// clocks) bounds it.  (In us: 34 column by column, with one chain of 64 dependent
-// steps; 28 with all inverses formed here first and one chain a product.)
+// factored diagonal block: eight rows per CTA (136 CTAs at n = 1152).  Sixteen
+// columns at a time: times the inverse of L_ll (Dinv; the last one is formed here by
+// warp 4 meanwhile), then the later columns less X_l L_jl^T, with DMMA m8n8k4.
+// A scheduler's unit takes 576 clocks for one of those, so that each product of
+// 16 columns is dealt to the four warps: warp (y, z) takes its columns 8 y .. 8 y + 7
+// and the terms 8 z .. 8 z + 7 of its sums; the two parts meet in shared memory.
+// (In us: 34 column by column, with one chain of 64 dependent steps; 28 with a
+// warp for each 16 columns and all inverses formed here first, 22 without those.)
 __global__ void __launch_bounds__(160) panel_solve_kernel(double *V, int n, int k0, const double *Dinv) {
-  __shared__ double Ls[NB][PS];     // L(j, c)
-  __shared__ double Inv[4][16][17];  // inverses of the 16 x 16 diagonal blocks
-  __shared__ double Xs[8][PS];      // the rows
+  __shared__ double Ls[NB][PS];     // L(j, c), with the inverses of its 16 x 16 diagonal blocks
+  __shared__ double Ps[2][8][20];   // sixteen columns of the rows after the updates, in two parts
+  __shared__ double Xs[2][8][PS];   // the solution, in two parts
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
   const int row0 = k0 + NB + blockIdx.x * 8;
+  const int y = w & 1, z = w >> 1;
+  double acc[4][2];  // rows gid, columns 16 j + 8 y + 2 tig + {0, 1}
   if (w < 4) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        acc[j][h] = z == 0 && row0 + gid < n
+                        ? V[(size_t)(row0 + gid) + (size_t)n * (k0 + 16 * j + 8 * y + 2 * tig + h)]
+                        : 0.0;
 #pragma unroll 16
     for (int x = 0; x < NB * NB / 128; ++x) {
       const int t = threadIdx.x + 128 * x, j = t & (NB - 1), c = t >> 6;
-      Ls[j][c] = V[(size_t)(k0 + j) + (size_t)n * (k0 + c)];
-    }
-#pragma unroll
-    for (int x = 0; x < 8 * NB / 128; ++x) {
-      const int t = threadIdx.x + 128 * x, r = t & 7, c = t >> 3;
-      Xs[r][c] = row0 + r < n ? V[(size_t)(row0 + r) + (size_t)n * (k0 + c)] : 0.0;
-    }
-#pragma unroll
-    for (int x = 0; x < 6; ++x) {
-      const int t = threadIdx.x + 128 * x;
-      Inv[t >> 8][(t >> 4) & 15][t & 15] = Dinv[t];
+      const bool inv = (j >> 4) == (c >> 4) && c < 48;
+      Ls[j][c] = inv ? Dinv[(c >> 4) * 256 + (j & 15) * 16 + (c & 15)] : V[(size_t)(k0 + j) + (size_t)n * (k0 + c)];
     }
   }
   __syncthreads();
-  if (w == 4) {  // column `lane` of the inverse of L_33 by forward substitution
+  if (w == 4) {  // inverse of L_33 by forward substitution: lane (c, h), column c's rows 2 j + h
     constexpr int o = 48;
-    double x[16], q[16];
+    const int c = lane & 15, h = lane >> 4;
+    const double mine = recip_f64(Ls[o + c][o + c]);
+    double x[8];
 #pragma unroll
-    for (int r = 0; r < 16; ++r) {
-      x[r] = r == lane ? 1.0 : 0.0;
-      q[r] = recip_f64(Ls[o + r][o + r]);
+    for (int j = 0; j < 8; ++j) x[j] = 2 * j + h == c ? 1.0 : 0.0;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const double q = __shfl_sync(0xffffffffu, mine, i);
+      const double xi = __shfl_sync(0xffffffffu, x[i >> 1] * q, c + 16 * (i & 1));
+      if (h == (i & 1)) x[i >> 1] = xi;
+#pragma unroll
+      for (int j = (i + 1) >> 1; j < 8; ++j) {
+        double l = Ls[o + 2 * j + h][o + i];
+        if (2 * j == i) l = h ? l : 0.0;
+        x[j] = fma(-l, xi, x[j]);
+      }
     }
+    __syncwarp();
 #pragma unroll
-    for (int r = 0; r < 16; ++r) {
-      x[r] *= q[r];
-#pragma unroll
-      for (int p = r + 1; p < 16; ++p) x[p] = fma(-Ls[o + p][o + r], x[r], x[p]);
-    }
-    if (lane < 16)
-#pragma unroll
-      for (int r = 0; r < 16; ++r) Inv[3][r][lane] = x[r];
+    for (int j = 0; j < 8; ++j) Ls[o + 2 * j + h][o + c] = x[j];
     asm volatile("bar.arrive 2, 160;" ::: "memory");
     return;
   }
-  double acc[2][2];  // rows gid, columns 16 w + 8 y + 2 tig + {0, 1}
 #pragma unroll
-  for (int y = 0; y < 2; ++y)
-#pragma unroll
-    for (int h = 0; h < 2; ++h) acc[y][h] = Xs[gid][16 * w + 8 * y + 2 * tig + h];
-#pragma unroll 1
   for (int l = 0; l < 4; ++l) {
-    if (l == 3) asm volatile("bar.sync 2, 160;" ::: "memory");
-    if (w == l) {
-      if (l) {  // the rows' columns after the updates, as the left operand
 #pragma unroll
-        for (int y = 0; y < 2; ++y)
+    for (int h = 0; h < 2; ++h) Ps[z][gid][8 * y + 2 * tig + h] = acc[l][h];
+    if (l < 3)
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+    else
+      asm volatile("bar.sync 2, 160;" ::: "memory");  // and the last inverse
+    double x[2] = {0.0, 0.0};
 #pragma unroll
-          for (int h = 0; h < 2; ++h) Xs[gid][16 * w + 8 * y + 2 * tig + h] = acc[y][h];
-        __syncwarp();
-      }
-      double x[2][2][2] = {};
+    for (int k = 8 * z; k < 8 * z + 8; k += 4)  // X(r, c) = sum_k P(r, k) Inv(c, k)
+      dmma(x[0], x[1], Ps[0][gid][k + tig] + Ps[1][gid][k + tig], Ls[16 * l + 8 * y + gid][16 * l + k + tig]);
 #pragma unroll
-      for (int k = 0; k < 8; k += 4)
-#pragma unroll
-        for (int y = 0; y < 2; ++y)  // X(r, c) = sum_k P(r, k) Inv(c, k)
-#pragma unroll
-          for (int z = 0; z < 2; ++z)
-            dmma(x[z][y][0], x[z][y][1], Xs[gid][16 * w + 8 * z + k + tig], Inv[w][8 * y + gid][8 * z + k + tig]);
-      __syncwarp();
-#pragma unroll
-      for (int y = 0; y < 2; ++y)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) Xs[gid][16 * w + 8 * y + 2 * tig + h] = x[0][y][h] + x[1][y][h];
-    }
+    for (int h = 0; h < 2; ++h) Xs[z][gid][16 * l + 8 * y + 2 * tig + h] = x[h];
     asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (w > l) {
-      double u[2][2] = {};
 #pragma unroll
-      for (int k = 0; k < 8; k += 4)
+    for (int k = 8 * z; k < 8 * z + 8; k += 4) {
+      if (l == 3) break;
+      const double v = -(Xs[0][gid][16 * l + k + tig] + Xs[1][gid][16 * l + k + tig]);
 #pragma unroll
-        for (int y = 0; y < 2; ++y) {
-          dmma(acc[y][0], acc[y][1], -Xs[gid][16 * l + k + tig], Ls[16 * w + 8 * y + gid][16 * l + k + tig]);
-          dmma(u[y][0], u[y][1], -Xs[gid][16 * l + 8 + k + tig], Ls[16 * w + 8 * y + gid][16 * l + 8 + k + tig]);
-        }
-#pragma unroll
-      for (int y = 0; y < 2; ++y)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) acc[y][h] += u[y][h];
+      for (int j = l + 1; j < 4; ++j) dmma(acc[j][0], acc[j][1], v, Ls[16 * j + 8 * y + gid][16 * l + k + tig]);
     }
   }
   for (int t = threadIdx.x; t < 8 * NB; t += 128) {
     const int r = t & 7, c = t >> 3;
-    if (row0 + r < n) V[(size_t)(row0 + r) + (size_t)n * (k0 + c)] = Xs[r][c];
+    if (row0 + r < n) V[(size_t)(row0 + r) + (size_t)n * (k0 + c)] = Xs[0][r][c] + Xs[1][r][c];
   }
 }
 
