@@ -34,8 +34,8 @@
 // Kernels: row_scale (norms -> exponents), residue (17 FP16 planes per
 // operand), mod_gemm (persistent CTA pairs, 256 x 256 tiles, TMA + tcgen05,
 // one product per plane; the epilogue reduces modulo p and stores bytes),
-// crt_epilogue (fixed-point reconstruction, scaling, denominators, the
-// elements to be summed in FP64), dmma_tiles (whole tiles in FP64).
+// crt_epilogue (fixed-point reconstruction, scaling, denominators; the
+// elements and tiles to be summed in FP64).
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -190,9 +190,8 @@ struct OpArgs {
 // along the fast direction: a block takes 32 rows, each warp a part of K.
 // Both operands of a product in one launch (short ones are launch-bound).
 __global__ void __launch_bounds__(256) row_scale_kernel(const __grid_constant__ OpArgs A,
-                                                        const __grid_constant__ OpArgs B, unsigned *list) {
+                                                        const __grid_constant__ OpArgs B) {
   __shared__ RowStat sh[8][32];
-  if (blockIdx.x == 0 && threadIdx.x == 0) *list = 0;  // the count of tiles left to FP64
   const bool second = (int)blockIdx.x >= A.blocks;
   const OpArgs &P = second ? B : A;
   const RowMap &M = P.M;
@@ -307,9 +306,8 @@ __device__ __forceinline__ void residues8(const double (&v)[8], int e, bool live
 // the eight threads of a row find its scale themselves (no row_scale launch).
 template <bool SCALE>
 __global__ void __launch_bounds__(256) residue_kernel(const __grid_constant__ OpArgs A,
-                                                      const __grid_constant__ OpArgs B, unsigned *list) {
+                                                      const __grid_constant__ OpArgs B) {
   __shared__ double sh[64][33];
-  if (SCALE && blockIdx.x == 0 && threadIdx.x == 0) *list = 0;  // the count of tiles left to FP64
   const bool second = (int)blockIdx.x >= A.blocks;
   const OpArgs &P = second ? B : A;
   const RowMap &M = P.M;
@@ -742,7 +740,6 @@ struct CrtParams {
   int denom, lower;
   int nfast;                 // C's fast direction is n
   int sym;                   // rows and columns are the same vectors: C(n,m) comes with C(m,n)
-  unsigned *list;            // [0] count, then tiles (tn * tiles_m + tm) left to FP64
 };
 
 // Whether an element is left to FP64: the flags of its row and column, and
@@ -781,12 +778,14 @@ __device__ __forceinline__ Side side(const CrtParams &P, const RowMap &M, int r)
 // of one set of vectors with itself) has only the tiles m >= n: C(n,m) is
 // written along with C(m,n) through shared memory, with the same denominator
 // (the reference subtracts the two virtual energies in the other order there).
+constexpr int DK = 16, DP = 20;
 template <int MODE>
 __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_constant__ CrtParams P) {
   __shared__ int count;
   __shared__ Side sr[64], sc[64];           // the tile's rows and columns
   __shared__ long long rows[64], cols[64];  // symmetric: offsets of the mirror's columns
-  extern __shared__ double S[];             // symmetric: [64][65]
+  extern __shared__ double S[];             // symmetric: [64][65]; a tile summed in FP64: its operands
+  double(*As)[DP] = reinterpret_cast<double(*)[DP]>(S), (*Bs)[DP] = As + 64;
   const int tm = blockIdx.x, tn = blockIdx.y;
   if ((P.lower || P.sym) && tm < tn) return;
   const int t0 = threadIdx.x & 15, t1 = threadIdx.x >> 4;
@@ -821,25 +820,60 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
   }
   if (todo) atomicAdd(&count, __popc(todo));
   __syncthreads();
-  if (count > MG_TILE_MAX) {
-    if (threadIdx.x == 0) P.list[1 + atomicAdd(P.list, 1u)] = tn * gridDim.x + tm;
-    return;
-  }
   const int lane = threadIdx.x & 31;
-  int ea[4];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) ea[k] = m0 + k < P.nm ? P.ea[m0 + k] : 0;
-  auto put = [&](int k, int y, double v) {
-    const Side &a = sr[mq + k], &b = sc[nq + 32 * y];
+  auto put = [&](int ml, int nl, double v) {
+    const Side &a = sr[ml], &b = sc[nl];
     if (MODE == CRT_QUOTIENT || (MODE == CRT_ANY && P.denom))
       v = div_f64(v, a.eo + b.eo - b.ev - a.ev);  // RIMP2.F90:403-404
     if (MODE == CRT_ANY && P.alpha != 1.0) v *= P.alpha;
-    if (mirror) S[(mq + k) * 65 + nq + 32 * y] = v;
+    if (mirror) S[ml * 65 + nl] = v;
     double *c = P.C + a.off + b.off;
     if (MODE == CRT_MINUS) v = *c - v;
     if (MODE == CRT_ANY && P.beta != 0.0) v += P.beta * *c;
     *c = v;
   };
+  if (count > MG_TILE_MAX) {
+    // the whole tile with FP64 tensor operations: 16 x 16 of it a warp
+    const int gid = lane >> 2, tig = lane & 3, warp = threadIdx.x >> 5;
+    const int wm = (warp & 3) * 16, wn = (warp >> 2) * 16;
+    double acc[2][2][2] = {};
+    for (int q0 = 0; q0 < P.A.K; q0 += DK) {
+      __syncthreads();
+#pragma unroll 1
+      for (int t = threadIdx.x; t < 2 * 64 * DK; t += 512) {
+        const bool cols = t >= 64 * DK;
+        const RowMap &M = cols ? P.B : P.A;
+        const int u = t & (64 * DK - 1), i = M.sk == 1 ? u / DK : u & 63, q = M.sk == 1 ? u % DK : u >> 6;
+        const bool live = q0 + q < M.K && (cols ? tn * 64 + i < P.nn : tm * 64 + i < P.nm);
+        const int row = cols ? P.col0 + tn * 64 + i : P.row0 + tm * 64 + i;
+        (cols ? Bs : As)[i][q] = live ? M.base[row_off(M, row) + (long long)(q0 + q) * M.sk] : 0.0;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int ks = 0; ks < DK; ks += 4)
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+          for (int y = 0; y < 2; ++y)
+            asm volatile(
+                "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                : "+d"(acc[x][y][0]), "+d"(acc[x][y][1])
+                : "d"(As[wm + 8 * x + gid][ks + tig]), "d"(Bs[wn + 8 * y + gid][ks + tig]));
+    }
+    __syncthreads();  // the operands give way to the mirror
+#pragma unroll 1
+    for (int e = 0; e < 8; ++e) {
+      const int ml = wm + 8 * (e >> 2) + gid, nl = wn + 8 * ((e >> 1) & 1) + 2 * tig + (e & 1);
+      double v = 0.0;
+#pragma unroll
+      for (int x = 0; x < 8; ++x) v = e == x ? acc[x >> 2][(x >> 1) & 1][x & 1] : v;
+      if (tm * 64 + ml < P.nm && tn * 64 + nl < P.nn) put(ml, nl, v);
+    }
+  }
+  if (count <= MG_TILE_MAX) {
+  int ea[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) ea[k] = m0 + k < P.nm ? P.ea[m0 + k] : 0;
   unsigned small = 0;
 #pragma unroll 1
   for (int y = 0; y < 2; ++y) {
@@ -866,7 +900,7 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
         double v;
         if (m0 + k >= P.nm || ((todo >> (4 * y + k)) & 1u)) continue;
         if (crt_value(r[k], ea[k] + eb, v))
-          put(k, y, v);
+          put(mq + k, nq + 32 * y, v);
         else
           small |= 1u << (4 * y + k);
       }
@@ -878,7 +912,7 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
     for (int x = 0; x < 8; ++x) {
       const int k = x & 3, y = x >> 2, n = n0 + 32 * y;
       if ((small >> x) & 1u)
-        put(k, y, crt_small(P.res + n * P.ldm + m0 + k, plane, P.ea[m0 + k] + P.eb[n]));
+        put(mq + k, nq + 32 * y, crt_small(P.res + n * P.ldm + m0 + k, plane, P.ea[m0 + k] + P.eb[n]));
       unsigned mask = __ballot_sync(0xffffffffu, (todo >> x) & 1u);
       while (mask) {
         const int src = __ffs(mask) - 1;
@@ -890,9 +924,10 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
         for (int q = lane; q < P.A.K; q += 32) s = fma(a[q * P.A.sk], b[q * P.B.sk], s);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == src) put(k, y, s);
+        if (lane == src) put(mq + k, nq + 32 * y, s);
       }
     }
+  }
   }
   if (!mirror) return;
   __syncthreads();
@@ -901,72 +936,6 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
   if (tn * 64 + c < P.nn)
     for (int r = threadIdx.x >> 6; r < 64 && tm * 64 + r < P.nm; r += 8)
       P.C[cols[c] + rows[r]] = S[r * 65 + c];
-}
-
-// The listed 64 x 64 tiles with FP64 tensor operations (DMMA m8n8k4).
-constexpr int DK = 16, DP = 20;
-__global__ void __launch_bounds__(256) dmma_tiles_kernel(const __grid_constant__ CrtParams P, int tiles_m) {
-  __shared__ double As[64][DP], Bs[64][DP];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int wm = (warp & 1) * 32, wn = (warp >> 1) * 16, gid = lane >> 2, tig = lane & 3;
-  const unsigned ntile = min(P.list[0], (unsigned)(tiles_m * ((P.nn + 63) / 64)));
-  for (unsigned t = blockIdx.x; t < ntile; t += gridDim.x) {
-    const int id = (int)P.list[1 + t], m0 = (id % tiles_m) * 64, n0 = (id / tiles_m) * 64;
-    double acc[4][2][2];
-#pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-      for (int y = 0; y < 2; ++y) acc[x][y][0] = acc[x][y][1] = 0.0;
-    // this thread's four (row, k) places of each operand
-    const double *pa[4], *pb[4];
-    int ra[4], rb[4], ka[4], kb[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      ra[q] = P.A.sk == 1 ? (tid >> 4) + 16 * q : tid & 63;
-      ka[q] = P.A.sk == 1 ? tid & 15 : (tid >> 6) + 4 * q;
-      rb[q] = P.B.sk == 1 ? (tid >> 4) + 16 * q : tid & 63;
-      kb[q] = P.B.sk == 1 ? tid & 15 : (tid >> 6) + 4 * q;
-      pa[q] = m0 + ra[q] < P.nm ? P.A.base + row_off(P.A, P.row0 + m0 + ra[q]) : nullptr;
-      pb[q] = n0 + rb[q] < P.nn ? P.B.base + row_off(P.B, P.col0 + n0 + rb[q]) : nullptr;
-    }
-    for (int k0 = 0; k0 < P.A.K; k0 += DK) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        As[ra[q]][ka[q]] = pa[q] && k0 + ka[q] < P.A.K ? pa[q][(long long)(k0 + ka[q]) * P.A.sk] : 0.0;
-        Bs[rb[q]][kb[q]] = pb[q] && k0 + kb[q] < P.A.K ? pb[q][(long long)(k0 + kb[q]) * P.B.sk] : 0.0;
-      }
-      __syncthreads();
-#pragma unroll
-      for (int ks = 0; ks < DK; ks += 4) {
-        double af[4], bf[2];
-#pragma unroll
-        for (int x = 0; x < 4; ++x) af[x] = As[wm + 8 * x + gid][ks + tig];
-#pragma unroll
-        for (int y = 0; y < 2; ++y) bf[y] = Bs[wn + 8 * y + gid][ks + tig];
-#pragma unroll
-        for (int x = 0; x < 4; ++x)
-#pragma unroll
-          for (int y = 0; y < 2; ++y)
-            asm volatile(
-                "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                : "+d"(acc[x][y][0]), "+d"(acc[x][y][1])
-                : "d"(af[x]), "d"(bf[y]));
-      }
-      __syncthreads();
-    }
-#pragma unroll
-    for (int x = 0; x < 4; ++x)
-#pragma unroll
-      for (int y = 0; y < 2; ++y)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          const int m = m0 + wm + 8 * x + gid, n = n0 + wn + 8 * y + 2 * tig + h;
-          if (m < P.nm && n < P.nn) {
-            put_c(P, P.row0 + m, P.col0 + n, acc[x][y][h]);
-            if (P.sym && m0 != n0) put_c(P, n, m, acc[x][y][h]);
-          }
-        }
-  }
 }
 
 // --------------------------------------------------------------------------
@@ -1017,22 +986,22 @@ OpArgs op_args(ModOperand &op, const RowMap &M, int row0, bool used) {
 }
 
 // Residues of rows [r0, ..) of A into Q and of columns [c0, ..) of B into L;
-// either may be in place already.  Clears the list of tiles left to FP64.
+// either may be in place already.
 int fill_operands(ModOperand &Q, const RowMap &A, int r0, bool rows, ModOperand &L, const RowMap &B,
-                  int c0, bool cols, unsigned *list, cudaStream_t s) {
+                  int c0, bool cols, cudaStream_t s) {
   OpArgs a = op_args(Q, A, r0, rows), b = op_args(L, B, c0, cols);
   const bool one = a.nkc == 1 && a.blocks + b.blocks > 0;
   if (!one) {
-    row_scale_kernel<<<(unsigned)std::max(1, a.blocks + b.blocks), 256, 0, s>>>(a, b, list);
+    row_scale_kernel<<<(unsigned)std::max(1, a.blocks + b.blocks), 256, 0, s>>>(a, b);
     count_launch(1);
   }
   a.blocks = rows ? a.nkc * ((a.rows + 31) / 32) : 0;
   b.blocks = cols ? b.nkc * ((b.rows + 31) / 32) : 0;
   if (a.blocks + b.blocks > 0) {
     if (one)
-      residue_kernel<true><<<(unsigned)(a.blocks + b.blocks), 256, 0, s>>>(a, b, list);
+      residue_kernel<true><<<(unsigned)(a.blocks + b.blocks), 256, 0, s>>>(a, b);
     else
-      residue_kernel<false><<<(unsigned)(a.blocks + b.blocks), 256, 0, s>>>(a, b, list);
+      residue_kernel<false><<<(unsigned)(a.blocks + b.blocks), 256, 0, s>>>(a, b);
     count_launch(1);
   }
   RIMP2_CK(cudaGetLastError());
@@ -1188,7 +1157,6 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
   const int rb = (int)std::min<long long>(B.rows, std::min(cap_rows, cap_cols));
   if (g.lower && (ra < A.rows || rb < B.rows)) return RIMP2_OK;
   if ((rb + 63) / 64 > 65535) return RIMP2_OK;
-  const long long tiles_m = (ra + 63) / 64, tiles_n = (rb + 63) / 64;
   ModOperand Q, L;
   Q.rows = ra;
   L.rows = rb;
@@ -1196,17 +1164,16 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
   // a product of one set of vectors with itself needs their residues once
   const bool same = ra == A.rows && rb == B.rows && A.rows == B.rows && A.base == B.base && A.sk == B.sk &&
                     memcmp(A.ext, B.ext, sizeof A.ext) == 0 && memcmp(A.st, B.st, sizeof A.st) == 0;
-  DevBuf arena, res, list;
+  DevBuf arena, res;
   {
-    DevBuf *const buf[] = {&Q.planes, &L.planes, &res, &Q.e, &L.e, &Q.flag, &L.flag, &list};
+    DevBuf *const buf[] = {&Q.planes, &L.planes, &res, &Q.e, &L.e, &Q.flag, &L.flag};
     const size_t bytes[] = {mod_operand_bytes(ra, g.K),
                             same ? 0 : mod_operand_bytes(rb, g.K),
                             (size_t)MG_PLANES * rb * ldm,
                             sizeof(int) * (size_t)ra,
                             sizeof(int) * (size_t)rb,
                             (size_t)ra,
-                            (size_t)rb,
-                            sizeof(unsigned) * (size_t)(tiles_m * tiles_n + 1)};
+                            (size_t)rb};
     if (alloc_parts(arena, buf, bytes, s) != RIMP2_OK) {
       (void)cudaGetLastError();  // no room: the FP64 kernel needs none
       clear_error();
@@ -1234,12 +1201,11 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
   P.lower = g.lower;
   P.nfast = B.cst[0] < A.cst[0];
   P.sym = same && !g.lower && g.beta == 0.0 && A.rows > 256 && memcmp(A.role, B.role, sizeof A.role) == 0;
-  constexpr int mirror_smem = 64 * 65 * (int)sizeof(double);
+  const int crt_smem = (P.sym ? 64 * 65 : 2 * 64 * DP) * (int)sizeof(double);
   const bool plain = g.alpha == 1.0 && g.beta == 0.0;
   auto *crt = plain ? (g.denom ? crt_epilogue_kernel<CRT_QUOTIENT> : crt_epilogue_kernel<CRT_PLAIN>)
               : !g.denom && g.alpha == -1.0 && g.beta == 1.0 ? crt_epilogue_kernel<CRT_MINUS>
                                                              : crt_epilogue_kernel<CRT_ANY>;
-  P.list = list.as<unsigned>();
   P.ea = Q.e.as<int>();
   P.fa = Q.flag.as<unsigned char>();
   P.eb = L.e.as<int>();
@@ -1250,7 +1216,7 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
       const int nc = std::min(rb, B.rows - c0);
       const bool cols = !same && (r0 == 0 || rb < B.rows);
       if (cols || same) L.rows = nc;
-      RIMP2_TRY(fill_operands(Q, A, r0, c0 == 0, L, B, c0, cols, list.as<unsigned>(), s));
+      RIMP2_TRY(fill_operands(Q, A, r0, c0 == 0, L, B, c0, cols, s));
       P.row0 = r0;
       P.col0 = c0;
       P.nm = Q.rows;
@@ -1258,10 +1224,8 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
       P.ldm = ((long long)Q.rows + 255) / 256 * 256;
       RIMP2_TRY(mod_product(L, Q, res.as<signed char>(), P.ldm, g.lower || P.sym, s));
       dim3 grid((unsigned)((P.nm + 63) / 64), (unsigned)((P.nn + 63) / 64));
-      crt<<<grid, 512, P.sym ? mirror_smem : 0, s>>>(P);
-      const long long nt = (long long)grid.x * grid.y;
-      dmma_tiles_kernel<<<(unsigned)std::min<long long>(nt, 304), 256, 0, s>>>(P, (int)grid.x);
-      count_launch(2);
+      crt<<<grid, 512, crt_smem, s>>>(P);
+      count_launch(1);
       RIMP2_CK(cudaGetLastError());
     }
   }

@@ -187,7 +187,7 @@ def test_fp64_energies(api, nocc, nvirt, nba, spread):
     Er, Tr = fp64_energies(nocc, nvirt, nba, Ca, eo, ev)
     before = api.kernel_launch_count()
     E, T = api.energy(nvirt, nocc, nba, Ca, eo, ev)
-    assert api.kernel_launch_count() - before > 8, "expected the residue form"
+    assert api.kernel_launch_count() - before > 7, "expected the residue form"
     # both sides sum FP64 terms of g and 1/D that are a few ulp off; the terms
     # of a pair cancel by no more than their number: sums of magnitudes over
     # |e_ij| stay below ~10 here, the sums' rounding below sqrt(nvirt) u each
@@ -202,7 +202,7 @@ def test_fp64_amplitudes(api, nocc, nvirt, nba):
     eo, ev = np.sort(-r.random(nocc) - 0.3), np.sort(r.random(nvirt) + 0.1)
     before = api.kernel_launch_count()
     E, T, t = api.energy(nvirt, nocc, nba, Ca, eo, ev, amplitudes=True)
-    assert api.kernel_launch_count() - before > 8, "expected the residue form"
+    assert api.kernel_launch_count() - before > 7, "expected the residue form"
     g = np.tensordot(Ca, Ca, (0, 0))
     mag = np.tensordot(np.abs(Ca), np.abs(Ca), (0, 0))
     d = eo[None, :, None, None] + eo - ev[:, None, None, None] - ev[None, None, :, None]
