@@ -160,6 +160,66 @@ __global__ void __launch_bounds__(BM / WM * (BN / WN) * 32) gemm_f64_kernel(MapG
   }
 }
 
+// C of at most eight columns: two rows of A a thread, the columns' operand in shared
+// memory, plain FMAs (rows whose sums are contiguous too: a thread's next terms
+// are in the sectors it has read, and the FP64 pipe waits longer than L1 does).  A scheduler's FP64 unit takes 64
+// clocks for 32 of them and 576 for the 256 of a DMMA, which also computes the
+// columns up to eight and the terms up to four: 2.33 -> 1.41 ms for 4.1 million
+// rows, 7 columns and sums of 30 (the FP64 pipe bounds both).  PLAIN: C = A B.
+constexpr int THIN_K = 64, THIN_ROWS = 2 * 256;
+template <int N, bool PLAIN>
+__global__ void __launch_bounds__(256) thin_f64_kernel(MapGemm g) {
+  __shared__ double2 U[THIN_K][4];  // B(k, n), pairs of columns
+  const int M = g.A.rows, K = g.A.K;
+  const long long m = (long long)blockIdx.x * THIN_ROWS + threadIdx.x;
+  const bool live[2] = {m < M, m + 256 < M};
+  const double *a[2];
+  double acc[2][N];
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    a[r] = g.A.base + (live[r] ? row_off(g.A, (int)(m + 256 * r)) : 0);
+#pragma unroll
+    for (int n = 0; n < N; ++n) acc[r][n] = 0.0;
+  }
+  for (int k0 = 0; k0 < K; k0 += THIN_K) {
+    __syncthreads();
+    for (int t = threadIdx.x; t < THIN_K * N; t += 256) {
+      const int k = t % THIN_K, n = t / THIN_K;
+      if (k0 + k < K)
+        reinterpret_cast<double *>(U[k])[n] = g.B.base[row_off(g.B, n) + (long long)(k0 + k) * g.B.sk];
+    }
+    __syncthreads();
+    const int kn = min(THIN_K, K - k0);
+#pragma unroll 4
+    for (int k = 0; k < kn; ++k) {
+      double x[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) x[r] = live[r] ? a[r][(long long)(k0 + k) * g.A.sk] : 0.0;
+#pragma unroll
+      for (int n = 0; n < N; n += 2) {
+        const double2 u = U[k][n / 2];
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          acc[r][n] = fma(x[r], u.x, acc[r][n]);
+          if (n + 1 < N) acc[r][n + 1] = fma(x[r], u.y, acc[r][n + 1]);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    if (!live[r]) continue;
+    const long long o = c_off(g.A, (int)(m + 256 * r));
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      if (PLAIN)
+        g.C[o + c_off(g.B, n)] = acc[r][n];
+      else
+        put_c(g, (int)(m + 256 * r), n, acc[r][n]);
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
 // Fused FP64 energy kernel
 // ---------------------------------------------------------------------------
@@ -746,6 +806,11 @@ static int dmma_form(double m, double n, double k, bool lower, int nsm, double *
   return best;
 }
 
+// Time of thin_f64_kernel: 1.15 TFLOP/s over all SMs, 7.6 GFLOP/s on one.
+static double thin_time(double m, double n, double k, int nsm) {
+  return 5e-6 + std::ceil(m / THIN_ROWS / nsm) * THIN_ROWS * n * k * 2.0 / 7.6e9;
+}
+
 static double gemm_time(double m, double n, double k, bool lower, int nsm) {
   double t;
   dmma_form(m, n, k, lower, nsm, &t);
@@ -762,6 +827,19 @@ static int launch_dmma(const MapGemm &P, cudaStream_t s) {
   return RIMP2_OK;
 }
 
+template <int N>
+static int launch_thin(const MapGemm &P, cudaStream_t s) {
+  const bool plain = P.alpha == 1.0 && P.beta == 0.0 && !P.denom;
+  const unsigned blocks = (unsigned)(((long long)P.A.rows + THIN_ROWS - 1) / THIN_ROWS);
+  if (plain)
+    thin_f64_kernel<N, true><<<blocks, 256, 0, s>>>(P);
+  else
+    thin_f64_kernel<N, false><<<blocks, 256, 0, s>>>(P);
+  count_launch(1);
+  RIMP2_CK(cudaGetLastError());
+  return RIMP2_OK;
+}
+
 static int launch_folded(const GemmDesc &g, RowMap A, RowMap B, cudaStream_t s) {
   int dev = 0, nsm = 0;
   RIMP2_CK(cudaGetDevice(&dev));
@@ -772,6 +850,12 @@ static int launch_folded(const GemmDesc &g, RowMap A, RowMap B, cudaStream_t s) 
   const double m = thin_rows ? B.rows : A.rows, n = thin_rows ? A.rows : B.rows;
   double t;
   const int form = dmma_form(m, n, g.K, g.lower != 0, nsm, &t);
+  // at most eight columns: plain FMAs, where the rows fill the SMs and rows or
+  // sums run along the fast direction
+  const RowMap &rows = thin_rows ? B : A;
+  const bool thin = !g.lower && n <= 8 && (rows.sk == 1 || (rows.st[0] == 1 && rows.ext[0] >= 16)) &&
+                    thin_time(m, n, g.K, nsm) < t;
+  if (thin) t = thin_time(m, n, g.K, nsm);
   // large ones go to the FP16 tensor cores as residues
   if (mod_gemm_time(A.rows, B.rows, g.K, g.lower != 0) < 0.9 * t) {
     bool done = false;
@@ -788,6 +872,18 @@ static int launch_folded(const GemmDesc &g, RowMap A, RowMap B, cudaStream_t s) 
   P.ev = g.ev;
   P.denom = g.denom;
   P.lower = g.lower;
+  if (thin) {
+    switch (P.B.rows) {
+      case 1: return launch_thin<1>(P, s);
+      case 2: return launch_thin<2>(P, s);
+      case 3: return launch_thin<3>(P, s);
+      case 4: return launch_thin<4>(P, s);
+      case 5: return launch_thin<5>(P, s);
+      case 6: return launch_thin<6>(P, s);
+      case 7: return launch_thin<7>(P, s);
+      default: return launch_thin<8>(P, s);
+    }
+  }
   if (form == 1) return launch_dmma<32, 32, 16, 16>(P, s);
   if (form == 2) return launch_dmma<16, 16, 16, 16>(P, s);
   if (form == 3) return launch_dmma<128, 8, 32, 8>(P, s);

@@ -76,6 +76,25 @@ def test_product_forms(api, residues, ta, tb, m, n, k, alpha, beta, pad):
         assert abs(C[i, j] - ref) <= tol
 
 
+@pytest.mark.parametrize("n", range(1, 9))
+@pytest.mark.parametrize("ta,m,k,alpha,beta", [
+    ("N", 160001, 33, 1.0, 0.0),   # rows along the fast direction, one past a block
+    ("N", 156000, 65, -1.0, 1.0),  # two chunks of the columns' operand
+    ("T", 160001, 30, 1.0, 0.0),   # sums along it
+    ("T", 158000, 64, 0.5, -2.0),
+])
+def test_thin_products(api, ta, m, n, k, alpha, beta):
+    """At most eight columns: FP64's own bound, K u sum|a||b|, then alpha and beta."""
+    r = np.random.Generator(np.random.Philox(key=[n, k]))
+    A, B = r.standard_normal((m, k)), r.standard_normal((k, n))
+    C0 = np.asfortranarray(r.standard_normal((m, n)))
+    C = C0.copy(order="F")
+    assert product(api, ta, "N", A, B, alpha, beta, C) == 1
+    ref, mag = A @ B, np.abs(A) @ np.abs(B)  # numpy's own error: the same bound
+    tol = 2 * abs(alpha) * k * U * mag + 3 * U * (np.abs(alpha * ref) + np.abs(beta * C0))
+    assert (np.abs(C - (alpha * ref + beta * C0)) <= tol).all()
+
+
 def test_product_exact_and_special_values(api):
     r = np.random.Generator(np.random.Philox(key=[5, 9]))
     m = n = k = 640
