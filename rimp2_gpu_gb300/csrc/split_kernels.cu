@@ -520,6 +520,7 @@ __global__ void __launch_bounds__(BATCH_THREADS, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_wait();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -958,6 +959,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
   cluster_sync_all();  // both CTAs' barriers are initialised before any remote access
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  grid_wait();
 
   if (warp == 0) {
     // --------------------- TMA producers (both CTAs) ---------------------
@@ -2277,6 +2279,7 @@ __global__ void __launch_bounds__(256, 6) single_inputs_kernel(const __grid_cons
   if ((int)blockIdx.x < P.slice_blocks) {
     const int col = (blockIdx.x * 256 + threadIdx.x) >> 5;
     if (col < P.F.ncol) slice_column(P.F, col, P.nsl, P.plane, P.slices, P.inv, P.vplane, P.dcorr);
+    grid_trigger();
     return;
   }
   const int t = ((int)blockIdx.x - P.slice_blocks) * 256 + threadIdx.x;
@@ -2287,6 +2290,7 @@ __global__ void __launch_bounds__(256, 6) single_inputs_kernel(const __grid_cons
   eps_entry(P.F, t, P.eo2, P.ev2);
   if (t < P.nitems) P.items[t] = work_item(P.F, 0, t);
   if (t < P.npitems) P.pitems[t] = pair_item(P.F, 0, t);
+  grid_trigger();
 }
 
 // One warp per pair; the last block to finish sums the total.
@@ -2295,6 +2299,7 @@ __global__ void __launch_bounds__(256) single_reduce_kernel(const __grid_constan
   __shared__ bool last;
   const FragDesc &F = P.F;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, p = blockIdx.x * 8 + w;
+  grid_wait();
   if (p < F.nocc * (F.nocc + 1) / 2) {
     const double *src = P.part + (long long)p * F.ntp;
     double s = 0.0, c = 0.0;
@@ -2388,15 +2393,15 @@ int pair_stages_for(const std::vector<FragDesc> &fh) {
   return 3;
 }
 
-int launch_pair(const Group &g, PairParams Q, int npair, cudaStream_t s) {
+int launch_pair(const Group &g, PairParams Q, int npair, cudaStream_t s, bool overlap = false) {
   Q.xbuf = g.xbuf.as<float>();
   cudaError_t e;
   if (g.pair_nstage == 4)
-    e = launch_hi(split_pair_kernel<4, true>, 2 * npair, NTHREADS, pair_smem_bytes(4, true), s,
-                  g.tm, g.tmB, Q);
+    e = launch_ex(true, overlap, split_pair_kernel<4, true>, 2 * npair, NTHREADS,
+                  pair_smem_bytes(4, true), s, g.tm, g.tmB, Q);
   else
-    e = launch_hi(split_pair_kernel<3, false>, 2 * npair, NTHREADS, pair_smem_bytes(3, false),
-                  s, g.tm, g.tmB, Q);
+    e = launch_ex(true, overlap, split_pair_kernel<3, false>, 2 * npair, NTHREADS,
+                  pair_smem_bytes(3, false), s, g.tm, g.tmB, Q);
   if (e != cudaSuccess) {
     set_error("paired energy kernel launch failed: %s", cudaGetErrorString(e));
     return RIMP2_ERR_CUDA;
@@ -2552,6 +2557,14 @@ int record_group(Group &g, cudaStream_t s, int nsm, cudaEvent_t *ev /* 3 or null
   const FragDesc *fr = g.frags.as<FragDesc>();
   if (ev) RIMP2_CK(cudaEventRecord(ev[0], s));
   SingleArgs A;
+  // the kernels of one fragment are set up at the end of the one before (not in a
+  // graph under capture, nor between timing events): 27 -> 23 us a call at nocc = 8,
+  // nvirt = 96, NBA = 256, 271 -> 266 at 24/301/1203.  The inputs' blocks say so when
+  // they are done; with the energy kernel saying so at its start, the waiting
+  // reduction cost 6 to 16 us.
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const bool overlap = single && !ev && cudaStreamIsCapturing(s, &cap) == cudaSuccess &&
+                       cap == cudaStreamCaptureStatusNone;
   if (single) {
     A.F = g.fh[0];
     A.frag = g.frags.as<FragDesc>();
@@ -2609,21 +2622,22 @@ int record_group(Group &g, cudaStream_t s, int nsm, cudaEvent_t *ev /* 3 or null
     Q.part = P.part;
     Q.err = P.err;
     const int npair = (int)std::min<long long>(g.npitems, std::max(1, nsm / 2));
-    RIMP2_TRY(launch_pair(g, Q, npair, s));
+    RIMP2_TRY(launch_pair(g, Q, npair, s, overlap));
     note_split_kernel(2);
   } else if (g.nsl == 2) {
     note_split_kernel(1);
-    RIMP2_CK(launch_hi(split_batch_kernel<2, 3>, grid, BATCH_THREADS, smem_bytes(2, 3), s, g.tm, P));
+    RIMP2_CK(launch_ex(true, overlap, split_batch_kernel<2, 3>, grid, BATCH_THREADS, smem_bytes(2, 3), s,
+                       g.tm, P));
   } else {
     note_split_kernel(1);
-    RIMP2_CK(launch_hi(split_batch_kernel<3, 2>, grid, BATCH_THREADS, smem_bytes(3, 2), s, g.tm, P));
+    RIMP2_CK(launch_ex(true, overlap, split_batch_kernel<3, 2>, grid, BATCH_THREADS, smem_bytes(3, 2), s,
+                       g.tm, P));
   }
   count_launch(1);
   if (ev) RIMP2_CK(cudaEventRecord(ev[2], s));
   if (single) {
-    single_reduce_kernel<<<(unsigned)((g.npairs_total + 7) / 8), 256, 0, s>>>(A);
+    RIMP2_CK(launch_ex(false, overlap, single_reduce_kernel, (unsigned)((g.npairs_total + 7) / 8), 256, 0, s, A));
     count_launch(1);
-    RIMP2_CK(cudaGetLastError());
     return RIMP2_OK;
   }
   pair_reduce_batch_kernel<<<(unsigned)((g.npairs_total + 7) / 8), 256, 0, s>>>(

@@ -67,6 +67,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   return true;
 }
 
+// The kernels before this one in the stream are complete, their writes visible
+// (at once for a kernel that was launched after them).
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel may be set up once every block got here.
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap *map, uint32_t bar,
                                             int c0, int c1, int c2) {
   asm volatile(
@@ -285,20 +291,35 @@ int energy_priority() {
   return prio;
 }
 
+// overlap: the kernel may be set up while the one before it in the stream still
+// runs; it calls grid_wait() before it touches memory.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_hi(void (*k)(KArgs...), unsigned grid, unsigned block, size_t smem,
-                      cudaStream_t s, Args... args) {
+cudaError_t launch_ex(bool high, bool overlap, void (*k)(KArgs...), unsigned grid, unsigned block,
+                      size_t smem, cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributePriority;
-  at[0].val.priority = energy_priority();
+  cudaLaunchAttribute at[2];
+  int n = 0;
+  if (high) {
+    at[n].id = cudaLaunchAttributePriority;
+    at[n++].val.priority = energy_priority();
+  }
+  if (overlap) {
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
   cfg.attrs = at;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = n;
   return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
+template <typename... KArgs, typename... Args>
+cudaError_t launch_hi(void (*k)(KArgs...), unsigned grid, unsigned block, size_t smem,
+                      cudaStream_t s, Args... args) {
+  return launch_ex(true, false, k, grid, block, smem, s, args...);
 }
 
 }  // namespace
