@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "mod_gemm.cuh"
+#include "tc.cuh"
 
 namespace rimp2 {
 void count_launch(int n);
@@ -160,6 +161,7 @@ __global__ void __launch_bounds__(PT) potrf_block_kernel(double *V, int n, int k
   __shared__ double rd[NB];  // 1 / L(k, k)
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
   const int r = lane & 15, h = lane >> 4;
+  grid_wait();
 #pragma unroll
   for (int t = threadIdx.x; t < NB * NB; t += PT) {
     const int i = t & (NB - 1), c = t >> 6;
@@ -271,6 +273,7 @@ __global__ void __launch_bounds__(160) panel_solve_kernel(double *V, int n, int 
   __shared__ double Xs[2][8][PS];   // the solution, in two parts
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
   const int row0 = k0 + NB + blockIdx.x * 8;
+  grid_wait();
   const int y = w & 1, z = w >> 1;
   double acc[4][2];  // rows gid, columns 16 j + 8 y + 2 tig + {0, 1}
   if (w < 4) {
@@ -420,11 +423,12 @@ int dev_cholesky(int n, double *V, cudaStream_t s) {
     const int p1 = n - p0 < CH_PANEL ? n : p0 + CH_PANEL;
     for (int k0 = p0; k0 < p1; k0 += NB) {
       const int b = n - k0 < NB ? n - k0 : NB;
-      potrf_block_kernel<<<1, PT, 0, s>>>(V, n, k0, b, bad.as<int>(), dinv.as<double>());
+      RIMP2_CK(launch_ex(false, true, potrf_block_kernel, 1, PT, 0, s, V, n, k0, b, bad.as<int>(), dinv.as<double>()));
       count_launch(1);
       const int r0 = k0 + b;
       if (r0 >= n) break;
-      panel_solve_kernel<<<(n - r0 + 7) / 8, 160, 0, s>>>(V, n, k0, dinv.as<double>());
+      RIMP2_CK(launch_ex(false, true, panel_solve_kernel, (n - r0 + 7) / 8, 160, 0, s, V, n, k0,
+                         (const double *)dinv.as<double>()));
       count_launch(1);
       if (r0 < p1) RIMP2_TRY(update(r0, r0, p1 - r0, k0, NB, false));
     }

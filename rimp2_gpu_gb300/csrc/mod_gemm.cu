@@ -218,6 +218,7 @@ __global__ void __launch_bounds__(256) row_scale_kernel(const __grid_constant__ 
       stat_merge(s, e2, s2, l2, b2);
     }
     if (lane == 0) stat_store(s, P.e + r, P.flag + r);
+    grid_trigger();
     return;
   }
   const int r = blk * 32 + lane;
@@ -240,6 +241,7 @@ __global__ void __launch_bounds__(256) row_scale_kernel(const __grid_constant__ 
     }
     stat_store(s, P.e + r, P.flag + r);
   }
+  grid_trigger();
 }
 
 // |x| 2^e rounded to an integer (< 2^63)
@@ -308,6 +310,7 @@ template <bool SCALE>
 __global__ void __launch_bounds__(256) residue_kernel(const __grid_constant__ OpArgs A,
                                                       const __grid_constant__ OpArgs B) {
   __shared__ double sh[64][33];
+  grid_wait();
   const bool second = (int)blockIdx.x >= A.blocks;
   const OpArgs &P = second ? B : A;
   const RowMap &M = P.M;
@@ -369,6 +372,7 @@ __global__ void __launch_bounds__(256) residue_kernel(const __grid_constant__ Op
   const bool live = !(flag & MG_ROW_FP64);
   __half *out = P.out + ((size_t)kc * P.rows + r) * 64 + kq * 8;
   residues8(v, e, live, out, P.plane);
+  grid_trigger();
 }
 
 // --------------------------------------------------------------------------
@@ -477,6 +481,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
   const uint32_t tmem = *tmem_slot;
   if (warp == 1)  // both CTAs hold their columns
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  grid_wait();
 
   if (warp == 0) {
     // --------------------- TMA producers (both CTAs) ---------------------
@@ -787,6 +792,7 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
   extern __shared__ double S[];             // symmetric: [64][65]; a tile summed in FP64: its operands
   double(*As)[DP] = reinterpret_cast<double(*)[DP]>(S), (*Bs)[DP] = As + 64;
   const int tm = blockIdx.x, tn = blockIdx.y;
+  grid_wait();
   if ((P.lower || P.sym) && tm < tn) return;
   const int t0 = threadIdx.x & 15, t1 = threadIdx.x >> 4;
   const int mq = (P.nfast ? t1 & 15 : t0) * 4, nq = P.nfast ? t0 + (t1 & 16) : t1;
@@ -1001,7 +1007,7 @@ int fill_operands(ModOperand &Q, const RowMap &A, int r0, bool rows, ModOperand 
     if (one)
       residue_kernel<true><<<(unsigned)(a.blocks + b.blocks), 256, 0, s>>>(a, b);
     else
-      residue_kernel<false><<<(unsigned)(a.blocks + b.blocks), 256, 0, s>>>(a, b);
+      RIMP2_CK(launch_ex(false, true, residue_kernel<false>, (unsigned)(a.blocks + b.blocks), 256, 0, s, a, b));
     count_launch(1);
   }
   RIMP2_CK(cudaGetLastError());
@@ -1025,7 +1031,8 @@ static int launch_product(const CUtensorMap &tl, const CUtensorMap &tq, const Mg
   RIMP2_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const long long nitems = (long long)MG_PLANES * mg_tiles(P);
   const int npair = (int)std::min<long long>(nitems, nsm / 2);
-  RIMP2_CK(launch_hi(mod_gemm_kernel<TQ>, 2 * npair, MG_THREADS, mg_smem(TQ), s, tl, tq, P));
+  // each kernel of a contraction is set up at the end of the one before
+  RIMP2_CK(launch_ex(true, true, mod_gemm_kernel<TQ>, 2 * npair, MG_THREADS, mg_smem(TQ), s, tl, tq, P));
   count_launch(1);
   return RIMP2_OK;
 }
@@ -1224,7 +1231,7 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
       P.ldm = ((long long)Q.rows + 255) / 256 * 256;
       RIMP2_TRY(mod_product(L, Q, res.as<signed char>(), P.ldm, g.lower || P.sym, s));
       dim3 grid((unsigned)((P.nm + 63) / 64), (unsigned)((P.nn + 63) / 64));
-      crt<<<grid, 512, crt_smem, s>>>(P);
+      RIMP2_CK(launch_ex(false, true, crt, grid, 512, crt_smem, s, P));
       count_launch(1);
       RIMP2_CK(cudaGetLastError());
     }

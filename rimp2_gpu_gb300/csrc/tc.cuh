@@ -294,10 +294,10 @@ int energy_priority() {
 // overlap: the kernel may be set up while the one before it in the stream still
 // runs; it calls grid_wait() before it touches memory.
 template <typename... KArgs, typename... Args>
-cudaError_t launch_ex(bool high, bool overlap, void (*k)(KArgs...), unsigned grid, unsigned block,
+cudaError_t launch_ex(bool high, bool overlap, void (*k)(KArgs...), dim3 grid, unsigned block,
                       size_t smem, cudaStream_t s, Args... args) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
