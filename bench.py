@@ -505,14 +505,18 @@ def run_ours(args):
                 break
         with Clocks(local) as pclk:
             fp64_peak = api.probe_fp64_peak()  # one launch of >= 1 s
-        # performed DMMA work: i<j pairs compute T1 and T2 of every 64x64 tile
-        # pair A<=B, i=j pairs T1 only; K is padded to the 16-wide slab
+        # FP64 products of the pair energies, as a DMMA kernel performs them: i<j
+        # pairs compute T1 and T2 of every 64x64 tile pair A<=B, i=j pairs T1 only; K
+        # is padded to the 16-wide slab.  One fragment's integrals come as residue
+        # products on the FP16 tensor cores, far above the FP64 pipe's own rate.
         nt64 = (NVIRT + 63) // 64
         performed = 2.0 * (NOCC * (NOCC - 1) // 2 * 2 + NOCC) * (nt64 * (nt64 + 1) // 2) * \
             64 * 64 * ((NBA + 15) // 16 * 16)
         plain = {"ms": pms, "eff_tflops": eff_flop() / pms / 1e9,
                  "performed_tflops": performed / pms / 1e9, "fp64_dmma_peak_tflops": fp64_peak,
                  "frac_of_fp64_peak": performed / pms / 1e9 / fp64_peak,
+                 "performed_is": "FP64 products a DMMA kernel would perform; they run as residues "
+                                 "on the FP16 tensor cores",
                  "fp64_peak_probe": "independent DMMA chains on every SM, one launch of >= 1 s "
                                     "(the library's rimp2_probe_fp64_peak)",
                  "fp64_peak_probe_clocks": pclk.summary()}

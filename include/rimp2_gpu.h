@@ -36,7 +36,7 @@ extern "C" {
 #define RIMP2_ERR_TIMEOUT 5 /* a device-side bounded wait ran out */
 #define RIMP2_ERR_UNSUPPORTED 6
 
-#define RIMP2_PREC_FP64 0  /* plain FP64 (DMMA) fused kernel */
+#define RIMP2_PREC_FP64 0  /* plain FP64 (residue products or DMMA) */
 #define RIMP2_PREC_SPLIT 1 /* split-precision tcgen05 alpha contraction */
 
 /* ---- library state ----------------------------------------------------- */
@@ -181,7 +181,7 @@ int rimp2_first_order(const int *nvirt, const int *nocc, const int *noccEOS, con
  * Po = UoccEOST UoccEOST^T, Pv = UvirtT UvirtT^T (occupied partitioning) or
  * Po = UoccT UoccT^T, Pv = UvirtEOST UvirtEOST^T (virtual partitioning).
  * With U = I both are the canonical MP2 energy.  precision: RIMP2_PREC_FP64
- * (FP64 DMMA) or RIMP2_PREC_SPLIT (tcgen05 split form with the slice count of
+ * (FP64) or RIMP2_PREC_SPLIT (tcgen05 split form with the slice count of
  * the shape-bucket table; relative error within 1e-7).  Ct is formed with
  * FP64 GEMMs either way. */
 int rimp2_energy_eos(const int *nvirt, const int *nocc, const int *noccEOS, const int *nvirtEOS,
@@ -212,7 +212,8 @@ int rimp2_datafile_write(const char *path, const int *hdr, int first_order,
  * RIMP2_calc_toccA, RIMP2.F90:397-404) --------------------------------------
  * e_ij = sum_ab t_ij^ab (2 g_ij^ab - g_ij^ba),  t = g / (e_i+e_j-e_a-e_b),
  * Epair(nocc,nocc) symmetric, Etot = sum_ij e_ij.
- * precision: RIMP2_PREC_FP64 (FP64 DMMA, 1e-11 of the FP64 oracle) or
+ * precision: RIMP2_PREC_FP64 (1e-11 of the FP64 oracle; sums in FP64 or exact
+ * before one rounding, by size) or
  * RIMP2_PREC_SPLIT (FP16 Ozaki slices on tcgen05: every pair energy and the
  * total within 1e-7 relative of FP64; the integer part of each product is
  * accumulated exactly, the corrections in FP32, the epilogue in FP32 with

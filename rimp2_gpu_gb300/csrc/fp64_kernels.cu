@@ -1,10 +1,16 @@
-// fp64_kernels.cu -- FP64 kernels on the DMMA (mma.sync .f64) tensor path.
+// fp64_kernels.cu -- FP64 contractions and energies.
 //
-//  * gemm_f64_kernel: strided, batched column-major-agnostic FP64 contraction
+//  * launch_gemm_f64: strided, batched column-major-agnostic FP64 contraction
 //    C(m,n) = alpha * sum_k A(m,k) B(k,n) + beta * C(m,n) with an optional
 //    orbital-energy denominator epilogue.  It carries every FP64 product of
 //    the drop-in subroutines (toccA/tvirtA g/D and projections, toccB/tvirtB,
-//    TransAlpha1/2, gocc/gvirt/gen4DimFO, the driver's DGEMMs).
+//    TransAlpha1/2, gocc/gvirt/gen4DimFO, the driver's DGEMMs): as residues on
+//    the FP16 tensor cores (mod_gemm.cu) where that is faster, else with FP64
+//    tensor operations (gemm_f64_kernel, mma.sync .f64) or, for at most eight
+//    columns, plain FMAs (thin_f64_kernel).
+//  * FP64 energies of one fragment: the integrals of occupied blocks by that
+//    product, then g_energy_kernel; small ones and captured calls by the
+//    fused kernel.
 //  * the fused FP64 energy: a work item is the tile pair (A,B) of occupied
 //    pair (i<=j): T1 = G_ij[A,B] = C_iA^T C_jB and T2 = G_ji[A,B] =
 //    C_jA^T C_iB share the (a,b) layout, so the exchange integral g_ij(b,a)
@@ -16,7 +22,7 @@
 //    local-orbital fragment energy).
 //
 // GB300 FP64 throughput is a small fraction of its low-precision tensor
-// rate, so these kernels are arithmetic-bound by construction: shared-memory
+// rate, so the FP64 kernels are arithmetic-bound by construction: shared-memory
 // staging is simple (cp.async double buffering in the GEMM), padding keeps
 // fragment loads bank-conflict free, and two CTAs per SM keep the FP64 pipe
 // busy.
@@ -464,8 +470,9 @@ __global__ void __launch_bounds__(NTHR, 2) eos_energy_kernel(const double *__res
 // through shared memory, so that both are read along the fast direction.  Off
 // the diagonal tile the two orders share a denominator:
 // 2 (g1^2 - g1 g2 + g2^2) / D.  It reads each integral once (8 bytes; twice on
-// diagonal tiles) and keeps to about ten FP64 operations per pair of elements:
-// at 1/64 of the FP32 rate these take as long as the reads.  The reciprocal is
+// diagonal tiles) and keeps to eight FP64 operations per pair of elements, which
+// bound it (386 us at nocc = 16, nvirt = 512; 464 with the diagonal tiles' form
+// computed beside the other and selected).  The reciprocal is
 // the FP32 one refined by a third-order Newton step (error about an ulp).
 struct GEnergyArgs {
   const double *G;
@@ -856,7 +863,10 @@ static int launch_folded(const GemmDesc &g, RowMap A, RowMap B, cudaStream_t s) 
   const bool thin = !g.lower && n <= 8 && (rows.sk == 1 || (rows.st[0] == 1 && rows.ext[0] >= 16)) &&
                     thin_time(m, n, g.K, nsm) < t;
   if (thin) t = thin_time(m, n, g.K, nsm);
-  // large ones go to the FP16 tensor cores as residues
+  // large ones go to the FP16 tensor cores as residues (2709 x 2709, sums of 1203:
+  // 0.22 ms against 18.4 with DMMA); short or small ones lose to that form's four
+  // launches and its operands' conversion (1000 x 192, sums of 64: 31 us with DMMA,
+  // 45 as residues)
   if (mod_gemm_time(A.rows, B.rows, g.K, g.lower != 0) < 0.9 * t) {
     bool done = false;
     RIMP2_TRY(mod_gemm(g, A, B, s, &done));

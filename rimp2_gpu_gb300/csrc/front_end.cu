@@ -5,7 +5,7 @@
 //   Calpha(:,a,i) = L^{-1} (:|a i)
 // so that sum_alpha Calpha(alpha,a,i) Calpha(alpha,b,j) = (ai|V^{-1}|bj).
 // The reference starts from Calpha (RIMP2.F90:48-49); this front end has no
-// counterpart there.  The AO->MO transform runs either on the FP64 DMMA GEMM
+// counterpart there.  The AO->MO transform runs either on the FP64 contraction
 // of fp64_kernels.cu or on the tcgen05 split GEMM (two residual FP16 slices,
 // ~2^-33 relative per product); the Cholesky and the solve are FP64, blocked
 // (64) so that all but O(n*64^2) of their work is GEMM:

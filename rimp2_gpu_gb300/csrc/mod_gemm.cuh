@@ -71,9 +71,9 @@ __device__ __forceinline__ bool recip_f32(double d, double &r0) {
   return true;
 }
 
-// 1/d: that reciprocal refined by a third-order Newton step, about an ulp.
-// FP64 operations run at 1/64 of the FP32 rate here: three instead of a
-// division's nine or so.
+// 1/d: that reciprocal refined by a third-order step of Householder's method,
+// r (1 + e + e^2) with e = 1 - d r: about an ulp.  FP64 operations run at 1/64 of
+// the FP32 rate here: three of them.
 __device__ __forceinline__ double recip_f64(double d) {
   double r0;
   if (!recip_f32(d, r0)) return 1.0 / d;
@@ -82,7 +82,7 @@ __device__ __forceinline__ double recip_f64(double d) {
 }
 
 // v / d: the quotient by that reciprocal corrected twice by its remainder
-// (22, 44, 66 bits before the last rounding), five operations
+// v - d q (Markstein; 22, 44, 66 bits before the last rounding), five operations
 __device__ __forceinline__ double div_f64(double v, double d) {
   const int ev = (__double2hiint(v) >> 20) & 0x7FF;
   double r;

@@ -4311,7 +4311,8 @@ int ao_half_fused(const double *ao, int NBA, int nbas, const double *Cmo, int no
 }
 
 // Local-orbital fragment energy in the split form: slices of Calpha and of its
-// projected copy Ct in one buffer, one persistent split_eos_kernel launch,
+// projected copies Ct in one buffer, one persistent launch (split_eos_pair_kernel;
+// split_eos_kernel with two residual slices),
 // compensated FP64 pair and total reductions.
 // Fragment energies of one or two projected copies of Calpha: Etot[c] from
 // copy Ct[c].
