@@ -226,6 +226,27 @@ def test_short_last_block_both_kernels(api, kernel_choice, rem):
         assert abs(E - Er) <= 1e-7 * abs(Er)
 
 
+@pytest.mark.parametrize("kern", ["0", "1"])
+@pytest.mark.parametrize("nocc,nvirt,NBA", [(9, 385, 128), (8, 257, 64), (7, 128, 64), (2, 640, 64)])
+def test_queue_order_leaves_results_alone(api, kernel_choice, kern, nocc, nvirt, NBA):
+    """One fragment's items in the order of their length, the same fragment as a batch
+    of one in pair order: the partial energies have their own places, equal bits."""
+    import torch
+    kernel_choice(kern)
+    Ca, eo, ev = O.gen_fragment(1700 + nvirt, nocc, nvirt, NBA)
+    Ep, E = dev_energy(api, Ca, eo, ev, 1)
+    d = [torch.from_numpy(x).cuda() for x in (Ca.ravel(order="F"), eo, ev)]
+    dE = torch.zeros(nocc * nocc, dtype=torch.float64, device="cuda")
+    dT = torch.zeros(1, dtype=torch.float64, device="cuda")
+    plan = api.BatchPlan([(nocc, nvirt, NBA) + tuple(x.data_ptr() for x in d + [dE, dT])], nslices=[1])
+    torch.cuda.synchronize()
+    plan.execute()
+    torch.cuda.synchronize()
+    plan.close()
+    assert np.array_equal(dE.cpu().numpy().reshape(nocc, nocc, order="F"), Ep)
+    assert dT.item() == E
+
+
 def test_pair_kernel_batched(api, kernel_choice):
     """Uneven fragments through one paired-CTA launch (graph-captured plan)."""
     import torch
