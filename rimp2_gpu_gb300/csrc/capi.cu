@@ -51,6 +51,8 @@ int collect_device_error(cudaStream_t s) {
   return RIMP2_OK;
 }
 
+void report_device_error(int code) { *(volatile int *)g_host_err = code; }
+
 void set_error(const char *fmt, ...) {
   va_list ap;
   va_start(ap, fmt);

@@ -21,6 +21,7 @@ cudaStream_t current_stream();
 int ensure_device();  // RIMP2_OK or an error status (message set)
 int *device_error_word();  // persistent device int that kernels set on a failed bounded wait
 int collect_device_error(cudaStream_t s);  // sync s, read + clear the word, map to a status
+void report_device_error(int code);        // sets that word from the host (fault injection)
 // optional per-phase event timing of the split path (ms of the last call)
 bool timing_enabled();
 void record_timing(int slot, float ms);
@@ -93,7 +94,8 @@ int alloc_parts(DevBuf &arena, DevBuf *const (&buf)[N], const size_t (&bytes)[N]
 
 // Host fault injection for failure-path tests: RIMP2_FAULT_INJECT=alloc makes
 // the next device allocation report out-of-memory, =launch makes the next
-// kernel-launch check report a launch failure.  Nothing touches the GPU.
+// kernel-launch check report a launch failure, =wait makes a residue product
+// report that one of its bounded waits ran out.  Nothing touches the GPU.
 bool inject_fault(const char *what);
 
 // ---- FP64 DMMA kernels (fp64_kernels.cu) -------------------------------------

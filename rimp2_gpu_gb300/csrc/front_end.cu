@@ -439,7 +439,8 @@ int dev_cholesky(int n, double *V, cudaStream_t s) {
   RIMP2_CK(cudaGetLastError());
   int h = 0;
   RIMP2_CK(cudaMemcpyAsync(&h, bad.p, sizeof(int), cudaMemcpyDeviceToHost, s));
-  RIMP2_CK(cudaStreamSynchronize(s));
+  // an update that gave up leaves anything behind, also a pivot that is not positive
+  RIMP2_TRY(collect_device_error(s));
   if (h) {
     set_error("auxiliary metric is not positive definite (pivot %d)", h - 1);
     return RIMP2_ERR_ARG;
@@ -654,7 +655,7 @@ extern "C" int rimp2_calpha_from_ao(const int *NBA, const int *nbas, const int *
   RIMP2_CK(cudaMemcpyAsync(Calpha, dOut.p, sizeof(double) * no, cudaMemcpyDeviceToHost, s));
   RIMP2_CK(cudaStreamSynchronize(s));
   RIMP2_CK(cudaGetLastError());
-  return RIMP2_OK;
+  return collect_device_error(s);
 }
 
 extern "C" int rimp2_cholesky_dev(int n, double *dV, void *stream) {

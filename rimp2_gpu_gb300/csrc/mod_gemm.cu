@@ -1241,6 +1241,7 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
       RIMP2_CK(cudaGetLastError());
     }
   }
+  if (inject_fault("wait")) report_device_error(24);
   *handled = true;
   return RIMP2_OK;
 }
