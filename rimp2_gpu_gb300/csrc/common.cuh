@@ -202,7 +202,7 @@ cudaStream_t slice_stream();  // the streamed host path's slicing
 struct SlicedOp {
   int nsl = 2, nks = 0;
   long long rows_per_group = 0, ncol = 0, R = 0;
-  DevBuf slices, inv, desc;
+  DevBuf slices, inv;
 };
 // rows = columns of a column-major array: group g, row r at src + K*(r + nrows*g)
 int sliced_cols(SlicedOp &op, const double *src, int K, int nrows, int ngroups, int nsl,

@@ -573,6 +573,11 @@ __device__ __forceinline__ void decode_pair_ij(int p, int &i, int &j) {
   i = p - jj * (jj + 1) / 2;
 }
 
+// One fragment's descriptor into device memory, as a kernel parameter: a copy from
+// the host's vector would be read again by every replay of a captured call, when
+// the vector is gone.
+__global__ void plain_frag_kernel(PlainFrag *fr, const __grid_constant__ PlainFrag F) { *fr = F; }
+
 __global__ void __launch_bounds__(NTHR) plain_batch_kernel(const PlainFrag *__restrict__ fr,
                                                            int nfrag, long long nitems,
                                                            unsigned int *queue,
@@ -1214,9 +1219,16 @@ int plain_plan_create(PlainPlan **out, int nfrag, const PlainFrag *in, cudaStrea
   if (rc == RIMP2_OK) rc = P->part.alloc(sizeof(double) * (size_t)std::max<long long>(item, 1), s);
   if (rc == RIMP2_OK) rc = P->queue.alloc(sizeof(unsigned int), s);
   P->fh = fh;
-  if (rc == RIMP2_OK &&
-      cudaMemcpyAsync(P->frags.p, P->fh.data(), sizeof(PlainFrag) * (size_t)nfrag,
-                      cudaMemcpyHostToDevice, s) != cudaSuccess) {
+  if (rc == RIMP2_OK && nfrag == 1) {
+    plain_frag_kernel<<<1, 1, 0, s>>>(P->frags.as<PlainFrag>(), fh[0]);
+    count_launch(1);
+    if (cudaGetLastError() != cudaSuccess) {
+      set_error("plain batch descriptor launch failed");
+      rc = RIMP2_ERR_CUDA;
+    }
+  } else if (rc == RIMP2_OK &&
+             cudaMemcpyAsync(P->frags.p, P->fh.data(), sizeof(PlainFrag) * (size_t)nfrag,
+                             cudaMemcpyHostToDevice, s) != cudaSuccess) {
     set_error("plain batch descriptor copy failed");
     rc = RIMP2_ERR_CUDA;
   }

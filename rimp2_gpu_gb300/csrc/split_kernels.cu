@@ -407,6 +407,15 @@ __global__ void __launch_bounds__(256, 6)
   slice_column(F, col, nsl, plane, slices, inv_scale, vplane, dcorr);
 }
 
+// The columns of one set, its descriptor a kernel parameter (a captured call may be
+// replayed when the host's copy is gone).
+__global__ void __launch_bounds__(256, 6)
+    slice_one_kernel(const __grid_constant__ FragDesc F, int nsl, long long plane,
+                     __half *__restrict__ slices, float *__restrict__ inv_scale) {
+  const int col = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (col < F.ncol) slice_column(F, col, nsl, plane, slices, inv_scale, 0, nullptr);
+}
+
 // orbital energies as hi/lo float pairs (padded virtuals get a large value so
 // their denominators stay finite; their g is exactly zero). grid.y = fragment
 __device__ __forceinline__ void eps_entry(const FragDesc &F, int t, float2 *eo2, float2 *ev2) {
@@ -4103,13 +4112,10 @@ int sliced_cols(SlicedOp &op, const double *src, int K, int nrows, int ngroups, 
     set_error("split GEMM operand too large (%lld rows)", op.R);
     return RIMP2_ERR_ARG;
   }
-  RIMP2_TRY(op.desc.alloc(sizeof(FragDesc), s));
-  RIMP2_CK(cudaMemcpyAsync(op.desc.p, &F, sizeof F, cudaMemcpyHostToDevice, s));
   RIMP2_TRY(op.slices.alloc(sizeof(__half) * (size_t)nsl * op.R * 64, s));
   RIMP2_TRY(op.inv.alloc(sizeof(float) * (size_t)op.ncol, s));
-  slice_batch_kernel<<<(unsigned)(((long long)F.ncol * 32 + 255) / 256), 256, 0, s>>>(
-      op.desc.as<FragDesc>(), nsl, op.R * 64, op.slices.as<__half>(), op.inv.as<float>(), 0,
-      0x7fffffff);
+  slice_one_kernel<<<(unsigned)(((long long)F.ncol * 32 + 255) / 256), 256, 0, s>>>(
+      F, nsl, op.R * 64, op.slices.as<__half>(), op.inv.as<float>());
   count_launch(1);
   RIMP2_CK(cudaGetLastError());
   return RIMP2_OK;
