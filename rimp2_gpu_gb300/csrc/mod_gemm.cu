@@ -399,6 +399,7 @@ constexpr int mg_stage(int tq) { return PANEL_BYTES + tq / 2 * KSTEP * 2; }
 constexpr int mg_nst(int tq) { return tq == 256 ? 6 : 8; }
 constexpr int mg_nacc(int tq) { return tq == 256 ? 2 : 4; }  // accumulators: short sums need more in flight
 constexpr int mg_smem(int tq) { return mg_nst(tq) * mg_stage(tq) + 1024 + 256; }
+static_assert(tmem_alone(mg_smem(64)) && tmem_alone(mg_smem(128)) && tmem_alone(mg_smem(256)), "tensor memory");
 
 struct MgParams {
   int rows_l, rows_q;        // rows per K chunk of the two operands
@@ -623,6 +624,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
         }
         tc_fence_before();
         __syncwarp();
+        // nothing to release: the accumulator's loads are complete (tcgen05.wait::ld), and
+        // the arrival says no more than that; not for a barrier that stores rely on
         if (lane == 0) mbar_arrive_relaxed(tempty0_L + 8 * u);
       }
       if (ok && n < nl) {

@@ -883,6 +883,7 @@ struct PairParams {
 constexpr int pair_smem_bytes(int nstage, bool gx) {
   return nstage * PAIR_STAGE_BYTES + 1024 + 512 + (gx ? 0 : 64 * TP * 4);
 }
+static_assert(tmem_alone(pair_smem_bytes(3, false)) && tmem_alone(pair_smem_bytes(4, true)), "tensor memory");
 
 // Exchange-tile transpose through memory, for the GX form: each thread stores
 // its 64 values of tile row `row` (columns [cbase, cbase+64)) as 16-byte
@@ -961,13 +962,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(
                      smem_u32(tmem_slot))
                  : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
   cluster_sync_all();  // both CTAs' barriers are initialised before any remote access
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  if (warp == 1)  // both CTAs hold their columns
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   grid_wait();
 
   if (warp == 0) {
@@ -1788,6 +1790,7 @@ __device__ __forceinline__ void eos_pair_decode(const EosPairParams &P, long lon
 
 constexpr int EP_NSTAGE = 3;
 constexpr int EP_SMEM = EP_NSTAGE * PAIR_STAGE_BYTES + 1024 + 512;
+static_assert(tmem_alone(EP_SMEM), "tensor memory");
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
     split_eos_pair_kernel(const __grid_constant__ CUtensorMap tmA,
@@ -2147,9 +2150,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(NTHREADS, 1)
   }
 }
 
-int eos_smem_bytes(int nsl, int nstage) {
+constexpr int eos_smem_bytes(int nsl, int nstage) {
   return nstage * eos_stage_bytes(nsl) + 1024 + 512;
 }
+static_assert(eos_smem_bytes(3, 3) >= TMEM_SMEM_MIN, "tensor memory");
 
 // Self-test of the bounded-wait path: one thread waits on an mbarrier that
 // nothing ever completes, with a short clock budget.  The wait must give up,
@@ -2380,10 +2384,11 @@ __global__ void __launch_bounds__(256) single_reduce_kernel(const __grid_constan
 // --------------------------------------------------------------------------
 // host side
 // --------------------------------------------------------------------------
-int smem_bytes(int nsl, int nstage) {
+constexpr int smem_bytes(int nsl, int nstage) {
   return nstage * nsl * 2 * PANEL_BYTES + 1024 /*align*/ + 512 /*barriers, ring, etc*/ +
          64 * TP * 4 /*diagonal-tile transpose buffer*/;
 }
+static_assert(smem_bytes(2, 3) >= TMEM_SMEM_MIN && smem_bytes(3, 2) >= TMEM_SMEM_MIN, "tensor memory");
 
 // One launch group of a batch: its fragments share a slice count and an
 // energy kernel (one-CTA or paired), a slices buffer, the tensor maps and one
@@ -2712,6 +2717,7 @@ constexpr int gemm_stage_bytes(int nsl, int NT) { return nsl * (PANEL_BYTES + NT
 constexpr int gemm_smem_bytes(int nsl, int NT) {
   return GEMM_NST * gemm_stage_bytes(nsl, NT) + 1024 + 256;
 }
+static_assert(gemm_smem_bytes(2, 16) >= TMEM_SMEM_MIN, "tensor memory");
 
 constexpr int GEMM_EPI = 8;                       // epilogue warps: two per lane quadrant
 constexpr int GEMM_THREADS = 64 + 32 * GEMM_EPI;
@@ -3001,6 +3007,7 @@ constexpr int ah_smem_bytes(int form, int NT) {
   return 1024 + 2 * ah_stage_bytes(NT) + ah_slot_bytes(form) + 2 * 4 * 128 * 4 /*row max exchange*/ +
          4 * 128 /*row exponents*/ + 256 /*barriers, slot*/;
 }
+static_assert(ah_smem_bytes(AH_BOX, 16) >= TMEM_SMEM_MIN, "tensor memory");
 
 // 8-byte asynchronous global -> shared copy; src_bytes = 0 fills zeros and
 // reads nothing

@@ -18,6 +18,17 @@ constexpr int KSTEP = 64;      // K per stage (one 128-byte swizzle row of FP16)
 constexpr int PANEL_BYTES = TILE * KSTEP * 2;  // 16 KB
 constexpr long long WAIT_BUDGET = 4000000000LL;  // ~2 s of SM clock per wait
 
+// Two waits have no bound: the allocation of tensor memory and the cluster
+// barriers.  A CTA of a pair allocates all 512 columns on both its SMs, where two
+// pairs holding one SM each would wait for one another; but no SM has room
+// for a CTA of a pair and another CTA of these kernels that allocates at all
+// (228 KB of shared memory, 1 KB of each CTA's taken by the system), so
+// the columns are free when such a CTA starts.  And the CTAs of a cluster start
+// together, every other wait before a cluster barrier is bounded, so each arrives.
+constexpr int SM_SMEM = 228 * 1024;
+constexpr int TMEM_SMEM_MIN = 75008;  // least shared memory of a kernel that allocates
+constexpr bool tmem_alone(int smem) { return smem + TMEM_SMEM_MIN + 2 * 1024 > SM_SMEM; }
+
 // --------------------------------------------------------------------------
 // small PTX helpers
 // --------------------------------------------------------------------------
