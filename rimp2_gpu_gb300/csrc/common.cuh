@@ -95,7 +95,8 @@ int alloc_parts(DevBuf &arena, DevBuf *const (&buf)[N], const size_t (&bytes)[N]
 // Host fault injection for failure-path tests: RIMP2_FAULT_INJECT=alloc makes
 // the next device allocation report out-of-memory, =launch makes the next
 // kernel-launch check report a launch failure, =wait makes a residue product
-// report that one of its bounded waits ran out.  Nothing touches the GPU.
+// report that one of its bounded waits ran out, =record that the event of its
+// end could not be recorded.  Nothing touches the GPU.
 bool inject_fault(const char *what);
 
 // ---- FP64 DMMA kernels (fp64_kernels.cu) -------------------------------------

@@ -42,6 +42,7 @@
 #include <cmath>
 #include <cstring>
 #include <mutex>
+#include <vector>
 
 #include "tc.cuh"
 #include "mod_gemm.cuh"
@@ -1100,34 +1101,54 @@ bool make_map(RowMap &M, Dim *d, int nd, const double *base, long long sk, int K
   return true;
 }
 
-// One contraction's kernels at a time on the device: a later one, on whatever
+// One contraction's kernels at a time on a device: a later one, on whatever
 // stream and from whatever thread, starts when the earlier one's have ended.
-// Each fills the GPU by itself, so nothing is lost; several at once (persistent
-// CTA pairs between the operands' and the epilogue's many small blocks on other
-// streams) were seen to stop the GPU's scheduling.  Held while a contraction
-// is queued.
+// Contractions on three streams at once, without this order, stopped making
+// progress on the GPU.  The cause is not known: what is left unbounded in the
+// kernels, the tensor memory's allocation and the cluster barriers, cannot wait for
+// another kernel (TMEM_SMEM_MIN, tc.cuh).  So they do not run at once.  The price: a
+// contraction also waits for what stands before the last one on that one's stream,
+// and small ones on several streams do not overlap (eight streams, nocc 6, nvirt 53,
+// NBA 187: 69 us an energy, against 89 in the FP64 kernels that did overlap).
+// Held while a contraction is queued; one that fails half way, or whose end could not
+// be recorded, is waited for by the host before the next may be queued.
 class ModOrder {
   static std::mutex mu;
-  static cudaEvent_t last;
+  static std::vector<cudaEvent_t> last;  // by device
   std::unique_lock<std::mutex> lk;
   cudaStream_t s;
+  cudaEvent_t *ev = nullptr;
+  bool open = false;
 
  public:
   explicit ModOrder(cudaStream_t st) : lk(mu), s(st) {}
   int begin() {
-    if (!last) {
-      RIMP2_CK(cudaEventCreateWithFlags(&last, cudaEventDisableTiming));
-      return RIMP2_OK;
+    int dev = 0;
+    RIMP2_CK(cudaGetDevice(&dev));
+    if ((size_t)dev >= last.size()) last.resize(dev + 1, nullptr);
+    ev = &last[dev];
+    if (*ev)
+      RIMP2_CK(cudaStreamWaitEvent(s, *ev, 0));
+    else
+      RIMP2_CK(cudaEventCreateWithFlags(ev, cudaEventDisableTiming));
+    open = true;
+    return RIMP2_OK;
+  }
+  int end() {
+    if (inject_fault("record")) {
+      set_error("injected event failure (RIMP2_FAULT_INJECT=record)");
+      return RIMP2_ERR_CUDA;
     }
-    RIMP2_CK(cudaStreamWaitEvent(s, last, 0));
+    RIMP2_CK(cudaEventRecord(*ev, s));
+    open = false;
     return RIMP2_OK;
   }
   ~ModOrder() {
-    if (last) cudaEventRecord(last, s);
+    if (open) cudaStreamSynchronize(s);
   }
 };
 std::mutex ModOrder::mu;
-cudaEvent_t ModOrder::last = nullptr;
+std::vector<cudaEvent_t> ModOrder::last;
 
 constexpr size_t MG_PLANE_CAP = (size_t)6 << 30;  // bytes of one operand's planes per part
 constexpr size_t MG_RES_CAP = (size_t)4 << 30;    // bytes of the residues of a part of C
@@ -1244,6 +1265,7 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
       RIMP2_CK(cudaGetLastError());
     }
   }
+  RIMP2_TRY(order.end());
   if (inject_fault("wait")) report_device_error(24);
   *handled = true;
   return RIMP2_OK;

@@ -51,3 +51,87 @@ def test_product_that_gave_up(api, monkeypatch, call):
     monkeypatch.delenv("RIMP2_FAULT_INJECT")
     api.sync_status()
     run()
+
+
+def fragment(seed, no=6, nv=90, nb=400):
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    f64 = dict(dtype=torch.float64, device="cuda")
+    C = torch.randn(no, nv, nb, generator=g, **f64) * 0.05
+    eo = torch.sort(torch.rand(no, generator=g, **f64) - 1.5)[0]
+    ev = torch.sort(torch.rand(nv, generator=g, **f64) + 0.1)[0]
+    return (nv, no, nb), (C, eo, ev, torch.zeros(no, no, **f64), torch.zeros(1, **f64))
+
+
+def enqueue(api, frag, stream):
+    sizes, t = frag
+    api.energy_dev(*sizes, *(x.data_ptr() for x in t), precision=api.PREC_FP64, stream=stream.cuda_stream)
+
+
+@pytest.mark.parametrize("threads", [1, 3])
+def test_contractions_on_several_streams(api, threads):
+    """Energies in turn on three streams, from one thread and from a thread for
+    each stream: the bits of every call alone, and no error afterwards."""
+    import threading
+
+    import torch
+    streams = [torch.cuda.Stream() for _ in range(3)]
+    frags = [[fragment(10 * k + r) for r in range(4)] for k in range(3)]
+    want = []
+    for k in range(3):
+        for f in frags[k]:
+            torch.cuda.synchronize()
+            before = api.kernel_launch_count()
+            enqueue(api, f, streams[0])
+            assert api.kernel_launch_count() - before > 6  # residue products
+            torch.cuda.synchronize()
+            want.append(f[1][3].clone())
+            f[1][3].zero_()
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(ks):
+        try:
+            for _ in range(5):
+                for r in range(4):
+                    for k in ks:
+                        enqueue(api, frags[k][r], streams[k])
+        except Exception as e:  # shown by the assertion below
+            errors.append(e)
+
+    parts = [[0, 1, 2]] if threads == 1 else [[0], [1], [2]]
+    ts = [threading.Thread(target=work, args=(p,)) for p in parts]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    torch.cuda.synchronize()
+    assert not errors
+    api.sync_status()
+    for w, f in zip(want, (f for k in range(3) for f in frags[k])):
+        assert torch.equal(w, f[1][3])
+
+
+def test_end_that_cannot_be_recorded(api, monkeypatch):
+    """The call fails (the order of contractions would be lost otherwise), has
+    waited for its kernels, and later calls run."""
+    import torch
+    from rimp2_gpu_gb300._lib import Rimp2Error
+    s = torch.cuda.Stream()
+    f = fragment(1)
+    torch.cuda.synchronize()
+    enqueue(api, f, s)
+    torch.cuda.synchronize()
+    want = f[1][3].clone()
+    f[1][3].zero_()
+    torch.cuda.synchronize()
+    monkeypatch.setenv("RIMP2_FAULT_INJECT", "record")
+    with pytest.raises(Rimp2Error):
+        enqueue(api, f, s)
+    assert s.query()
+    monkeypatch.delenv("RIMP2_FAULT_INJECT")
+    enqueue(api, f, s)
+    torch.cuda.synchronize()
+    api.sync_status()
+    assert torch.equal(want, f[1][3])
