@@ -69,11 +69,21 @@ bool inject_fault(const char *what) {
   return v && strcmp(v, what) == 0;
 }
 
+// alloc: every allocation; alloc:N: the N-th one since the variable was last another
+static bool inject_alloc_fault() {
+  static std::atomic<int> at{0}, seen{0};
+  const char *v = getenv("RIMP2_FAULT_INJECT");
+  const int n = v && strncmp(v, "alloc:", 6) == 0 ? atoi(v + 6) : 0;
+  if (at.exchange(n) != n) seen = 0;
+  if (n > 0) return ++seen == n;
+  return v && strcmp(v, "alloc") == 0;
+}
+
 int DevBuf::alloc(size_t bytes, cudaStream_t st) {
   s = st;
   n = bytes;
   if (bytes == 0) bytes = 16;
-  if (inject_fault("alloc")) {
+  if (inject_alloc_fault()) {
     set_error("injected device allocation failure (RIMP2_FAULT_INJECT=alloc)");
     return RIMP2_ERR_NOMEM;
   }
@@ -736,6 +746,15 @@ int rimp2_steps5to8(const int *nvirt_, const int *nocc_, const int *noccEOS_, co
   RIMP2_TRY(h2d(dUvE, UvirtEOST, nv * ve, s));
   const double *Ca = dC.as<double>(), *eo = deo.as<double>(), *ev = dev.as<double>();
   DevBuf tv1;  // Step 6's first array, from the g/D that Step 5 forms
+  // it gives way where a later array of Step 5 finds no room: Step 6 forms it again
+  auto room = [&](DevBuf &b, size_t n) -> int {
+    const int rc = dalloc(b, n, s);
+    if (rc != RIMP2_ERR_NOMEM || !tv1.p) return rc;
+    (void)cudaGetLastError();
+    clear_error();
+    tv1.release();
+    return dalloc(b, n, s);
+  };
   {  // Step 5 (RIMP2.F90:71-93)
     DevBuf X, t1, t2, t3, out;
     RIMP2_TRY(dalloc(X, no * no * nv * nv, s));
@@ -750,14 +769,14 @@ int rimp2_steps5to8(const int *nvirt_, const int *nocc_, const int *noccEOS_, co
       clear_error();
     }
     X.release();
-    RIMP2_TRY(dalloc(t2, ne * ne * nv * nv, s));
+    RIMP2_TRY(room(t2, ne * ne * nv * nv));
     RIMP2_TRY(dev_dgemm('T', 'N', noccEOS, noccEOS * nvirt * nvirt, nocc, 1.0, dUoE.as<double>(),
                         nocc, t1.as<double>(), nocc, 0.0, t2.as<double>(), noccEOS, s));
-    RIMP2_TRY(dalloc(t3, nv * nv * ne * ne, s));
+    RIMP2_TRY(room(t3, nv * nv * ne * ne));
     RIMP2_TRY(dev_dgemm('N', 'N', noccEOS * noccEOS * nvirt, nvirt, nvirt, 1.0, t2.as<double>(),
                         noccEOS * noccEOS * nvirt, dUvT.as<double>(), nvirt, 0.0, t3.as<double>(),
                         noccEOS * noccEOS * nvirt, s));
-    RIMP2_TRY(dalloc(out, nv * ne * nv * ne, s));
+    RIMP2_TRY(room(out, nv * ne * nv * ne));
     RIMP2_TRY(dev_toccb(nvirt, noccEOS, t3.as<double>(), dUvT.as<double>(), out.as<double>(), s));
     RIMP2_TRY(d2h(toccEOS, out, nv * ne * nv * ne, s));
     RIMP2_CK(cudaStreamSynchronize(s));
@@ -779,6 +798,7 @@ int rimp2_steps5to8(const int *nvirt_, const int *nocc_, const int *noccEOS_, co
     RIMP2_TRY(dev_tvirtb(nvirtEOS, nocc, t3.as<double>(), dUoT.as<double>(), out.as<double>(), s));
     RIMP2_TRY(d2h(tvirtEOS, out, ve * no * ve * no, s));
     RIMP2_CK(cudaStreamSynchronize(s));
+    tv1.release();
   }
   {  // Step 7 (RIMP2.F90:133-147)
     DevBuf c2, c3, out;

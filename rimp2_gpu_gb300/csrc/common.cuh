@@ -93,7 +93,7 @@ int alloc_parts(DevBuf &arena, DevBuf *const (&buf)[N], const size_t (&bytes)[N]
 }
 
 // Host fault injection for failure-path tests: RIMP2_FAULT_INJECT=alloc makes
-// the next device allocation report out-of-memory, =launch makes the next
+// the next device allocation report out-of-memory, =alloc:N the N-th one only, =launch makes the next
 // kernel-launch check report a launch failure, =wait makes a residue product
 // report that one of its bounded waits ran out, =record that the event of its
 // end could not be recorded.  Nothing touches the GPU.

@@ -5,7 +5,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-ERR_TIMEOUT = 5
+ERR_NOMEM, ERR_TIMEOUT = 3, 5
 
 
 @pytest.fixture(scope="module")
@@ -135,3 +135,62 @@ def test_end_that_cannot_be_recorded(api, monkeypatch):
     torch.cuda.synchronize()
     api.sync_status()
     assert torch.equal(want, f[1][3])
+
+
+def lost_allocations(api, monkeypatch, run, tol=4 * 600 * 2.0 ** -53, count=60):
+    """run() with the first, the second, ... of its device allocations failing (of
+    `count`, more than it makes): how many of them it did not get over."""
+    from rimp2_gpu_gb300._lib import Rimp2Error
+    want = run()
+    lost = 0
+    for n in range(1, count + 1):
+        monkeypatch.setenv("RIMP2_FAULT_INJECT", f"alloc:{n}")
+        try:
+            got = run()
+        except Rimp2Error as e:
+            assert e.status == ERR_NOMEM
+            lost += 1
+            got = want
+        monkeypatch.delenv("RIMP2_FAULT_INJECT")
+        api.sync_status()
+        for w, g in zip(want, got):
+            # FP64 kernels instead of residues: four products in a row, sums of at most 600 terms
+            assert np.abs(w - g).max() <= tol * np.abs(w).max()
+    return lost
+
+
+def local_orbitals(nv, no, ne, ve, nb):
+    rng = np.random.default_rng(2)
+    q = lambda n: np.asfortranarray(np.linalg.qr(rng.standard_normal((n, n)))[0])  # noqa: E731
+    C = np.asfortranarray(rng.standard_normal((nb, nv, no)) * 0.05)
+    eo, ev = np.sort(rng.random(no) - 1.5), np.sort(rng.random(nv) + 0.1)
+    Uo, Uv = q(no), q(nv)
+    return C, eo, ev, np.asfortranarray(Uo[:, :ne]), Uv, Uo, np.asfortranarray(Uv[:, :ve])
+
+
+def test_steps5to8_short_of_memory(api, monkeypatch):
+    """What the call cannot do without are its seven inputs, g/D and its first
+    projection, and the last three arrays of Steps 6, 7 and 8 each.  Neither the
+    products' workspaces nor what it keeps for Step 6 beside Step 5 may make it fail."""
+    nv, no, ne, ve, nb = 100, 8, 3, 30, 300
+    x = local_orbitals(nv, no, ne, ve, nb)
+    run = lambda: api.steps5to8(nv, no, ne, ve, nb, *x)  # noqa: E731
+    assert lost_allocations(api, monkeypatch, run) == 7 + 2 + 3 * 3
+
+
+def test_energies_short_of_memory(api, monkeypatch):
+    """One fragment in FP64 cannot do without its three inputs and its results."""
+    nv, no, nb = 100, 8, 300
+    x = local_orbitals(nv, no, 3, 30, nb)
+    assert lost_allocations(api, monkeypatch, lambda: api.energy(nv, no, nb, *x[:3])) == 4
+
+
+def test_local_energies_short_of_memory(api, monkeypatch):
+    """Local orbitals in split form, one residual slice: the seven inputs, three
+    results and checks, the two projectors of more than half rank, both halves of
+    the two low-rank projections; not both partitionings' slices at once."""
+    nv, no, ne, ve, nb = 300, 8, 3, 30, 300
+    assert api.split_nslices(nv, no, nb) == 1
+    x = local_orbitals(nv, no, ne, ve, nb)
+    run = lambda: [np.array(api.energy_eos(nv, no, ne, ve, nb, *x, api.PREC_SPLIT))]  # noqa: E731
+    assert lost_allocations(api, monkeypatch, run, tol=1e-7) == 7 + 3 + 2 + 4  # accuracy of the split form
