@@ -55,14 +55,6 @@ __device__ __forceinline__ void dmma884(double &d0, double &d1, double a, double
 // ---------------------------------------------------------------------------
 // Strided batched GEMM
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void cp_async8(double *dst, const double *src, bool valid) {
-  // 8-byte global -> shared copy; an invalid element is zero-filled (no read)
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src),
-               "r"(valid ? 8 : 0)
-               : "memory");
-}
-
 struct MapGemm {
   RowMap A, B;  // C's rows and columns
   double *C;

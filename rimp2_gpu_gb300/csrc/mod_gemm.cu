@@ -785,37 +785,45 @@ __device__ __forceinline__ Side side(const CrtParams &P, const RowMap &M, int r)
   return s;
 }
 
-// A block takes 64 rows x 64 columns of C; a thread four consecutive rows of
+// A block takes 64 rows x CN columns of C; a thread four consecutive rows of
 // two columns.  It reads 17 bytes and writes 8 per element; its instructions
 // (some 170 an element) bound it, so what only depends on the row or the column
 // (offsets with their divisions, orbital energies) is formed once a block.  A symmetric product (g
 // of one set of vectors with itself) has only the tiles m >= n: C(n,m) is
 // written along with C(m,n) through shared memory, with the same denominator
 // (the reference subtracts the two virtual energies in the other order there).
+// Values whose large elements meet only small ones leave whole tiles to FP64, where
+// the FP64 unit bounds a block (19 us of an SM for 64 x 64 x 16).
 constexpr int DK = 16, DP = 20;
-template <int MODE>
-__global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_constant__ CrtParams P) {
+constexpr int crt_tile_max(int cn) { return 64 * cn / 8; }  // of a tile's elements; beyond it the whole tile is summed in FP64
+constexpr int crt_dmma_bytes(int cn) { return (2 * (64 + cn) * DP + 64 + cn) * (int)sizeof(double); }
+constexpr int crt_mirror_bytes(int cn) { return 64 * (cn + 1) * (int)sizeof(double); }
+
+template <int MODE, int CN>
+__global__ void __launch_bounds__(8 * CN, 1024 / (8 * CN)) crt_epilogue_kernel(const __grid_constant__ CrtParams P) {
+  constexpr int NT = 8 * CN, HALF = CN / 2, SP = CN + 1, LANES = HALF < 16 ? HALF : 16;
   __shared__ int count;
-  __shared__ Side sr[64], sc[64];           // the tile's rows and columns
-  __shared__ long long rows[64], cols[64];  // symmetric: offsets of the mirror's columns
-  extern __shared__ double S[];             // symmetric: [64][65]; a tile summed in FP64: its operands
-  double(*As)[DP] = reinterpret_cast<double(*)[DP]>(S), (*Bs)[DP] = As + 64;
-  const int tm = blockIdx.x, tn = blockIdx.y;
+  __shared__ Side sr[64], sc[CN];           // the tile's rows and columns
+  __shared__ long long rows[64], cols[CN];  // symmetric: offsets of the mirror's columns
+  extern __shared__ double S[];             // symmetric: [64][SP]; a tile summed in FP64: its operands
+  const int tm = blockIdx.x, tn = blockIdx.y, td = tn * CN / 64;  // td: the diagonal's row tile
   grid_wait();
-  if ((P.lower || P.sym) && tm < tn) return;
-  const int t0 = threadIdx.x & 15, t1 = threadIdx.x >> 4;
-  const int mq = (P.nfast ? t1 & 15 : t0) * 4, nq = P.nfast ? t0 + (t1 & 16) : t1;
-  const int m0 = tm * 64 + mq, n0 = tn * 64 + nq;
+  const bool sym = CN == 64 && P.sym;  // narrower blocks of a diagonal tile would choose each for itself
+  if ((P.lower || sym) && tm < td) return;
+  const int tid = threadIdx.x;
+  const int mq = (P.nfast ? tid / LANES % 16 : tid % 16) * 4;
+  const int nq = P.nfast ? tid % LANES + tid / (16 * LANES) * LANES : tid / 16;
+  const int m0 = tm * 64 + mq, n0 = tn * CN + nq;
   const long long plane = (long long)P.nn * P.ldm;
-  const bool mirror = P.sym && tm != tn;
-  if (threadIdx.x == 0) count = 0;
-  if (threadIdx.x < 64 && tm * 64 + threadIdx.x < P.nm)
-    sr[threadIdx.x] = side<MODE>(P, P.A, P.row0 + tm * 64 + threadIdx.x);
-  else if (threadIdx.x >= 64 && threadIdx.x < 128 && tn * 64 + threadIdx.x - 64 < P.nn)
-    sc[threadIdx.x - 64] = side<MODE>(P, P.B, P.col0 + tn * 64 + threadIdx.x - 64);
-  if (mirror && threadIdx.x < 64) {
-    if (tm * 64 + threadIdx.x < P.nm) rows[threadIdx.x] = c_off(P.B, tm * 64 + threadIdx.x);
-    if (tn * 64 + threadIdx.x < P.nn) cols[threadIdx.x] = c_off(P.A, tn * 64 + threadIdx.x);
+  const bool mirror = sym && tm != td;
+  if (tid == 0) count = 0;
+  if (tid < 64 && tm * 64 + tid < P.nm)
+    sr[tid] = side<MODE>(P, P.A, P.row0 + tm * 64 + tid);
+  else if (tid >= 64 && tid < 64 + CN && tn * CN + tid - 64 < P.nn)
+    sc[tid - 64] = side<MODE>(P, P.B, P.col0 + tn * CN + tid - 64);
+  if (mirror) {
+    if (tid < 64 && tm * 64 + tid < P.nm) rows[tid] = c_off(P.B, tm * 64 + tid);
+    if (tid < CN && tn * CN + tid < P.nn) cols[tid] = c_off(P.A, tn * CN + tid);
   }
   __syncthreads();
   // which elements are summed in FP64
@@ -825,7 +833,7 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
   for (int k = 0; k < 4; ++k) fm |= (unsigned)(m0 + k < P.nm ? P.fa[m0 + k] : (unsigned)MG_ROW_ZERO) << (8 * k);
 #pragma unroll
   for (int y = 0; y < 2; ++y) {
-    const int n = n0 + 32 * y;
+    const int n = n0 + HALF * y;
     if (n >= P.nn) continue;
     const unsigned g = *reinterpret_cast<const unsigned *>(P.res + MG_P * plane + n * P.ldm + m0);
     const unsigned fn = P.fb[n];
@@ -835,37 +843,62 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
   }
   if (todo) atomicAdd(&count, __popc(todo));
   __syncthreads();
-  const int lane = threadIdx.x & 31;
+  const int lane = tid & 31;
   auto put = [&](int ml, int nl, double v) {
     const Side &a = sr[ml], &b = sc[nl];
     if (MODE == CRT_QUOTIENT || (MODE == CRT_ANY && P.denom))
       v = div_f64(v, a.eo + b.eo - b.ev - a.ev);  // RIMP2.F90:403-404
     if (MODE == CRT_ANY && P.alpha != 1.0) v *= P.alpha;
-    if (mirror) S[ml * 65 + nl] = v;
+    if (mirror) S[ml * SP + nl] = v;
     double *c = P.C + a.off + b.off;
     if (MODE == CRT_MINUS) v = *c - v;
     if (MODE == CRT_ANY && P.beta != 0.0) v += P.beta * *c;
     *c = v;
   };
-  if (count > MG_TILE_MAX) {
-    // the whole tile with FP64 tensor operations: 16 x 16 of it a warp
-    const int gid = lane >> 2, tig = lane & 3, warp = threadIdx.x >> 5;
-    const int wm = (warp & 3) * 16, wn = (warp >> 2) * 16;
+  if (count > crt_tile_max(CN)) {
+    // the whole tile with FP64 tensor operations: 16 x 16 of it a warp, the next 16
+    // terms on their way by cp.async.  Rows 0 .. 63 of a buffer are the tile's
+    // rows, the others its columns.
+    double(*buf)[64 + CN][DP] = reinterpret_cast<double(*)[64 + CN][DP]>(S);
+    long long *off = reinterpret_cast<long long *>(S + 2 * (64 + CN) * DP);
+    const int K = P.A.K;
+    if (tid < 64)
+      off[tid] = tm * 64 + tid < P.nm ? row_off(P.A, P.row0 + tm * 64 + tid) : -1;
+    else if (tid < 64 + CN)
+      off[tid] = tn * CN + tid - 64 < P.nn ? row_off(P.B, P.col0 + tn * CN + tid - 64) : -1;
+    __syncthreads();
+    auto load = [&](int b, int q0) {
+#pragma unroll 2
+      for (int t = tid; t < (64 + CN) * DK; t += NT) {
+        const bool col = t >= 64 * DK;
+        const RowMap &M = col ? P.B : P.A;
+        const int u = col ? t - 64 * DK : t, ext = col ? CN : 64;
+        const int i = M.sk == 1 ? u / DK : u % ext, q = M.sk == 1 ? u % DK : u / ext, r = col ? 64 + i : i;
+        const bool live = off[r] >= 0 && q0 + q < K;
+        cp_async8(&buf[b][r][q], live ? M.base + off[r] + (long long)(q0 + q) * M.sk : M.base, live);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // the warps of 16 rows on the four schedulers: rows that a narrow product does not
+    // have leave none idle
+    const int gid = lane >> 2, tig = lane & 3, warp = tid >> 5;
+    const int wm = warp / (CN / 16) * 16, wn = warp % (CN / 16) * 16;
+    const bool work = tm * 64 + wm < P.nm && tn * CN + wn < P.nn;
     double acc[2][2][2] = {};
-    for (int q0 = 0; q0 < P.A.K; q0 += DK) {
-      __syncthreads();
+    load(0, 0);
+    int cur = 0;
 #pragma unroll 1
-      for (int t = threadIdx.x; t < 2 * 64 * DK; t += 512) {
-        const bool cols = t >= 64 * DK;
-        const RowMap &M = cols ? P.B : P.A;
-        const int u = t & (64 * DK - 1), i = M.sk == 1 ? u / DK : u & 63, q = M.sk == 1 ? u % DK : u >> 6;
-        const bool live = q0 + q < M.K && (cols ? tn * 64 + i < P.nn : tm * 64 + i < P.nm);
-        const int row = cols ? P.col0 + tn * 64 + i : P.row0 + tm * 64 + i;
-        (cols ? Bs : As)[i][q] = live ? M.base[row_off(M, row) + (long long)(q0 + q) * M.sk] : 0.0;
+    for (int q0 = 0; q0 < K; q0 += DK, cur ^= 1) {
+      if (q0 + DK < K) {
+        load(cur ^ 1, q0 + DK);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+      } else {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
       }
       __syncthreads();
 #pragma unroll
-      for (int ks = 0; ks < DK; ks += 4)
+      for (int ks = 0; ks < DK; ks += 4) {
+        if (!work || q0 + ks >= K) break;  // zeros from here on
 #pragma unroll
         for (int x = 0; x < 2; ++x)
 #pragma unroll
@@ -873,26 +906,26 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
             asm volatile(
                 "mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                 : "+d"(acc[x][y][0]), "+d"(acc[x][y][1])
-                : "d"(As[wm + 8 * x + gid][ks + tig]), "d"(Bs[wn + 8 * y + gid][ks + tig]));
+                : "d"(buf[cur][wm + 8 * x + gid][ks + tig]), "d"(buf[cur][64 + wn + 8 * y + gid][ks + tig]));
+      }
+      __syncthreads();  // the buffer is refilled two slabs later; after the last one: the operands give way to the mirror
     }
-    __syncthreads();  // the operands give way to the mirror
 #pragma unroll 1
     for (int e = 0; e < 8; ++e) {
       const int ml = wm + 8 * (e >> 2) + gid, nl = wn + 8 * ((e >> 1) & 1) + 2 * tig + (e & 1);
       double v = 0.0;
 #pragma unroll
       for (int x = 0; x < 8; ++x) v = e == x ? acc[x >> 2][(x >> 1) & 1][x & 1] : v;
-      if (tm * 64 + ml < P.nm && tn * 64 + nl < P.nn) put(ml, nl, v);
+      if (tm * 64 + ml < P.nm && tn * CN + nl < P.nn) put(ml, nl, v);
     }
-  }
-  if (count <= MG_TILE_MAX) {
+  } else {
   int ea[4];
 #pragma unroll
   for (int k = 0; k < 4; ++k) ea[k] = m0 + k < P.nm ? P.ea[m0 + k] : 0;
   unsigned small = 0;
 #pragma unroll 1
   for (int y = 0; y < 2; ++y) {
-    const int n = n0 + 32 * y;
+    const int n = n0 + HALF * y;
     if (n < P.nn) {
       unsigned w[MG_P];
       const signed char *src = P.res + n * P.ldm + m0;
@@ -915,7 +948,7 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
         double v;
         if (m0 + k >= P.nm || ((todo >> (4 * y + k)) & 1u)) continue;
         if (crt_value(r[k], ea[k] + eb, v))
-          put(mq + k, nq + 32 * y, v);
+          put(mq + k, nq + HALF * y, v);
         else
           small |= 1u << (4 * y + k);
       }
@@ -925,9 +958,9 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
   if (__any_sync(0xffffffffu, small | todo)) {
 #pragma unroll 1
     for (int x = 0; x < 8; ++x) {
-      const int k = x & 3, y = x >> 2, n = n0 + 32 * y;
+      const int k = x & 3, y = x >> 2, n = n0 + HALF * y;
       if ((small >> x) & 1u)
-        put(mq + k, nq + 32 * y, crt_small(P.res + n * P.ldm + m0 + k, plane, P.ea[m0 + k] + P.eb[n]));
+        put(mq + k, nq + HALF * y, crt_small(P.res + n * P.ldm + m0 + k, plane, P.ea[m0 + k] + P.eb[n]));
       unsigned mask = __ballot_sync(0xffffffffu, (todo >> x) & 1u);
       while (mask) {
         const int src = __ffs(mask) - 1;
@@ -939,7 +972,7 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
         for (int q = lane; q < P.A.K; q += 32) s = fma(a[q * P.A.sk], b[q * P.B.sk], s);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == src) put(mq + k, nq + 32 * y, s);
+        if (lane == src) put(mq + k, nq + HALF * y, s);
       }
     }
   }
@@ -947,10 +980,10 @@ __global__ void __launch_bounds__(512, 2) crt_epilogue_kernel(const __grid_const
   if (!mirror) return;
   __syncthreads();
   // C(n, m): rows along n are the fast direction here
-  const int c = threadIdx.x & 63;
-  if (tn * 64 + c < P.nn)
-    for (int r = threadIdx.x >> 6; r < 64 && tm * 64 + r < P.nm; r += 8)
-      P.C[cols[c] + rows[r]] = S[r * 65 + c];
+  const int c = tid % CN;
+  if (tn * CN + c < P.nn)
+    for (int r = tid / CN; r < 64 && tm * 64 + r < P.nm; r += 8)
+      P.C[cols[c] + rows[r]] = S[r * SP + c];
 }
 
 // --------------------------------------------------------------------------
@@ -1101,6 +1134,38 @@ bool make_map(RowMap &M, Dim *d, int nd, const double *base, long long sk, int K
   return true;
 }
 
+template <int MODE, int CN>
+int launch_crt_form(const CrtParams &P, cudaStream_t s) {
+  const int bytes = std::max(crt_dmma_bytes(CN), P.sym ? crt_mirror_bytes(CN) : 0);
+  const dim3 grid((unsigned)((P.nm + 63) / 64), (unsigned)((P.nn + CN - 1) / CN));
+  RIMP2_CK(launch_ex(false, true, crt_epilogue_kernel<MODE, CN>, grid, 8 * CN, bytes, s, P));
+  count_launch(1);
+  return RIMP2_OK;
+}
+
+template <int CN>
+int launch_crt_mode(const CrtParams &P, int mode, cudaStream_t s) {
+  if (mode == CRT_PLAIN) return launch_crt_form<CRT_PLAIN, CN>(P, s);
+  if (mode == CRT_MINUS) return launch_crt_form<CRT_MINUS, CN>(P, s);
+  if (mode == CRT_QUOTIENT) return launch_crt_form<CRT_QUOTIENT, CN>(P, s);
+  return launch_crt_form<CRT_ANY, CN>(P, s);
+}
+
+// Columns of a block.  64 cost least where the blocks are many (3000 x 3000, sums of 370:
+// 212 us a product, 222 with 16); with up to six 64 x 64 tiles an SM sixteen are as
+// fast (1600 x 1600: 93 and 91), and tiles left to FP64 spread over the SMs: 1600 x 1600
+// with all of them 2189 and 1901 us, 300 x 300 with sums of 1000 1208 and 427.
+// Up to 48 rows have 64 columns, whose warps share the rows that there are, and
+// symmetric products have whole tiles, so that C(m,n) and C(n,m) are the same bits.
+int launch_crt(const CrtParams &P, int mode, cudaStream_t s) {
+  int dev = 0, nsm = 0;
+  RIMP2_CK(cudaGetDevice(&dev));
+  RIMP2_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const long long tiles = ((P.nm + 63) / 64) * (long long)((P.nn + 63) / 64) / (P.lower ? 2 : 1);
+  if (!P.sym && P.nm > 48 && tiles <= 6LL * nsm) return launch_crt_mode<16>(P, mode, s);
+  return launch_crt_mode<64>(P, mode, s);
+}
+
 // One contraction's kernels at a time on a device: a later one, on whatever
 // stream and from whatever thread, starts when the earlier one's have ended.
 // Contractions on three streams at once, without this order, stopped making
@@ -1237,11 +1302,9 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
   P.lower = g.lower;
   P.nfast = B.cst[0] < A.cst[0];
   P.sym = same && !g.lower && g.beta == 0.0 && A.rows > 256 && memcmp(A.role, B.role, sizeof A.role) == 0;
-  const int crt_smem = (P.sym ? 64 * 65 : 2 * 64 * DP) * (int)sizeof(double);
   const bool plain = g.alpha == 1.0 && g.beta == 0.0;
-  auto *crt = plain ? (g.denom ? crt_epilogue_kernel<CRT_QUOTIENT> : crt_epilogue_kernel<CRT_PLAIN>)
-              : !g.denom && g.alpha == -1.0 && g.beta == 1.0 ? crt_epilogue_kernel<CRT_MINUS>
-                                                             : crt_epilogue_kernel<CRT_ANY>;
+  const int mode = plain ? (g.denom ? CRT_QUOTIENT : CRT_PLAIN)
+                   : !g.denom && g.alpha == -1.0 && g.beta == 1.0 ? CRT_MINUS : CRT_ANY;
   P.ea = Q.e.as<int>();
   P.fa = Q.flag.as<unsigned char>();
   P.eb = L.e.as<int>();
@@ -1259,9 +1322,7 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
       P.nn = nc;
       P.ldm = ((long long)Q.rows + 255) / 256 * 256;
       RIMP2_TRY(mod_product(L, Q, res.as<signed char>(), P.ldm, g.lower || P.sym, s));
-      dim3 grid((unsigned)((P.nm + 63) / 64), (unsigned)((P.nn + 63) / 64));
-      RIMP2_CK(launch_ex(false, true, crt, grid, 512, crt_smem, s, P));
-      count_launch(1);
+      RIMP2_TRY(launch_crt(P, mode, s));
       RIMP2_CK(cudaGetLastError());
     }
   }

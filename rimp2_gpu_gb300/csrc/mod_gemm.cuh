@@ -10,7 +10,6 @@ constexpr int MG_PLANES = MG_P + 1;  // and the plane of magnitudes
 // least sum |a||b| of an element, as a part of ||a|| ||b|| = 2^24 in the units
 // of the magnitudes' plane, below which it is summed in FP64
 constexpr float MG_TAU = 65536.0f;
-constexpr int MG_TILE_MAX = 512;     // of a 64 x 64 tile's elements; beyond it the whole tile is
 
 constexpr int MG_K_MIN = 16, MG_K_MAX = 16384;  // lengths of a sum
 
@@ -54,6 +53,14 @@ __device__ __forceinline__ int role_index(const RowMap &M, int r, int role) {
   const int d0 = r % M.ext[0], q = r / M.ext[0];
   const int d1 = q % M.ext[1], d2 = q / M.ext[1];
   return (M.role[0] == role ? d0 : 0) + (M.role[1] == role ? d1 : 0) + (M.role[2] == role ? d2 : 0);
+}
+
+__device__ __forceinline__ void cp_async8(double *dst, const double *src, bool valid) {
+  // 8-byte global -> shared copy; an invalid element is zero-filled (no read)
+  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src),
+               "r"(valid ? 8 : 0)
+               : "memory");
 }
 
 // The hardware's FP32 reciprocal of d (its bits moved into a float and back).
