@@ -25,7 +25,8 @@
 // below what FP64 summation itself loses unless sum|a||b| is a tiny part of
 // ||a|| ||b|| (rows whose large elements meet only small ones).  A 17th
 // product of the magnitudes, in FP16, measures sum|a||b| for every element
-// (from below); an element whose measure is under 2^-8 of ||a|| ||b|| is
+// (from below, over all of K); an element whose measure is under 2^-8 of the largest
+// norms' product (2^-8 to 2^-6 of ||a|| ||b||, as the scales are powers of two) is
 // summed in FP64 instead (one warp per element, or a DMMA tile where an
 // eighth of a 64 x 64 tile needs it).  Rows with infinities, NaNs or extreme
 // exponents take that way too, so every element is what FP64 arithmetic would
@@ -412,6 +413,9 @@ struct MgParams {
   int *err;
 };
 
+// K chunks of one sum: the magnitudes need not be exact and are measured over all of K
+__device__ __forceinline__ int mg_seg(const MgParams &P, int plane) { return plane == MG_P ? P.nkc : P.seg; }
+
 // Items are numbered without gaps and dealt in turn: every pair of CTAs gets
 // as many, also of a triangle's tiles.
 __host__ __device__ inline int mg_tiles(const MgParams &P) {
@@ -538,7 +542,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
       for (int item = pair; item < nitems && ok; item += npair) {
         int p, tl, tq;
         mg_item(P, item, p, tl, tq);
-        for (int s0 = 0; s0 < P.nkc && ok; s0 += P.seg, ++t) {
+        const int seg = mg_seg(P, p);
+        for (int s0 = 0; s0 < P.nkc && ok; s0 += seg, ++t) {
           const int u = (int)(t % NACC);
           if (t >= NACC && !pair_wait(tempty0 + 8 * u, (uint32_t)((t / NACC - 1) & 1), true, abort_flag,
                                    abort_peer, P.err, 22)) {
@@ -547,7 +552,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
           }
           tc_fence_after();
           const uint32_t d = tmem + (uint32_t)(u * TQ);
-          const int s1 = min(P.nkc, s0 + P.seg);
+          const int s1 = min(P.nkc, s0 + seg);
           for (int kc = s0; kc < s1; ++kc) {
             if (!pair_wait(full0 + 8 * stage, phase, false, abort_flag, abort_peer, P.err, 23)) {
               ok = false;
@@ -585,7 +590,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
       const bool mag = p == MG_P;
       const float pf = mag ? 1.0f : DT.p[p], inv = mag ? 1.0f : DT.inv[p];
       uint32_t pk[NG][4];
-      for (int s0 = 0; s0 < P.nkc; s0 += P.seg, ++t) {
+      const int seg = mg_seg(P, p);
+      for (int s0 = 0; s0 < P.nkc; s0 += seg, ++t) {
         const int u = (int)(t % NACC);
         ok = pair_wait(tfull0 + 8 * u, (uint32_t)((t / NACC) & 1), false, abort_flag, abort_peer, P.err, 24);
         ok = __all_sync(0xffffffffu, ok);
@@ -600,7 +606,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
           if (mag) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-              uint32_t w = s0 ? pk[g][q] : 0u;
+              uint32_t w = 0u;
 #pragma unroll
               for (int k = 0; k < 4; ++k) w |= v[4 * q + k] >= MG_TAU ? 1u << (8 * k) : 0u;
               pk[g][q] = w;

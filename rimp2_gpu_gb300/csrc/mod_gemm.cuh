@@ -7,8 +7,9 @@ namespace rimp2 {
 
 constexpr int MG_P = 16;             // moduli
 constexpr int MG_PLANES = MG_P + 1;  // and the plane of magnitudes
-// least sum |a||b| of an element, as a part of ||a|| ||b|| = 2^24 in the units
-// of the magnitudes' plane, below which it is summed in FP64
+// least sum |a||b| of an element in the units of the magnitudes' plane, below
+// which it is summed in FP64: 2^-8 of 2^24.  Rows are scaled by powers of two to norms
+// between 2^11 and 2^12 of these units: 2^-8 to 2^-6 of ||a|| ||b||
 constexpr float MG_TAU = 65536.0f;
 
 constexpr int MG_K_MIN = 16, MG_K_MAX = 16384;  // lengths of a sum

@@ -81,3 +81,32 @@ def test_quotients(api, nvirt, nocc, nba):
     ref = np.einsum("iak,jbk->ijab", X3, X3, optimize=True) / d
     mag = np.einsum("iak,jbk->ijab", np.abs(X3), np.abs(X3), optimize=True) / np.abs(d)
     check(t, ref, mag + np.abs(ref), nba + nocc)
+
+
+def test_magnitudes_of_a_long_sum(api):
+    """sum |a||b| is 2^-5.8 of ||a|| ||b||, spread over sixteen sums of 1024 of which
+    none has 2^-8: no element is left to FP64, whose sums depend on the order of the
+    terms; residues' do not."""
+    rng = np.random.default_rng(4)
+    m, n, k, big = 64, 80, 16384, 1000.0
+
+    def rows(r, at):
+        x = (0.5 + 0.5 * rng.random((r, k))) * np.where(rng.random((r, k)) < 0.5, -1.0, 1.0)
+        x[:, at] = big * (0.75 + 1e-3 * rng.random(r))
+        return x
+    A, B = rows(m, 0), rows(n, 1)
+    norms = np.linalg.norm(A, axis=1)[:, None] * np.linalg.norm(B, axis=1)[None, :]
+    mag = np.abs(A) @ np.abs(B).T
+    assert (mag > norms / 64).all()  # whatever the scales
+    assert (np.abs(A[:, :1024]) @ np.abs(B[:, :1024]).T < norms / 256).all()
+
+    def product(p):
+        C = np.zeros((m, n), order="F")
+        api.dgemm("T", "N", m, n, k, 1.0, np.asfortranarray(A[:, p].T), k, np.asfortranarray(B[:, p].T), k, 0.0, C, m)
+        return C
+    same = np.arange(k)
+    C = product(same)
+    check(C, A @ B.T, mag, k)
+    for _ in range(3):
+        # the large terms stay in the first sum, the others change places
+        assert (C == product(np.concatenate([same[:2], 2 + rng.permutation(k - 2)]))).all()
