@@ -41,6 +41,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <vector>
@@ -1224,6 +1225,20 @@ std::vector<cudaEvent_t> ModOrder::last;
 constexpr size_t MG_PLANE_CAP = (size_t)6 << 30;  // bytes of one operand's planes per part
 constexpr size_t MG_RES_CAP = (size_t)4 << 30;    // bytes of the residues of a part of C
 
+// Most rows of an operand in a part, and most columns of a part whose rows take ldm
+// bytes.  RIMP2_RESIDUE_PARTS=rows,columns: smaller ones, to reach parts in tests.
+void part_caps(int K, long long *rows, long long ldm, long long *cols) {
+  *rows = std::max<long long>(256, (long long)(MG_PLANE_CAP / mod_operand_bytes(1, K)) / 256 * 256);
+  *cols = std::max<long long>(256, (long long)(MG_RES_CAP / (MG_PLANES * ldm)) / 256 * 256);
+  *cols = std::min(*cols, *rows);
+  const char *e = getenv("RIMP2_RESIDUE_PARTS");
+  int r = 0, c = 0;
+  if (e && sscanf(e, "%d,%d", &r, &c) == 2 && r >= 64 && c >= 64) {
+    *rows = std::min<long long>(*rows, r);
+    *cols = std::min<long long>(*cols, c);
+  }
+}
+
 }  // namespace
 
 bool fold_gemm(const GemmDesc &g, RowMap &A, RowMap &B) {
@@ -1257,11 +1272,12 @@ int mod_gemm(const GemmDesc &g, const RowMap &A0, const RowMap &B0, cudaStream_t
     return RIMP2_OK;
   }
   // parts: bounded workspaces, whatever the product's size
-  const long long cap_rows = std::max<long long>(256, (long long)(MG_PLANE_CAP / mod_operand_bytes(1, g.K)) / 256 * 256);
+  long long cap_rows, cap_cols;
+  part_caps(g.K, &cap_rows, 256, &cap_cols);
   const int ra = (int)std::min<long long>(A.rows, cap_rows);
   const long long ldm = ((long long)ra + 255) / 256 * 256;
-  const long long cap_cols = std::max<long long>(256, (long long)(MG_RES_CAP / (MG_PLANES * ldm)) / 256 * 256);
-  const int rb = (int)std::min<long long>(B.rows, std::min(cap_rows, cap_cols));
+  part_caps(g.K, &cap_rows, ldm, &cap_cols);
+  const int rb = (int)std::min<long long>(B.rows, cap_cols);
   if (g.lower && (ra < A.rows || rb < B.rows)) return RIMP2_OK;
   if ((rb + 63) / 64 > 65535) return RIMP2_OK;
   ModOperand Q, L;
@@ -1351,9 +1367,9 @@ double mod_gemm_time(double m, double n, double k, bool lower) {
 
 // Rows and columns of a square product that runs as one part.
 int mod_gemm_block(int K) {
-  const double rows = std::min((double)(MG_PLANE_CAP / mod_operand_bytes(1, K)),
-                               std::sqrt((double)(MG_RES_CAP / MG_PLANES)));
-  return (int)rows / 256 * 256;
+  long long rows, cols;
+  part_caps(K, &rows, (long long)std::sqrt((double)(MG_RES_CAP / MG_PLANES)) / 256 * 256, &cols);
+  return (int)std::min(rows, cols);
 }
 
 }  // namespace rimp2
