@@ -4240,7 +4240,7 @@ int ao_half_fused(const double *ao, int NBA, int nbas, const double *Cmo, int no
                   cudaStream_t s, bool *handled) {
   *handled = false;
   const int NT = (nocc + 15) / 16 * 16;
-  if (NT > AH_NT_MAX || nocc <= 0) return RIMP2_OK;
+  if (NT > AH_NT_MAX || nocc <= 0 || nbas < 2) return RIMP2_OK;  // callers: an occupied and a virtual orbital
   const char *env = getenv("RIMP2_AO_FUSED");  // =0: the sliced first half (for comparisons)
   if (env && env[0] == '0') return RIMP2_OK;
   auto encode = get_encode();
@@ -4294,7 +4294,7 @@ int ao_half_fused(const double *ao, int NBA, int nbas, const double *Cmo, int no
   // Their chunk takes 72 KB instead of 64, which NT = 80 has no room for: it
   // keeps the copies (nbas = 677: 4.05 ms, against 3.27 at 680 in one box).
   int form = NBA % 2 == 0 && (uintptr_t)ao % 16 == 0 ? AH_BOX
-             : nbas > 1 && NT < AH_NT_MAX            ? AH_BOX4
+             : NT < AH_NT_MAX                        ? AH_BOX4
                                                      : AH_COPY;
   AoMaps tmAO;
   memset(&tmAO, 0, sizeof tmAO);
@@ -4319,11 +4319,7 @@ int ao_half_fused(const double *ao, int NBA, int nbas, const double *Cmo, int no
   }
   void (*kern)(CUtensorMap, AoMaps, AoHalfParams) = nullptr;
   switch (NT) {
-    case 16:
-      kern = form == AH_BOX    ? ao_half_kernel<AH_BOX, 16>
-             : form == AH_BOX4 ? ao_half_kernel<AH_BOX4, 16>
-                               : ao_half_kernel<AH_COPY, 16>;  // one function
-      break;
+    case 16: kern = form == AH_BOX ? ao_half_kernel<AH_BOX, 16> : ao_half_kernel<AH_BOX4, 16>; break;
     case 32: kern = form == AH_BOX ? ao_half_kernel<AH_BOX, 32> : ao_half_kernel<AH_BOX4, 32>; break;
     case 48: kern = form == AH_BOX ? ao_half_kernel<AH_BOX, 48> : ao_half_kernel<AH_BOX4, 48>; break;
     case 64: kern = form == AH_BOX ? ao_half_kernel<AH_BOX, 64> : ao_half_kernel<AH_BOX4, 64>; break;
