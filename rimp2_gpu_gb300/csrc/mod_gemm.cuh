@@ -100,6 +100,36 @@ __device__ __forceinline__ double div_f64(double v, double d) {
   return fma(fma(-d, q, v), r, q);
 }
 
+// 1/d for a positive normal d: the FP32 reciprocal of its significand, its
+// exponent put back, refined by a third-order Newton step (Householder's method)
+// to about an ulp.  No branch, so that the steps around it can overlap; odd: d is
+// too near the ends of the range.
+__device__ __forceinline__ double recip_pos(double d, bool &odd) {
+  const int hi = __double2hiint(d), ed = (hi >> 20) & 0x7FF;
+  odd |= ed < 2 || ed > 2040;
+  const float f = __int_as_float(0x3F800000 | ((hi & 0xFFFFF) << 3) | ((unsigned)__double2loint(d) >> 29));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f));
+  const int b = __float_as_int(r);  // 0.5 .. 1
+  const double r0 = __hiloint2double((((b >> 23) + 1919 - ed) << 20) | ((b >> 3) & 0xFFFFF), b << 29);
+  const double e = fma(-d, r0, 1.0);
+  return fma(r0, fma(e, e, e), r0);
+}
+
+// 1/sqrt(d) likewise: FP32 seed for the significand in [1, 4), third-order step.
+__device__ __forceinline__ double rsqrt_pos(double d, bool &odd) {
+  const int hi = __double2hiint(d), ed = (hi >> 20) & 0x7FF;
+  odd |= ed < 2 || ed > 2040;
+  const int up = (ed & 1) ^ 1;  // exponent ed - 1023 = 2 half + up
+  const float f = __int_as_float(((127 + up) << 23) | ((hi & 0xFFFFF) << 3) | ((unsigned)__double2loint(d) >> 29));
+  float r;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(f));
+  const int b = __float_as_int(r), half = (ed - 1023 - up) / 2;
+  const double y = __hiloint2double((((b >> 23) + 896 - half) << 20) | ((b >> 3) & 0xFFFFF), b << 29);
+  const double e = fma(-d * y, y, 1.0);
+  return fma(y, e * fma(0.375, e, 0.5), y);
+}
+
 // C(m,n) = alpha v + beta C(m,n), v divided by the orbital-energy denominator
 // if the product has one; P: RowMap A, B; C, alpha, beta, denom, eo, ev
 template <class Params>
