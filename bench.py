@@ -512,9 +512,16 @@ def run_ours(args):
         nt64 = (NVIRT + 63) // 64
         performed = 2.0 * (NOCC * (NOCC - 1) // 2 * 2 + NOCC) * (nt64 * (nt64 + 1) // 2) * \
             64 * 64 * ((NBA + 15) // 16 * 16)
+        # the residue products themselves: 17 planes of the triangle's 256 x 256 tiles
+        ncol = NOCC * NVIRT
+        residue = 17.0 * ncol * (ncol + 256) * ((NBA + 63) // 64 * 64)
         plain = {"ms": pms, "eff_tflops": eff_flop() / pms / 1e9,
+                 "residue_fp16_tflops": residue / pms / 1e9,
                  "performed_tflops": performed / pms / 1e9, "fp64_dmma_peak_tflops": fp64_peak,
                  "frac_of_fp64_peak": performed / pms / 1e9 / fp64_peak,
+                 "frac_of_fp64_peak_is": "times the FP64 pipe's own rate, far above 1; what bounds "
+                                         "the call is residue_fp16_tflops, with conversion, "
+                                         "reconstruction and pair energies in the time",
                  "performed_is": "FP64 products a DMMA kernel would perform; they run as residues "
                                  "on the FP16 tensor cores",
                  "fp64_peak_probe": "independent DMMA chains on every SM, one launch of >= 1 s "
