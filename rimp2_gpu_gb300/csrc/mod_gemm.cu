@@ -407,7 +407,7 @@ static_assert(tmem_alone(mg_smem(64)) && tmem_alone(mg_smem(128)) && tmem_alone(
 struct MgParams {
   int rows_l, rows_q;        // rows per K chunk of the two operands
   int tiles_l, tiles_q;      // 256 columns, TQ rows
-  int nkc, seg;              // K chunks, and of one exact sum
+  int nkc, seg, nseg;        // K chunks, those of one exact sum, its number
   int lower;                 // square, only tiles with an element m >= n
   signed char *out;          // [plane][n][ldm]
   long long ldm;
@@ -591,8 +591,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(MG_THREADS, 1)
       const bool mag = p == MG_P;
       const float pf = mag ? 1.0f : DT.p[p], inv = mag ? 1.0f : DT.inv[p];
       uint32_t pk[NG][4];
-      const int seg = mg_seg(P, p);
-      for (int s0 = 0; s0 < P.nkc; s0 += seg, ++t) {
+      const int sums = mag ? 1 : P.nseg;  // counted: with the bound in K chunks 2% slower
+      for (int s0 = 0; s0 < sums; ++s0, ++t) {
         const int u = (int)(t % NACC);
         ok = pair_wait(tfull0 + 8 * u, (uint32_t)((t / NACC) & 1), false, abort_flag, abort_peer, P.err, 24);
         ok = __all_sync(0xffffffffu, ok);
@@ -1100,6 +1100,7 @@ int mod_product(const ModOperand &L, const ModOperand &Q, signed char *out, long
   P.nkc = L.nkc;
   const int nseg = (P.nkc + MG_SEG - 1) / MG_SEG;  // of about equal length
   P.seg = (P.nkc + nseg - 1) / nseg;
+  P.nseg = (P.nkc + P.seg - 1) / P.seg;
   P.lower = lower;
   P.out = out;
   P.ldm = ldm;
