@@ -18,6 +18,16 @@
  * compute entry returns RIMP2_ERR_NODEV.  The library works on the device
  * that is current at its first compute call (its stream, error word and
  * memory pool settings belong to that device); one process drives one GPU.
+ *
+ * Streams.  The *_dev calls are ordered by their stream.  FP64 products that run
+ * as residues (FP64 energies and transforms, Cholesky, solve) are ordered among
+ * one another as well, in the order of the calls, whatever their streams and threads: such a
+ * call also waits for what stands before the previous one on that one's stream.  Do not
+ * let a stream wait (in a host function, or for a value in memory) for work that comes
+ * after such a call made later on another stream; events cannot cause that.
+ * Captured calls take the FP64 kernels, are not ordered so, and may be replayed: they hold
+ * no host memory.  Calls that synchronise (host arrays, rimp2_cholesky_dev and the
+ * *_from_ao calls) cannot be captured.
  */
 #ifndef RIMP2_GPU_H
 #define RIMP2_GPU_H

@@ -28,7 +28,7 @@
 // (from below, over all of K); an element whose measure is under 2^-8 of the largest
 // norms' product (2^-8 to 2^-6 of ||a|| ||b||, as the scales are powers of two) is
 // summed in FP64 instead (one warp per element, or a DMMA tile where an
-// eighth of a 64 x 64 tile needs it).  Rows with infinities, NaNs or extreme
+// eighth of a tile needs it).  Rows with infinities, NaNs or extreme
 // exponents take that way too, so every element is what FP64 arithmetic would
 // make it, up to FP64's own rounding.
 //
