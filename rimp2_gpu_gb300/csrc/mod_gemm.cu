@@ -1177,8 +1177,9 @@ int launch_crt(const CrtParams &P, int mode, cudaStream_t s) {
 // One contraction's kernels at a time on a device: a later one, on whatever
 // stream and from whatever thread, starts when the earlier one's have ended.
 // Contractions on three streams at once, without this order, stopped making
-// progress on the GPU.  The cause is not known: what is left unbounded in the
-// kernels, the tensor memory's allocation and the cluster barriers, cannot wait for
+// progress on the GPU, when a CTA still gave up the allocation permit of its pair before
+// the other had its columns.  Whether that was all is not known; what is left
+// unbounded in the kernels, that allocation and the cluster barriers, cannot wait for
 // another kernel (TMEM_SMEM_MIN, tc.cuh).  So they do not run at once.  The price: a
 // contraction also waits for what stands before the last one on that one's stream,
 // and small ones on several streams do not overlap (eight streams, nocc 6, nvirt 53,

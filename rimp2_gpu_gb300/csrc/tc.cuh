@@ -25,6 +25,8 @@ constexpr long long WAIT_BUDGET = 4000000000LL;  // ~2 s of SM clock per wait
 // (228 KB of shared memory, 1 KB of each CTA's taken by the system), so
 // the columns are free when such a CTA starts.  And the CTAs of a cluster start
 // together, every other wait before a cluster barrier is bounded, so each arrives.
+// The permit to allocate is given up after such a barrier: no CTA may allocate once
+// its pair has, and blocks of other streams can hold one of the two back.
 constexpr int SM_SMEM = 228 * 1024;
 constexpr int TMEM_SMEM_MIN = 75008;  // least shared memory of a kernel that allocates
 constexpr bool tmem_alone(int smem) { return smem + TMEM_SMEM_MIN + 2 * 1024 > SM_SMEM; }
